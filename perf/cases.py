@@ -49,7 +49,7 @@ def listed():
         # the fluctuation task: subsystem counts and g(r) after every step
         dict(name="fluctuations_512", kind="fluct", n=512, rho=0.316, T=1.312, tvn=0, bc=0, fp64=1, dt=0.004, steps=20),
         # a parameter sweep: 256 boxes of uneven size, half of them walled, advanced together
-        dict(name="sweep_256_boxes", kind="batch", boxes=256, nmin=200, nmax=4000, mix=3, dt=0.004, steps=5),
+        dict(name="sweep_256_boxes", kind="batch", boxes=256, nmin=200, nmax=4000, mix=3, dt=0.004, steps=10),
         # structure of a stored configuration
         dict(name="rdf_16384", kind="rdf", n=16384, rho=0.85, mode=0, bins=256),
         # a gradient of time-averaged energy and pressure
@@ -83,7 +83,7 @@ def draw(rng):
     if kind == "batch":
         nmin = _log(rng, 100, 400)
         return dict(kind=kind, boxes=_log(rng, 8, 256), nmin=nmin, nmax=_log(rng, nmin + 100, 4000),
-                    mix=rng.randrange(1 << 30), dt=0.004, steps=5)
+                    mix=rng.randrange(1 << 30), dt=0.004, steps=10)
     if kind == "rdf":
         return dict(kind=kind, n=_log(rng, 200, 40000), rho=rho, mode=rng.randint(0, 2), bins=rng.choice([100, 200, 256]))
     if kind == "adjoint":
