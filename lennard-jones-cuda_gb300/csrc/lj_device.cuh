@@ -44,6 +44,30 @@ __device__ __forceinline__ int32_t fixed_coord(double x, double origin, double i
   return (int32_t)q;
 }
 
+// Wrapping difference of two fixed-point coordinates (the minimum image).
+__device__ __forceinline__ int fixed_diff(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
+
+// The i record of a thread is held with x, y, z in slots 1..3 of an aligned
+// register quadruple (.y, .z, .w), while the 128-bit shared loads of the j
+// records put theirs in slots 0..2.  Each integer difference then reads its
+// two operands from registers of opposite parity, which sit in different
+// register-file banks: with both records in slots 0..2 every difference
+// waited on a bank conflict (measured on GB300: 52.5 -> 49.4 cycles per
+// 64-pair warp step of the packed loop).  i_record_slots123 places it.
+__device__ __forceinline__ int4 i_record_slots123(const int4 q, int4* slot) {
+  volatile int4* v = slot;
+  v->x = 0;
+  v->y = q.x;
+  v->z = q.y;
+  v->w = q.z;
+  // volatile load: the compiler may not forward the stored registers
+  int4 r;
+  asm volatile("ld.volatile.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "r"((unsigned)__cvta_generic_to_shared(slot)));
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // mbarrier + bulk copy (cp.async.bulk, the non-tensor TMA path).
 // ---------------------------------------------------------------------------

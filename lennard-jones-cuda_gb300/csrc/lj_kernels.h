@@ -10,9 +10,6 @@
 namespace ljgb {
 
 constexpr int kMaxHistBins = 4096;
-// Shared-memory histogram of a pair-kernel CTA: nb 32-bit bins, rounded up to
-// 16 bytes.
-constexpr size_t hist_smem_bytes(int nb) { return (sizeof(unsigned) * (size_t)nb + 15) / 16 * 16; }
 
 // Pair-histogram request.  mode 0: r^2 bins, clamp overflow to the last bin
 // (MDSystem.cu:39); 1: r^2 bins, drop overflow (MDSystem.cpp:282-284);
@@ -39,9 +36,23 @@ struct PairArgs {
   const BoxArgs* boxes;       // per box constants
   float* partial;             // nseg x 5 x threads  (float, or double for FP64)
   int* status;                // device status word (timeouts)
-  HistArgs hist;
 };
 
+
+// Pair histogram of one box of n particles (lj_rdf.cu) over the fixed-point
+// shadow q: adds the counts of all ordered pairs to h.counts.  The ranges are
+// those of build_rdf_ranges for at most rdf_ctas_per_sm() CTAs an SM.
+struct RdfPass {
+  const int4* q;
+  const DevScalars* sc;    // the box's frame (k2)
+  int n;
+  const int* cta_block;    // first i-block of each CTA
+  const int* cta_chunk;    // first j-chunk of that block
+  const int* cta_units;    // chunks the CTA covers
+  HistArgs hist;
+};
+int rdf_ctas_per_sm();
+cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st);
 
 struct PairShape {
   int threads;  // CTA size = i-block length (one i per thread)
@@ -55,10 +66,7 @@ int fp64_block_threads();
 int fp64_tile();
 
 cudaError_t pair_occupancy(int prec, int shape, int* blocks_per_sm);
-// Resident CTAs per SM of the MIXED histogram-only pair kernel with nb bins.
-cudaError_t pair_hist_occupancy(int shape, int nb, int* blocks_per_sm);
-cudaError_t launch_pairs(int prec, int shape, bool forces, bool hist, const PairArgs& a, int grid,
-                         cudaStream_t st);
+cudaError_t launch_pairs(int prec, int shape, const PairArgs& a, int grid, cudaStream_t st);
 struct FusedPairArgs;
 cudaError_t launch_pairs_fused(int shape, int mode, const FusedPairArgs& a, int grid, cudaStream_t st);
 

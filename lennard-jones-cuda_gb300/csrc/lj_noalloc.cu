@@ -282,8 +282,7 @@ extern "C" lj_status lj_forces_static(const float* pos4, float* force4, double* 
   a.sc = sc;
   a.partial = partial;
   a.status = status;
-  a.hist = HistArgs{0, 1, 1.0f, 0.0f, nullptr};
-  if ((e = launch_pairs(0, kShape, true, false, a, G, st)) != cudaSuccess)
+  if ((e = launch_pairs(0, kShape, a, G, st)) != cudaSuccess)
     return (lj_status)static_fail(LJ_ERR_CUDA, cudaGetErrorString(e));
   k_static_reduce<<<nblocks, kBI, 0, st>>>(partial, blocks, sc, reinterpret_cast<float4*>(force4), blk);
   k_static_sums<<<1, 256, 0, st>>>(blk, nblocks, dsums);

@@ -1,4 +1,4 @@
-// lj_pairs.cu -- all-pairs Lennard-Jones force / energy / virial / RDF kernels.
+// lj_pairs.cu -- all-pairs Lennard-Jones force / energy / virial kernels.
 //
 // Replaces calculateForces + RDFmerger of the reference
 // (src/library/MDSystem.cu:21-153) and the O(N^2) CPU loop of
@@ -18,8 +18,7 @@
 //    TwoSum-compensated accumulators;
 //  * no per-pair global atomics: partial sums of each (CTA, i-block) segment
 //    go to a partial buffer reduced deterministically in FP64 by the
-//    integrator kernels; pair histograms (RDF) go to a shared-memory
-//    histogram flushed once per CTA.
+//    integrator kernels (pair histograms are lj_rdf.cu's).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -41,33 +40,9 @@ constexpr int kChunk = LJ_CHUNK;  // pairs per compensated force partial sum
 // tile; the unrolled chunk loop needs those to be whole chunks.
 static_assert(kSplitGrain % kChunk == 0, "schedule cuts must fall on chunk boundaries");
 
-// Wrapping difference of two fixed-point coordinates (the minimum image).
-__device__ __forceinline__ int fixed_diff(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
-
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// The i record of a thread is held with x, y, z in slots 1..3 of an aligned
-// register quadruple (.y, .z, .w), while the 128-bit shared loads of the j
-// records put theirs in slots 0..2.  Each integer difference then reads its
-// two operands from registers of opposite parity, which sit in different
-// register-file banks: with both records in slots 0..2 every difference
-// waited on a bank conflict (measured on GB300: 52.5 -> 49.4 cycles per
-// 64-pair warp step of the packed loop).  i_record_slots123 places it.
-__device__ __forceinline__ int4 i_record_slots123(const int4 q, int4* slot) {
-  volatile int4* v = slot;
-  v->x = 0;
-  v->y = q.x;
-  v->z = q.y;
-  v->w = q.z;
-  // volatile load: the compiler may not forward the stored registers
-  int4 r;
-  asm volatile("ld.volatile.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "r"((unsigned)__cvta_generic_to_shared(slot)));
   return r;
 }
 
@@ -168,33 +143,6 @@ __device__ __forceinline__ float lane_sum(f32x2 v) {
   return a + b;
 }
 
-// floor(x) for 0 <= x < 2^23: 2^23 + x rounded down is 2^23 + floor(x)
-// exactly, read back from the float's bits (an FP32 add and an integer
-// subtract instead of a round and a float -> int conversion).
-__device__ __forceinline__ int floor_small(float x) {
-  return __float_as_int(__fadd_rd(x, 8388608.0f)) - 0x4B000000;
-}
-
-// Histogram bin of a pair from its fixed-point separation (qi in slots 1..3);
-// the arithmetic is exactly what the oracle's emu_rdf_* reproduces on the CPU
-// (floor of the separately rounded products, clamped or dropped past the last
-// bin).
-__device__ __forceinline__ int pair_bin(const int4 qi, const int4 qj, float k2, const HistArgs& h) {
-  const float dx = __int2float_rn((int)((unsigned)qj.x - (unsigned)qi.y));
-  const float dy = __int2float_rn((int)((unsigned)qj.y - (unsigned)qi.z));
-  const float dz = __int2float_rn((int)((unsigned)qj.z - (unsigned)qi.w));
-  const float r2 = __fmul_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), k2);
-  if (h.mode == 2) {  // linear r bins, r < rmax (so r / w < nb, up to rounding)
-    if (!(r2 < h.rmax2)) return -1;
-    return min(floor_small(__fmul_rn(__fsqrt_rn(r2), h.inv_w)), h.nb - 1);
-  }
-  // r^2 bins; the quotient is capped at nb first, which keeps it in
-  // floor_small's range and changes no bin
-  const int fb = floor_small(fminf(__fmul_rn(r2, h.inv_w), (float)h.nb));
-  if (h.mode == 0) return min(fb, h.nb - 1);  // clamp (MDSystem.cu:39)
-  return fb < h.nb ? fb : -1;                  // drop (MDSystem.cpp:283)
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -206,10 +154,9 @@ __device__ __forceinline__ int pair_bin(const int4 qi, const int4 qj, float k2, 
 // Verlet step for that block (fused_block_step), and the CTA that finishes
 // the last block runs the per-box observables (EVN) or the TVN scale (TVN).
 // Completion is detected with atomic counters only; no CTA waits on another.
-template <int THREADS, int TILE, int STAGES, bool FORCES, bool HIST, int EPI>
+template <int THREADS, int TILE, int STAGES, int EPI>
 __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& st, unsigned char* smem_raw) {
   int4* sq = reinterpret_cast<int4*>(smem_raw);
-  unsigned* shist = reinterpret_cast<unsigned*>(smem_raw + sizeof(int4) * STAGES * TILE);
   __shared__ uint64_t bars[STAGES];
   __shared__ double shd[EPI ? 4 * 32 : 1];
   __shared__ int sflag;
@@ -248,9 +195,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
   __shared__ volatile int sfail;
   const int lane = tid & 31;
 
-  if (HIST) {
-    for (int b = tid; b < a.hist.nb; b += THREADS) shist[b] = 0u;
-  }
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&bars[s], 1);
@@ -284,12 +228,9 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
   bool valid_i = tid < bi.n_i;
   int4 qi = i_record_slots123(a.q[bi.p0 + (valid_i ? i_local : bi.i0)], &sirec[tid]);
   float k2inv = a.sc[bi.sys].k2inv;
-  float k2 = a.sc[bi.sys].k2;
   FloatAcc acc[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) acc[c] = FloatAcc{0.f, 0.f};
-  unsigned nclamp = 0;  // HIST, clamped r^2 bins: pairs in the last bin
-  unsigned nself = 0;   // HIST: self pairs binned into bin 0
 
   // A warp whose wait times out (or that sees another warp's timeout) keeps
   // walking the tile sequence without computing, so every CTA-wide barrier
@@ -313,88 +254,61 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
     if (!failed) {
       const int4* st = sq + s * TILE;
       const bool masked = j0 < bi.i0 + bi.n_i && j0 + cnt > bi.i0;  // tile holds this block's own i's
-      if (FORCES) {
-        // Force sums are folded into the TwoSum accumulators every kChunk
-        // pairs, so a large near-neighbour term rounds at most kChunk-1 later
-        // additions.  Energy sums go chunk -> tile (plain FP32) -> TwoSum: a
-        // chunk partial is never small next to the tile sum, so the far-field
-        // (s/r)^6 tail is not truncated.
-        float ta = 0.f, tb = 0.f;
-        if (cnt == TILE) {
-          // Full tile: unrolled chunks.  Only the diagonal tile (the j-range
-          // holding this CTA's own i's) needs the self-pair excluded; it
-          // keeps the unrolled loop and pays one compare + select per pair.
-          const bool diag = masked;
+      // Force sums are folded into the TwoSum accumulators every kChunk
+      // pairs, so a large near-neighbour term rounds at most kChunk-1 later
+      // additions.  Energy sums go chunk -> tile (plain FP32) -> TwoSum: a
+      // chunk partial is never small next to the tile sum, so the far-field
+      // (s/r)^6 tail is not truncated.
+      float ta = 0.f, tb = 0.f;
+      if (cnt == TILE) {
+        // Full tile: unrolled chunks.  Only the diagonal tile (the j-range
+        // holding this CTA's own i's) needs the self-pair excluded; it
+        // keeps the unrolled loop and pays one compare + select per pair.
+        const bool diag = masked;
 #pragma unroll 1
-          for (int c0 = jlo; c0 < jhi; c0 += kChunk) {
-            const f32x2 k2i2 = pk2(k2inv, k2inv);
-            f32x2 FX = 0ull, FY = 0ull, FZ = 0ull, PA = 0ull, PB = 0ull;
-            if (!diag) {
+        for (int c0 = jlo; c0 < jhi; c0 += kChunk) {
+          const f32x2 k2i2 = pk2(k2inv, k2inv);
+          f32x2 FX = 0ull, FY = 0ull, FZ = 0ull, PA = 0ull, PB = 0ull;
+          if (!diag) {
 #pragma unroll
-              for (int jj = c0; jj < c0 + kChunk; jj += 2)
-                pair_mixed2<false>(qi, st[jj], st[jj + 1], k2i2, false, false, FX, FY, FZ, PA, PB);
-            } else {
-              const int self = i_local - j0;  // tile-local index of this thread's i
+            for (int jj = c0; jj < c0 + kChunk; jj += 2)
+              pair_mixed2<false>(qi, st[jj], st[jj + 1], k2i2, false, false, FX, FY, FZ, PA, PB);
+          } else {
+            const int self = i_local - j0;  // tile-local index of this thread's i
 #pragma unroll
-              for (int jj = c0; jj < c0 + kChunk; jj += 2)
-                pair_mixed2<true>(qi, st[jj], st[jj + 1], k2i2, jj == self, jj + 1 == self, FX, FY, FZ, PA, PB);
-            }
-            const float fx = lane_sum(FX), fy = lane_sum(FY), fz = lane_sum(FZ), pa = lane_sum(PA),
-                        pb = lane_sum(PB);
-            two_sum_add(acc[0], fx);
-            two_sum_add(acc[1], fy);
-            two_sum_add(acc[2], fz);
-            ta += pa;
-            tb += pb;
-          }
-        } else {
-          // Ragged last tile of a box: packed pairs with the self pair
-          // excluded, an odd last record on its own.
-          const int self = i_local - j0;
-          for (int c0 = jlo; c0 < jhi; c0 += kChunk) {
-            const int c1 = min(jhi, c0 + kChunk);
-            const f32x2 k2i2 = pk2(k2inv, k2inv);
-            f32x2 FX = 0ull, FY = 0ull, FZ = 0ull, PA = 0ull, PB = 0ull;
-            int jj = c0;
-            for (; jj + 1 < c1; jj += 2)
+            for (int jj = c0; jj < c0 + kChunk; jj += 2)
               pair_mixed2<true>(qi, st[jj], st[jj + 1], k2i2, jj == self, jj + 1 == self, FX, FY, FZ, PA, PB);
-            float fx = lane_sum(FX), fy = lane_sum(FY), fz = lane_sum(FZ), pa = lane_sum(PA), pb = lane_sum(PB);
-            if (jj < c1) pair_mixed<true>(qi, st[jj], k2inv, jj == self, fx, fy, fz, pa, pb);
-            two_sum_add(acc[0], fx);
-            two_sum_add(acc[1], fy);
-            two_sum_add(acc[2], fz);
-            ta += pa;
-            tb += pb;
           }
+          const float fx = lane_sum(FX), fy = lane_sum(FY), fz = lane_sum(FZ), pa = lane_sum(PA),
+                      pb = lane_sum(PB);
+          two_sum_add(acc[0], fx);
+          two_sum_add(acc[1], fy);
+          two_sum_add(acc[2], fz);
+          ta += pa;
+          tb += pb;
         }
-        two_sum_add(acc[3], ta);
-        two_sum_add(acc[4], tb);
-      }
-      if (HIST && valid_i) {
-        // The self pair (separation 0) is binned with the others, into bin 0
-        // in every mode, and taken out of bin 0 once at the end: no per-pair
-        // index test.
+      } else {
+        // Ragged last tile of a box: packed pairs with the self pair
+        // excluded, an odd last record on its own.
         const int self = i_local - j0;
-        if (self >= jlo && self < jhi) ++nself;
-        if (a.hist.mode == 0) {
-          // Clamped r^2 bins: most pairs of a box land in the last bin.  They
-          // are counted in a register and added once per warp at the end
-          // instead of by a same-address shared atomic per pair.
-          const int last_bin = a.hist.nb - 1;
-#pragma unroll 4
-          for (int jj = jlo; jj < jhi; ++jj) {
-            const int b = pair_bin(qi, st[jj], k2, a.hist);
-            if (b == last_bin) ++nclamp;
-            else atomicAdd(&shist[b], 1u);
-          }
-        } else {
-#pragma unroll 4
-          for (int jj = jlo; jj < jhi; ++jj) {
-            const int b = pair_bin(qi, st[jj], k2, a.hist);
-            if (b >= 0) atomicAdd(&shist[b], 1u);
-          }
+        for (int c0 = jlo; c0 < jhi; c0 += kChunk) {
+          const int c1 = min(jhi, c0 + kChunk);
+          const f32x2 k2i2 = pk2(k2inv, k2inv);
+          f32x2 FX = 0ull, FY = 0ull, FZ = 0ull, PA = 0ull, PB = 0ull;
+          int jj = c0;
+          for (; jj + 1 < c1; jj += 2)
+            pair_mixed2<true>(qi, st[jj], st[jj + 1], k2i2, jj == self, jj + 1 == self, FX, FY, FZ, PA, PB);
+          float fx = lane_sum(FX), fy = lane_sum(FY), fz = lane_sum(FZ), pa = lane_sum(PA), pb = lane_sum(PB);
+          if (jj < c1) pair_mixed<true>(qi, st[jj], k2inv, jj == self, fx, fy, fz, pa, pb);
+          two_sum_add(acc[0], fx);
+          two_sum_add(acc[1], fy);
+          two_sum_add(acc[2], fz);
+          ta += pa;
+          tb += pb;
         }
       }
+      two_sum_add(acc[3], ta);
+      two_sum_add(acc[4], tb);
     }
     // This warp is done reading stage s; the last warp done refills it.
     __syncwarp();
@@ -421,7 +335,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
     const bool last = (k == ntiles - 1);
     const bool block_end = (jt + 1 == bi.njt);
     if (block_end || last) {
-      if (FORCES && valid_i && !failed) {
+      if (valid_i && !failed) {
         const int seg = bi.seg_first + (g - bi.g_first);
         float* out = a.partial + (size_t)seg * 5 * THREADS;
 #pragma unroll
@@ -453,7 +367,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
         valid_i = tid < bi.n_i;
         qi = i_record_slots123(a.q[bi.p0 + (valid_i ? i_local : bi.i0)], &sirec[tid]);
         k2inv = a.sc[bi.sys].k2inv;
-        k2 = a.sc[bi.sys].k2;
         jt = 0;
       }
     } else {
@@ -487,29 +400,18 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
     }
     return;
   }
-  if (HIST) {
-    const unsigned wclamp = __reduce_add_sync(0xffffffffu, nclamp);
-    const unsigned wself = __reduce_add_sync(0xffffffffu, nself);
-    if (lane == 0) {
-      if (wclamp) atomicAdd(&shist[a.hist.nb - 1], wclamp);
-      if (wself) atomicSub(&shist[0], wself);
-    }
-    __syncthreads();
-    for (int b = tid; b < a.hist.nb; b += THREADS)
-      if (shist[b]) atomicAdd(a.hist.counts + b, (unsigned long long)shist[b]);
-  }
 }
 
-template <int THREADS, int TILE, int STAGES, int MINB, bool FORCES, bool HIST>
+template <int THREADS, int TILE, int STAGES, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_pairs_mixed(PairArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  pairs_body<THREADS, TILE, STAGES, FORCES, HIST, 0>(a, StateArgs{}, smem_raw);
+  pairs_body<THREADS, TILE, STAGES, 0>(a, StateArgs{}, smem_raw);
 }
 
 template <int THREADS, int TILE, int STAGES, int MINB, int EPI>
 __global__ void __launch_bounds__(THREADS, MINB) k_pairs_mixed_fused(FusedPairArgs f) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  pairs_body<THREADS, TILE, STAGES, true, false, EPI>(f.pair, f.st, smem_raw);
+  pairs_body<THREADS, TILE, STAGES, EPI>(f.pair, f.st, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -642,12 +544,11 @@ __global__ void __launch_bounds__(THREADS) k_pairs_fp64(PairArgs a) {
 // ---------------------------------------------------------------------------
 namespace {
 
-template <int THREADS, int TILE, int STAGES, int MINB, bool FORCES, bool HIST>
+template <int THREADS, int TILE, int STAGES, int MINB>
 cudaError_t launch_mixed_t(const PairArgs& a, int grid, cudaStream_t st) {
-  // <= 48 KB: 16 B x STAGES x TILE staging (+ the histogram's bins, at most
-  // 16 KB), no opt-in needed.
-  const size_t smem = sizeof(int4) * STAGES * TILE + (HIST ? hist_smem_bytes(a.hist.nb) : 0);
-  k_pairs_mixed<THREADS, TILE, STAGES, MINB, FORCES, HIST><<<grid, THREADS, smem, st>>>(a);
+  // <= 48 KB: 16 B x STAGES x TILE staging, no opt-in needed.
+  const size_t smem = sizeof(int4) * STAGES * TILE;
+  k_pairs_mixed<THREADS, TILE, STAGES, MINB><<<grid, THREADS, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -662,16 +563,8 @@ cudaError_t launch_fused_t(int mode, const FusedPairArgs& f, int grid, cudaStrea
 template <int THREADS, int TILE, int STAGES, int MINB>
 cudaError_t occupancy_mixed_t(int* blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks_per_sm, k_pairs_mixed<THREADS, TILE, STAGES, MINB, true, false>, THREADS,
+      blocks_per_sm, k_pairs_mixed<THREADS, TILE, STAGES, MINB>, THREADS,
       sizeof(int4) * STAGES * TILE);
-}
-
-// Resident CTAs per SM of the histogram-only variant with nb bins.
-template <int THREADS, int TILE, int STAGES, int MINB>
-cudaError_t occupancy_hist_t(int nb, int* blocks_per_sm) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks_per_sm, k_pairs_mixed<THREADS, TILE, STAGES, MINB, false, true>, THREADS,
-      sizeof(int4) * STAGES * TILE + hist_smem_bytes(nb));
 }
 
 template <int THREADS, int TILE, int STAGES>
@@ -706,8 +599,6 @@ const PairShape kShapes[] = {
 };
 const int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
-// FP64 i-block and j-tile match MIXED shape 0 so the histogram kernel can
-// run on an FP64 handle's schedule.
 constexpr int kFp64Threads = 128, kFp64Tile = 256, kFp64Stages = 3;
 
 int fp64_block_threads() { return kFp64Threads; }
@@ -725,26 +616,12 @@ cudaError_t pair_occupancy(int prec, int shape, int* blocks_per_sm) {
   return cudaErrorInvalidValue;
 }
 
-cudaError_t pair_hist_occupancy(int shape, int nb, int* blocks_per_sm) {
-  switch (shape) {
-#define LJ_HOCC_CASE(i, T, TL, S, M) \
-  case i:                            \
-    return occupancy_hist_t<T, TL, S, M>(nb, blocks_per_sm);
-    LJ_SHAPES(LJ_HOCC_CASE)
-#undef LJ_HOCC_CASE
-  }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_pairs(int prec, int shape, bool forces, bool hist, const PairArgs& a, int grid,
-                         cudaStream_t st) {
+cudaError_t launch_pairs(int prec, int shape, const PairArgs& a, int grid, cudaStream_t st) {
   if (prec == 1) return launch_fp64_t<kFp64Threads, kFp64Tile, kFp64Stages>(a, grid, st);
   switch (shape) {
-#define LJ_LAUNCH_CASE(i, T, TL, S, M)                                                  \
-  case i:                                                                               \
-    if (forces && !hist) return launch_mixed_t<T, TL, S, M, true, false>(a, grid, st); \
-    if (forces && hist) return launch_mixed_t<T, TL, S, M, true, true>(a, grid, st);   \
-    return launch_mixed_t<T, TL, S, M, false, true>(a, grid, st);
+#define LJ_LAUNCH_CASE(i, T, TL, S, M) \
+  case i:                              \
+    return launch_mixed_t<T, TL, S, M>(a, grid, st);
     LJ_SHAPES(LJ_LAUNCH_CASE)
 #undef LJ_LAUNCH_CASE
   }

@@ -1,0 +1,137 @@
+// lj_rdf.cu -- pair histograms (RDF) of one box.
+//
+// Replaces the per-pair global atomics and RDFmerger of the reference
+// (src/library/MDSystem.cu:36-42, 140-153) and the bin counting of its CPU
+// loop (src/library/MDSystem.cpp:281-285).  Counts are those of all ordered
+// pairs j != i, as the reference's.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "lj_device.cuh"
+#include "lj_kernels.h"
+#include "lj_schedule.h"
+
+namespace ljgb {
+namespace {
+
+// floor(x) for 0 <= x < 2^23: 2^23 + x rounded down is 2^23 + floor(x)
+// exactly, read back from the float's bits (an FP32 add and an integer
+// subtract instead of a round and a float -> int conversion).
+__device__ __forceinline__ int floor_small(float x) {
+  return __float_as_int(__fadd_rd(x, 8388608.0f)) - 0x4B000000;
+}
+
+constexpr int kTile = 256;  // j records staged in shared memory
+
+// One pair into the CTA's histogram, from its fixed-point separation (qi in
+// slots 1..3, see i_record_slots123).  The arithmetic is exactly what the
+// oracle's emu_rdf_* reproduces on the CPU: floor of the separately rounded
+// products, clamped to or dropped past the last bin.
+template <int MODE>
+__device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float k2, float inv_w, float limit, int last,
+                                         unsigned* shist, unsigned& nclamp) {
+  const float dx = __int2float_rn(fixed_diff(qj.x, qi.y));
+  const float dy = __int2float_rn(fixed_diff(qj.y, qi.z));
+  const float dz = __int2float_rn(fixed_diff(qj.z, qi.w));
+  const float r2 = __fmul_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), k2);
+  if (MODE == 2) {  // linear r bins; limit = rmax^2 (so r / w < nb, up to rounding)
+    if (r2 < limit) atomicAdd(&shist[min(floor_small(__fmul_rn(__fsqrt_rn(r2), inv_w)), last)], 1u);
+  } else {
+    const float b = __fmul_rn(r2, inv_w);
+    if (MODE == 1) {  // r^2 bins, overflow dropped (MDSystem.cpp:283); limit = nb
+      if (b < limit) atomicAdd(&shist[floor_small(b)], 1u);
+    } else {  // overflow counted in the last bin (MDSystem.cu:39); limit = nb - 1
+      // most pairs of a box land there: counted in a register
+      if (b >= limit) ++nclamp;
+      else atomicAdd(&shist[min(floor_small(fminf(b, limit)), last)], 1u);
+    }
+  }
+}
+
+// Each unordered pair once: block b of 256 i's (one per thread) runs over the
+// j's from its own first particle on and skips j <= i inside its own square;
+// the wrapping difference is antisymmetric, so (j, i) falls into the bin of
+// (i, j) exactly and the flush adds every count twice.  The loop is bound by
+// issue (about 17 instructions a pair, no memory traffic: the shadow stays in
+// L2), so halving the pairs is what shortens it; N = 16384, 256 clamped bins:
+// the call took 234 us over ordered pairs, 131 us so.  A CTA owns a contiguous range of
+// (block, 32-j chunk) units (build_rdf_ranges), flushing its shared histogram
+// once: a grid of single tiles would flush 256 bins thousands of times.
+template <int MODE>
+__global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
+  extern __shared__ unsigned shist[];
+  __shared__ int4 tile[kTile];
+  __shared__ int4 sirec[kRdfBlock];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const HistArgs h = a.hist;
+  const int last = h.nb - 1;
+  const float limit = MODE == 2 ? h.rmax2 : (float)(MODE == 1 ? h.nb : last);
+  const float k2 = a.sc->k2;
+  for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
+  unsigned nclamp = 0;
+  auto flush = [&]() {
+    const unsigned wclamp = __reduce_add_sync(0xffffffffu, nclamp);
+    nclamp = 0;
+    if (MODE == 0 && lane == 0 && wclamp) atomicAdd(&shist[last], wclamp);
+    __syncthreads();
+    for (int b = tid; b < h.nb; b += kRdfBlock)
+      if (shist[b]) atomicAdd(h.counts + b, 2ull * shist[b]);
+  };
+  int B = a.cta_block[blockIdx.x], c = a.cta_chunk[blockIdx.x], left = a.cta_units[blockIdx.x];
+  const int nchunks = (a.n + kRdfChunk - 1) / kRdfChunk;
+  int counted = 0;  // units since the last flush
+  for (; left > 0; ++B, c = 0) {
+    const int i0 = B * kRdfBlock, i = i0 + tid;
+    const int4 qi = i_record_slots123(a.q[min(i, a.n - 1)], &sirec[tid]);
+    int take = min(left, nchunks - B * (kRdfBlock / kRdfChunk) - c);
+    left -= take;
+    // 2^19 units are 2^32 pairs, what a 32-bit bin can hold
+    for (; take > 0;) {
+      const int part = min(take, (1 << 18));
+      if (counted + part > (1 << 18)) {
+        __syncthreads();
+        flush();
+        __syncthreads();
+        for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
+        counted = 0;
+      }
+      counted += part;
+      const int j1 = min(a.n, i0 + (c + part) * kRdfChunk);
+      for (int j0 = i0 + c * kRdfChunk; j0 < j1; j0 += kTile) {
+        const int cnt = min(kTile, j1 - j0);
+        __syncthreads();
+        if (tid < cnt) tile[tid] = a.q[j0 + tid];
+        __syncthreads();
+        if (i >= a.n) continue;
+        if (j0 >= i0 + kRdfBlock) {
+#pragma unroll 4
+          for (int jj = 0; jj < cnt; ++jj) bin_pair<MODE>(qi, tile[jj], k2, h.inv_w, limit, last, shist, nclamp);
+        } else {
+          for (int jj = 0; jj < cnt; ++jj)
+            if (j0 + jj > i) bin_pair<MODE>(qi, tile[jj], k2, h.inv_w, limit, last, shist, nclamp);
+        }
+      }
+      take -= part;
+      c += part;
+    }
+  }
+  __syncthreads();
+  flush();
+}
+
+}  // namespace
+
+// 6 CTAs of 256 threads an SM at 40 registers; their shared memory (4 + 4 KB
+// and at most 16 KB of bins each) fits beside each other for any bin count.
+int rdf_ctas_per_sm() { return 6; }
+
+cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st) {
+  const size_t smem = sizeof(unsigned) * (size_t)a.hist.nb;
+  if (a.hist.mode == 0) k_rdf<0><<<grid, kRdfBlock, smem, st>>>(a);
+  else if (a.hist.mode == 1) k_rdf<1><<<grid, kRdfBlock, smem, st>>>(a);
+  else k_rdf<2><<<grid, kRdfBlock, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+}  // namespace ljgb

@@ -115,4 +115,28 @@ bool build_schedule(const int* n, int nsys, int BI, int TILE, int G, int tile_ov
   return true;
 }
 
+bool build_rdf_ranges(int n, int ctas, RdfRanges* out) {
+  if (n < 1 || ctas < 1 || !out) return false;
+  constexpr int kPerBlock = kRdfBlock / kRdfChunk;
+  const int nb = (n + kRdfBlock - 1) / kRdfBlock, nch = (n + kRdfChunk - 1) / kRdfChunk;
+  const int64_t total = (int64_t)nb * nch - (int64_t)kPerBlock * nb * (nb - 1) / 2;
+  RdfRanges r;
+  r.G = (int)std::min<int64_t>(ctas, total);
+  int b = 0;
+  int64_t first = 0;  // chunks before block b
+  for (int g = 0; g < r.G; ++g) {
+    const int64_t lo = total * g / r.G, hi = total * (g + 1) / r.G;
+    while (lo >= first + nch - (int64_t)b * kPerBlock) {
+      first += nch - (int64_t)b * kPerBlock;
+      ++b;
+    }
+    r.cta_block.push_back(b);
+    r.cta_chunk.push_back((int)(lo - first));
+    if (hi - lo > INT32_MAX) return false;
+    r.cta_units.push_back((int)(hi - lo));
+  }
+  *out = std::move(r);
+  return true;
+}
+
 }  // namespace ljgb

@@ -43,4 +43,16 @@ constexpr int kSplitGrain = 32;
 bool build_schedule(const int* n, int nsys, int BI, int TILE, int G, int tile_overhead, Schedule* out,
                     int grain = kSplitGrain);
 
+// Work split of the pair histogram of one box: i-blocks of kRdfBlock particles,
+// each against the j's from the block's own first particle on, in chunks of
+// kRdfChunk (pairs j <= i inside the block's own square are skipped by the
+// kernel), cut into G contiguous ranges of equal chunk counts.
+constexpr int kRdfBlock = 256;
+constexpr int kRdfChunk = 32;
+struct RdfRanges {
+  int G = 0;
+  std::vector<int> cta_block, cta_chunk, cta_units;  // G each
+};
+bool build_rdf_ranges(int n, int ctas, RdfRanges* out);
+
 }  // namespace ljgb

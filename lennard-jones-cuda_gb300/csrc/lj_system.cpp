@@ -265,12 +265,9 @@ struct lj_system {
   DevBuf<unsigned long long> rdf_sum;
   DevBuf<int4> qhist;
   long long rdf_samples = 0;
-  // CTA ranges of the histogram-only pair pass: the same blocks and tiles as
-  // `sched`, cut for the CTAs the histogram variant holds resident (more per
-  // SM than the force kernel: fewer registers, a small shared histogram).
-  Schedule hsched;
-  int hist_shape = -1, hist_nb = -1;
-  DevBuf<int> h_cta_tile_begin, h_cta_lo, h_cta_block, h_cta_jt;
+  // CTA ranges of the pair-histogram pass (they depend on N alone)
+  int hist_grid = 0;  // 0: not built yet
+  DevBuf<int> h_cta_block, h_cta_chunk, h_cta_units;
 
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
@@ -361,7 +358,6 @@ PairArgs pair_args(lj_system* s) {
   a.boxes = s->dboxes.p;
   a.partial = s->partial.p;
   a.status = s->status.p;
-  a.hist = HistArgs{0, 1, 1.0f, 0.0f, nullptr};
   return a;
 }
 
@@ -501,7 +497,6 @@ lj_status build_and_swap_schedule(lj_system* s) {
   s->partial.swap(partial);
   s->sched = std::move(sch);
   s->BI = threads;
-  s->hist_shape = -1;  // the histogram pass re-cuts its ranges on next use
   s->pred_ready = false;
   s->sched_shape = s->shape;
   s->sched_split = s->split_cap;
@@ -530,63 +525,45 @@ lj_status enqueue_frame_all(lj_system* s) {
   return LJ_OK;
 }
 
-lj_status enqueue_pairs(lj_system* s, bool forces, bool hist, const HistArgs* h) {
-  PairArgs p = pair_args(s);
-  if (h) p.hist = *h;
-  LJ_CUDA(s, launch_pairs(s->prec, s->shape, forces, hist, p, s->sched.G, s->stream));
+// The current shadow becomes that of the positions; a periodic box's frame is
+// its box, so only walled and open boxes have theirs rebuilt.
+lj_status enqueue_shadow(lj_system* s) {
+  if (s->any_nonperiodic) return enqueue_frame_all(s);
+  s->pred_ready = false;
+  LJ_CUDA(s, launch_quantize(state_args(s), nblocks(s), s->BI, false, s->stream));
   s->launches += 1;
   return LJ_OK;
 }
 
-// Arguments and grid of a histogram-only pair pass over shadow q with
-// histogram h, on `shape` (the geometry of the active schedule).  The CTA
-// ranges are cut for as many CTAs as that variant holds resident with h.nb
-// bins, and kept until the shape, the bin count or the schedule changes.
-lj_status hist_pass_args(lj_system* s, int shape, const int4* q, const HistArgs& h, PairArgs* out, int* grid) {
-  if (shape != s->hist_shape || h.nb != s->hist_nb) {
-    int per_sm = 0;
-    LJ_CUDA(s, pair_hist_occupancy(shape, h.nb, &per_sm));
-    if (per_sm < 1) return fail(s, LJ_ERR_NO_DEVICE, "histogram pair kernel cannot be resident on this device");
-    std::vector<int> n(s->nsys);
-    for (int k = 0; k < s->nsys; ++k) n[k] = s->cfg[k].n;
-    Schedule sch;
-    if (!build_schedule(n.data(), s->nsys, kShapes[shape].threads, kShapes[shape].tile, s->num_sms * per_sm,
-                        kTileOverhead, &sch))
-      return fail(s, LJ_ERR_INVALID, "cannot build the histogram schedule");
-    if (sch.BI != s->sched.BI || sch.TILE != s->sched.TILE || sch.blocks.size() != s->sched.blocks.size())
-      return fail(s, LJ_ERR_INVALID, "histogram schedule does not match the pair schedule's blocks");
-    // new range tables beside the old ones, swapped in once complete
-    const int G = sch.G;
-    DevBuf<int> ctb, clo, cb, cj;
-    LJ_CUDA(s, ctb.alloc(G + 1));
-    LJ_CUDA(s, clo.alloc(G + 1));
-    LJ_CUDA(s, cb.alloc(G));
-    LJ_CUDA(s, cj.alloc(G));
-    LJ_CUDA(s, cudaMemcpyAsync(ctb.p, sch.cta_tile_begin.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice,
-                               s->stream));
-    LJ_CUDA(s, cudaMemcpyAsync(clo.p, sch.cta_lo.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, s->stream));
-    LJ_CUDA(s, cudaMemcpyAsync(cb.p, sch.cta_block.data(), sizeof(int) * G, cudaMemcpyHostToDevice, s->stream));
-    LJ_CUDA(s, cudaMemcpyAsync(cj.p, sch.cta_jt.data(), sizeof(int) * G, cudaMemcpyHostToDevice, s->stream));
-    LJ_CUDA(s, cudaStreamSynchronize(s->stream));
-    s->h_cta_tile_begin.swap(ctb);
-    s->h_cta_lo.swap(clo);
-    s->h_cta_block.swap(cb);
-    s->h_cta_jt.swap(cj);
-    s->hsched = std::move(sch);
-    // step graphs that accumulate the RDF name the old tables (freed on return)
-    if (s->rdf_acc) clear_graphs(s);
-    s->hist_shape = shape;
-    s->hist_nb = h.nb;
-  }
+lj_status enqueue_pairs(lj_system* s) {
   PairArgs p = pair_args(s);
-  p.q = q;
-  p.hist = h;
-  p.cta_tile_begin = s->h_cta_tile_begin.p;
-  p.cta_lo = s->h_cta_lo.p;
-  p.cta_block = s->h_cta_block.p;
-  p.cta_jt = s->h_cta_jt.p;
-  *out = p;
-  *grid = s->hsched.G;
+  LJ_CUDA(s, launch_pairs(s->prec, s->shape, p, s->sched.G, s->stream));
+  s->launches += 1;
+  return LJ_OK;
+}
+
+// Arguments of a pair-histogram pass of box 0 over shadow q.  The CTA ranges
+// are built and uploaded on the first use.
+lj_status rdf_pass(lj_system* s, const int4* q, const HistArgs& h, RdfPass* out) {
+  if (s->hist_grid == 0) {
+    RdfRanges r;
+    if (!build_rdf_ranges(s->cfg[0].n, s->num_sms * rdf_ctas_per_sm(), &r))
+      return fail(s, LJ_ERR_INVALID, "cannot build the histogram ranges");
+    // new tables beside the (empty) old ones, swapped in once complete
+    DevBuf<int> cb, cc, cu;
+    LJ_CUDA(s, cb.alloc(r.G));
+    LJ_CUDA(s, cc.alloc(r.G));
+    LJ_CUDA(s, cu.alloc(r.G));
+    LJ_CUDA(s, cudaMemcpyAsync(cb.p, r.cta_block.data(), sizeof(int) * r.G, cudaMemcpyHostToDevice, s->stream));
+    LJ_CUDA(s, cudaMemcpyAsync(cc.p, r.cta_chunk.data(), sizeof(int) * r.G, cudaMemcpyHostToDevice, s->stream));
+    LJ_CUDA(s, cudaMemcpyAsync(cu.p, r.cta_units.data(), sizeof(int) * r.G, cudaMemcpyHostToDevice, s->stream));
+    LJ_CUDA(s, cudaStreamSynchronize(s->stream));
+    s->h_cta_block.swap(cb);
+    s->h_cta_chunk.swap(cc);
+    s->h_cta_units.swap(cu);
+    s->hist_grid = r.G;
+  }
+  *out = RdfPass{q, s->sc.p, s->cfg[0].n, s->h_cta_block.p, s->h_cta_chunk.p, s->h_cta_units.p, h};
   return LJ_OK;
 }
 
@@ -597,7 +574,7 @@ lj_status enqueue_compute_forces(lj_system* s) {
   if (st) return st;
   st = enqueue_frame_all(s);
   if (st) return st;
-  st = enqueue_pairs(s, true, false, nullptr);
+  st = enqueue_pairs(s);
   if (st) return st;
   StateArgs a = state_args(s);
   LJ_CUDA(s, launch_reduce(a, nblocks(s), s->BI, MODE_FORCES_ONLY, s->stream));
@@ -637,7 +614,7 @@ lj_status enqueue_step(lj_system* s, int mode, cudaEvent_t* ev, bool capture, in
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[1], s->stream, flags));
   {
     PairArgs p = pair_args(s);
-    LJ_CUDA(s, launch_pairs(s->prec, s->shape, true, false, p, s->sched.G, s->stream));
+    LJ_CUDA(s, launch_pairs(s->prec, s->shape, p, s->sched.G, s->stream));
     ++k;
   }
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[2], s->stream, flags));
@@ -690,7 +667,7 @@ int step_mode(const lj_system* s) {
   return MODE_EVN;
 }
 
-lj_status enqueue_after_step(lj_system* s, const PairArgs* hist, int hist_grid, int* kernels);
+lj_status enqueue_after_step(lj_system* s, const RdfPass& rdf, int* kernels);
 
 lj_status get_graph(lj_system* s, int mode, GraphEntry** out) {
   const bool fused = use_fused(s);
@@ -704,11 +681,9 @@ lj_status get_graph(lj_system* s, int mode, GraphEntry** out) {
   }
   // The RDF pass's range tables are built before the capture (building them
   // may allocate and synchronise).
-  PairArgs hist{};
-  int hist_grid = 0;
+  RdfPass pass{};
   if (rdf) {
-    const int shape = (s->prec == LJ_PREC_MIXED) ? s->shape : 0;
-    lj_status hst = hist_pass_args(s, shape, s->qhist.p, s->rdf_args, &hist, &hist_grid);
+    lj_status hst = rdf_pass(s, s->qhist.p, s->rdf_args, &pass);
     if (hst) return hst;
   }
   GraphEntry ge;
@@ -722,7 +697,7 @@ lj_status get_graph(lj_system* s, int mode, GraphEntry** out) {
   LJ_CUDA(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   lj_status st = fused ? enqueue_step_fused(s, mode, ge.profiled ? ev : nullptr, true, &ge.kernels)
                        : enqueue_step(s, mode, ge.profiled ? ev : nullptr, true, &ge.kernels);
-  if (!st && (counters || rdf)) st = enqueue_after_step(s, &hist, hist_grid, &ge.kernels);
+  if (!st && (counters || rdf)) st = enqueue_after_step(s, pass, &ge.kernels);
   cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
   if (st || ce != cudaSuccess) {  // nothing of a failed capture is kept
     if (g) cudaGraphDestroy(g);
@@ -777,9 +752,9 @@ lj_status flush_observables(lj_system* s) {
 // row, counting phase -- lives on the device): the counters' bookkeeping and
 // histogram, and the RDF of the step's positions (quantized into a shadow of
 // their own: the step's shadow buffer holds the next step's prediction) added
-// into the running sum.  `hist` are the histogram pass's arguments, prepared
+// into the running sum.  `rdf` are the histogram pass's arguments, prepared
 // before the capture.
-lj_status enqueue_after_step(lj_system* s, const PairArgs* hist, int hist_grid, int* kernels) {
+lj_status enqueue_after_step(lj_system* s, const RdfPass& rdf, int* kernels) {
   if (s->counter_cap > 0) {
     LJ_CUDA(s, launch_counters(state_args(s), s->dcounters.p, (int)s->counters.size(), s->counter_bins,
                                s->counter_state.p, s->counter_ring.p, s->counter_part.p, s->ntotal, s->stream));
@@ -789,8 +764,7 @@ lj_status enqueue_after_step(lj_system* s, const PairArgs* hist, int hist_grid, 
     StateArgs a = state_args(s);
     a.q = s->qhist.p;
     LJ_CUDA(s, launch_quantize(a, nblocks(s), s->BI, false, s->stream));
-    const int shape = (s->prec == LJ_PREC_MIXED) ? s->shape : 0;
-    LJ_CUDA(s, launch_pairs(LJ_PREC_MIXED, shape, false, true, *hist, hist_grid, s->stream));
+    LJ_CUDA(s, launch_rdf(rdf, s->hist_grid, s->stream));
     *kernels += 2;
   }
   return LJ_OK;
@@ -1143,10 +1117,9 @@ lj_status lj_destroy(lj_system* s) {
   s->counter_part.free();
   s->rdf_sum.free();
   s->qhist.free();
-  s->h_cta_tile_begin.free();
-  s->h_cta_lo.free();
   s->h_cta_block.free();
-  s->h_cta_jt.free();
+  s->h_cta_chunk.free();
+  s->h_cta_units.free();
   s->cta_lo.free();
   s->cta_block.free();
   s->cta_jt.free();
@@ -1664,7 +1637,7 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   if (!(width > 0)) return fail(s, LJ_ERR_INVALID, "bin width must be > 0");
   if (s->nsys != 1) return fail(s, LJ_ERR_UNSUPPORTED, "RDF counts apply to single-box handles");
   DeviceGuard device_guard(s->device);
-  lj_status st = enqueue_frame_all(s);
+  lj_status st = enqueue_shadow(s);
   if (st) return st;
   LJ_CUDA(s, cudaMemsetAsync(s->hist.p, 0, sizeof(unsigned long long) * nbins, s->stream));
   HistArgs h{};
@@ -1682,14 +1655,10 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   }
   h.counts = s->hist.p;
   // The histogram path always runs on the fixed-point shadow.
-  // FP64 handles schedule 128-particle i-blocks and 256-record j-tiles,
-  // the geometry of MIXED shape 0, so that shape reads their tables.
-  const int shape = (s->prec == LJ_PREC_MIXED) ? s->shape : 0;
-  PairArgs p;
-  int grid = 0;
-  st = hist_pass_args(s, shape, pair_args(s).q, h, &p, &grid);
+  RdfPass p{};
+  st = rdf_pass(s, pair_args(s).q, h, &p);
   if (st) return st;
-  LJ_CUDA(s, launch_pairs(LJ_PREC_MIXED, shape, false, true, p, grid, s->stream));
+  LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
   s->launches += 1;
   LJ_CUDA(s, cudaMemcpyAsync(counts, s->hist.p, sizeof(unsigned long long) * nbins, cudaMemcpyDeviceToHost,
                              s->stream));
