@@ -134,7 +134,7 @@ bool ensure_ctx(int n, int block_hint) {
     g_ctx.release();
   }
   REF_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  REF_CHECK(pair_occupancy(0, shape, &per_sm));
+  REF_CHECK(pair_occupancy(shape, &per_sm));
   Schedule s;
   // at most 8 CTAs per i-block (a block's epilogue sums one segment per CTA)
   const int nb_i = (n + kShapes[shape].threads - 1) / kShapes[shape].threads;
@@ -226,7 +226,7 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   a.status = c.status;
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.hist, 0, sizeof(unsigned long long) * kRefBins, c.stream));
-  REF_CHECK(launch_pairs(0, c.shape, a, c.sched.G, c.stream));
+  REF_CHECK(launch_pairs(c.shape, a, c.sched.G, c.stream));
   if (want_rdf)
     REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.hist}},
                          c.rdf_grid, c.stream));

@@ -102,7 +102,11 @@ __global__ void k_drift(StateArgs s) {
       if (MODE == MODE_EVN) s.v[k] = fma(box.hdt, f, v[c]);
       if (MODE == MODE_TVN) s.tf[k] = 0.5 * f;
     }
-    if (box.bc == 0) store_shadow(s, s.sc[bi.sys], p, x[0], x[1], x[2], box);
+    if (box.bc == 0) {
+      // an FP64 step reads the FP64 shadow alone
+      if (s.prec) s.xd[p] = make_double4_32a(x[0], x[1], x[2], 0.0);
+      else store_shadow(s, s.sc[bi.sys], p, x[0], x[1], x[2], box);
+    }
   }
   if (box.bc != 0) block_bbox(s, B, valid, x, sh);
 }
@@ -204,12 +208,12 @@ __global__ void k_quantize(StateArgs s, int only_nonperiodic) {
 }
 
 // ---------------------------------------------------------------------------
-// Sum of the pair-kernel segments into FP64 forces and per-particle sums,
-// then (EVN) the second half-kick + boundaries, or (TVN) the averaged force
+// Sum of the MIXED pair kernel's segments into FP64 forces and per-particle
+// sums (k_reduce64 is FP64's), then (EVN) the second half-kick + boundaries, or (TVN) the averaged force
 // and the half-kicked velocity whose kinetic temperature sets chi.
 // Block partials: [0] K, [1] V, [2] W, [3] sum tv^2.
 // ---------------------------------------------------------------------------
-template <int MODE, int PREC>
+template <int MODE>
 __global__ void k_reduce(StateArgs s) {
   __shared__ double sh[4 * 32];
   const int B = blockIdx.x;
@@ -220,18 +224,9 @@ __global__ void k_reduce(StateArgs s) {
   const BoxArgs box = s.boxes[bi.sys];
   double part[4] = {0., 0., 0., 0.};
   if (valid) {
-    double S[5] = {0., 0., 0., 0., 0.};
-    if (PREC == 0) {
-      segment_sums(s, bi, tid, S);
-    } else {
-      const double* pd = reinterpret_cast<const double*>(s.partial);
-      for (int k = 0; k < bi.seg_count; ++k) {
-        const size_t base = (size_t)(bi.seg_first + k) * 5 * s.bi_threads + tid;
-#pragma unroll
-        for (int c = 0; c < 5; ++c) S[c] += pd[base + (size_t)c * s.bi_threads];
-      }
-    }
-    const double fs = (PREC == 0) ? s.sc[bi.sys].fscale : 4.0 * box.eps / (box.sigma * box.sigma);
+    double S[5];
+    segment_sums(s, bi, tid, S);
+    const double fs = s.sc[bi.sys].fscale;
     double F[3] = {fs * S[0], fs * S[1], fs * S[2]};
     const double e = box.eps4 * (S[3] - S[4]);
     const double w = box.eps4 * fma(12.0, S[3], -6.0 * S[4]);
@@ -847,15 +842,9 @@ cudaError_t launch_quantize(const StateArgs& s, int nblocks, int bi, bool only_n
 }
 
 cudaError_t launch_reduce(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st) {
-  if (s.prec == 0) {
-    if (mode == MODE_FORCES_ONLY) k_reduce<MODE_FORCES_ONLY, 0><<<nblocks, bi, 0, st>>>(s);
-    else if (mode == MODE_EVN) k_reduce<MODE_EVN, 0><<<nblocks, bi, 0, st>>>(s);
-    else k_reduce<MODE_TVN, 0><<<nblocks, bi, 0, st>>>(s);
-  } else {
-    if (mode == MODE_FORCES_ONLY) k_reduce<MODE_FORCES_ONLY, 1><<<nblocks, bi, 0, st>>>(s);
-    else if (mode == MODE_EVN) k_reduce<MODE_EVN, 1><<<nblocks, bi, 0, st>>>(s);
-    else k_reduce<MODE_TVN, 1><<<nblocks, bi, 0, st>>>(s);
-  }
+  if (mode == MODE_FORCES_ONLY) k_reduce<MODE_FORCES_ONLY><<<nblocks, bi, 0, st>>>(s);
+  else if (mode == MODE_EVN) k_reduce<MODE_EVN><<<nblocks, bi, 0, st>>>(s);
+  else k_reduce<MODE_TVN><<<nblocks, bi, 0, st>>>(s);
   return cudaGetLastError();
 }
 

@@ -122,6 +122,8 @@ struct BoxArgs {
   double kP;     // rho / N:    P = (W / 6 + N T) kP
   double inv3N;  // 1 / (3 N):  Tkin = inv3N sum tv^2
   double invT0;  // 1 / T0 (0 when T0 = 0)
+  double fscale64;  // 4 eps / sigma^2: F = fscale64 sum s d of the FP64 pair pass
+  long long image_lo, image_hi;  // bits of the separations where the FP64 nearest image turns (ImageBounds)
   double wall_margin;  // walls: m = max(sigma, L / 20), the frame's margin beyond [0, L] and the positions
 };
 

@@ -25,7 +25,6 @@ struct HistArgs {
 // Arguments of the persistent pair kernels (by value).
 struct PairArgs {
   const int4* q;              // MIXED: fixed-point shadow (x, y, z, pad), all boxes
-  const double4_32a* xd;          // FP64: position shadow (x, y, z, 0)
   const BlockInfo* blocks;    // i-blocks of the schedule
   const int* cta_tile_begin;  // G+1 tile ranges
   const int* cta_block;       // first i-block of each CTA
@@ -34,7 +33,7 @@ struct PairArgs {
                               // last tile, 0 = whole tile); nullptr = whole tiles only
   const DevScalars* sc;       // per box frame / scalars
   const BoxArgs* boxes;       // per box constants
-  float* partial;             // nseg x 5 x threads  (float, or double for FP64)
+  float* partial;             // nseg x 5 x threads
   int* status;                // device status word (timeouts)
 };
 
@@ -62,11 +61,9 @@ struct PairShape {
 
 extern const PairShape kShapes[];
 extern const int kNumShapes;
-int fp64_block_threads();
-int fp64_tile();
 
-cudaError_t pair_occupancy(int prec, int shape, int* blocks_per_sm);
-cudaError_t launch_pairs(int prec, int shape, const PairArgs& a, int grid, cudaStream_t st);
+cudaError_t pair_occupancy(int shape, int* blocks_per_sm);
+cudaError_t launch_pairs(int shape, const PairArgs& a, int grid, cudaStream_t st);
 struct FusedPairArgs;
 cudaError_t launch_pairs_fused(int shape, int mode, const FusedPairArgs& a, int grid, cudaStream_t st);
 
@@ -112,6 +109,32 @@ struct FusedPairArgs {
   PairArgs pair;
   StateArgs st;
 };
+
+// FP64 pair pass over unordered pairs (lj_pairs64.cu).  Each box's particles
+// form tiles of 32 (the FP64 handles' i-blocks), `group` tiles a square side;
+// a tile's sums lie in groups + 1 slots of 5 x 32 doubles: slot ga from the
+// squares (ga, its own group), slot gb + 1 from (its own group, gb).  parts:
+// warps that share a square (1 unless group is 1).
+struct Pair64Task {
+  int sys, ga, gb;
+};
+struct Pair64Box {
+  int p0, n, tiles, groups;
+  long long tile0_slot;  // slot of the box's tile 0
+};
+struct Pair64Args {
+  const double4_32a* xd;  // position shadow (x, y, z, 0)
+  const Pair64Task* tasks;
+  const Pair64Box* boxes64;
+  const BoxArgs* boxes;
+  double* part;
+  int ntasks, group, parts, nsys;
+};
+// BoxArgs::image_lo / image_hi of a period L (bits of two separations).
+void fp64_image_bounds(double L, double invL, long long* lo, long long* hi);
+cudaError_t launch_pairs64(const Pair64Args& a, cudaStream_t st);
+// With the observables of every box, except for MODE_TVN.
+cudaError_t launch_reduce64(const StateArgs& s, const Pair64Args& a, int nblocks, int mode, cudaStream_t st);
 
 cudaError_t launch_drift_mode(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st);
 cudaError_t launch_bbox(const StateArgs& s, int nblocks, int bi, cudaStream_t st);

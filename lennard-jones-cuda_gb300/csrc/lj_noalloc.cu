@@ -248,7 +248,7 @@ extern "C" lj_status lj_forces_static(const float* pos4, float* force4, double* 
   // array until a call with another n replaces it.
   if (g_static_plan_n[dev] != n) {
     int per_sm = 0;
-    e = pair_occupancy(0, kShape, &per_sm);
+    e = pair_occupancy(kShape, &per_sm);
     if (e != cudaSuccess) return (lj_status)static_fail(LJ_ERR_CUDA, cudaGetErrorString(e));
     plan_static(n, g_static_sms[dev] * per_sm, &g_static_plan);
     const StaticPlan& p = g_static_plan;
@@ -282,7 +282,7 @@ extern "C" lj_status lj_forces_static(const float* pos4, float* force4, double* 
   a.sc = sc;
   a.partial = partial;
   a.status = status;
-  if ((e = launch_pairs(0, kShape, a, G, st)) != cudaSuccess)
+  if ((e = launch_pairs(kShape, a, G, st)) != cudaSuccess)
     return (lj_status)static_fail(LJ_ERR_CUDA, cudaGetErrorString(e));
   k_static_reduce<<<nblocks, kBI, 0, st>>>(partial, blocks, sc, reinterpret_cast<float4*>(force4), blk);
   k_static_sums<<<1, 256, 0, st>>>(blk, nblocks, dsums);

@@ -415,131 +415,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_pairs_mixed_fused(FusedPairAr
 }
 
 // ---------------------------------------------------------------------------
-// All-FP64 persistent pair kernel (the comparator path): double positions,
-// minimum image by rint, double accumulators.  Same schedule and partials
-// layout (5 doubles per particle per segment).
-// ---------------------------------------------------------------------------
-template <int THREADS, int TILE, int STAGES>
-__global__ void __launch_bounds__(THREADS) k_pairs_fp64(PairArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  double4_32a* sx = reinterpret_cast<double4_32a*>(smem_raw);
-  __shared__ uint64_t bars[STAGES];
-
-  const int g = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int t0 = a.cta_tile_begin[g], t1 = a.cta_tile_begin[g + 1];
-  const int lo0 = a.cta_lo ? a.cta_lo[g] : 0, lo1 = a.cta_lo ? a.cta_lo[g + 1] : 0;
-  const int ntiles = t1 - t0 + (lo1 > 0 ? 1 : 0);
-  if (ntiles <= 0) return;
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) mbar_init(&bars[s], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-
-  int pB = a.cta_block[g], pjt = a.cta_jt[g], issued = 0;
-  if (tid == 0) {
-    const int pre = ntiles < STAGES ? ntiles : STAGES;
-    for (; issued < pre; ++issued) {
-      const BlockInfo bi = a.blocks[pB];
-      const int j0 = pjt * TILE;
-      const int cnt = min(TILE, bi.n_sys - j0);
-      const int s = issued % STAGES;
-      mbar_arrive_expect_tx(&bars[s], (uint32_t)cnt * 32u);
-      bulk_g2s(sx + s * TILE, a.xd + bi.p0 + j0, (uint32_t)cnt * 32u, &bars[s]);
-      if (++pjt == bi.njt) { ++pB; pjt = 0; }
-    }
-  }
-
-  int B = a.cta_block[g], jt = a.cta_jt[g];
-  BlockInfo bi = a.blocks[B];
-  int i_local = bi.i0 + tid;
-  bool valid_i = tid < bi.n_i;
-  double4_32a xi = a.xd[bi.p0 + (valid_i ? i_local : bi.i0)];
-  BoxArgs box = a.boxes[bi.sys];
-  double s2 = box.sigma * box.sigma;
-  bool periodic = box.bc == 0;
-  double ax = 0., ay = 0., az = 0., aa = 0., ab = 0.;
-
-  int k = 0;
-  bool failed = false;
-  for (; k < ntiles; ++k) {
-    const int s = k % STAGES;
-    const bool ok = mbar_wait_bounded(&bars[s], (uint32_t)((k / STAGES) & 1));
-    const int j0 = jt * TILE;
-    const int cnt = min(TILE, bi.n_sys - j0);
-    const int jlo = k == 0 ? lo0 : 0;
-    const int jhi = (k == ntiles - 1 && lo1 > 0) ? lo1 : cnt;
-    if (ok) {
-      const double4_32a* st = sx + s * TILE;
-      for (int jj = jlo; jj < jhi; ++jj) {
-        const double4_32a xj = st[jj];
-        double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        if (periodic) {  // nearest image, ties away from zero (fast_round, MDSystem.cpp:732-739)
-          dx = fma(-box.L, round(dx * box.invL), dx);
-          dy = fma(-box.L, round(dy * box.invL), dy);
-          dz = fma(-box.L, round(dz * box.invL), dz);
-        }
-        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-        double ri = s2 / r2;
-        if (j0 + jj == i_local) ri = 0.0;
-        const double r6 = ri * ri * ri;
-        const double sf = r6 * ri * fma(12.0, r6, -6.0);
-        ax = fma(sf, dx, ax);
-        ay = fma(sf, dy, ay);
-        az = fma(sf, dz, az);
-        aa = fma(r6, r6, aa);
-        ab += r6;
-      }
-    }
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      break;
-    }
-    if (tid == 0 && issued < ntiles) {
-      const BlockInfo pbi = a.blocks[pB];
-      const int pj0 = pjt * TILE;
-      const int pcnt = min(TILE, pbi.n_sys - pj0);
-      mbar_arrive_expect_tx(&bars[s], (uint32_t)pcnt * 32u);
-      bulk_g2s(sx + s * TILE, a.xd + pbi.p0 + pj0, (uint32_t)pcnt * 32u, &bars[s]);
-      if (++pjt == pbi.njt) { ++pB; pjt = 0; }
-      ++issued;
-    }
-    const bool last = (k == ntiles - 1);
-    const bool block_end = (jt + 1 == bi.njt);
-    if (block_end || last) {
-      if (valid_i) {
-        const int seg = bi.seg_first + (g - bi.g_first);
-        double* out = reinterpret_cast<double*>(a.partial) + (size_t)seg * 5 * THREADS;
-        out[0 * THREADS + tid] = ax;
-        out[1 * THREADS + tid] = ay;
-        out[2 * THREADS + tid] = az;
-        out[3 * THREADS + tid] = aa;
-        out[4 * THREADS + tid] = ab;
-      }
-      ax = ay = az = aa = ab = 0.;
-      if (block_end && !last) {
-        ++B;
-        bi = a.blocks[B];
-        i_local = bi.i0 + tid;
-        valid_i = tid < bi.n_i;
-        xi = a.xd[bi.p0 + (valid_i ? i_local : bi.i0)];
-        box = a.boxes[bi.sys];
-        s2 = box.sigma * box.sigma;
-        periodic = box.bc == 0;
-        jt = 0;
-      }
-    } else {
-      ++jt;
-    }
-  }
-  if (failed && tid == 0) {
-    for (int kk = k; kk < issued; ++kk) mbar_wait_bounded(&bars[kk % STAGES], (uint32_t)((kk / STAGES) & 1));
-    atomicOr(a.status, LJ_DEVFLAG_TIMEOUT);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Shape table and launchers.
 // ---------------------------------------------------------------------------
 namespace {
@@ -567,19 +442,6 @@ cudaError_t occupancy_mixed_t(int* blocks_per_sm) {
       sizeof(int4) * STAGES * TILE);
 }
 
-template <int THREADS, int TILE, int STAGES>
-cudaError_t launch_fp64_t(const PairArgs& a, int grid, cudaStream_t st) {
-  const size_t smem = sizeof(double4_32a) * STAGES * TILE;
-  k_pairs_fp64<THREADS, TILE, STAGES><<<grid, THREADS, smem, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int THREADS, int TILE, int STAGES>
-cudaError_t occupancy_fp64_t(int* blocks_per_sm) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_pairs_fp64<THREADS, TILE, STAGES>,
-                                                       THREADS, sizeof(double4_32a) * STAGES * TILE);
-}
-
 }  // namespace
 
 // Kernel shapes the autotuner chooses among (threads = i-block size; MINB =
@@ -599,13 +461,7 @@ const PairShape kShapes[] = {
 };
 const int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
-constexpr int kFp64Threads = 128, kFp64Tile = 256, kFp64Stages = 3;
-
-int fp64_block_threads() { return kFp64Threads; }
-int fp64_tile() { return kFp64Tile; }
-
-cudaError_t pair_occupancy(int prec, int shape, int* blocks_per_sm) {
-  if (prec == 1) return occupancy_fp64_t<kFp64Threads, kFp64Tile, kFp64Stages>(blocks_per_sm);
+cudaError_t pair_occupancy(int shape, int* blocks_per_sm) {
   switch (shape) {
 #define LJ_OCC_CASE(i, T, TL, S, M) \
   case i:                           \
@@ -616,8 +472,7 @@ cudaError_t pair_occupancy(int prec, int shape, int* blocks_per_sm) {
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_pairs(int prec, int shape, const PairArgs& a, int grid, cudaStream_t st) {
-  if (prec == 1) return launch_fp64_t<kFp64Threads, kFp64Tile, kFp64Stages>(a, grid, st);
+cudaError_t launch_pairs(int shape, const PairArgs& a, int grid, cudaStream_t st) {
   switch (shape) {
 #define LJ_LAUNCH_CASE(i, T, TL, S, M) \
   case i:                              \

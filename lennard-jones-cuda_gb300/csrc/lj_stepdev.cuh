@@ -114,20 +114,14 @@ __device__ __forceinline__ void box_sum3(const StateArgs& s, int b0, int b1, dou
   out[2] = acc[2];
 }
 
-// CalculateParameters (MDSystem.cpp:325-359) for box `sys`, plus t += dt for
-// steps (MDSystem.cpp:582) and the optional per-step record.  Block-wide call;
-// thread 0 writes.  sh: 3 x 32 doubles.
+// CalculateParameters (MDSystem.cpp:325-359) for box `sys` from its sums K, V,
+// W, plus t += dt for steps (MDSystem.cpp:582) and the optional per-step
+// record; one thread.
 // rec_parity >= 0: the record's Tkin is Tkin_rec[rec_parity] (TVN steps
 // whose observables were left pending), else the box's Tkin.
 template <int MODE>
-__device__ __forceinline__ void observables_box(const StateArgs& s, int sys, double* sh, int slot = 0,
-                                                int rec_parity = -1) {
-  const BoxArgs box = s.boxes[sys];
-  const int b0 = s.sys_block_first[sys], b1 = s.sys_block_first[sys + 1];
-  double kvw[3];
-  box_sum3(s, b0, b1, sh, kvw, slot);
-  const double K = kvw[0], V = kvw[1], W = kvw[2];
-  if (threadIdx.x != 0) return;
+__device__ __forceinline__ void write_observables(const StateArgs& s, int sys, const BoxArgs& box, double K, double V,
+                                                  double W, int rec_parity) {
   DevScalars& sc = s.sc[sys];
   const double N = (double)box.N;
   const double T = K * box.kT;                           // 2 K / 3 / N
@@ -167,6 +161,18 @@ __device__ __forceinline__ void observables_box(const StateArgs& s, int sys, dou
     r.step = sc.step;
     sc.rec_count += 1;
   }
+}
+
+// The same for the sums of the box's block partials.  Block-wide call; thread
+// 0 writes.  sh: 3 x 32 doubles.
+template <int MODE>
+__device__ __forceinline__ void observables_box(const StateArgs& s, int sys, double* sh, int slot = 0,
+                                                int rec_parity = -1) {
+  const BoxArgs box = s.boxes[sys];
+  const int b0 = s.sys_block_first[sys], b1 = s.sys_block_first[sys + 1];
+  double kvw[3];
+  box_sum3(s, b0, b1, sh, kvw, slot);
+  if (threadIdx.x == 0) write_observables<MODE>(s, sys, box, kvw[0], kvw[1], kvw[2], rec_parity);
 }
 
 // Observables of the boxes whose fused step of parity `parity` left them

@@ -242,7 +242,12 @@ struct lj_system {
   DevBuf<DevScalars> sc;
   DevBuf<BoxArgs> dboxes;
   DevBuf<double> blk_part;
-  DevBuf<float> partial;  // sized in bytes/4 to also hold doubles
+  DevBuf<float> partial;  // MIXED: nseg x 5 x BI
+  // FP64 pair pass: tasks, boxes and sums (Pair64Args)
+  int p64_group = 1, p64_parts = 1;
+  DevBuf<Pair64Task> p64_tasks;
+  DevBuf<Pair64Box> p64_boxes;
+  DevBuf<double> p64_part;
   DevBuf<int> status;
   DevBuf<DevRecord> records;
   DevBuf<unsigned long long> hist;
@@ -348,7 +353,6 @@ StateArgs state_args(lj_system* s) {
 PairArgs pair_args(lj_system* s) {
   PairArgs a{};
   a.q = s->qpar ? s->q2.p : s->q.p;
-  a.xd = s->xd.p;
   a.blocks = s->blocks.p;
   a.cta_tile_begin = s->cta_tile_begin.p;
   a.cta_block = s->cta_block.p;
@@ -359,6 +363,11 @@ PairArgs pair_args(lj_system* s) {
   a.partial = s->partial.p;
   a.status = s->status.p;
   return a;
+}
+
+Pair64Args pair64_args(const lj_system* s) {
+  return Pair64Args{s->xd.p,       s->p64_tasks.p,        s->p64_boxes.p, s->dboxes.p,
+                    s->p64_part.p, (int)s->p64_tasks.n, s->p64_group,   s->p64_parts,  s->nsys};
 }
 
 int nblocks(const lj_system* s) { return (int)s->sched.blocks.size(); }
@@ -418,6 +427,8 @@ lj_status upload_boxes(lj_system* s) {
     b.inv3N = 1.0 / (3.0 * b.N);
     b.invT0 = b.T0 > 0 ? 1.0 / b.T0 : 0.0;
     b.wall_margin = std::max(b.sigma, 0.05 * b.L);
+    b.fscale64 = 4.0 * b.eps / (b.sigma * b.sigma);
+    fp64_image_bounds(b.L, b.invL, &b.image_lo, &b.image_hi);
     s->any_open |= (b.bc == 2);
   }
   LJ_CUDA(s, cudaMemcpyAsync(s->dboxes.p, s->boxes.data(), sizeof(BoxArgs) * s->nsys, cudaMemcpyHostToDevice,
@@ -430,16 +441,60 @@ lj_status upload_boxes(lj_system* s) {
 // filled beside the old ones and swapped in only once complete, so a
 // failure (an allocation, say) leaves the handle on its previous schedule,
 // with shape and split cap put back to the ones that schedule was built for.
-lj_status build_and_swap_schedule(lj_system* s) {
-  int threads, tile, blocks_per_sm = 0;
-  if (s->prec == LJ_PREC_FP64) {
-    threads = fp64_block_threads();
-    tile = fp64_tile();
-  } else {
-    threads = kShapes[s->shape].threads;
-    tile = kShapes[s->shape].tile;
+// Squares and tasks of the FP64 pair pass for boxes of sizes n (Pair64Args).
+// The square side grows while there are still about 80 tasks an SM: a tile
+// then has at most ~256 slots, so the sums stay at 10 KB a particle whatever
+// N is.  With fewer than 8 tasks an SM the turns of a task are shared by 2, 4
+// or 8 warps: N = 512 gives 136 tasks for 152 SMs.
+struct Pair64Plan {
+  int group = 1, parts = 1;
+  long long slots = 0;
+  std::vector<Pair64Task> tasks;
+  std::vector<Pair64Box> boxes;
+};
+
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
+  Pair64Plan p;
+  auto squares = [&](long long group) {
+    long long t = 0;
+    for (int k : n) {
+      const long long g = ((k + 31) / 32 + group - 1) / group;
+      t += g * (g + 1) / 2;
+    }
+    return t;
+  };
+  while (squares(2ll * p.group) >= 80ll * sms) p.group *= 2;
+  if (p.group == 1)
+    while (p.parts < 8 && squares(1) * p.parts < 8ll * sms) p.parts *= 2;
+  int p0 = 0;
+  for (int k : n) {
+    Pair64Box b{};
+    b.p0 = p0;
+    b.n = k;
+    b.tiles = (k + 31) / 32;
+    b.groups = (b.tiles + p.group - 1) / p.group;
+    b.tile0_slot = p.slots;
+    p.slots += (long long)b.tiles * (b.groups + 1);
+    p.boxes.push_back(b);
+    p0 += k;
   }
-  LJ_CUDA(s, pair_occupancy(s->prec, s->shape, &blocks_per_sm));
+  // the squares on a box's diagonal hold half the pairs: they come last
+  for (int diag = 0; diag < 2; ++diag)
+    for (int k = 0; k < (int)n.size(); ++k)
+      for (int ga = 0; ga < p.boxes[k].groups; ++ga)
+        for (int gb = diag ? ga : ga + 1; gb < (diag ? ga + 1 : p.boxes[k].groups); ++gb)
+          p.tasks.push_back(Pair64Task{k, ga, gb});
+  return p;
+}
+
+lj_status build_and_swap_schedule(lj_system* s) {
+  const bool fp64 = s->prec == LJ_PREC_FP64;
+  // FP64: i-blocks of one tile; its pair pass has tasks of its own, so the
+  // stream-K ranges of the schedule are not used (one CTA, one j-tile).
+  const int threads = fp64 ? 32 : kShapes[s->shape].threads;
+  const int tile = fp64 ? 1 << 30 : kShapes[s->shape].tile;
+  int blocks_per_sm = 1;
+  if (!fp64) LJ_CUDA(s, pair_occupancy(s->shape, &blocks_per_sm));
   if (blocks_per_sm < 1) return fail(s, LJ_ERR_NO_DEVICE, "pair kernel cannot be resident on this device");
   std::vector<int> n(s->nsys);
   for (int k = 0; k < s->nsys; ++k) n[k] = s->cfg[k].n;
@@ -450,7 +505,9 @@ lj_status build_and_swap_schedule(lj_system* s) {
   // occupancy / 128 is unaffected).
   long long nbt = 0;
   for (int k = 0; k < s->nsys; ++k) nbt += (n[k] + threads - 1) / threads;
-  const int G = (int)std::min<long long>((long long)s->num_sms * blocks_per_sm, nbt * s->split_cap);
+  const int G = fp64 ? 1 : (int)std::min<long long>((long long)s->num_sms * blocks_per_sm, nbt * s->split_cap);
+  Pair64Plan p64;
+  if (fp64) p64 = plan_pairs64(n, s->num_sms);
   Schedule sch;
   if (!build_schedule(n.data(), s->nsys, threads, tile, G, kTileOverhead, &sch))
     return fail(s, LJ_ERR_INVALID, "cannot build the pair schedule");
@@ -468,9 +525,20 @@ lj_status build_and_swap_schedule(lj_system* s) {
   LJ_CUDA(s, bpart.alloc((size_t)nb * 8));
   LJ_CUDA(s, bcnt.alloc(nb));
   LJ_CUDA(s, gcnt.alloc(4));
-  // partial: nseg x 5 x BI values of 8 bytes (FP64) or 4 bytes (MIXED)
-  const size_t vals = (size_t)sch.nseg * 5 * threads;
-  LJ_CUDA(s, partial.alloc(vals * (s->prec == LJ_PREC_FP64 ? 2 : 1)));
+  DevBuf<Pair64Task> p64_tasks;
+  DevBuf<Pair64Box> p64_boxes;
+  DevBuf<double> p64_part;
+  if (fp64) {
+    LJ_CUDA(s, p64_tasks.alloc(p64.tasks.size()));
+    LJ_CUDA(s, p64_boxes.alloc(p64.boxes.size()));
+    LJ_CUDA(s, p64_part.alloc((size_t)p64.slots * 5 * 32));
+    LJ_CUDA(s, cudaMemcpyAsync(p64_tasks.p, p64.tasks.data(), sizeof(Pair64Task) * p64.tasks.size(),
+                               cudaMemcpyHostToDevice, s->stream));
+    LJ_CUDA(s, cudaMemcpyAsync(p64_boxes.p, p64.boxes.data(), sizeof(Pair64Box) * p64.boxes.size(),
+                               cudaMemcpyHostToDevice, s->stream));
+  } else {
+    LJ_CUDA(s, partial.alloc((size_t)sch.nseg * 5 * threads));
+  }
   LJ_CUDA(s, cudaMemsetAsync(bcnt.p, 0, sizeof(int) * nb, s->stream));
   LJ_CUDA(s, cudaMemsetAsync(gcnt.p, 0, sizeof(int) * gcnt.n, s->stream));
   LJ_CUDA(s, cudaMemcpyAsync(blocks.p, sch.blocks.data(), sizeof(BlockInfo) * nb, cudaMemcpyHostToDevice, s->stream));
@@ -495,6 +563,11 @@ lj_status build_and_swap_schedule(lj_system* s) {
   s->blk_cnt.swap(bcnt);
   s->glob_cnt.swap(gcnt);
   s->partial.swap(partial);
+  s->p64_tasks.swap(p64_tasks);
+  s->p64_boxes.swap(p64_boxes);
+  s->p64_part.swap(p64_part);
+  s->p64_group = p64.group;
+  s->p64_parts = p64.parts;
   s->sched = std::move(sch);
   s->BI = threads;
   s->pred_ready = false;
@@ -535,10 +608,30 @@ lj_status enqueue_shadow(lj_system* s) {
   return LJ_OK;
 }
 
+// The pair pass at the current shadow, and the sums of its parts with the
+// second half of a step of `mode`.
 lj_status enqueue_pairs(lj_system* s) {
-  PairArgs p = pair_args(s);
-  LJ_CUDA(s, launch_pairs(s->prec, s->shape, p, s->sched.G, s->stream));
-  s->launches += 1;
+  if (s->prec == LJ_PREC_FP64) LJ_CUDA(s, launch_pairs64(pair64_args(s), s->stream));
+  else LJ_CUDA(s, launch_pairs(s->shape, pair_args(s), s->sched.G, s->stream));
+  return LJ_OK;
+}
+
+// ... TVN's rescale and the observables (k_reduce64 forms them itself unless
+// the rescale has to come first); *kernels counts the launches.
+lj_status enqueue_reduce(lj_system* s, int mode, int* kernels) {
+  const StateArgs a = state_args(s);
+  const bool fp64 = s->prec == LJ_PREC_FP64;
+  if (fp64) LJ_CUDA(s, launch_reduce64(a, pair64_args(s), nblocks(s), mode, s->stream));
+  else LJ_CUDA(s, launch_reduce(a, nblocks(s), s->BI, mode, s->stream));
+  *kernels += 1;
+  if (mode == MODE_TVN) {
+    LJ_CUDA(s, launch_tvn_finish(a, nblocks(s), s->BI, s->stream));
+    *kernels += 1;
+  }
+  if (!fp64 || mode == MODE_TVN) {
+    LJ_CUDA(s, launch_observables(a, s->nsys, mode, s->stream));
+    *kernels += 1;
+  }
   return LJ_OK;
 }
 
@@ -574,12 +667,10 @@ lj_status enqueue_compute_forces(lj_system* s) {
   if (st) return st;
   st = enqueue_frame_all(s);
   if (st) return st;
-  st = enqueue_pairs(s);
-  if (st) return st;
-  StateArgs a = state_args(s);
-  LJ_CUDA(s, launch_reduce(a, nblocks(s), s->BI, MODE_FORCES_ONLY, s->stream));
-  LJ_CUDA(s, launch_observables(a, s->nsys, MODE_FORCES_ONLY, s->stream));
-  s->launches += 2;
+  if ((st = enqueue_pairs(s))) return st;
+  int kernels = 1;
+  if ((st = enqueue_reduce(s, MODE_FORCES_ONLY, &kernels))) return st;
+  s->launches += kernels;
   return LJ_OK;
 }
 
@@ -612,20 +703,11 @@ lj_status enqueue_step(lj_system* s, int mode, cudaEvent_t* ev, bool capture, in
     k += 2;
   }
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[1], s->stream, flags));
-  {
-    PairArgs p = pair_args(s);
-    LJ_CUDA(s, launch_pairs(s->prec, s->shape, p, s->sched.G, s->stream));
-    ++k;
-  }
+  lj_status pst = enqueue_pairs(s);
+  if (pst) return pst;
+  ++k;
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[2], s->stream, flags));
-  LJ_CUDA(s, launch_reduce(a, nb, s->BI, mode, s->stream));
-  ++k;
-  if (mode == MODE_TVN) {
-    LJ_CUDA(s, launch_tvn_finish(a, nb, s->BI, s->stream));
-    ++k;
-  }
-  LJ_CUDA(s, launch_observables(a, s->nsys, mode, s->stream));
-  ++k;
+  if ((pst = enqueue_reduce(s, mode, &k))) return pst;
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[3], s->stream, flags));
   if (kernels) *kernels = k;
   return LJ_OK;
@@ -1128,6 +1210,9 @@ lj_status lj_destroy(lj_system* s) {
   s->dboxes.free();
   s->blk_part.free();
   s->partial.free();
+  s->p64_tasks.free();
+  s->p64_boxes.free();
+  s->p64_part.free();
   s->status.free();
   s->records.free();
   s->hist.free();
@@ -1927,10 +2012,14 @@ lj_status lj_set_split_cap(lj_system* s, int32_t cap) {
 lj_status lj_split_info(lj_system* s, int32_t* cap, int32_t* ctas, int32_t* max_segments) {
   if (!s) return LJ_ERR_INVALID;
   if (cap) *cap = s->split_cap;
-  if (ctas) *ctas = s->sched.G;
+  const bool fp64 = s->prec == LJ_PREC_FP64;
+  if (ctas) *ctas = fp64 ? (int)s->p64_tasks.n : s->sched.G;
   if (max_segments) {
     int m = 0;
     for (const BlockInfo& b : s->sched.blocks) m = std::max(m, b.seg_count);
+    if (fp64)
+      for (const lj_config& c : s->cfg)
+        m = std::max(m, (((c.n + 31) / 32 + s->p64_group - 1) / s->p64_group + 1));
     *max_segments = m;
   }
   return LJ_OK;

@@ -24,6 +24,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = [
     "lj_pairs.cu",
     "lj_rdf.cu",
+    "lj_pairs64.cu",
     "lj_integrate.cu",
     "lj_compat.cu",
     "lj_noalloc.cu",
