@@ -20,7 +20,11 @@
 //   Xb_m = dl_m/dx_m + Xb_{m+1} + H(x_m) z_m,   H = dF/dx (symmetric)
 //   d/d(eps, sigma) += G(x_m)^T z_m + dl_m/d(eps, sigma),  G = dF/d(eps, sigma)
 // dloss/dx_0 = Xb_0, dloss/dv_0 = bb_0.  One pair pass per reverse step
-// gives F, dF/dsigma, H z and the energy / virial sums at x_m.
+// gives dl_m/dx_m + H z and the sums G^T z, V, W and dW/dsigma at x_m.
+//
+// Two launches a step either way: the pair pass, and one that sums its parts
+// and does all of the per-particle work up to the next pass (forward: kick,
+// states kept, drift; reverse: Xb_m, then z_{m-1}).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -32,201 +36,355 @@
 #include "lj_device.cuh"
 #include "lj_gb300.h"
 #include "lj_init.h"
+#include "lj_pair64.cuh"
+#include "lj_schedule.h"
 
 namespace ljgb {
 namespace {
 
-constexpr int kAdjThreads = 128;  // i per CTA of the pair pass (and of the per-particle kernels)
-constexpr int kAdjTile = 64;      // j records staged in shared memory per tile
-constexpr int kParts = 12;        // per-i sums: F(3), dF/dsigma(3), Hz(3), e, w, dw/dsigma
+constexpr int kScalars = 5;  // sums over pairs of a task: e, u, then (reverse) u_sigma, z.F, z.dF/dsigma
 
 struct AdjBox {
   int n, npad;
   double L, invL;
   double eps4, sigma2, inv_sigma;
+  ImageBounds ib;  // round-half-even images
 };
 
-// All-pairs pass over j in [blockIdx.y * jchunk, +jchunk) for the i of this
-// CTA (one i per thread), minimum image d = d - L rint(d / L).  Per pair,
-// with s6 = (sigma^2/r^2)^3, s12 = s6^2:
-//   f = g d,  g = 4 eps (12 s12 - 6 s6) / r^2
-//   dg/dsigma = 4 eps (144 s12 - 36 s6) / (sigma r^2)
-//   H z: J (z_i - z_j),  J = g I + (g'/r) d d^T,  g'/r = 4 eps (-168 s12 + 48 s6) / r^4
-// Partial sums go to part[blockIdx.y][c][i] (summed in a fixed order later).
+// The pair pass's work split (Pair64Plan of one box) and sums.
+struct AdjPass {
+  const Pair64Task* tasks;
+  int ntasks, tiles, groups, group, parts;
+  double* part;  // [tile][groups + 1][3][32]: F (forward), or dl/dx + H z
+  double* scal;  // [task][kScalars]
+};
+
+struct AdjSums {
+  double x, y, z;
+};
+
+// Pairs of tiles ta and tb, turns r0 .. r1-1, as in lj_pairs64.cu: lane = i,
+// positions (and z) and sums of the j's move around the warp, so each pair is
+// evaluated once for both particles.  Per pair, with s6 = (sigma^2/r^2)^3 and
+// c = 4 eps s6 / r^2 (one factor of all three):
+//   f = g d,  g = c (12 s6 - 6)
+//   dg/dsigma = gs / sigma,  gs = c (144 s6 - 36)
+//   H z: J (z_i - z_j),  J = g I + h d d^T,  h = c / r^2 (-168 s6 + 48)
+// The reverse step needs F and dF/dsigma only in dl/dx = cF F + cA dF/dsigma
+// and in the sums z.F and z.dF/dsigma, which over unordered pairs are those
+// of g d.dz and gs d.dz: six vector sums a pair are left of eighteen.
+// FP64 operations an unordered pair: 30 forward, 55 reverse (of 2 x 36 and
+// 2 x 66 over ordered pairs with an IEEE division).
+template <bool HVP, bool UNIT>
+__device__ __forceinline__ int adj_turns(const AdjBox& b, const double* x, const double* z, double cF, double cA,
+                                         int ta, int tb, int r0, int r1, const double (&xi)[3], const double (&zi)[3],
+                                         AdjSums& I, AdjSums& J, double (&S)[kScalars]) {
+  const int lane = threadIdx.x & 31;
+  const bool vi = ta * 32 + lane < b.n, diag = ta == tb;
+  int jl = (lane + r0) & 31;
+  const int j = min(tb * 32 + jl, b.n - 1);
+  double xj[3], zj[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    xj[c] = x[(size_t)c * b.npad + j];
+    if (HVP) zj[c] = z[(size_t)c * b.npad + j];
+  }
+#pragma unroll 2
+  for (int r = r0; r < r1; ++r) {
+    double d[3] = {xi[0] - xj[0], xi[1] - xj[1], xi[2] - xj[2]};
+    nearest_image<false>(d, b.L, b.invL, b.ib);
+    double r2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+    double y = rcp_seed(r2);
+    const bool meets = vi && tb * 32 + jl < b.n && !(diag && r == 16 && lane >= 16);
+    if (!meets || beyond_seed(r2)) {  // a seed of 0 makes the pair's terms 0
+      r2 = 1.0;
+      y = 0.0;
+    }
+    const double inv = rcp_from_seed(r2, y);
+    const double s2 = UNIT ? inv : b.sigma2 * inv;
+    const double s6 = s2 * s2 * s2;
+    const double c = b.eps4 * inv * s6;
+    const double t = fma(12.0, s6, -6.0);
+    const double g = c * t;
+    S[0] = fma(s6, s6 - 1.0, S[0]);
+    S[1] = fma(s6, t, S[1]);
+    double k = g;  // factor of d in i's sums
+    double gz[3] = {0.0, 0.0, 0.0};
+    if (HVP) {
+      const double ts = fma(144.0, s6, -36.0);
+      const double gs = c * ts;
+      const double h = c * inv * fma(-168.0, s6, 48.0);
+      double dz[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) dz[q] = zi[q] - zj[q];
+      const double dot = fma(d[2], dz[2], fma(d[1], dz[1], d[0] * dz[0]));
+      S[2] = fma(s6, ts, S[2]);
+      S[3] = fma(g, dot, S[3]);
+      S[4] = fma(gs, dot, S[4]);
+      k = fma(cF, g, fma(cA, gs, h * dot));
+#pragma unroll
+      for (int q = 0; q < 3; ++q) gz[q] = dz[q];
+    }
+    if (HVP) {
+      I.x = fma(g, gz[0], fma(k, d[0], I.x));
+      I.y = fma(g, gz[1], fma(k, d[1], I.y));
+      I.z = fma(g, gz[2], fma(k, d[2], I.z));
+      J.x = shfl_next(fma(-g, gz[0], fma(-k, d[0], J.x)), lane);
+      J.y = shfl_next(fma(-g, gz[1], fma(-k, d[1], J.y)), lane);
+      J.z = shfl_next(fma(-g, gz[2], fma(-k, d[2], J.z)), lane);
+    } else {
+      I.x = fma(k, d[0], I.x);
+      I.y = fma(k, d[1], I.y);
+      I.z = fma(k, d[2], I.z);
+      J.x = shfl_next(fma(-k, d[0], J.x), lane);
+      J.y = shfl_next(fma(-k, d[1], J.y), lane);
+      J.z = shfl_next(fma(-k, d[2], J.z), lane);
+    }
+    jl = (jl + 1) & 31;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      xj[q] = shfl_next(xj[q], lane);
+      if (HVP) zj[q] = shfl_next(zj[q], lane);
+    }
+  }
+  return jl;
+}
+
+__device__ __forceinline__ void store_adj(double* to, int at, const AdjSums& s) {
+  to[at] = s.x;
+  to[32 + at] = s.y;
+  to[64 + at] = s.z;
+}
+
+// One task: a square of tiles by one warp, or of one tile by `parts` warps.
+template <bool HVP, bool UNIT>
+__device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, const double* x, const double* z,
+                                         double cF, double cA, double* sh) {
+  const int lane = threadIdx.x & 31;
+  const Pair64Task tk = a.tasks[blockIdx.x];
+  const int slots = a.groups + 1;
+  constexpr int kS = HVP ? kScalars : 2;
+  double S[kScalars] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  auto load = [&](const double* from, int t, double (&to)[3]) {
+    const int i = min(t * 32 + lane, b.n - 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) to[c] = from[(size_t)c * b.npad + i];
+  };
+  double xi[3], zi[3] = {0.0, 0.0, 0.0};
+  if (a.parts > 1) {
+    const int w = threadIdx.x >> 5, ta = tk.ga, tb = tk.gb;
+    const int first = ta == tb ? 1 : 0, turns = (ta == tb ? 16 : 32) / a.parts;
+    load(x, ta, xi);
+    if (HVP) load(z, ta, zi);
+    AdjSums I{}, J{};
+    const int jl =
+        adj_turns<HVP, UNIT>(b, x, z, cF, cA, ta, tb, first + w * turns, first + (w + 1) * turns, xi, zi, I, J, S);
+    double* const mine = sh + w * (192 + kScalars);
+    store_adj(mine, lane, I);
+    store_adj(mine + 96, jl, J);
+#pragma unroll
+    for (int m = 0; m < kS; ++m) S[m] = warp_sum(S[m]);
+    if (lane == 0)
+#pragma unroll
+      for (int m = 0; m < kS; ++m) mine[192 + m] = S[m];
+    __syncthreads();
+    for (int k = threadIdx.x; k < 192 + kS; k += blockDim.x) {
+      double v = 0.0;
+      for (int p = 0; p < a.parts; ++p) v += sh[p * (192 + kScalars) + k];
+      if (k < 96) a.part[((size_t)ta * slots + tb + 1) * 96 + k] = v;
+      else if (k < 192) a.part[((size_t)tb * slots + ta) * 96 + k - 96] = v;
+      else a.scal[(size_t)blockIdx.x * kScalars + k - 192] = v;
+    }
+    return;
+  }
+  const int a0 = tk.ga * a.group, a1 = min(a.tiles, a0 + a.group);
+  const int b0 = tk.gb * a.group, b1 = min(a.tiles, b0 + a.group);
+  for (int ta = a0; ta < a1; ++ta) {
+    load(x, ta, xi);
+    if (HVP) load(z, ta, zi);
+    AdjSums I{};
+    for (int tb = max(ta, b0); tb < b1; ++tb) {
+      const int r0 = ta == tb ? 1 : 0, r1 = ta == tb ? 17 : 32;
+      double* const jslot = a.part + ((size_t)tb * slots + tk.ga) * 96;
+      const int at = (lane + r0) & 31;
+      AdjSums J{};
+      if (ta > a0) J = AdjSums{jslot[at], jslot[32 + at], jslot[64 + at]};  // earlier rows' sums
+      const int jl = adj_turns<HVP, UNIT>(b, x, z, cF, cA, ta, tb, r0, r1, xi, zi, I, J, S);
+      store_adj(jslot, jl, J);
+      __syncwarp();
+    }
+    store_adj(a.part + ((size_t)ta * slots + tk.gb + 1) * 96, lane, I);
+  }
+#pragma unroll
+  for (int m = 0; m < kS; ++m) S[m] = warp_sum(S[m]);
+  if (lane == 0)
+#pragma unroll
+    for (int m = 0; m < kS; ++m) a.scal[(size_t)blockIdx.x * kScalars + m] = S[m];
+}
+
+// FP64-pipe bound.  N = 1000: 37 us forward, 65 us reverse (79 and 142 over
+// ordered pairs).
 template <bool HVP>
-__global__ void __launch_bounds__(kAdjThreads) k_adj_pairs(AdjBox b, const double* __restrict__ x,
-                                                           const double* __restrict__ z, int jchunk,
-                                                           double* __restrict__ part) {
-  __shared__ double sx[3][kAdjTile];
-  __shared__ double sz[3][HVP ? kAdjTile : 1];
-  const int i = blockIdx.x * kAdjThreads + threadIdx.x;
-  const int j0 = blockIdx.y * jchunk;
-  const int j1 = min(b.n, j0 + jchunk);
-  const bool valid = i < b.n;
-  double xi[3], zi[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    xi[c] = valid ? x[(size_t)c * b.npad + i] : 0.0;
-    zi[c] = (HVP && valid) ? z[(size_t)c * b.npad + i] : 0.0;
-  }
-  double acc[kParts];
-#pragma unroll
-  for (int c = 0; c < kParts; ++c) acc[c] = 0.0;
-  for (int t0 = j0; t0 < j1; t0 += kAdjTile) {
-    const int cnt = min(kAdjTile, j1 - t0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < cnt; k += kAdjThreads) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sx[c][k] = x[(size_t)c * b.npad + t0 + k];
-        if (HVP) sz[c][k] = z[(size_t)c * b.npad + t0 + k];
-      }
-    }
-    __syncthreads();
-    if (!valid) continue;
-    for (int k = 0; k < cnt; ++k) {
-      if (t0 + k == i) continue;
-      double d[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double t = xi[c] - sx[c][k];
-        d[c] = fma(-b.L, rint(t * b.invL), t);
-      }
-      const double r2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
-      const double inv = 1.0 / r2;
-      const double s2 = b.sigma2 * inv;
-      const double s6 = s2 * s2 * s2;
-      const double s12 = s6 * s6;
-      const double u = fma(12.0, s12, -6.0 * s6);
-      const double g = b.eps4 * u * inv;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] = fma(g, d[c], acc[c]);
-      acc[9] += s12 - s6;
-      acc[10] += u;
-      if (HVP) {
-        const double us = fma(144.0, s12, -36.0 * s6);
-        const double gs = b.eps4 * us * inv * b.inv_sigma;
-        const double h = b.eps4 * fma(-168.0, s12, 48.0 * s6) * inv * inv;
-        double dz[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dz[c] = zi[c] - sz[c][k];
-        const double hd = h * fma(d[2], dz[2], fma(d[1], dz[1], d[0] * dz[0]));
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          acc[3 + c] = fma(gs, d[c], acc[3 + c]);
-          acc[6 + c] = fma(g, dz[c], fma(hd, d[c], acc[6 + c]));
-        }
-        acc[11] += us;
-      }
-    }
-  }
-  if (!valid) return;
-  acc[9] *= b.eps4;
-  acc[10] *= b.eps4;
-  acc[11] *= b.eps4 * b.inv_sigma;
-  double* out = part + (size_t)blockIdx.y * kParts * b.npad + i;
-#pragma unroll
-  for (int c = 0; c < kParts; ++c)
-    if (HVP || c < 3 || c == 9 || c == 10) out[(size_t)c * b.npad] = acc[c];
+__global__ void __launch_bounds__(256) k_adj_pairs(AdjBox b, AdjPass a, const double* __restrict__ x,
+                                                   const double* __restrict__ z, double cF, double cA) {
+  extern __shared__ double sh[];  // parts > 1: parts x (2 x 3 x 32 + kScalars)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (b.sigma2 == 1.0) adj_task<HVP, true>(b, a, x, z, cF, cA, sh);
+  else adj_task<HVP, false>(b, a, x, z, cF, cA, sh);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Sum of part[js][c][i] over js = 0..JS-1 (fixed order).
-__device__ __forceinline__ double part_sum(const double* part, int JS, int npad, int c, int i) {
-  double s = 0.0;
-  for (int js = 0; js < JS; ++js) s += part[((size_t)js * kParts + c) * npad + i];
-  return s;
-}
+// CTA of one tile for the per-particle kernels below: 12 warps sum its slots
+// (component c by four warps, a quarter of the slots each), a 13th sums this
+// tile's share of the tasks' scalars; then warp c holds component c of the
+// tile's particles.  Fixed order throughout.  (One CTA of 128 particles and
+// a thread per particle summed 12 values of 32 parts serially: 97 us at
+// N = 1000.)
+constexpr int kSumWarps = 4;
+constexpr int kAdjTileThreads = 32 * (3 * kSumWarps + 1);
 
-// x += dt v + dt^2 F / 2; v += dt F / 2; single +-L wrap.
-__global__ void k_adj_drift(AdjBox b, double* x, double* v, const double* f, double dt) {
-  const int i = blockIdx.x * kAdjThreads + threadIdx.x;
-  if (i >= b.n) return;
-  const double hdt = 0.5 * dt, hdt2 = 0.5 * dt * dt;
+template <int NS>
+__device__ __forceinline__ double adj_tile_sums(const AdjPass& a, double (&scal)[NS], bool* mine) {
+  __shared__ double sum[3 * kSumWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
+  if (warp < 3 * kSumWarps) {
+    const int c = warp % 3, u = warp / 3, slots = a.groups + 1;
+    const double* p = a.part + (size_t)t * slots * 96 + c * 32 + lane;
+    double q0 = 0.0, q1 = 0.0;
+    for (int k = u; k < slots; k += 8 * kSumWarps) {
+      double v[8];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const size_t k = (size_t)c * b.npad + i;
-    const double fc = f[k], vc = v[k];
-    double xc = fma(hdt2, fc, fma(dt, vc, x[k]));
-    if (xc < 0.) xc += b.L;
-    if (xc > b.L) xc -= b.L;
-    x[k] = xc;
-    v[k] = fma(hdt, fc, vc);
-  }
-}
-
-// F = pair sums; with kick: v += dt F / 2.  Block partials (K, V, W) into
-// blk[blockIdx.x * 3 + 0..2] when blk is non-null.
-__global__ void k_adj_forces(AdjBox b, const double* part, int JS, double* f, double* v, double hdt, double* blk) {
-  __shared__ double sh[3 * 32];
-  const int i = blockIdx.x * kAdjThreads + threadIdx.x;
-  double p[3] = {0.0, 0.0, 0.0};
-  if (i < b.n) {
-    double vv = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const size_t k = (size_t)c * b.npad + i;
-      const double fc = part_sum(part, JS, b.npad, c, i);
-      f[k] = fc;
-      if (v) {
-        const double vc = fma(hdt, fc, v[k]);
-        v[k] = vc;
-        vv = fma(vc, vc, vv);
-      }
+      for (int m = 0; m < 8; ++m) v[m] = k + m * kSumWarps < slots ? p[(size_t)(k + m * kSumWarps) * 96] : 0.0;
+      q0 += (v[0] + v[2]) + (v[4] + v[6]);
+      q1 += (v[1] + v[3]) + (v[5] + v[7]);
     }
-    p[0] = 0.5 * vv;
-    p[1] = 0.5 * part_sum(part, JS, b.npad, 9, i);
-    p[2] = part_sum(part, JS, b.npad, 10, i);
+    sum[warp][lane] = q0 + q1;
+  } else {
+    for (int k = t + lane * a.tiles; k < a.ntasks; k += 32 * a.tiles)
+#pragma unroll
+      for (int m = 0; m < NS; ++m) scal[m] += a.scal[(size_t)k * kScalars + m];
+#pragma unroll
+    for (int m = 0; m < NS; ++m) scal[m] = warp_sum(scal[m]);
+  }
+  __syncthreads();
+  *mine = warp < 3;
+  if (warp >= 3) return 0.0;
+  return (sum[warp][lane] + sum[warp + 3][lane]) + (sum[warp + 6][lane] + sum[warp + 9][lane]);
+}
+
+// x + dt v + dt^2 F / 2 with a single +-L wrap, and v + dt F / 2.
+__device__ __forceinline__ void adj_drift1(const AdjBox& b, double& x, double& v, double f, double dt) {
+  x = fma(0.5 * dt * dt, f, fma(dt, v, x));
+  if (x < 0.) x += b.L;
+  if (x > b.L) x -= b.L;
+  v = fma(0.5 * dt, f, v);
+}
+
+// Where a state is kept: x, v, f (any may be null).
+struct AdjKeep {
+  double *x, *v, *f;
+};
+
+// F of the current positions; with kick, v += dt F / 2.  The finished state
+// goes to `keep` and `keep2`; with drift, x and v become those half a step on.
+// Block partials (K, V, W) into blk[tile * 3 + 0..2] when blk is non-null.
+__global__ void __launch_bounds__(kAdjTileThreads) k_adj_forces(AdjBox b, AdjPass a, double* x, double* v, double dt,
+                                                                int kick, int drift, AdjKeep keep, AdjKeep keep2,
+                                                                double* blk) {
+  __shared__ double ksum[3];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  double scal[2] = {0.0, 0.0};
+  bool mine;
+  const double F = adj_tile_sums<2>(a, scal, &mine);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+  double vv = 0.0;
+  if (mine && i < b.n) {
+    const size_t k = (size_t)warp * b.npad + i;
+    double xc = x[k], vc = v[k];
+    if (kick) vc = fma(0.5 * dt, F, vc);
+    vv = vc * vc;
+    if (keep.x) keep.x[k] = xc;
+    if (keep.v) keep.v[k] = vc;
+    if (keep.f) keep.f[k] = F;
+    if (keep2.x) keep2.x[k] = xc;
+    if (keep2.v) keep2.v[k] = vc;
+    if (drift) {
+      adj_drift1(b, xc, vc, F, dt);
+      x[k] = xc;
+    }
+    v[k] = vc;
   }
   if (!blk) return;
-  block_sum<3>(p, sh);
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) blk[(size_t)blockIdx.x * 3 + c] = p[c];
-}
-
-// Reverse step m, first half: bb <- bb_m, z <- z_m (from Xb_{m+1}, bb_{m+1}).
-// cv = dl_m/dv_m / v_m (0 for m = 0); first = (m == 0).
-__global__ void k_adj_prep(AdjBox b, const double* vm, const double* Xb, double* bb, double* z, double cv,
-                           double dt, int first) {
-  const int i = blockIdx.x * kAdjThreads + threadIdx.x;
-  if (i >= b.n) return;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const size_t k = (size_t)c * b.npad + i;
-    const double X = Xb[k], bn = bb[k];
-    const double bm = fma(dt, X, fma(cv, vm[k], bn));
-    const double y = fma(0.5 * dt * dt, X, 0.5 * dt * bn);
-    z[k] = first ? y : fma(0.5 * dt, bm, y);
-    bb[k] = bm;
+  if (mine) {
+    vv = warp_sum(vv);
+    if (lane == 0) ksum[warp] = vv;
+  }
+  __syncthreads();
+  if (warp == 3 * kSumWarps && lane == 0) {
+    double* const o = blk + (size_t)blockIdx.x * 3;
+    o[0] = 0.5 * (ksum[0] + ksum[1] + ksum[2]);
+    o[1] = b.eps4 * scal[0];        // V: each unordered pair once
+    o[2] = 2.0 * (b.eps4 * scal[1]);  // W: ordered pairs
   }
 }
 
-// Reverse step m, second half: Xb <- dl_m/dx_m + Xb + H z, with
-// dl_m/dx_m = cF F + cA dF/dsigma (both 0 for m = 0).  Block partials
-// (z.F, z.dF/dsigma, V, W, dW/dsigma) into blk[blockIdx.x * 5 + 0..4].
-__global__ void k_adj_finish(AdjBox b, const double* part, int JS, const double* z, double* Xb, double cF,
-                             double cA, double* blk) {
-  __shared__ double sh[5 * 32];
-  const int i = blockIdx.x * kAdjThreads + threadIdx.x;
-  double p[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (i < b.n) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const size_t k = (size_t)c * b.npad + i;
-      const double F = part_sum(part, JS, b.npad, c, i);
-      const double A = part_sum(part, JS, b.npad, 3 + c, i);
-      const double Hz = part_sum(part, JS, b.npad, 6 + c, i);
-      Xb[k] = fma(cF, F, fma(cA, A, Xb[k] + Hz));
-      const double zc = z[k];
-      p[0] = fma(zc, F, p[0]);
-      p[1] = fma(zc, A, p[1]);
-    }
-    p[2] = 0.5 * part_sum(part, JS, b.npad, 9, i);
-    p[3] = part_sum(part, JS, b.npad, 10, i);
-    p[4] = part_sum(part, JS, b.npad, 11, i);
+// A replay's start from a checkpoint: the state into `keep`, x and v half a
+// step on.
+__global__ void k_adj_start(AdjBox b, const double* ckpt, size_t s3, double* x, double* v, double dt, AdjKeep keep) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= 3 * b.npad || k % b.npad >= b.n) return;
+  double xc = ckpt[k], vc = ckpt[s3 + k];
+  keep.x[k] = xc;
+  keep.v[k] = vc;
+  adj_drift1(b, xc, vc, ckpt[2 * s3 + k], dt);
+  x[k] = xc;
+  v[k] = vc;
+}
+
+// Reverse step m, first half, one component: bb_m and z_m from Xb_{m+1} = X
+// and bb_{m+1}.  cv = dl_m/dv_m / v_m (0 for m = 0); first = (m == 0).
+__device__ __forceinline__ void adj_prep1(double X, double vm, double cv, double dt, int first, double* bb,
+                                          double* z) {
+  const double bn = *bb;
+  const double bm = fma(dt, X, fma(cv, vm, bn));
+  const double y = fma(0.5 * dt * dt, X, 0.5 * dt * bn);
+  *z = first ? y : fma(0.5 * dt, bm, y);
+  *bb = bm;
+}
+
+__global__ void k_adj_prep(AdjBox b, const double* vm, const double* Xb, double* bb, double* z, double cv, double dt) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= 3 * b.npad || k % b.npad >= b.n) return;
+  adj_prep1(Xb[k], vm[k], cv, dt, 0, bb + k, z + k);
+}
+
+// Reverse step m, second half: Xb <- dl_m/dx_m + Xb + H z (the pass's sums),
+// then, for m > 0 (vm non-null), the first half of step m - 1 with its v.
+// Block partials (z.F, z.dF/dsigma, V, W, dW/dsigma) into blk[tile * 5 + 0..4].
+__global__ void __launch_bounds__(kAdjTileThreads) k_adj_finish(AdjBox b, AdjPass a, const double* vm, double* Xb,
+                                                                double* bb, double* z, double cv, double dt,
+                                                                int first, double* blk) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  double scal[kScalars] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  bool mine;
+  const double H = adj_tile_sums<kScalars>(a, scal, &mine);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+  if (mine && i < b.n) {
+    const size_t k = (size_t)warp * b.npad + i;
+    const double X = Xb[k] + H;
+    Xb[k] = X;
+    if (vm) adj_prep1(X, vm[k], cv, dt, first, bb + k, z + k);
   }
-  block_sum<5>(p, sh);
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 5; ++c) blk[(size_t)blockIdx.x * 5 + c] = p[c];
+  if (warp == 3 * kSumWarps && lane == 0) {
+    double* const o = blk + (size_t)blockIdx.x * 5;
+    o[0] = scal[3];
+    o[1] = b.inv_sigma * scal[4];
+    o[2] = b.eps4 * scal[0];
+    o[3] = 2.0 * (b.eps4 * scal[1]);
+    o[4] = 2.0 * (b.eps4 * b.inv_sigma * scal[2]);
+  }
 }
 
 // (N x 3 interleaved) <-> component-major device layout.
@@ -272,15 +430,18 @@ using namespace ljgb;
 
 struct lj_adjoint {
   int device = 0;
-  int n = 0, npad = 0, nib = 0, JS = 1, jchunk = 0;
+  int n = 0, npad = 0;
   AdjBox box{};
+  AdjPass pass{};
   double rho = 0, eps = 1, sigma = 1;
   double wK = 0.0, wV = 1.0, wP = 1.0;
   int every = 20;
   cudaStream_t stream = nullptr;
-  DBuf<double> x, v, f, x0, v0, part, ckpt, seg, Xb, bb, z, blk, hostio;
+  DBuf<double> x, v, x0, v0, part, scal, ckpt, seg, Xb, bb, z, blk, hostio;
+  DBuf<Pair64Task> tasks;
   // last forward
   bool have_forward = false;
+  int seg_in_hand = -1;  // segment whose states `seg` holds (the forward pass leaves its last one there)
   double dt = 0.0;
   int S = 0;
   double loss = 0.0;
@@ -310,21 +471,22 @@ lj_status afail(lj_adjoint* a, lj_status code, const char* fmt, ...) {
 
 size_t xyz(const lj_adjoint* a) { return (size_t)3 * a->npad; }
 
-// F (and the energy sums) at the positions in x; kick v when v is non-null.
-lj_status adj_forces(lj_adjoint* a, double* x, double* f, double* v, double* blk) {
-  const dim3 grid(a->nib, a->JS);
-  k_adj_pairs<false><<<grid, kAdjThreads, 0, a->stream>>>(a->box, x, nullptr, a->jchunk, a->part.p);
-  k_adj_forces<<<a->nib, kAdjThreads, 0, a->stream>>>(a->box, a->part.p, a->JS, f, v, 0.5 * a->dt, blk);
-  ADJ_CUDA(a, cudaGetLastError());
+// The pair pass at positions x: forces, or (z non-null) the reverse step's.
+lj_status adj_pairs(lj_adjoint* a, const double* x, const double* z, double cF, double cA) {
+  const AdjPass& p = a->pass;
+  const size_t smem = p.parts > 1 ? sizeof(double) * (192 + kScalars) * p.parts : 0;
+  ADJ_CUDA(a, launch_dependent(z ? k_adj_pairs<true> : k_adj_pairs<false>, p.ntasks, 32 * p.parts, smem, a->stream,
+                               a->box, p, x, z, cF, cA));
   return LJ_OK;
 }
 
-// One forward step of the current state (x, v, f); observables partials of
-// step m into blk (nib x 3).
-lj_status adj_step(lj_adjoint* a, double* blk) {
-  k_adj_drift<<<a->nib, kAdjThreads, 0, a->stream>>>(a->box, a->x.p, a->v.p, a->f.p, a->dt);
-  ADJ_CUDA(a, cudaGetLastError());
-  return adj_forces(a, a->x.p, a->f.p, a->v.p, blk);
+// F at the current positions and what follows it (k_adj_forces).
+lj_status adj_forces(lj_adjoint* a, bool kick, bool drift, AdjKeep keep, AdjKeep keep2, double* blk) {
+  lj_status st = adj_pairs(a, a->x.p, nullptr, 0.0, 0.0);
+  if (st) return st;
+  ADJ_CUDA(a, launch_dependent(k_adj_forces, a->pass.tiles, kAdjTileThreads, 0, a->stream, a->box, a->pass, a->x.p,
+                               a->v.p, a->dt, kick ? 1 : 0, drift ? 1 : 0, keep, keep2, blk));
+  return LJ_OK;
 }
 
 lj_status adj_copy(lj_adjoint* a, double* dst, const double* src, size_t count) {
@@ -348,13 +510,13 @@ lj_status lj_adjoint_create(const lj_config* cfg, int32_t checkpoint_every, lj_a
   a->device = cfg->device;
   a->n = cfg->n;
   a->npad = (cfg->n + 31) / 32 * 32;
-  a->nib = (cfg->n + kAdjThreads - 1) / kAdjThreads;
   a->rho = cfg->density;
   a->eps = cfg->epsilon;
   a->sigma = cfg->sigma;
   a->every = checkpoint_every;
   const double L = std::cbrt((double)cfg->n / cfg->density);
-  a->box = AdjBox{cfg->n, a->npad, L, 1.0 / L, 4.0 * cfg->epsilon, cfg->sigma * cfg->sigma, 1.0 / cfg->sigma};
+  a->box = AdjBox{cfg->n, a->npad, L, 1.0 / L, 4.0 * cfg->epsilon, cfg->sigma * cfg->sigma, 1.0 / cfg->sigma,
+                  image_bounds(L, 1.0 / L, false)};
   auto bail = [&](lj_status st) {
     lj_adjoint_destroy(a);
     return st;
@@ -364,16 +526,18 @@ lj_status lj_adjoint_create(const lj_config* cfg, int32_t checkpoint_every, lj_a
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device) != cudaSuccess)
     return bail(LJ_ERR_NO_DEVICE);
-  // j split: about four CTAs per SM, j chunks a multiple of 32 records
-  const int want = std::max(1, (4 * sms + a->nib - 1) / a->nib);
-  a->jchunk = std::max(32, ((a->n + want - 1) / want + 31) / 32 * 32);
-  a->JS = (a->n + a->jchunk - 1) / a->jchunk;
+  const Pair64Plan plan = plan_pairs64({a->n}, sms);
   if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(LJ_ERR_CUDA);
   const size_t s3 = xyz(a);
-  if (a->x.alloc(s3) || a->v.alloc(s3) || a->f.alloc(s3) || a->x0.alloc(s3) || a->v0.alloc(s3) || a->Xb.alloc(s3) ||
-      a->bb.alloc(s3) || a->z.alloc(s3) || a->hostio.alloc(s3) ||
-      a->part.alloc((size_t)a->JS * kParts * a->npad))
+  if (a->x.alloc(s3) || a->v.alloc(s3) || a->x0.alloc(s3) || a->v0.alloc(s3) || a->Xb.alloc(s3) ||
+      a->bb.alloc(s3) || a->z.alloc(s3) || a->hostio.alloc(s3) || a->part.alloc((size_t)plan.slots * 96) ||
+      a->scal.alloc(plan.tasks.size() * kScalars) || a->tasks.alloc(plan.tasks.size()))
     return bail(LJ_ERR_OUT_OF_MEMORY);
+  if (cudaMemcpyAsync(a->tasks.p, plan.tasks.data(), sizeof(Pair64Task) * plan.tasks.size(), cudaMemcpyHostToDevice,
+                      a->stream) != cudaSuccess)
+    return bail(LJ_ERR_CUDA);
+  a->pass = AdjPass{a->tasks.p, (int)plan.tasks.size(), plan.boxes[0].tiles, plan.boxes[0].groups,
+                    plan.group, plan.parts,             a->part.p,           a->scal.p};
   std::vector<double> pos((size_t)3 * a->n), vel((size_t)3 * a->n);
   if (!sample_initial_state(a->n, L, cfg->temperature, cfg->lattice, cfg->jitter, cfg->sigma, cfg->seed, pos.data(),
                             vel.data()))
@@ -388,9 +552,10 @@ lj_status lj_adjoint_destroy(lj_adjoint* a) {
   if (!a) return LJ_OK;
   DeviceGuard device_guard(a->device);
   if (a->stream) cudaStreamSynchronize(a->stream);
-  for (DBuf<double>* b : {&a->x, &a->v, &a->f, &a->x0, &a->v0, &a->part, &a->ckpt, &a->seg, &a->Xb, &a->bb, &a->z,
+  for (DBuf<double>* b : {&a->x, &a->v, &a->x0, &a->v0, &a->part, &a->scal, &a->ckpt, &a->seg, &a->Xb, &a->bb, &a->z,
                           &a->blk, &a->hostio})
     b->free();
+  a->tasks.free();
   if (a->stream) cudaStreamDestroy(a->stream);
   delete a;
   return LJ_OK;
@@ -433,24 +598,33 @@ lj_status lj_adjoint_forward(lj_adjoint* a, double dt, int32_t nsteps, double* l
   a->dt = dt;
   a->S = nsteps;
   a->have_forward = false;
+  a->seg_in_hand = -1;
   const size_t s3 = xyz(a);
   const int J = (nsteps + a->every - 1) / a->every;
+  const int nt = a->pass.tiles;
   if (a->ckpt.alloc((size_t)J * 3 * s3) || a->seg.alloc((size_t)(a->every + 1) * 2 * s3) ||
-      a->blk.alloc((size_t)(nsteps + 1) * a->nib * 5))
+      a->blk.alloc((size_t)(nsteps + 1) * nt * 5))
     return afail(a, LJ_ERR_OUT_OF_MEMORY, "cannot allocate %d checkpoints of %d particles", J, a->n);
   lj_status st;
   if ((st = adj_copy(a, a->x.p, a->x0.p, s3)) || (st = adj_copy(a, a->v.p, a->v0.p, s3))) return st;
-  if ((st = adj_forces(a, a->x.p, a->f.p, nullptr, nullptr))) return st;
-  for (int m = 0; m < nsteps; ++m) {
-    if (m % a->every == 0) {
+  // State m: the pass at x_m, then kick, what is kept of it (a checkpoint,
+  // and the last segment's states, which the reverse sweep starts with), and
+  // the drift to x_{m+1}.
+  const int last0 = (J - 1) * a->every;
+  for (int m = 0; m <= nsteps; ++m) {
+    AdjKeep ck{}, sg{};
+    if (m < nsteps && m % a->every == 0) {
       double* c = a->ckpt.p + (size_t)(m / a->every) * 3 * s3;
-      if ((st = adj_copy(a, c, a->x.p, s3)) || (st = adj_copy(a, c + s3, a->v.p, s3)) ||
-          (st = adj_copy(a, c + 2 * s3, a->f.p, s3)))
-        return st;
+      ck = AdjKeep{c, c + s3, c + 2 * s3};
     }
-    if ((st = adj_step(a, a->blk.p + (size_t)m * a->nib * 3))) return st;
+    if (m >= last0) {
+      double* sl = a->seg.p + (size_t)(m - last0) * 2 * s3;
+      sg = AdjKeep{sl, sl + s3, nullptr};
+    }
+    double* const blk = m == 0 ? nullptr : a->blk.p + (size_t)(m - 1) * nt * 3;
+    if ((st = adj_forces(a, m > 0, m < nsteps, ck, sg, blk))) return st;
   }
-  std::vector<double> h((size_t)nsteps * a->nib * 3);
+  std::vector<double> h((size_t)nsteps * nt * 3);
   ADJ_CUDA(a, cudaMemcpyAsync(h.data(), a->blk.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, a->stream));
   ADJ_CUDA(a, cudaStreamSynchronize(a->stream));
   const double N = (double)a->n;
@@ -460,8 +634,8 @@ lj_status lj_adjoint_forward(lj_adjoint* a, double dt, int32_t nsteps, double* l
   double l = 0.0;
   for (int m = 0; m < nsteps; ++m) {
     double s[3] = {0.0, 0.0, 0.0};
-    for (int b = 0; b < a->nib; ++b)
-      for (int c = 0; c < 3; ++c) s[c] += h[((size_t)m * a->nib + b) * 3 + c];
+    for (int b = 0; b < nt; ++b)
+      for (int c = 0; c < 3; ++c) s[c] += h[((size_t)m * nt + b) * 3 + c];
     a->K[m] = s[0];
     a->V[m] = s[1];
     a->W[m] = s[2];
@@ -472,6 +646,7 @@ lj_status lj_adjoint_forward(lj_adjoint* a, double dt, int32_t nsteps, double* l
   if (!std::isfinite(l)) return afail(a, LJ_ERR_NONFINITE, "the loss is not finite");
   a->loss = l;
   a->have_forward = true;
+  a->seg_in_hand = J - 1;
   if (loss) *loss = l;
   return LJ_OK;
 }
@@ -502,40 +677,42 @@ lj_status lj_adjoint_backward(lj_adjoint* a, double* d_epsilon, double* d_sigma,
   ADJ_CUDA(a, cudaMemsetAsync(a->Xb.p, 0, sizeof(double) * s3, a->stream));
   ADJ_CUDA(a, cudaMemsetAsync(a->bb.p, 0, sizeof(double) * s3, a->stream));
   lj_status st;
+  const int nt = a->pass.tiles, grid3 = (3 * a->npad + 255) / 256;
   for (int j = J - 1; j >= 0; --j) {
     const int c0 = j * k, c1 = std::min(c0 + k, S);
-    // replay the segment from its checkpoint (same kernels as the forward)
-    const double* c = a->ckpt.p + (size_t)j * 3 * s3;
-    if ((st = adj_copy(a, a->x.p, c, s3)) || (st = adj_copy(a, a->v.p, c + s3, s3)) ||
-        (st = adj_copy(a, a->f.p, c + 2 * s3, s3)))
-      return st;
-    for (int m = c0; m <= c1; ++m) {
-      if (m > c0 && (st = adj_step(a, nullptr))) return st;
-      double* sl = a->seg.p + (size_t)(m - c0) * 2 * s3;
-      if ((st = adj_copy(a, sl, a->x.p, s3)) || (st = adj_copy(a, sl + s3, a->v.p, s3))) return st;
+    auto state = [&](int m) { return a->seg.p + (size_t)(m - c0) * 2 * s3; };
+    if (a->seg_in_hand != j) {
+      // replay the segment from its checkpoint (same kernels as the forward)
+      a->seg_in_hand = -1;
+      const double* c = a->ckpt.p + (size_t)j * 3 * s3;
+      ADJ_CUDA(a, launch_dependent(k_adj_start, grid3, 256, 0, a->stream, a->box, c, s3, a->x.p, a->v.p, dt,
+                                   AdjKeep{state(c0), state(c0) + s3, nullptr}));
+      for (int m = c0 + 1; m <= c1; ++m)
+        if ((st = adj_forces(a, true, m < c1, AdjKeep{state(m), state(m) + s3, nullptr}, AdjKeep{}, nullptr)))
+          return st;
+      a->seg_in_hand = j;
     }
-    // reverse sweep over m = c1 .. c0+1 (.. 0 in the first segment)
+    if (j == J - 1)
+      ADJ_CUDA(a, launch_dependent(k_adj_prep, grid3, 256, 0, a->stream, a->box, (const double*)(state(S) + s3),
+                                   (const double*)a->Xb.p, a->bb.p, a->z.p, cv, dt));
+    // reverse sweep over m = c1 .. c0+1 (.. 0 in the first segment); state
+    // c0 is the previous segment's last, and this one's checkpoint
     for (int m = c1; m >= (j == 0 ? 0 : c0 + 1); --m) {
-      const double* xm = a->seg.p + (size_t)(m - c0) * 2 * s3;
-      const double* vm = xm + s3;
-      k_adj_prep<<<a->nib, kAdjThreads, 0, a->stream>>>(a->box, vm, a->Xb.p, a->bb.p, a->z.p, m >= 1 ? cv : 0.0, dt,
-                                                        m == 0 ? 1 : 0);
-      k_adj_pairs<true><<<dim3(a->nib, a->JS), kAdjThreads, 0, a->stream>>>(a->box, xm, a->z.p, a->jchunk,
-                                                                             a->part.p);
-      k_adj_finish<<<a->nib, kAdjThreads, 0, a->stream>>>(a->box, a->part.p, a->JS, a->z.p, a->Xb.p,
-                                                          m >= 1 ? cF : 0.0, m >= 1 ? cA : 0.0,
-                                                          a->blk.p + (size_t)m * a->nib * 5);
-      ADJ_CUDA(a, cudaGetLastError());
+      if ((st = adj_pairs(a, state(m), a->z.p, m >= 1 ? cF : 0.0, m >= 1 ? cA * a->box.inv_sigma : 0.0))) return st;
+      const double* vm = m >= 1 ? state(m - 1) + s3 : nullptr;
+      ADJ_CUDA(a, launch_dependent(k_adj_finish, nt, kAdjTileThreads, 0, a->stream, a->box, a->pass, vm, a->Xb.p,
+                                   a->bb.p, a->z.p, m >= 2 ? cv : 0.0, dt, m == 1 ? 1 : 0,
+                                   a->blk.p + (size_t)m * nt * 5));
     }
   }
   // parameter gradients: fixed-order sums of the block partials
-  std::vector<double> h((size_t)(S + 1) * a->nib * 5);
+  std::vector<double> h((size_t)(S + 1) * nt * 5);
   ADJ_CUDA(a, cudaMemcpyAsync(h.data(), a->blk.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, a->stream));
   double de = 0.0, ds = 0.0;
   for (int m = 0; m <= S; ++m) {
     double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int b = 0; b < a->nib; ++b)
-      for (int q = 0; q < 5; ++q) s[q] += h[((size_t)m * a->nib + b) * 5 + q];
+    for (int b = 0; b < nt; ++b)
+      for (int q = 0; q < 5; ++q) s[q] += h[((size_t)m * nt + b) * 5 + q];
     de += s[0] / a->eps;  // G_eps^T z = z.F / eps
     ds += s[1];           // G_sigma^T z = z.dF/dsigma
     if (m >= 1) {         // explicit: dV/deps = V/eps, dV/dsigma = W/(2 sigma), dW/deps = W/eps

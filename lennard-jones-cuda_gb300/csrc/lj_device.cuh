@@ -193,4 +193,20 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   __syncthreads();
 }
 
+// Launch as a programmatic dependent of the kernel queued before.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 }  // namespace ljgb

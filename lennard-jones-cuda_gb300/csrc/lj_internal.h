@@ -127,4 +127,17 @@ struct BoxArgs {
   double wall_margin;  // walls: m = max(sigma, L / 20), the frame's margin beyond [0, L] and the positions
 };
 
+// FP64 pair pass over unordered pairs (lj_pairs64.cu).  Each box's particles
+// form tiles of 32 (the FP64 handles' i-blocks), `group` tiles a square side;
+// a tile's sums lie in groups + 1 slots of 5 x 32 doubles: slot ga from the
+// squares (ga, its own group), slot gb + 1 from (its own group, gb).  parts:
+// warps that share a square (1 unless group is 1).
+struct Pair64Task {
+  int sys, ga, gb;
+};
+struct Pair64Box {
+  int p0, n, tiles, groups;
+  long long tile0_slot;  // slot of the box's tile 0
+};
+
 }  // namespace ljgb

@@ -253,22 +253,6 @@ __global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair6
   if (lane == 0) write_observables<MODE>(s, bi.sys, box, kvw[0], kvw[1], kvw[2], -1);
 }
 
-// Launch as a programmatic dependent of the kernel queued before.
-template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 }  // namespace
 
 void fp64_image_bounds(double L, double invL, long long* lo, long long* hi) {

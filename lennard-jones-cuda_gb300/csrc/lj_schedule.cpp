@@ -139,4 +139,38 @@ bool build_rdf_ranges(int n, int ctas, RdfRanges* out) {
   return true;
 }
 
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
+  Pair64Plan p;
+  auto squares = [&](long long group) {
+    long long t = 0;
+    for (int k : n) {
+      const long long g = ((k + 31) / 32 + group - 1) / group;
+      t += g * (g + 1) / 2;
+    }
+    return t;
+  };
+  while (squares(2ll * p.group) >= 80ll * sms) p.group *= 2;
+  if (p.group == 1)
+    while (p.parts < 8 && squares(1) * p.parts < 8ll * sms) p.parts *= 2;
+  int p0 = 0;
+  for (int k : n) {
+    Pair64Box b{};
+    b.p0 = p0;
+    b.n = k;
+    b.tiles = (k + 31) / 32;
+    b.groups = (b.tiles + p.group - 1) / p.group;
+    b.tile0_slot = p.slots;
+    p.slots += (long long)b.tiles * (b.groups + 1);
+    p.boxes.push_back(b);
+    p0 += k;
+  }
+  // the squares on a box's diagonal hold half the pairs: they come last
+  for (int diag = 0; diag < 2; ++diag)
+    for (int k = 0; k < (int)n.size(); ++k)
+      for (int ga = 0; ga < p.boxes[k].groups; ++ga)
+        for (int gb = diag ? ga : ga + 1; gb < (diag ? ga + 1 : p.boxes[k].groups); ++gb)
+          p.tasks.push_back(Pair64Task{k, ga, gb});
+  return p;
+}
+
 }  // namespace ljgb

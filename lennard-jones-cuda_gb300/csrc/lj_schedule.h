@@ -55,4 +55,17 @@ struct RdfRanges {
 };
 bool build_rdf_ranges(int n, int ctas, RdfRanges* out);
 
+// Squares and tasks of the FP64 pair pass for boxes of sizes n (Pair64Task).
+// The square side grows while there are still about 80 tasks an SM: a tile
+// then has at most ~256 slots, so the sums stay at 10 KB a particle whatever
+// N is.  With fewer than 8 tasks an SM the turns of a task are shared by 2, 4
+// or 8 warps: N = 512 gives 136 tasks for 152 SMs.
+struct Pair64Plan {
+  int group = 1, parts = 1;
+  long long slots = 0;
+  std::vector<Pair64Task> tasks;
+  std::vector<Pair64Box> boxes;
+};
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms);
+
 }  // namespace ljgb

@@ -441,52 +441,6 @@ lj_status upload_boxes(lj_system* s) {
 // filled beside the old ones and swapped in only once complete, so a
 // failure (an allocation, say) leaves the handle on its previous schedule,
 // with shape and split cap put back to the ones that schedule was built for.
-// Squares and tasks of the FP64 pair pass for boxes of sizes n (Pair64Args).
-// The square side grows while there are still about 80 tasks an SM: a tile
-// then has at most ~256 slots, so the sums stay at 10 KB a particle whatever
-// N is.  With fewer than 8 tasks an SM the turns of a task are shared by 2, 4
-// or 8 warps: N = 512 gives 136 tasks for 152 SMs.
-struct Pair64Plan {
-  int group = 1, parts = 1;
-  long long slots = 0;
-  std::vector<Pair64Task> tasks;
-  std::vector<Pair64Box> boxes;
-};
-
-Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
-  Pair64Plan p;
-  auto squares = [&](long long group) {
-    long long t = 0;
-    for (int k : n) {
-      const long long g = ((k + 31) / 32 + group - 1) / group;
-      t += g * (g + 1) / 2;
-    }
-    return t;
-  };
-  while (squares(2ll * p.group) >= 80ll * sms) p.group *= 2;
-  if (p.group == 1)
-    while (p.parts < 8 && squares(1) * p.parts < 8ll * sms) p.parts *= 2;
-  int p0 = 0;
-  for (int k : n) {
-    Pair64Box b{};
-    b.p0 = p0;
-    b.n = k;
-    b.tiles = (k + 31) / 32;
-    b.groups = (b.tiles + p.group - 1) / p.group;
-    b.tile0_slot = p.slots;
-    p.slots += (long long)b.tiles * (b.groups + 1);
-    p.boxes.push_back(b);
-    p0 += k;
-  }
-  // the squares on a box's diagonal hold half the pairs: they come last
-  for (int diag = 0; diag < 2; ++diag)
-    for (int k = 0; k < (int)n.size(); ++k)
-      for (int ga = 0; ga < p.boxes[k].groups; ++ga)
-        for (int gb = diag ? ga : ga + 1; gb < (diag ? ga + 1 : p.boxes[k].groups); ++gb)
-          p.tasks.push_back(Pair64Task{k, ga, gb});
-  return p;
-}
-
 lj_status build_and_swap_schedule(lj_system* s) {
   const bool fp64 = s->prec == LJ_PREC_FP64;
   // FP64: i-blocks of one tile; its pair pass has tasks of its own, so the
