@@ -452,15 +452,18 @@ __global__ void k_tvn_close(StateArgs s) {
   block_sum<3>(part, sh);
   if (tid == 0) {
     // halving the block sums gives the bits of summing halved terms
-    s.blk_part[(size_t)B * 8 + 0] = 0.5 * part[0];
-    s.blk_part[(size_t)B * 8 + 1] = 0.5 * part[1];
-    s.blk_part[(size_t)B * 8 + 2] = part[2];
+    // (slots by parity: the next step may be an EVN one, whose epilogues write
+    // theirs while these are summed)
+    s.blk_part[(size_t)B * 8 + s.obs_slot + 0] = 0.5 * part[0];
+    s.blk_part[(size_t)B * 8 + s.obs_slot + 1] = 0.5 * part[1];
+    s.blk_part[(size_t)B * 8 + s.obs_slot + 2] = part[2];
     if (B == s.sys_block_first[bi.sys]) {
       const int par = s.ticket - 2;  // this step's parity
       sc.Tkin = tkin_sh;
       sc.Tkin_rec[par] = tkin_sh;
       sc.chi = chi;
-      sc.obs_slot[par] = 0;
+      sc.obs_slot[par] = s.obs_slot;
+      sc.obs_nblk[par] = 0;
       sc.obs_pending[par] = MODE_TVN;
     }
   }

@@ -78,8 +78,11 @@ struct DevScalars {
   // for its record.  A step marks its own parity's entry and the next step's
   // pair kernel consumes it, so the two never touch the same entry at once.
   double Tkin_rec[2];
+  // obs_nblk[p] > 0: the partials are those of the row step, one set per CTA
+  // (row_part); 0: one per i-block (blk_part).
   int obs_pending[2];
   int obs_slot[2];
+  int obs_nblk[2];
 };
 
 // Observable record layout written by the device (matches lj_observables).

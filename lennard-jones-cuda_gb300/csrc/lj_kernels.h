@@ -98,6 +98,7 @@ struct StateArgs {
   int nblocks;                 // i-blocks of all boxes
   int nsys;                    // boxes
   int obs_slot;                // fused EVN: first block-partial slot of this step's K, V, W (0 or 4, by parity)
+  double* row_part;            // row step (lj_rows.cu): 8 partial sums per CTA, in place of blk_part
   int ticket;                  // fused: glob_cnt index of this step's pending-observables tickets (2 or 3)
 };
 
@@ -109,6 +110,16 @@ struct FusedPairArgs {
   PairArgs pair;
   StateArgs st;
 };
+
+// Row step of one box (lj_rows.cu): ctas = 0 where the box is too large for it.
+struct RowPlan {
+  int rows, ctas, close_ctas;
+  size_t smem;
+};
+RowPlan plan_rows(int n, int sms);
+cudaError_t rows_setup();
+cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, cudaStream_t st);
+cudaError_t launch_rows_close(const StateArgs& s, const RowPlan& p, int n, cudaStream_t st);
 
 // Arguments of the FP64 pair pass (lj_pairs64.cu; Pair64Plan).
 struct Pair64Args {

@@ -88,6 +88,18 @@ __device__ __forceinline__ int4 shadow_of_bc(const DevScalars& sc, int bc, doubl
                    fixed_coord_scaled(z - sc.origin[2], scale), 0);
 }
 
+// check_wall_frame and shadow_of_bc for component c of particle p alone.
+__device__ __forceinline__ void predict_coord(const StateArgs& s, const DevScalars& sc, const BoxArgs& box, int c,
+                                              int p, double x) {
+  const double o = box.bc == 0 ? 0.0 : sc.origin[c];
+  if (box.bc == 1) {
+    const double u = (x - o) * sc.invP;
+    if (!(u >= 0.0 && u < 0.4999)) atomicOr(s.status, LJ_DEVFLAG_ESCAPED);
+  }
+  const double scale = sc.invP * 4294967296.0;
+  reinterpret_cast<int*>(s.q_next + p)[c] = fixed_coord_scaled(box.bc == 0 ? x : x - o, scale);
+}
+
 // Sum of blk_part[b][slot] over the blocks of one box, fixed order, valid in
 // thread 0 (every CTA that calls this obtains the same bits).
 __device__ __forceinline__ double box_sum(const StateArgs& s, int b0, int b1, int slot, double* sh) {
@@ -97,13 +109,14 @@ __device__ __forceinline__ double box_sum(const StateArgs& s, int b0, int b1, in
   return acc[0];
 }
 
-// Sums of blk_part[b][0..2] (K, V, W) over the blocks of one box in one
-// block reduction (fixed order); valid in thread 0.  sh: 3 x 32 doubles.
-__device__ __forceinline__ void box_sum3(const StateArgs& s, int b0, int b1, double* sh, double (&out)[3],
+// Sums of part[b][0..2] (K, V, W; 8 values per block) over the blocks of one
+// box in one block reduction (fixed order); valid in thread 0.  sh: 3 x 32
+// doubles.
+__device__ __forceinline__ void box_sum3(const double* part, int b0, int b1, double* sh, double (&out)[3],
                                          int slot = 0) {
   double acc[3] = {0.0, 0.0, 0.0};
   for (int b = b0 + (int)threadIdx.x; b < b1; b += blockDim.x) {
-    const double* bp = s.blk_part + (size_t)b * 8 + slot;
+    const double* bp = part + (size_t)b * 8 + slot;
     acc[0] += __ldcg(bp);
     acc[1] += __ldcg(bp + 1);
     acc[2] += __ldcg(bp + 2);
@@ -171,8 +184,25 @@ __device__ __forceinline__ void observables_box(const StateArgs& s, int sys, dou
   const BoxArgs box = s.boxes[sys];
   const int b0 = s.sys_block_first[sys], b1 = s.sys_block_first[sys + 1];
   double kvw[3];
-  box_sum3(s, b0, b1, sh, kvw, slot);
+  box_sum3(s.blk_part, b0, b1, sh, kvw, slot);
   if (threadIdx.x == 0) write_observables<MODE>(s, sys, box, kvw[0], kvw[1], kvw[2], rec_parity);
+}
+
+// The same for the row step's partials (a few hundred at most), by the first
+// warp: no barrier and no serial sum over warps.
+__device__ __forceinline__ void row_observables(const StateArgs& s, int sys, int mode, int nblk, int slot,
+                                                int parity) {
+  if (threadIdx.x >= 32) return;
+  double kvw[3] = {0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblk; b += 32)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) kvw[k] += __ldcg(s.row_part + (size_t)b * 8 + slot + k);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) kvw[k] = warp_sum(kvw[k]);
+  if (threadIdx.x != 0) return;
+  const BoxArgs box = s.boxes[sys];
+  if (mode == MODE_TVN) write_observables<MODE_TVN>(s, sys, box, kvw[0], kvw[1], kvw[2], parity);
+  else write_observables<MODE_EVN>(s, sys, box, kvw[0], kvw[1], kvw[2], -1);
 }
 
 // Observables of the boxes whose fused step of parity `parity` left them
@@ -181,14 +211,16 @@ __device__ __forceinline__ void observables_box(const StateArgs& s, int sys, dou
 // takes boxes k, k + tickets, ...  Block-wide call.
 __device__ __forceinline__ void pending_observables_parity(const StateArgs& s, int parity, int ticket, int tickets,
                                                            double* sh) {
-  __shared__ int pend, slot;
+  __shared__ int pend, slot, nblk;
   for (int sys = ticket; sys < s.nsys; sys += tickets) {
     if (threadIdx.x == 0) {
       pend = s.sc[sys].obs_pending[parity];
       slot = s.sc[sys].obs_slot[parity];
+      nblk = s.sc[sys].obs_nblk[parity];
     }
     __syncthreads();
-    if (pend == MODE_TVN) observables_box<MODE_TVN>(s, sys, sh, slot, parity);
+    if (pend && nblk) row_observables(s, sys, pend, nblk, slot, parity);
+    else if (pend == MODE_TVN) observables_box<MODE_TVN>(s, sys, sh, slot, parity);
     else if (pend == MODE_EVN) observables_box<MODE_EVN>(s, sys, sh, slot);
     if (pend && threadIdx.x == 0) s.sc[sys].obs_pending[parity] = 0;
     __syncthreads();

@@ -242,6 +242,10 @@ struct lj_system {
   DevBuf<DevScalars> sc;
   DevBuf<BoxArgs> dboxes;
   DevBuf<double> blk_part;
+  // row step of a single box (lj_rows.cu); rows.ctas = 0: not for this box
+  RowPlan rows{};
+  bool rows_off = false;  // the autotuner found a stream-K shape faster, or is timing one
+  DevBuf<double> row_part;
   DevBuf<float> partial;  // MIXED: nseg x 5 x BI
   // FP64 pair pass: tasks, boxes and sums (Pair64Args)
   int p64_group = 1, p64_parts = 1;
@@ -335,6 +339,7 @@ StateArgs state_args(lj_system* s) {
   a.sc = s->sc.p;
   a.sys_block_first = s->sys_block_first.p;
   a.blk_part = s->blk_part.p;
+  a.row_part = s->row_part.p;
   a.partial = s->partial.p;
   a.prec = s->prec;
   a.bi_threads = s->BI;
@@ -673,6 +678,24 @@ lj_status enqueue_step(lj_system* s, int mode, cudaEvent_t* ev, bool capture, in
 // shadow frame (periodic or walled boxes, not open ones) and the MIXED kernel.
 bool use_fused(const lj_system* s) { return s->prec == LJ_PREC_MIXED && !s->any_open; }
 
+// The row step takes the fused steps of a box it is built for, unless a
+// stream-K shape or split cap was chosen.
+bool use_rows(const lj_system* s) {
+  return use_fused(s) && s->rows.ctas > 0 && !s->rows_off && s->forced_shape < 0 && s->forced_split == 0;
+}
+
+lj_status enqueue_rows(lj_system* s, int mode, cudaEvent_t pair_end, unsigned flags, int* kernels) {
+  const StateArgs a = state_args(s);
+  LJ_CUDA(s, launch_rows(a, s->rows, s->cfg[0].n, mode, s->stream));
+  *kernels += 1;
+  if (pair_end) LJ_CUDA(s, cudaEventRecordWithFlags(pair_end, s->stream, flags));
+  if (mode == MODE_TVN) {
+    LJ_CUDA(s, launch_rows_close(a, s->rows, s->cfg[0].n, s->stream));
+    *kernels += 1;
+  }
+  return LJ_OK;
+}
+
 lj_status enqueue_step_fused(lj_system* s, int mode, cudaEvent_t* ev, bool capture, int* kernels) {
   StateArgs a = state_args(s);
   const int nb = nblocks(s);
@@ -680,15 +703,20 @@ lj_status enqueue_step_fused(lj_system* s, int mode, cudaEvent_t* ev, bool captu
   int k = 0;
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[0], s->stream, flags));
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[1], s->stream, flags));
-  FusedPairArgs f{};
-  f.pair = pair_args(s);
-  f.st = a;
-  LJ_CUDA(s, launch_pairs_fused(s->shape, mode, f, s->sched.G, s->stream));
-  ++k;
-  if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[2], s->stream, flags));
-  if (mode == MODE_TVN) {
-    LJ_CUDA(s, launch_tvn_close(a, nb, s->BI, s->stream));
+  if (use_rows(s)) {
+    lj_status st = enqueue_rows(s, mode, ev ? ev[2] : nullptr, flags, &k);
+    if (st) return st;
+  } else {
+    FusedPairArgs f{};
+    f.pair = pair_args(s);
+    f.st = a;
+    LJ_CUDA(s, launch_pairs_fused(s->shape, mode, f, s->sched.G, s->stream));
     ++k;
+    if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[2], s->stream, flags));
+    if (mode == MODE_TVN) {
+      LJ_CUDA(s, launch_tvn_close(a, nb, s->BI, s->stream));
+      ++k;
+    }
   }
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[3], s->stream, flags));
   if (kernels) *kernels = k;
@@ -708,7 +736,7 @@ lj_status enqueue_after_step(lj_system* s, const RdfPass& rdf, int* kernels);
 lj_status get_graph(lj_system* s, int mode, GraphEntry** out) {
   const bool fused = use_fused(s);
   const bool counters = s->counter_cap > 0, rdf = s->rdf_acc;
-  const int key = mode * 128 + (rdf ? 64 : 0) + (counters ? 32 : 0) + (fused ? 8 : 0) + (fused && s->qpar ? 4 : 0) +
+  const int key = mode * 256 + (fused && use_rows(s) ? 128 : 0) + (rdf ? 64 : 0) + (counters ? 32 : 0) + (fused ? 8 : 0) + (fused && s->qpar ? 4 : 0) +
                   (s->any_nonperiodic ? 2 : 0) + (s->profiling ? 1 : 0);
   auto it = s->graphs.find(key);
   if (it != s->graphs.end()) {
@@ -909,6 +937,7 @@ lj_status alloc_state(lj_system* s) {
   LJ_CUDA(s, s->sc.alloc(s->nsys));
   LJ_CUDA(s, s->dboxes.alloc(s->nsys));
   LJ_CUDA(s, s->status.alloc(1));
+  if (s->rows.ctas > 0) LJ_CUDA(s, s->row_part.alloc(8 * (size_t)std::max(s->rows.ctas, s->rows.close_ctas)));
   LJ_CUDA(s, s->hist.alloc(kMaxHistBins));
   LJ_CUDA(s, cudaMemsetAsync(s->x.p, 0, sizeof(double) * n3, s->stream));
   LJ_CUDA(s, cudaMemsetAsync(s->v.p, 0, sizeof(double) * n3, s->stream));
@@ -1043,6 +1072,9 @@ lj_status create_impl(const lj_config* cfgs, int nsys, lj_system** out) {
   if (cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(s, LJ_ERR_CUDA, "cudaStreamCreate failed"));
   s->stream = s->own_stream;
+  if (nsys == 1 && s->prec == LJ_PREC_MIXED) s->rows = plan_rows(s->cfg[0].n, s->num_sms);
+  if (s->rows.ctas > 0 && rows_setup() != cudaSuccess)
+    return bail(fail(s, LJ_ERR_CUDA, "cudaFuncSetAttribute failed"));
   lj_status st = alloc_state(s);
   if (st) return bail(st);
   st = upload_boxes(s);
@@ -1163,6 +1195,7 @@ lj_status lj_destroy(lj_system* s) {
   s->sc.free();
   s->dboxes.free();
   s->blk_part.free();
+  s->row_part.free();
   s->partial.free();
   s->p64_tasks.free();
   s->p64_boxes.free();
@@ -1436,7 +1469,20 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
     s->pred_ready = true;
     s->pred_dt = dt;
   }
+  // The row step's launches go to the stream directly: each is a programmatic
+  // dependent of the one before, across steps too, which graphs of one step
+  // would not be.
+  const bool direct = fused && use_rows(s) && !s->profiling && s->counter_cap == 0 && !s->rdf_acc;
   for (int k = 0; k < nsteps; ++k) {
+    if (direct) {
+      int kernels = 0;
+      lj_status st = enqueue_rows(s, mode, nullptr, 0, &kernels);
+      if (st) return st;
+      s->launches += kernels;
+      s->qpar ^= 1;
+      s->obs_maybe_pending = true;
+      continue;
+    }
     GraphEntry* ge = nullptr;
     lj_status st = get_graph(s, mode, &ge);
     if (st) return st;
@@ -1936,6 +1982,7 @@ lj_status lj_set_kernel_shape(lj_system* s, int32_t shape) {
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_shape;
   s->forced_shape = shape;
+  s->rows_off = false;
   s->shape = shape < 0 ? 0 : shape;
   lj_status st = setup_schedule(s);
   if (st) {
@@ -1953,6 +2000,7 @@ lj_status lj_set_split_cap(lj_system* s, int32_t cap) {
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_split;
   s->forced_split = cap;
+  s->rows_off = false;
   s->split_cap = cap > 0 ? cap : kMaxSegmentsPerBlock;
   lj_status st = setup_schedule(s);
   if (st) {
@@ -2032,8 +2080,12 @@ lj_status lj_autotune(lj_system* s) {
   // handle goes back to its own shape and split cap where it can, and to the
   // snapshotted state, before the error is returned.
   const int orig_shape = s->shape, orig_split = s->split_cap;
+  const bool orig_rows_off = s->rows_off;
+  const int orig_forced = s->forced_shape;
   auto give_up = [&](lj_status err) -> lj_status {
     const std::string msg = s->err;
+    s->rows_off = orig_rows_off;
+    s->forced_shape = orig_forced;
     s->profiling = was_profiling;
     s->shape = orig_shape;
     s->split_cap = orig_split;
@@ -2061,6 +2113,40 @@ lj_status lj_autotune(lj_system* s) {
   // only matters while it keeps the grid below SMs x resident CTAs; larger
   // caps give the same schedule and are skipped.
   static const int kSplitCaps[] = {1, 2, 4, 8, 16, 32};
+  // One trial of the step as it is set up now: ms per step.
+  auto trial = [&](float* out) -> lj_status {
+    if ((st = restore())) return st;
+    if ((st = enqueue_compute_forces(s))) return st;
+    // two warm-up steps (timed, to size the rounds), then the fastest of
+    // three rounds of about 1 ms each (2..10 steps): neighbouring shapes
+    // differ by ~1%, about the spread of a single short round
+    LJ_CUDA(s, cudaEventRecord(e0, s->stream));
+    if ((st = lj_step(s, dt, 2))) return st;
+    LJ_CUDA(s, cudaEventRecord(e1, s->stream));
+    LJ_CUDA(s, cudaEventSynchronize(e1));
+    float warm_ms = 0;
+    LJ_CUDA(s, cudaEventElapsedTime(&warm_ms, e0, e1));
+    const int reps = std::max(2, std::min(10, (int)(1.0f / std::max(warm_ms * 0.5f, 1e-3f))));
+    float ms = 1e30f;
+    for (int round = 0; round < 3; ++round) {
+      LJ_CUDA(s, cudaEventRecord(e0, s->stream));
+      if ((st = lj_step(s, dt, reps))) return st;
+      LJ_CUDA(s, cudaEventRecord(e1, s->stream));
+      LJ_CUDA(s, cudaEventSynchronize(e1));
+      float r_ms = 0;
+      LJ_CUDA(s, cudaEventElapsedTime(&r_ms, e0, e1));
+      ms = std::min(ms, r_ms / reps);
+    }
+    if ((st = check_status(s))) return st;
+    *out = ms;
+    return LJ_OK;
+  };
+  // The row step, where this box has it, competes with the best stream-K shape.
+  float rows_ms = 1e30f;
+  s->rows_off = false;
+  s->forced_shape = -1;  // a block hint gives way to the measurement
+  if (use_rows(s) && (st = trial(&rows_ms))) return give_up(st);
+  s->rows_off = true;
   int best = 0, best_split = s->split_cap;
   float best_ms = 1e30f;
   for (int k = 0; k < kNumShapes; ++k) {
@@ -2072,29 +2158,8 @@ lj_status lj_autotune(lj_system* s) {
       if ((st = setup_schedule(s))) return give_up(st);
       if (s->sched.G == prev_G) break;
       prev_G = s->sched.G;
-      if ((st = restore())) return give_up(st);
-      if ((st = enqueue_compute_forces(s))) return give_up(st);
-      // two warm-up steps (timed, to size the rounds), then the fastest of
-      // three rounds of about 1 ms each (2..10 steps): neighbouring shapes
-      // differ by ~1%, about the spread of a single short round
-      LJ_CUDA(s, cudaEventRecord(e0, s->stream));
-      if ((st = lj_step(s, dt, 2))) return give_up(st);
-      LJ_CUDA(s, cudaEventRecord(e1, s->stream));
-      LJ_CUDA(s, cudaEventSynchronize(e1));
-      float warm_ms = 0;
-      LJ_CUDA(s, cudaEventElapsedTime(&warm_ms, e0, e1));
-      const int reps = std::max(2, std::min(10, (int)(1.0f / std::max(warm_ms * 0.5f, 1e-3f))));
-      float ms = 1e30f;
-      for (int round = 0; round < 3; ++round) {
-        LJ_CUDA(s, cudaEventRecord(e0, s->stream));
-        if ((st = lj_step(s, dt, reps))) return give_up(st);
-        LJ_CUDA(s, cudaEventRecord(e1, s->stream));
-        LJ_CUDA(s, cudaEventSynchronize(e1));
-        float r_ms = 0;
-        LJ_CUDA(s, cudaEventElapsedTime(&r_ms, e0, e1));
-        ms = std::min(ms, r_ms / reps);
-      }
-      if ((st = check_status(s))) return give_up(st);
+      float ms = 0;
+      if ((st = trial(&ms))) return give_up(st);
       if (ms < best_ms) {
         best_ms = ms;
         best = k;
@@ -2102,6 +2167,7 @@ lj_status lj_autotune(lj_system* s) {
       }
     }
   }
+  s->rows_off = rows_ms > best_ms;
   s->shape = best;
   s->split_cap = best_split;
   s->profiling = was_profiling;

@@ -23,6 +23,7 @@ LIB_PATH = os.path.join(PKG_DIR, "liblj_gb300.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = [
     "lj_pairs.cu",
+    "lj_rows.cu",
     "lj_rdf.cu",
     "lj_pairs64.cu",
     "lj_integrate.cu",
