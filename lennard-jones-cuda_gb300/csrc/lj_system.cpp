@@ -1454,7 +1454,9 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
       changed = true;
     }
   if (changed) {
-    lj_status st = upload_boxes(s);
+    // pending observables advance the clock by the dt of their own step
+    lj_status st = flush_observables(s);
+    if (!st) st = upload_boxes(s);
     if (st) return st;
   }
   const int mode = step_mode(s);

@@ -78,3 +78,15 @@ def test_row_step_observables_by_route(ljgb_mod, canonical):
     for k in ("U", "K", "P", "av_U_tot", "t", "step", "av_iters"):
         assert o[k] == pytest.approx(runs[0][1][k], rel=1e-6), k
     s.close()
+
+
+@pytest.mark.parametrize("shape", [-1, 0])
+def test_change_of_time_step_keeps_the_clock(ljgb_mod, shape):
+    """The last step before a change of dt advances the clock by its own dt,
+    although its observables are formed after the change."""
+    s = ljgb_mod.System(n=700, density=0.7, temperature=1.0)
+    s.set_kernel_shape(shape)
+    s.integrate(0.004, 3)
+    s.integrate(0.002, 2)
+    assert s.observables()["t"] == pytest.approx(0.016, rel=1e-12)
+    s.close()
