@@ -121,6 +121,11 @@ cudaError_t rows_setup();
 cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, cudaStream_t st);
 cudaError_t launch_rows_close(const StateArgs& s, const RowPlan& p, int n, cudaStream_t st);
 
+// Steps of one small box in one launch (lj_cluster.cu).
+constexpr int kClusterMaxN = 512;
+cudaError_t cluster_setup(bool* usable);
+cudaError_t launch_cluster(const StateArgs& s, int n, int mode, int nsteps, cudaStream_t st);
+
 // Arguments of the FP64 pair pass (lj_pairs64.cu; Pair64Plan).
 struct Pair64Args {
   const double4_32a* xd;  // position shadow (x, y, z, 0)

@@ -246,6 +246,7 @@ struct lj_system {
   RowPlan rows{};
   bool rows_off = false;  // the autotuner found a stream-K shape faster, or is timing one
   DevBuf<double> row_part;
+  bool cluster_ok = false;  // the box may step in one cluster (lj_cluster.cu)
   DevBuf<float> partial;  // MIXED: nseg x 5 x BI
   // FP64 pair pass: tasks, boxes and sums (Pair64Args)
   int p64_group = 1, p64_parts = 1;
@@ -1075,6 +1076,8 @@ lj_status create_impl(const lj_config* cfgs, int nsys, lj_system** out) {
   if (nsys == 1 && s->prec == LJ_PREC_MIXED) s->rows = plan_rows(s->cfg[0].n, s->num_sms);
   if (s->rows.ctas > 0 && rows_setup() != cudaSuccess)
     return bail(fail(s, LJ_ERR_CUDA, "cudaFuncSetAttribute failed"));
+  if (s->rows.ctas > 0 && s->cfg[0].n <= kClusterMaxN && cluster_setup(&s->cluster_ok) != cudaSuccess)
+    return bail(fail(s, LJ_ERR_CUDA, "cluster set-up failed"));
   lj_status st = alloc_state(s);
   if (st) return bail(st);
   st = upload_boxes(s);
@@ -1474,7 +1477,24 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
   // The row step's launches go to the stream directly: each is a programmatic
   // dependent of the one before, across steps too, which graphs of one step
   // would not be.
-  const bool direct = fused && use_rows(s) && !s->profiling && s->counter_cap == 0 && !s->rdf_acc;
+  // (A stream being captured keeps the graphs' route: single launches would be
+  // recorded with this call's step parity.)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+  const bool plain = !s->profiling && s->counter_cap == 0 && !s->rdf_acc && capture == cudaStreamCaptureStatusNone;
+  if (fused && use_rows(s) && s->cluster_ok && plain) {
+    // Small boxes: all steps in one launch (at most kClusterSteps, ~10 ms, so
+    // that the stream gets its turn).
+    constexpr int kClusterSteps = 4096;
+    lj_status st = flush_observables(s);
+    if (st) return st;
+    for (int done = 0; done < nsteps; done += kClusterSteps) {
+      LJ_CUDA(s, launch_cluster(state_args(s), s->cfg[0].n, mode, std::min(kClusterSteps, nsteps - done), s->stream));
+      s->launches += 1;
+    }
+    return LJ_OK;
+  }
+  const bool direct = fused && use_rows(s) && plain;
   for (int k = 0; k < nsteps; ++k) {
     if (direct) {
       int kernels = 0;
