@@ -143,4 +143,12 @@ struct Pair64Box {
   long long tile0_slot;  // slot of the box's tile 0
 };
 
+// Task of a warp of the unordered-pair kernel (lj_newton.cu): `count` tiles of
+// 32 j's, from tile `tile` of i-block `block` (256 i's) on.  Block I meets the
+// tiles from its own first one (8 I) to the box's last, then block I + 1.
+constexpr int kNewtonBlock = 256;
+struct NewtonTask {
+  int block, tile, count;
+};
+
 }  // namespace ljgb

@@ -111,15 +111,35 @@ struct FusedPairArgs {
   StateArgs st;
 };
 
-// Row step of one box (lj_rows.cu): ctas = 0 where the box is too large for it.
+// Step of one box of kNewtonMinN particles or more over unordered pairs
+// (lj_newton.cu; NewtonPlan).  The line lies where it overtakes the row step:
+// us a step, rows / unordered pairs, N = 6000 31 / 36, N = 8000 48.9 / 48.7,
+// N = 9000 64 / 59, N = 14 000 139 / 111.
+constexpr int kNewtonMinN = 8192;
+struct NewtonArgs {
+  const int4* q;
+  const DevScalars* sc;
+  const NewtonTask* tasks;
+  const int* block_part;  // per block of 256: first part of its i sums, count
+  float* jpart;           // per tile t (block b = t / 8) b + 1 parts of 5 x 32, tile-major
+  float* ipart;           // part (task + block): 5 x 256
+  int n, ntasks;
+};
+cudaError_t newton_setup(int* ctas_per_sm);
+constexpr int kNewtonWarps = 4;  // tasks of a CTA
+cudaError_t launch_newton(const NewtonArgs& a, cudaStream_t st);
+cudaError_t launch_newton_sum(const StateArgs& s, const NewtonArgs& a, int mode, cudaStream_t st);
+
+// Row step of one smaller box (lj_rows.cu): ctas = 0 where it does not apply.
 struct RowPlan {
-  int rows, ctas, close_ctas;
+  int rows, ctas;
   size_t smem;
 };
 RowPlan plan_rows(int n, int sms);
 cudaError_t rows_setup();
 cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, cudaStream_t st);
-cudaError_t launch_rows_close(const StateArgs& s, const RowPlan& p, int n, cudaStream_t st);
+// parts: CTAs (row step) or tiles whose sums of tv^2 make chi
+cudaError_t launch_rows_close(const StateArgs& s, int n, int parts, cudaStream_t st);
 
 // Steps of one small box in one launch (lj_cluster.cu).
 constexpr int kClusterMaxN = 512;

@@ -1,4 +1,4 @@
-// lj_rows.cu -- the MIXED step of one box of up to about 14 000 particles,
+// lj_rows.cu -- the MIXED step of one box of fewer than 8192 particles,
 // a CTA per SM, each owning its rows (i's) outright.
 //
 // The stream-K kernel (lj_pairs.cu) cuts every i-block's j range over several
@@ -26,23 +26,8 @@ namespace {
 
 constexpr int kRowWarps = 16;    // 12 to 20 warps measure alike (N = 400 to 8000)
 constexpr int kRowThreads = 32 * kRowWarps;
-// The j records are staged whole (192 KB) up to kRowWhole of them, so that a
-// warp's share of the work is one or two long runs; larger boxes in tiles of
-// at most kRowTile, two in flight.
-constexpr int kRowWhole = 12288;
-constexpr int kRowTile = 6144;
-constexpr int kRowStages = 2;
-__host__ __device__ constexpr int row_tile(int n) {
-  const int k = (n + kRowTile - 1) / kRowTile;
-  return n <= kRowWhole ? n : ((n + k - 1) / k + 31) / 32 * 32;
-}
 constexpr int kRowFold = 32;     // j's a lane sums in plain FP32 before the compensated sum takes them
-// Rows of a CTA: 4 threads each in the second half, and the largest boxes this
-// kernel is the faster one for (14 496 particles on 152 SMs): us a step, here
-// and with the best stream-K shape, N = 8000 52 / 70, 11 000 87 / 104, 14 000
-// 139 / 148, 15 000 163 / 160, 16 384 192 / 185.  There the tail that this
-// kernel does not have is a smaller share, and its tiles' portions shorter.
-constexpr int kMaxRows = 96;
+constexpr int kMaxRows = 64;     // rows of a CTA: 4 threads each in the second half
 
 __device__ __forceinline__ int4 load_slots(const int4* rec) {
   int4 r;  // volatile: kept a 128-bit load into an aligned register quadruple
@@ -52,17 +37,17 @@ __device__ __forceinline__ int4 load_slots(const int4* rec) {
   return r;
 }
 
-// Pairs of two rows with chunks c0 .. c1-1 (32 j's each, one a lane) of a
-// tile of cnt records; the lanes' sums added up into out[row * 5 + value].
-// self: the first row's own place in the tile (even).
-__device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, int cnt, int c0, int c1, int self,
+// Pairs of two rows with chunks c0 .. c1-1 (32 j's each, one a lane) of the n
+// records st; the lanes' sums added up into out[row * 5 + value].  self: the
+// first row's index (even).
+__device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, int n, int c0, int c1, int self,
                                             f32x2 k2i2, float* out) {
   const int lane = threadIdx.x & 31;
   const int4 qa = load_slots(rowq), qb = load_slots(rowq + 1);
   Float2Acc acc[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) acc[k] = Float2Acc{0ull, 0ull};
-  const int ragged = (cnt & 31) ? cnt >> 5 : -1;  // chunk that ends before its 32nd record
+  const int ragged = (n & 31) ? n >> 5 : -1;  // chunk that ends before its 32nd record
   const int cself = self >> 5;                    // chunk that holds the rows themselves
   for (int c = c0; c < c1;) {
     const int special = cself >= c && cself < c1 ? cself : (ragged >= c && ragged < c1 ? ragged : c1);
@@ -74,7 +59,7 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
         pair_mixed_rows<false>(qa, qb, st[c * 32 + lane], k2i2, false, false, f[0], f[1], f[2], f[3], f[4]);
     } else {
       const int j = c * 32 + lane;
-      const bool out_of = j >= cnt;
+      const bool out_of = j >= n;
       pair_mixed_rows<true>(qa, qb, st[out_of ? 0 : j], k2i2, out_of || j == self, out_of || j == self + 1, f[0], f[1],
                             f[2], f[3], f[4]);
       ++c;
@@ -109,10 +94,10 @@ __device__ __forceinline__ int warp_of_unit(int u, int U) { return ((u + 1) * kR
 // CTA computes the observables the previous step left pending.  MODE_EVN: the
 // whole step; MODE_TVN: up to sum tv^2 (k_rows_close follows).
 //
-// A tile's work is groups x chunks units (two rows x 32 j's) in one sequence,
-// cut evenly over the warps; the portion of group g by warp w has slot w + g
-// of the tile (the sequence visits (w, g) monotonically, so no two portions
-// share a slot), and the second half adds a row's slots in a fixed order.
+// The work is groups x chunks units (two rows x 32 j's) in one sequence, cut
+// evenly over the warps; the portion of group g by warp w has slot w + g (the
+// sequence visits (w, g) monotonically, so no two portions share a slot), and
+// the second half adds a row's slots in a fixed order.
 //
 // Bound: from N ~ 8000 the pair loop's issue and register reads as in
 // lj_pairs.cu; below ~2000 the fixed parts (launch, first copy, reductions, a
@@ -122,15 +107,13 @@ __device__ __forceinline__ int warp_of_unit(int u, int U) { return ((u + 1) * kR
 template <int MODE>
 __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int rows, int ctas) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint64_t bars[kRowStages];
-  __shared__ int done[kRowStages];
+  __shared__ uint64_t bar;
   __shared__ volatile int sfail;
   __shared__ int4 srow[kMaxRows];
-  __shared__ double red[5][4];
+  __shared__ double red[5][2];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int tile = row_tile(n), ntile = (n + tile - 1) / tile;
-  int4* const sq = reinterpret_cast<int4*>(smem_raw);
-  float* const part = reinterpret_cast<float*>(smem_raw + sizeof(int4) * (size_t)min(ntile, kRowStages) * tile);
+  int4* const sq = reinterpret_cast<int4*>(smem_raw);              // all n records
+  float* const part = reinterpret_cast<float*>(smem_raw + sizeof(int4) * (size_t)n);
 
   if ((int)blockIdx.x == ctas) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -141,14 +124,11 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   const int i0 = blockIdx.x * rows, nr = min(rows, n - i0), groups = (nr + 1) / 2;
   const int slots = kRowWarps + groups;
   if (tid == 0) {
-    for (int k = 0; k < kRowStages; ++k) {
-      mbar_init(&bars[k], 1);
-      done[k] = 0;
-    }
+    mbar_init(&bar, 1);
     sfail = 0;
     fence_mbar_init();
   }
-  for (int k = tid; k < ntile * slots * 10; k += kRowThreads) part[k] = 0.0f;
+  for (int k = tid; k < slots * 10; k += kRowThreads) part[k] = 0.0f;
   const BoxArgs box = s.boxes[0];
   __syncthreads();
   // What the previous step's kernels write is read from here on.
@@ -158,13 +138,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   // the few SMs left free and take turns at their FP64 pipes (N = 2001: the
   // close added 8.1 us to the step, and 4 us so).
   if (MODE == MODE_EVN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  auto fetch = [&](int t) {
-    const uint32_t bytes = (uint32_t)min(tile, n - t * tile) * 16u;
-    mbar_arrive_expect_tx(&bars[t % kRowStages], bytes);
-    bulk_g2s(sq + (size_t)(t % kRowStages) * tile, s.q + (size_t)t * tile, bytes, &bars[t % kRowStages]);
-  };
-  if (tid == 0)
-    for (int t = 0; t < min(ntile, kRowStages); ++t) fetch(t);
+  if (tid == 0) {
+    mbar_arrive_expect_tx(&bar, (uint32_t)n * 16u);
+    bulk_g2s(sq, s.q, (uint32_t)n * 16u, &bar);
+  }
   if (tid < 2 * groups) {
     const int4 q = s.q[min(i0 + tid, n - 1)];
     srow[tid] = make_int4(0, q.x, q.y, q.z);
@@ -191,57 +168,34 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   }
   __syncthreads();
 
-  const f32x2 k2i2 = pk2(k2inv, k2inv);
-  bool failed = false;
-  for (int t = 0; t < ntile; ++t) {
-    const int stage = t % kRowStages;
-    if (!failed) {
-      const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bars[stage], (uint32_t)((t / kRowStages) & 1)));
-      failed = !ok || sfail;
-      if (!ok && lane == 0) sfail = 1;
+  const int C = (n + 31) / 32, U = groups * C;
+  if (__all_sync(0xffffffffu, mbar_wait_bounded(&bar, 0))) {
+    const f32x2 k2i2 = pk2(k2inv, k2inv);
+    const int hi = (w + 1) * U / kRowWarps;
+    for (int u = w * U / kRowWarps; u < hi;) {
+      const int g = u / C, c0 = u - g * C, c1 = min(C, c0 + hi - u);
+      row_portion(srow + 2 * g, sq, n, c0, c1, i0 + 2 * g, k2i2, part + (w + g) * 10);
+      u += c1 - c0;
     }
-    if (!failed) {
-      const int cnt = min(tile, n - t * tile), C = (cnt + 31) / 32, U = groups * C;
-      const int hi = (w + 1) * U / kRowWarps;
-      for (int u = w * U / kRowWarps; u < hi;) {
-        const int g = u / C, c0 = u - g * C, c1 = min(C, c0 + hi - u);
-        row_portion(srow + 2 * g, sq + (size_t)stage * tile, cnt, c0, c1, i0 + 2 * g - t * tile, k2i2,
-                    part + ((size_t)t * slots + w + g) * 10);
-        u += c1 - c0;
-      }
-    }
-    if (t + kRowStages < ntile || failed) {  // the last warp done with the stage refills it
-      __syncwarp();
-      if (lane == 0) {
-        __threadfence_block();
-        if (atomicAdd(&done[stage], 1) == kRowWarps - 1) {
-          done[stage] = 0;
-          if (t + kRowStages < ntile) fetch(t + kRowStages);
-        }
-      }
-    }
+  } else if (lane == 0) {
+    sfail = 1;
   }
   __syncthreads();
   if (sfail) {
-    // Every copy that was issued is waited for before the shared memory goes.
+    // The copy is waited for once more before the shared memory goes.
     if (tid == 0) {
-      for (int t = max(0, ntile - kRowStages); t < ntile; ++t)
-        mbar_wait_bounded(&bars[t % kRowStages], (uint32_t)((t / kRowStages) & 1));
+      mbar_wait_bounded(&bar, 0);
       atomicOr(s.status, LJ_DEVFLAG_TIMEOUT);
     }
     return;
   }
 
-  // A row's value k: its slots over tiles and warps, in FP32 TwoSum, then FP64.
+  // A row's value k: its slots, in FP32 TwoSum, then FP64.
   auto row_sum = [&](int k) {
     FloatAcc a{0.f, 0.f};
-    const int g = r >> 1;
-    for (int t = 0; t < ntile; ++t) {
-      const int C = (min(tile, n - t * tile) + 31) / 32, U = groups * C;
-      const int w1 = warp_of_unit((g + 1) * C - 1, U);
-      const float* p = part + ((size_t)t * slots + g) * 10 + (r & 1) * 5 + k;
-      for (int ww = warp_of_unit(g * C, U); ww <= w1; ++ww) two_sum_add(a, p[ww * 10]);
-    }
+    const int g = r >> 1, w1 = warp_of_unit((g + 1) * C - 1, U);
+    const float* p = part + g * 10 + (r & 1) * 5 + k;
+    for (int ww = warp_of_unit(g * C, U); ww <= w1; ++ww) two_sum_add(a, p[ww * 10]);
     return (double)a.hi + (double)a.lo;
   };
   double p0 = 0.0, p1 = 0.0;  // c < 3: v^2 (EVN) or tv^2; c = 3: e, w
@@ -271,26 +225,25 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
     }
   }
   if (c < 4) {  // whole warps
-    const int nw = rpad / 32, wi = r / 32;
+    const int wi = r / 32;
     if (MODE == MODE_EVN || c < 3) p0 = warp_sum(p0);
     if (MODE == MODE_EVN && c == 3) p1 = warp_sum(p1);
     if (lane == 0) {
       red[c][wi] = p0;
       if (c == 3) red[4][wi] = p1;
-      for (int k = nw; k < 4; ++k)
-        if (wi == 0) red[c][k] = 0.0, red[c == 3 ? 4 : c][k] = 0.0;
+      if (rpad == 32) red[c][1] = red[c == 3 ? 4 : c][1] = 0.0;
     }
   }
   __syncthreads();
   if (w == 0 && lane < 3) {
-    auto four = [&](int k) { return (red[k][0] + red[k][1]) + (red[k][2] + red[k][3]); };
+    auto both = [&](int k) { return red[k][0] + red[k][1]; };
     double* const o = s.row_part + (size_t)blockIdx.x * 8;
     if (MODE == MODE_EVN) {
-      if (lane == 0) o[s.obs_slot + 0] = 0.5 * (four(0) + four(1) + four(2));
-      if (lane == 1) o[s.obs_slot + 1] = 0.5 * four(3);
-      if (lane == 2) o[s.obs_slot + 2] = four(4);
+      if (lane == 0) o[s.obs_slot + 0] = 0.5 * (both(0) + both(1) + both(2));
+      if (lane == 1) o[s.obs_slot + 1] = 0.5 * both(3);
+      if (lane == 2) o[s.obs_slot + 2] = both(4);
     } else if (lane == 0) {
-      o[3] = four(0) + four(1) + four(2);
+      o[3] = both(0) + both(1) + both(2);
     }
   }
 }
@@ -365,23 +318,20 @@ __global__ void __launch_bounds__(128) k_rows_close(StateArgs s, int n, int ctas
 // Rows in pairs, and one SM left to the observables' CTA.
 RowPlan plan_rows(int n, int sms) {
   RowPlan p{};
-  if (sms < 2) return p;
+  if (sms < 2 || n >= kNewtonMinN) return p;
   const int unit = 2 * (sms - 1);
   p.rows = 2 * ((n + unit - 1) / unit);
   if (p.rows > kMaxRows) return RowPlan{};
   p.ctas = (n + p.rows - 1) / p.rows;
-  const int tile = row_tile(n), ntile = (n + tile - 1) / tile;
-  p.smem = sizeof(int4) * (size_t)(ntile < kRowStages ? ntile : kRowStages) * tile +
-           sizeof(float) * 10 * (size_t)ntile * (kRowWarps + p.rows / 2);
+  p.smem = sizeof(int4) * (size_t)n + sizeof(float) * 10 * (size_t)(kRowWarps + p.rows / 2);
   if (p.smem < sizeof(double) * 3 * 32) p.smem = sizeof(double) * 3 * 32;  // the observables' sums
-  p.close_ctas = (n + 31) / 32;
   return p;
 }
 
 cudaError_t rows_setup() {
-  cudaError_t e = cudaFuncSetAttribute(k_rows<MODE_EVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_rows<MODE_TVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+  constexpr int kMost = sizeof(int4) * kNewtonMinN + sizeof(float) * 10 * (kRowWarps + kMaxRows / 2);
+  cudaError_t e = cudaFuncSetAttribute(k_rows<MODE_EVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows<MODE_TVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   return e;
 }
 
@@ -390,8 +340,8 @@ cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, c
                           s, n, p.rows, p.ctas);
 }
 
-cudaError_t launch_rows_close(const StateArgs& s, const RowPlan& p, int n, cudaStream_t st) {
-  return launch_dependent(k_rows_close, p.close_ctas, 128, 0, st, s, n, p.ctas);
+cudaError_t launch_rows_close(const StateArgs& s, int n, int parts, cudaStream_t st) {
+  return launch_dependent(k_rows_close, (n + 31) / 32, 128, 0, st, s, n, parts);
 }
 
 }  // namespace ljgb

@@ -173,4 +173,27 @@ Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
   return p;
 }
 
+NewtonPlan plan_newton(int n, int warps) {
+  NewtonPlan p;
+  constexpr int kTiles = kNewtonBlock / 32;  // tiles of a block
+  const int tiles = (n + 31) / 32, blocks = (tiles + kTiles - 1) / kTiles;
+  std::vector<int64_t> first(blocks + 1, 0);  // units before block I
+  for (int I = 0; I < blocks; ++I) first[I + 1] = first[I] + tiles - (int64_t)kTiles * I;
+  const int64_t total = first[blocks];
+  const int64_t W = std::min<int64_t>(warps, total);
+  p.block_part.assign(2 * blocks, 0);
+  int I = 0;
+  for (int64_t w = 0; w < W; ++w) {
+    const int64_t lo = total * w / W, hi = total * (w + 1) / W;
+    while (first[I + 1] <= lo) ++I;
+    p.tasks.push_back(NewtonTask{I, kTiles * I + (int)(lo - first[I]), (int)(hi - lo)});
+    for (int B = I; B < blocks && first[B] < hi; ++B) {
+      if (p.block_part[2 * B + 1]++ == 0) p.block_part[2 * B] = (int)w + B;
+    }
+  }
+  p.iparts = (int)W + blocks;
+  for (int t = 0; t < tiles; ++t) p.jparts += t / kTiles + 1;
+  return p;
+}
+
 }  // namespace ljgb

@@ -68,4 +68,16 @@ struct Pair64Plan {
 };
 Pair64Plan plan_pairs64(const std::vector<int>& n, int sms);
 
+// Tasks of the unordered-pair kernel for n particles and `warps` warps: equal
+// shares (+-1) of the (block, tile) sequence.  The i sums of (task, block) are
+// part task + block, so a block's parts are consecutive: block_part holds the
+// first and the count.
+struct NewtonPlan {
+  std::vector<NewtonTask> tasks;
+  std::vector<int> block_part;
+  long long jparts = 0;  // parts of the j sums
+  int iparts = 0;
+};
+NewtonPlan plan_newton(int n, int warps);
+
 }  // namespace ljgb

@@ -70,6 +70,9 @@ thread_local std::string g_create_error;
 // weight ragged tiles in the stream-K split.
 constexpr int kTileOverhead = 8;
 constexpr int kMaxSegmentsPerBlock = 8;
+// The unordered-pair step's j sums are 10 KB a particle at N = 2^18 (2.7 GB)
+// and grow with N; larger boxes keep the stream-K kernel.
+constexpr int kNewtonMaxN = 1 << 18;
 
 // Owned device array.  Movable, not copyable; freed on destruction (or
 // explicitly).
@@ -247,6 +250,11 @@ struct lj_system {
   bool rows_off = false;  // the autotuner found a stream-K shape faster, or is timing one
   DevBuf<double> row_part;
   bool cluster_ok = false;  // the box may step in one cluster (lj_cluster.cu)
+  // unordered-pair step of a single large box (lj_newton.cu); newton = tasks, 0: not for this box
+  int newton = 0;
+  DevBuf<NewtonTask> newton_tasks;
+  DevBuf<int> newton_blocks;
+  DevBuf<float> newton_j, newton_i;
   DevBuf<float> partial;  // MIXED: nseg x 5 x BI
   // FP64 pair pass: tasks, boxes and sums (Pair64Args)
   int p64_group = 1, p64_parts = 1;
@@ -679,19 +687,59 @@ lj_status enqueue_step(lj_system* s, int mode, cudaEvent_t* ev, bool capture, in
 // shadow frame (periodic or walled boxes, not open ones) and the MIXED kernel.
 bool use_fused(const lj_system* s) { return s->prec == LJ_PREC_MIXED && !s->any_open; }
 
-// The row step takes the fused steps of a box it is built for, unless a
-// stream-K shape or split cap was chosen.
+// The row step (boxes below kNewtonMinN) or the unordered-pair step takes the
+// fused steps of a single box, unless a stream-K shape or split cap was chosen.
 bool use_rows(const lj_system* s) {
-  return use_fused(s) && s->rows.ctas > 0 && !s->rows_off && s->forced_shape < 0 && s->forced_split == 0;
+  return use_fused(s) && (s->rows.ctas > 0 || s->newton > 0) && !s->rows_off && s->forced_shape < 0 && s->forced_split == 0;
+}
+
+void free_newton(lj_system* s) {
+  s->newton = 0;
+  s->newton_tasks.free();
+  s->newton_blocks.free();
+  s->newton_j.free();
+  s->newton_i.free();
+}
+
+// The unordered-pair step's tables and sums, built when the box is created.
+lj_status setup_newton(lj_system* s) {
+  const int n = s->cfg[0].n;
+  int per_sm = 0;
+  LJ_CUDA(s, newton_setup(&per_sm));
+  if (per_sm < 1) return LJ_OK;
+  const NewtonPlan p = plan_newton(n, s->num_sms * per_sm * kNewtonWarps);
+  LJ_CUDA(s, s->newton_tasks.alloc(p.tasks.size()));
+  LJ_CUDA(s, s->newton_blocks.alloc(p.block_part.size()));
+  LJ_CUDA(s, s->newton_j.alloc((size_t)p.jparts * 160));
+  LJ_CUDA(s, s->newton_i.alloc((size_t)p.iparts * 5 * kNewtonBlock));
+  LJ_CUDA(s, s->row_part.alloc(8 * (size_t)((n + 31) / 32)));
+  LJ_CUDA(s, cudaMemcpyAsync(s->newton_tasks.p, p.tasks.data(), sizeof(NewtonTask) * p.tasks.size(),
+                             cudaMemcpyHostToDevice, s->stream));
+  LJ_CUDA(s, cudaMemcpyAsync(s->newton_blocks.p, p.block_part.data(), sizeof(int) * p.block_part.size(),
+                             cudaMemcpyHostToDevice, s->stream));
+  LJ_CUDA(s, cudaStreamSynchronize(s->stream));
+  s->newton = (int)p.tasks.size();
+  return LJ_OK;
+}
+
+NewtonArgs newton_args(const lj_system* s, const StateArgs& a) {
+  return NewtonArgs{a.q, a.sc, s->newton_tasks.p, s->newton_blocks.p, s->newton_j.p, s->newton_i.p, s->cfg[0].n,
+                    s->newton};
 }
 
 lj_status enqueue_rows(lj_system* s, int mode, cudaEvent_t pair_end, unsigned flags, int* kernels) {
   const StateArgs a = state_args(s);
-  LJ_CUDA(s, launch_rows(a, s->rows, s->cfg[0].n, mode, s->stream));
+  const int n = s->cfg[0].n;
+  if (s->newton) LJ_CUDA(s, launch_newton(newton_args(s, a), s->stream));
+  else LJ_CUDA(s, launch_rows(a, s->rows, n, mode, s->stream));
   *kernels += 1;
+  if (s->newton) {
+    LJ_CUDA(s, launch_newton_sum(a, newton_args(s, a), mode, s->stream));
+    *kernels += 1;
+  }
   if (pair_end) LJ_CUDA(s, cudaEventRecordWithFlags(pair_end, s->stream, flags));
   if (mode == MODE_TVN) {
-    LJ_CUDA(s, launch_rows_close(a, s->rows, s->cfg[0].n, s->stream));
+    LJ_CUDA(s, launch_rows_close(a, n, s->newton ? (n + 31) / 32 : s->rows.ctas, s->stream));
     *kernels += 1;
   }
   return LJ_OK;
@@ -938,7 +986,7 @@ lj_status alloc_state(lj_system* s) {
   LJ_CUDA(s, s->sc.alloc(s->nsys));
   LJ_CUDA(s, s->dboxes.alloc(s->nsys));
   LJ_CUDA(s, s->status.alloc(1));
-  if (s->rows.ctas > 0) LJ_CUDA(s, s->row_part.alloc(8 * (size_t)std::max(s->rows.ctas, s->rows.close_ctas)));
+  if (s->rows.ctas > 0) LJ_CUDA(s, s->row_part.alloc(8 * (size_t)std::max(s->rows.ctas, (s->ntotal + 31) / 32)));
   LJ_CUDA(s, s->hist.alloc(kMaxHistBins));
   LJ_CUDA(s, cudaMemsetAsync(s->x.p, 0, sizeof(double) * n3, s->stream));
   LJ_CUDA(s, cudaMemsetAsync(s->v.p, 0, sizeof(double) * n3, s->stream));
@@ -1080,6 +1128,11 @@ lj_status create_impl(const lj_config* cfgs, int nsys, lj_system** out) {
     return bail(fail(s, LJ_ERR_CUDA, "cluster set-up failed"));
   lj_status st = alloc_state(s);
   if (st) return bail(st);
+  if (nsys == 1 && s->prec == LJ_PREC_MIXED && s->cfg[0].n >= kNewtonMinN && s->cfg[0].n <= kNewtonMaxN) {
+    // (without memory for its sums the box steps by the stream-K kernel)
+    if ((st = setup_newton(s)) == LJ_ERR_OUT_OF_MEMORY) free_newton(s);
+    else if (st) return bail(st);
+  }
   st = upload_boxes(s);
   if (st) return bail(st);
   // Shape: the reference's CUDABlockSize picks the nearest i-block size.
@@ -1199,6 +1252,7 @@ lj_status lj_destroy(lj_system* s) {
   s->dboxes.free();
   s->blk_part.free();
   s->row_part.free();
+  free_newton(s);
   s->partial.free();
   s->p64_tasks.free();
   s->p64_boxes.free();

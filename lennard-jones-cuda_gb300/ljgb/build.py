@@ -24,6 +24,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = [
     "lj_pairs.cu",
     "lj_rows.cu",
+    "lj_newton.cu",
     "lj_cluster.cu",
     "lj_rdf.cu",
     "lj_pairs64.cu",
