@@ -24,28 +24,44 @@ __device__ __forceinline__ int floor_small(float x) {
 
 constexpr int kTile = 256;  // j records staged in shared memory
 
-// One pair into the CTA's histogram, from its fixed-point separation (qi in
-// slots 1..3, see i_record_slots123).  The arithmetic is exactly what the
-// oracle's emu_rdf_* reproduces on the CPU: floor of the separately rounded
-// products, clamped to or dropped past the last bin.
+// Bin position of a squared fixed-point separation x, before floor, in the
+// separately rounded products that the oracle's emu_rdf_* repeats on the CPU:
+// r^2 bins (modes 0, 1) x k2 inv_w; linear bins (mode 2) only x k2, compared
+// with rmax^2 before the root.
 template <int MODE>
-__device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float k2, float inv_w, float limit, int last,
-                                         unsigned* shist, unsigned& nclamp) {
+__device__ __forceinline__ float bin_pos(float x, float k2, float inv_w) {
+  const float r2 = __fmul_rn(x, k2);
+  return MODE == 2 ? r2 : __fmul_rn(r2, inv_w);
+}
+
+// Smallest x >= 0 whose bin position reaches `limit`, by bisection on the
+// bits: rounded products by positive constants are monotonic in x, so `x <
+// bound` decides as comparing the position itself would, without forming it.
+template <int MODE>
+__device__ float bin_bound(float k2, float inv_w, float limit) {
+  int lo = 0, hi = 0x7f800000;
+  while (lo < hi) {
+    const int mid = lo + (hi - lo) / 2;
+    if (bin_pos<MODE>(__int_as_float(mid), k2, inv_w) >= limit) hi = mid;
+    else lo = mid + 1;
+  }
+  return __int_as_float(lo);
+}
+
+// One pair into the CTA's histogram, from its fixed-point separation (qi in
+// slots 1..3, see i_record_slots123).  Pairs at or past the bound are not
+// counted here: dropped (modes 1, 2), or the last bin's (mode 0), which gets
+// all pairs less the counted ones at the end.
+template <int MODE>
+__device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float bound, float k2, float inv_w, int last,
+                                         unsigned* shist) {
   const float dx = __int2float_rn(fixed_diff(qj.x, qi.y));
   const float dy = __int2float_rn(fixed_diff(qj.y, qi.z));
   const float dz = __int2float_rn(fixed_diff(qj.z, qi.w));
-  const float r2 = __fmul_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), k2);
-  if (MODE == 2) {  // linear r bins; limit = rmax^2 (so r / w < nb, up to rounding)
-    if (r2 < limit) atomicAdd(&shist[min(floor_small(__fmul_rn(__fsqrt_rn(r2), inv_w)), last)], 1u);
-  } else {
-    const float b = __fmul_rn(r2, inv_w);
-    if (MODE == 1) {  // r^2 bins, overflow dropped (MDSystem.cpp:283); limit = nb
-      if (b < limit) atomicAdd(&shist[floor_small(b)], 1u);
-    } else {  // overflow counted in the last bin (MDSystem.cu:39); limit = nb - 1
-      // most pairs of a box land there: counted in a register
-      if (b >= limit) ++nclamp;
-      else atomicAdd(&shist[min(floor_small(fminf(b, limit)), last)], 1u);
-    }
+  const float x = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+  if (x < bound) {
+    const float b = bin_pos<MODE>(x, k2, inv_w);
+    atomicAdd(&shist[MODE == 2 ? min(floor_small(__fmul_rn(__fsqrt_rn(b), inv_w)), last) : floor_small(b)], 1u);
   }
 }
 
@@ -53,11 +69,12 @@ __device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float k2,
 // j's from its own first particle on and skips j <= i inside its own square;
 // the wrapping difference is antisymmetric, so (j, i) falls into the bin of
 // (i, j) exactly and the flush adds every count twice.  The loop is bound by
-// issue (about 17 instructions a pair, no memory traffic: the shadow stays in
-// L2), so halving the pairs is what shortens it; N = 16384, 256 clamped bins:
-// the call took 234 us over ordered pairs, 131 us so.  A CTA owns a contiguous range of
-// (block, 32-j chunk) units (build_rdf_ranges), flushing its shared histogram
-// once: a grid of single tiles would flush 256 bins thousands of times.
+// issue (no memory traffic: the shadow stays in L2): 11 instructions for a pair
+// past the bound, which most are.  N = 16384, 256 clamped bins, us a call: 234
+// over ordered pairs, 131 over unordered ones, 119 with the bound in place of
+// the products and a counter.  A CTA owns a contiguous range of (block, 32-j
+// chunk) units (build_rdf_ranges), flushing its shared histogram once: a grid
+// of single tiles would flush 256 bins thousands of times.
 template <int MODE>
 __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
   extern __shared__ unsigned shist[];
@@ -66,17 +83,24 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
   const int tid = threadIdx.x, lane = tid & 31;
   const HistArgs h = a.hist;
   const int last = h.nb - 1;
-  const float limit = MODE == 2 ? h.rmax2 : (float)(MODE == 1 ? h.nb : last);
   const float k2 = a.sc->k2;
+  const float bound = bin_bound<MODE>(k2, h.inv_w, MODE == 2 ? h.rmax2 : (float)(MODE == 1 ? h.nb : last));
   for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
-  unsigned nclamp = 0;
+  unsigned npairs = 0;  // of this thread's i, since the last flush
   auto flush = [&]() {
-    const unsigned wclamp = __reduce_add_sync(0xffffffffu, nclamp);
-    nclamp = 0;
-    if (MODE == 0 && lane == 0 && wclamp) atomicAdd(&shist[last], wclamp);
     __syncthreads();
+    unsigned counted = 0;
     for (int b = tid; b < h.nb; b += kRdfBlock)
-      if (shist[b]) atomicAdd(h.counts + b, 2ull * shist[b]);
+      if (shist[b]) {
+        counted += shist[b];
+        atomicAdd(h.counts + b, 2ull * shist[b]);
+      }
+    if (MODE == 0) {
+      // (sums of a CTA stay below 2^32; the difference may be negative for a warp)
+      const unsigned all = __reduce_add_sync(0xffffffffu, npairs), binned = __reduce_add_sync(0xffffffffu, counted);
+      if (lane == 0) atomicAdd(h.counts + last, 2ull * all - 2ull * binned);
+    }
+    npairs = 0;
   };
   int B = a.cta_block[blockIdx.x], c = a.cta_chunk[blockIdx.x], left = a.cta_units[blockIdx.x];
   const int nchunks = (a.n + kRdfChunk - 1) / kRdfChunk;
@@ -90,7 +114,6 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
     for (; take > 0;) {
       const int part = min(take, (1 << 18));
       if (counted + part > (1 << 18)) {
-        __syncthreads();
         flush();
         __syncthreads();
         for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
@@ -105,18 +128,19 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
         __syncthreads();
         if (i >= a.n) continue;
         if (j0 >= i0 + kRdfBlock) {
-#pragma unroll 4
-          for (int jj = 0; jj < cnt; ++jj) bin_pair<MODE>(qi, tile[jj], k2, h.inv_w, limit, last, shist, nclamp);
+#pragma unroll 8
+          for (int jj = 0; jj < cnt; ++jj) bin_pair<MODE>(qi, tile[jj], bound, k2, h.inv_w, last, shist);
+          npairs += cnt;
         } else {
           for (int jj = 0; jj < cnt; ++jj)
-            if (j0 + jj > i) bin_pair<MODE>(qi, tile[jj], k2, h.inv_w, limit, last, shist, nclamp);
+            if (j0 + jj > i) bin_pair<MODE>(qi, tile[jj], bound, k2, h.inv_w, last, shist);
+          npairs += max(0, j0 + cnt - max(j0, i + 1));
         }
       }
       take -= part;
       c += part;
     }
   }
-  __syncthreads();
   flush();
 }
 

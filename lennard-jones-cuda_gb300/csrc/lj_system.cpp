@@ -1821,9 +1821,11 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   if (st) return st;
   LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
   s->launches += 1;
+  // the status word first: the copy into pageable memory returns once both are there
+  if ((st = flush_observables(s)) || (st = enqueue_status_read(s))) return st;
   LJ_CUDA(s, cudaMemcpyAsync(counts, s->hist.p, sizeof(unsigned long long) * nbins, cudaMemcpyDeviceToHost,
                              s->stream));
-  return check_status(s);
+  return finish_status(s);
 }
 
 lj_status lj_velocity_counts(lj_system* s, double step, int32_t nbins, uint64_t* counts) {
