@@ -8,12 +8,13 @@
 // kernel (forces, energies, virial) -> per-particle float4 forces and one FP64
 // virial sum; the 256-bin r^2 RDF, where it is asked for, is the histogram
 // kernel's (lj_rdf.cu): a call of N = 8000 took 203 us with both in one kernel and
-// takes 155 us in two, since the force loop evaluates ordered pairs and the
+// took 155 us in two, since the force loop evaluates ordered pairs and the
 // histogram each unordered pair once.  Work buffers
 // are cached per particle count on a private stream.
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -32,34 +33,56 @@ namespace {
 constexpr int kRefBins = 256;  // NdNdr2 size (MDSystem.cpp:97)
 constexpr int kBlk = kFloat4Threads;
 
-// Force[i] = (F, sum_j r^-12 - r^-6); block partial of sum_j s r^2.
+// What a call reads back, in one copy.
+struct RefResult {
+  unsigned long long hist[kRefBins];
+  float pressure;
+  int status;
+};
+
+// Force[i] = (F, sum_j r^-12 - r^-6), the segments added in FP32 TwoSum as the
+// integrators do; block partial of sum_j s r^2.  The last CTA to finish adds
+// the partials: pressure = (4/6) sum_i sum_j s r^2 (MDSystem.cu:105-108, 136).
 __global__ void k_ref_reduce(const float* partial, const BlockInfo* blocks, int bi_threads, const DevScalars* sc,
-                             float4* force, double* blk) {
+                             float4* force, double* blk, int* ticket, RefResult* result) {
   __shared__ double sh[32];
+  __shared__ bool last;
   const BlockInfo bi = blocks[blockIdx.x];
   const int tid = threadIdx.x;
   double part[1] = {0.0};
   if (tid < bi.n_i) {
-    double S[5] = {0, 0, 0, 0, 0};
+    FloatAcc acc[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) acc[c] = FloatAcc{0.f, 0.f};
+#pragma unroll 4
     for (int k = 0; k < bi.seg_count; ++k) {
       const size_t base = (size_t)(bi.seg_first + k) * 5 * bi_threads + tid;
-      for (int c = 0; c < 5; ++c) S[c] += (double)partial[base + (size_t)c * bi_threads];
+#pragma unroll
+      for (int c = 0; c < 5; ++c) two_sum_add(acc[c], partial[base + (size_t)c * bi_threads]);
     }
+    double S[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) S[c] = (double)acc[c].hi + (double)acc[c].lo;
     const double fs = sc->fscale;
     force[bi.i0 + tid] = make_float4((float)(fs * S[0]), (float)(fs * S[1]), (float)(fs * S[2]), (float)(S[3] - S[4]));
     part[0] = 12.0 * S[3] - 6.0 * S[4];
   }
   block_sum<1>(part, sh);
-  if (tid == 0) blk[(size_t)blockIdx.x * 8] = part[0];
-}
-
-// pressure = (4/6) sum_i sum_j s r^2   (MDSystem.cu:105-108, 136)
-__global__ void k_ref_pressure(const double* blk, int nb, float* out) {
-  __shared__ double sh[32];
+  if (tid == 0) {
+    blk[(size_t)blockIdx.x * 8] = part[0];
+    __threadfence();
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   double acc[1] = {0.0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) acc[0] += blk[(size_t)b * 8];
+  for (int b = tid; b < (int)gridDim.x; b += blockDim.x) acc[0] += __ldcg(blk + (size_t)b * 8);
   block_sum<1>(acc, sh);
-  if (threadIdx.x == 0) *out = (float)(acc[0] * 4.0 / 6.0);
+  if (tid == 0) {
+    result->pressure = (float)(acc[0] * 4.0 / 6.0);
+    *ticket = 0;
+  }
 }
 
 struct CompatCtx {
@@ -77,9 +100,9 @@ struct CompatCtx {
   int *rb = nullptr, *rc = nullptr, *ru = nullptr;  // ranges of the histogram pass
   float* partial = nullptr;
   double* blk = nullptr;
-  unsigned long long* hist = nullptr;
-  int* status = nullptr;
-  float* pressure = nullptr;
+  RefResult* result = nullptr;       // device
+  RefResult* host_result = nullptr;  // page-locked
+  int* ticket = nullptr;             // [0] reduce, [1] bounding box (0 between launches)
   void release() {
     if (stream) cudaStreamSynchronize(stream);
     cudaFree(q);
@@ -94,9 +117,9 @@ struct CompatCtx {
     cudaFree(ru);
     cudaFree(partial);
     cudaFree(blk);
-    cudaFree(hist);
-    cudaFree(status);
-    cudaFree(pressure);
+    cudaFree(result);
+    cudaFree(ticket);
+    if (host_result) cudaFreeHost(host_result);
     if (stream) cudaStreamDestroy(stream);
     *this = CompatCtx();
   }
@@ -176,11 +199,12 @@ bool ensure_ctx(int n, int block_hint) {
     REF_CHECK(device_alloc((void**)&c.ru, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.partial, sizeof(float) * (size_t)s.nseg * 5 * s.BI));
     REF_CHECK(device_alloc((void**)&c.blk, sizeof(double) * 8 * (size_t)std::max(nb, c.nb_bbox)));
-    REF_CHECK(device_alloc((void**)&c.hist, sizeof(unsigned long long) * kRefBins));
-    REF_CHECK(device_alloc((void**)&c.status, sizeof(int)));
-    REF_CHECK(device_alloc((void**)&c.pressure, sizeof(float)));
+    REF_CHECK(device_alloc((void**)&c.result, sizeof(RefResult)));
+    REF_CHECK(device_alloc((void**)&c.ticket, 2 * sizeof(int)));
+    REF_CHECK(pinned_alloc((void**)&c.host_result, sizeof(RefResult)));
     REF_CHECK(cudaMemset(c.sc, 0, sizeof(DevScalars)));
-    REF_CHECK(cudaMemset(c.status, 0, sizeof(int)));
+    REF_CHECK(cudaMemset(c.result, 0, sizeof(RefResult)));
+    REF_CHECK(cudaMemset(c.ticket, 0, 2 * sizeof(int)));
     REF_CHECK(cudaMemcpy(c.blocks, s.blocks.data(), sizeof(BlockInfo) * nb, cudaMemcpyHostToDevice));
     REF_CHECK(cudaMemcpy(c.ctb, s.cta_tile_begin.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
     REF_CHECK(cudaMemcpy(c.clo, s.cta_lo.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
@@ -211,9 +235,7 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   if (!ensure_ctx(n, block_size > 0 ? block_size : 128)) return false;
   CompatCtx& c = g_ctx;
   const float4* pos = reinterpret_cast<const float4*>(Pos);
-  if (!periodic) REF_CHECK(launch_float4_bbox(pos, n, c.blk, c.stream));
-  REF_CHECK(launch_float4_frame(c.blk, c.nb_bbox, periodic, (double)L, c.sc, nullptr, c.stream));
-  REF_CHECK(launch_float4_quantize(pos, n, c.sc, c.q, c.stream));
+  REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));
   PairArgs a{};
   a.q = c.q;
   a.blocks = c.blocks;
@@ -223,33 +245,34 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   a.cta_jt = c.cj;
   a.sc = c.sc;
   a.partial = c.partial;
-  a.status = c.status;
+  a.status = &c.result->status;
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
-  if (want_rdf) REF_CHECK(cudaMemsetAsync(c.hist, 0, sizeof(unsigned long long) * kRefBins, c.stream));
+  if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
   REF_CHECK(launch_pairs(c.shape, a, c.sched.G, c.stream));
   if (want_rdf)
-    REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.hist}},
+    REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}},
                          c.rdf_grid, c.stream));
   const int nb = (int)c.sched.blocks.size();
   k_ref_reduce<<<nb, c.sched.BI, 0, c.stream>>>(c.partial, c.blocks, c.sched.BI, c.sc,
-                                                  reinterpret_cast<float4*>(Force), c.blk);
+                                                  reinterpret_cast<float4*>(Force), c.blk, c.ticket, c.result);
   REF_CHECK(cudaGetLastError());
-  k_ref_pressure<<<1, 256, 0, c.stream>>>(c.blk, nb, c.pressure);
-  REF_CHECK(cudaGetLastError());
-  REF_CHECK(cudaMemcpyAsync(host_pressure, c.pressure, sizeof(float), cudaMemcpyDeviceToHost, c.stream));
-  unsigned long long h[kRefBins];
-  if (want_rdf) REF_CHECK(cudaMemcpyAsync(h, c.hist, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
-  int st = 0;
-  REF_CHECK(cudaMemcpyAsync(&st, c.status, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  // one copy into page-locked memory (three into the caller's and the stack
+  // waited for the stream one after another; with the frame by value and the
+  // pressure in the reduction, 155 -> 123 us a call at N = 8000)
+  RefResult* const r = c.host_result;
+  const size_t skip = want_rdf ? 0 : offsetof(RefResult, pressure);
+  REF_CHECK(cudaMemcpyAsync(reinterpret_cast<char*>(r) + skip, reinterpret_cast<const char*>(c.result) + skip,
+                            sizeof(RefResult) - skip, cudaMemcpyDeviceToHost, c.stream));
   REF_CHECK(cudaStreamSynchronize(c.stream));
-  if (st) {
-    cudaMemset(c.status, 0, sizeof(int));
+  *host_pressure = r->pressure;
+  if (r->status) {
+    cudaMemset(&c.result->status, 0, sizeof(int));
     g_status = LJ_ERR_DEVICE_TIMEOUT;
     g_error = "calculateNForces: a device-side wait timed out";
     return false;
   }
   if (want_rdf)
-    for (int b = 0; b < kRefBins; ++b) host_RDF[b] = (int)h[b];
+    for (int b = 0; b < kRefBins; ++b) host_RDF[b] = (int)r->hist[b];
   return true;
 }
 
@@ -355,97 +378,97 @@ const char* lj_reference_abi_error(void) { return g_error.c_str(); }
 namespace ljgb {
 namespace {
 
-// Per-CTA bounding box of kFloat4Threads positions: blk[b*8 + 0..2] = min,
-// blk[b*8 + 3..5] = max.
-__global__ void k_float4_bbox(const float4* pos, int n, double* blk) {
-  __shared__ double sh[6][32];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  if (i < n) {
-    const float4 p = pos[i];
-    lo[0] = hi[0] = p.x;
-    lo[1] = hi[1] = p.y;
-    lo[2] = hi[2] = p.z;
-  }
-  for (int c = 0; c < 3; ++c)
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[c] = fmin(lo[c], __shfl_down_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmax(hi[c], __shfl_down_sync(0xffffffffu, hi[c], o));
-    }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-    for (int c = 0; c < 3; ++c) {
-      sh[c][warp] = lo[c];
-      sh[3 + c][warp] = hi[c];
-    }
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) {
-      double a = 1e300, b = -1e300;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        a = fmin(a, sh[c][w]);
-        b = fmax(b, sh[3 + c][w]);
-      }
-      blk[(size_t)blockIdx.x * 8 + c] = a;
-      blk[(size_t)blockIdx.x * 8 + 3 + c] = b;
-    }
-}
-
-// One thread: frame of the fixed-point shadow (eps = sigma = 1).  Periodic:
-// origin 0, period L.  Otherwise the bounding box's low corner and a period
-// of twice its largest extent, so no separation wraps.  Clears *status when
-// given.
-__global__ void k_float4_frame(const double* blk, int nb, int periodic, double L, DevScalars* sc, int* status) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double origin[3] = {0, 0, 0};
-  double P = L;
-  if (!periodic) {
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int b = 0; b < nb; ++b)
-      for (int c = 0; c < 3; ++c) {
-        lo[c] = fmin(lo[c], blk[(size_t)b * 8 + c]);
-        hi[c] = fmax(hi[c], blk[(size_t)b * 8 + 3 + c]);
-      }
-    double ext = 0;
-    for (int c = 0; c < 3; ++c) {
-      ext = fmax(ext, hi[c] - lo[c]);
-      origin[c] = lo[c];
-    }
-    P = 2.002 * ext + 1e-3;
-  }
-  for (int c = 0; c < 3; ++c) sc->origin[c] = origin[c];
+// Frame of the fixed-point shadow (eps = sigma = 1).  Periodic: origin 0,
+// period L.  Otherwise the bounding box's low corner and a period of twice its
+// largest extent, so no separation wraps.
+__host__ __device__ inline void float4_frame(DevScalars* sc, double ox, double oy, double oz, double P) {
+  sc->origin[0] = ox;
+  sc->origin[1] = oy;
+  sc->origin[2] = oz;
   sc->P = P;
   sc->invP = 1.0 / P;
   const double ks = P / 4294967296.0;
   sc->k2 = (float)(ks * ks);
   sc->k2inv = (float)(1.0 / (ks * ks));
   sc->fscale = 4.0 * ks;
+}
+
+// Bounding box of the positions: per CTA (blk[b*8 + 0..2] = min, [3..5] =
+// max), then over the CTAs by the last one to finish, which writes the frame
+// (and clears *status when given).
+__global__ void k_float4_bbox(const float4* pos, int n, double* blk, int* ticket, DevScalars* sc, int* status) {
+  __shared__ float sh[6][32];
+  __shared__ bool last;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};  // min x, y, z, min -x, -y, -z
+  if (i < n) {
+    const float4 p = pos[i];
+    v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = -p.x, v[4] = -p.y, v[5] = -p.z;
+  }
+  auto over_block = [&]() {  // of v, in every thread
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      for (int o = 16; o > 0; o >>= 1) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+      if (lane == 0) sh[k][warp] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v[k] = fminf(v[k], sh[k][w]);
+    __syncthreads();
+  };
+  over_block();
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 6; ++k) blk[(size_t)blockIdx.x * 8 + k] = v[k];
+    __threadfence();
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    v[k] = INFINITY;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) v[k] = fminf(v[k], (float)__ldcg(blk + (size_t)b * 8 + k));
+  }
+  over_block();
+  if (threadIdx.x != 0) return;
+  double ext = 0;
+  for (int k = 0; k < 3; ++k) ext = fmax(ext, -(double)v[3 + k] - (double)v[k]);
+  float4_frame(sc, v[0], v[1], v[2], 2.002 * ext + 1e-3);
+  *ticket = 0;
   if (status) *status = 0;
 }
 
-__global__ void k_float4_quantize(const float4* pos, int n, const DevScalars* sc, int4* q) {
+// With PERIODIC the frame comes by value and is written to *sc for the
+// kernels that follow (and *status cleared when given).
+template <bool PERIODIC>
+__global__ void k_float4_quantize(const float4* pos, int n, DevScalars* sc, int4* q, DevScalars frame, int* status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (PERIODIC && i == 0) {
+    *sc = frame;
+    if (status) *status = 0;
+  }
   if (i >= n) return;
   const float4 p = pos[i];
-  q[i] = make_int4(fixed_coord(p.x, sc->origin[0], sc->invP), fixed_coord(p.y, sc->origin[1], sc->invP),
-                   fixed_coord(p.z, sc->origin[2], sc->invP), 0);
+  const DevScalars& f = PERIODIC ? frame : *sc;
+  q[i] = make_int4(fixed_coord(p.x, f.origin[0], f.invP), fixed_coord(p.y, f.origin[1], f.invP),
+                   fixed_coord(p.z, f.origin[2], f.invP), 0);
 }
 
 }  // namespace
 
-cudaError_t launch_float4_bbox(const float4* pos, int n, double* blk, cudaStream_t st) {
-  k_float4_bbox<<<(n + kFloat4Threads - 1) / kFloat4Threads, kFloat4Threads, 0, st>>>(pos, n, blk);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_float4_frame(const double* blk, int nb, int periodic, double L, DevScalars* sc, int* status,
-                                cudaStream_t st) {
-  k_float4_frame<<<1, 32, 0, st>>>(blk, nb, periodic, L, sc, status);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_float4_quantize(const float4* pos, int n, const DevScalars* sc, int4* q, cudaStream_t st) {
-  k_float4_quantize<<<(n + kFloat4Threads - 1) / kFloat4Threads, kFloat4Threads, 0, st>>>(pos, n, sc, q);
+cudaError_t launch_float4_shadow(const float4* pos, int n, int periodic, double L, DevScalars* sc, int* status,
+                                 double* blk, int* ticket, int4* q, cudaStream_t st) {
+  const int grid = (n + kFloat4Threads - 1) / kFloat4Threads;
+  DevScalars frame{};
+  if (periodic) {
+    float4_frame(&frame, 0.0, 0.0, 0.0, L);
+    k_float4_quantize<true><<<grid, kFloat4Threads, 0, st>>>(pos, n, sc, q, frame, status);
+  } else {
+    k_float4_bbox<<<grid, kFloat4Threads, 0, st>>>(pos, n, blk, ticket, sc, status);
+    k_float4_quantize<false><<<grid, kFloat4Threads, 0, st>>>(pos, n, sc, q, frame, nullptr);
+  }
   return cudaGetLastError();
 }
 

@@ -266,11 +266,8 @@ extern "C" lj_status lj_forces_static(const float* pos4, float* force4, double* 
   }
   const int G = g_static_G[dev], nblocks = g_static_nblocks[dev];
   const float4* pos = reinterpret_cast<const float4*>(pos4);
-  const int nbb = (n + kBboxThreads - 1) / kBboxThreads;
-  if (!periodic && (e = launch_float4_bbox(pos, n, blk, st)) != cudaSuccess)
-    return (lj_status)static_fail(LJ_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = launch_float4_frame(blk, nbb, periodic ? 1 : 0, (double)box, sc, status, st)) != cudaSuccess ||
-      (e = launch_float4_quantize(pos, n, sc, q, st)) != cudaSuccess)
+  int* ticket = status + 1;  // behind the status word; 0 since load, and again after every use
+  if ((e = launch_float4_shadow(pos, n, periodic ? 1 : 0, (double)box, sc, status, blk, ticket, q, st)) != cudaSuccess)
     return (lj_status)static_fail(LJ_ERR_CUDA, cudaGetErrorString(e));
   PairArgs a{};
   a.q = q;
