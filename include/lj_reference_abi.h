@@ -17,7 +17,8 @@
  *  - threadExit() synchronises and releases this layer's buffers; it does not
  *    reset the device for the whole process (MDSystem.cu:294-297);
  *  - `blockSize` (CUDABlockSize) selects the nearest i-block size of the
- *    kernel shapes; `q` stays unused as in the reference;
+ *    kernel shapes that boxes of more than 2^18 particles use (smaller ones
+ *    have kernels of their own); `q` stays unused as in the reference;
  *  - no per-call cudaMalloc/cudaFree: work buffers are cached per particle
  *    count (MDSystem.cu:265-287 allocated two RDF arrays on every call).
  */

@@ -4,15 +4,17 @@
 // contract and the deliberate differences.
 //
 // calculateNForces: float4 positions -> fixed-point shadow (frame from L or
-// from the bounding box for non-periodic boxes) -> persistent all-pairs
-// kernel (forces, energies, virial) -> per-particle float4 forces and one FP64
-// virial sum; the 256-bin r^2 RDF, where it is asked for, is the histogram
+// from the bounding box for non-periodic boxes) -> the pair kernels of a step
+// without the step (the row kernel below kNewtonMinN particles, unordered pairs
+// up to kNewtonMaxN, the stream-K kernel above) -> per-particle float4 forces
+// and one FP64 virial sum; the 256-bin r^2 RDF, where it is asked for, is the histogram
 // kernel's (lj_rdf.cu): a call of N = 8000 took 203 us with both in one kernel and
 // took 155 us in two, since the force loop evaluates ordered pairs and the
 // histogram each unordered pair once.  Work buffers
 // are cached per particle count on a private stream.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -94,6 +96,13 @@ struct CompatCtx {
   cudaStream_t stream = nullptr;
   int4* q = nullptr;
   DevScalars* sc = nullptr;
+  // the row or the unordered-pair kernel (rows.ctas > 0 or newton > 0) ...
+  RowPlan rows{};
+  int newton = 0;
+  NewtonTask* newton_tasks = nullptr;
+  int* newton_blocks = nullptr;
+  float *newton_j = nullptr, *newton_i = nullptr;
+  // ... or the stream-K kernel's schedule
   BlockInfo* blocks = nullptr;
   int *ctb = nullptr, *clo = nullptr, *cb = nullptr, *cj = nullptr;
   int rdf_grid = 0;
@@ -107,6 +116,10 @@ struct CompatCtx {
     if (stream) cudaStreamSynchronize(stream);
     cudaFree(q);
     cudaFree(sc);
+    cudaFree(newton_tasks);
+    cudaFree(newton_blocks);
+    cudaFree(newton_j);
+    cudaFree(newton_i);
     cudaFree(blocks);
     cudaFree(ctb);
     cudaFree(clo);
@@ -157,15 +170,19 @@ bool ensure_ctx(int n, int block_hint) {
     g_ctx.release();
   }
   REF_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  REF_CHECK(pair_occupancy(shape, &per_sm));
+  const RowPlan rows = plan_rows(n, sms);
+  const bool stream_k = n > kNewtonMaxN || (n < kNewtonMinN && rows.ctas == 0);
   Schedule s;
-  // at most 8 CTAs per i-block (a block's epilogue sums one segment per CTA)
-  const int nb_i = (n + kShapes[shape].threads - 1) / kShapes[shape].threads;
-  const int ctas = std::min(sms * per_sm, 8 * nb_i);
-  if (!build_schedule(&n, 1, kShapes[shape].threads, kShapes[shape].tile, ctas, 8, &s)) {
-    g_status = LJ_ERR_INVALID;
-    g_error = "cannot build the pair schedule";
-    return false;
+  if (stream_k) {
+    REF_CHECK(pair_occupancy(shape, &per_sm));
+    // at most 8 CTAs per i-block (a block's epilogue sums one segment per CTA)
+    const int nb_i = (n + kShapes[shape].threads - 1) / kShapes[shape].threads;
+    const int ctas = std::min(sms * per_sm, 8 * nb_i);
+    if (!build_schedule(&n, 1, kShapes[shape].threads, kShapes[shape].tile, ctas, 8, &s)) {
+      g_status = LJ_ERR_INVALID;
+      g_error = "cannot build the pair schedule";
+      return false;
+    }
   }
   RdfRanges rr;
   if (!build_rdf_ranges(n, sms * rdf_ctas_per_sm(), &rr)) {
@@ -189,27 +206,44 @@ bool ensure_ctx(int n, int block_hint) {
     const int nb = (int)s.blocks.size();
     REF_CHECK(device_alloc((void**)&c.q, sizeof(int4) * n));
     REF_CHECK(device_alloc((void**)&c.sc, sizeof(DevScalars)));
-    REF_CHECK(device_alloc((void**)&c.blocks, sizeof(BlockInfo) * nb));
-    REF_CHECK(device_alloc((void**)&c.ctb, sizeof(int) * (s.G + 1)));
-    REF_CHECK(device_alloc((void**)&c.clo, sizeof(int) * (s.G + 1)));
-    REF_CHECK(device_alloc((void**)&c.cb, sizeof(int) * s.G));
-    REF_CHECK(device_alloc((void**)&c.cj, sizeof(int) * s.G));
     REF_CHECK(device_alloc((void**)&c.rb, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.rc, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.ru, sizeof(int) * rr.G));
-    REF_CHECK(device_alloc((void**)&c.partial, sizeof(float) * (size_t)s.nseg * 5 * s.BI));
-    REF_CHECK(device_alloc((void**)&c.blk, sizeof(double) * 8 * (size_t)std::max(nb, c.nb_bbox)));
+    // 8 doubles per CTA, i-block, tile or bounding-box CTA, whichever are most
+    REF_CHECK(device_alloc((void**)&c.blk, sizeof(double) * 8 * (size_t)std::max({nb, c.nb_bbox, (n + 31) / 32, sms})));
+    if (stream_k) {
+      REF_CHECK(device_alloc((void**)&c.blocks, sizeof(BlockInfo) * nb));
+      REF_CHECK(device_alloc((void**)&c.ctb, sizeof(int) * (s.G + 1)));
+      REF_CHECK(device_alloc((void**)&c.clo, sizeof(int) * (s.G + 1)));
+      REF_CHECK(device_alloc((void**)&c.cb, sizeof(int) * s.G));
+      REF_CHECK(device_alloc((void**)&c.cj, sizeof(int) * s.G));
+      REF_CHECK(device_alloc((void**)&c.partial, sizeof(float) * (size_t)s.nseg * 5 * s.BI));
+      REF_CHECK(cudaMemcpy(c.blocks, s.blocks.data(), sizeof(BlockInfo) * nb, cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.ctb, s.cta_tile_begin.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.clo, s.cta_lo.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.cb, s.cta_block.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.cj, s.cta_jt.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
+    } else if (n < kNewtonMinN) {
+      c.rows = rows;
+      REF_CHECK(rows_setup());
+    } else {
+      int newton_per_sm = 0;
+      REF_CHECK(newton_setup(&newton_per_sm));
+      const NewtonPlan p = plan_newton(n, sms * newton_per_sm * kNewtonWarps);
+      REF_CHECK(device_alloc((void**)&c.newton_tasks, sizeof(NewtonTask) * p.tasks.size()));
+      REF_CHECK(device_alloc((void**)&c.newton_blocks, sizeof(int) * p.block_part.size()));
+      REF_CHECK(device_alloc((void**)&c.newton_j, sizeof(float) * 160 * (size_t)p.jparts));
+      REF_CHECK(device_alloc((void**)&c.newton_i, sizeof(float) * 5 * kNewtonBlock * (size_t)p.iparts));
+      REF_CHECK(cudaMemcpy(c.newton_tasks, p.tasks.data(), sizeof(NewtonTask) * p.tasks.size(), cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.newton_blocks, p.block_part.data(), sizeof(int) * p.block_part.size(), cudaMemcpyHostToDevice));
+      c.newton = (int)p.tasks.size();
+    }
     REF_CHECK(device_alloc((void**)&c.result, sizeof(RefResult)));
     REF_CHECK(device_alloc((void**)&c.ticket, 2 * sizeof(int)));
     REF_CHECK(pinned_alloc((void**)&c.host_result, sizeof(RefResult)));
     REF_CHECK(cudaMemset(c.sc, 0, sizeof(DevScalars)));
     REF_CHECK(cudaMemset(c.result, 0, sizeof(RefResult)));
     REF_CHECK(cudaMemset(c.ticket, 0, 2 * sizeof(int)));
-    REF_CHECK(cudaMemcpy(c.blocks, s.blocks.data(), sizeof(BlockInfo) * nb, cudaMemcpyHostToDevice));
-    REF_CHECK(cudaMemcpy(c.ctb, s.cta_tile_begin.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
-    REF_CHECK(cudaMemcpy(c.clo, s.cta_lo.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
-    REF_CHECK(cudaMemcpy(c.cb, s.cta_block.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
-    REF_CHECK(cudaMemcpy(c.cj, s.cta_jt.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
     REF_CHECK(cudaMemcpy(c.rb, rr.cta_block.data(), sizeof(int) * rr.G, cudaMemcpyHostToDevice));
     REF_CHECK(cudaMemcpy(c.rc, rr.cta_chunk.data(), sizeof(int) * rr.G, cudaMemcpyHostToDevice));
     REF_CHECK(cudaMemcpy(c.ru, rr.cta_units.data(), sizeof(int) * rr.G, cudaMemcpyHostToDevice));
@@ -236,26 +270,44 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   CompatCtx& c = g_ctx;
   const float4* pos = reinterpret_cast<const float4*>(Pos);
   REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));
-  PairArgs a{};
-  a.q = c.q;
-  a.blocks = c.blocks;
-  a.cta_tile_begin = c.ctb;
-  a.cta_lo = c.clo;
-  a.cta_block = c.cb;
-  a.cta_jt = c.cj;
-  a.sc = c.sc;
-  a.partial = c.partial;
-  a.status = &c.result->status;
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
-  REF_CHECK(launch_pairs(c.shape, a, c.sched.G, c.stream));
   if (want_rdf)
     REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}},
                          c.rdf_grid, c.stream));
-  const int nb = (int)c.sched.blocks.size();
-  k_ref_reduce<<<nb, c.sched.BI, 0, c.stream>>>(c.partial, c.blocks, c.sched.BI, c.sc,
-                                                  reinterpret_cast<float4*>(Force), c.blk, c.ticket, c.result);
-  REF_CHECK(cudaGetLastError());
+  if (c.rows.ctas > 0 || c.newton > 0) {
+    StateArgs st{};
+    st.q = c.q;
+    st.sc = c.sc;
+    st.status = &c.result->status;
+    st.row_part = c.blk;
+    st.blk_cnt = c.ticket;
+    st.force4 = reinterpret_cast<float4*>(Force);
+    st.pressure = &c.result->pressure;
+    if (c.newton > 0) {
+      const NewtonArgs na{c.q, c.sc, c.newton_tasks, c.newton_blocks, c.newton_j, c.newton_i, n, c.newton};
+      REF_CHECK(launch_newton(na, c.stream));
+      REF_CHECK(launch_newton_sum(st, na, MODE_FORCES_ONLY, c.stream));
+    } else {
+      REF_CHECK(launch_rows(st, c.rows, n, MODE_FORCES_ONLY, c.stream));
+    }
+  } else {
+    PairArgs a{};
+    a.q = c.q;
+    a.blocks = c.blocks;
+    a.cta_tile_begin = c.ctb;
+    a.cta_lo = c.clo;
+    a.cta_block = c.cb;
+    a.cta_jt = c.cj;
+    a.sc = c.sc;
+    a.partial = c.partial;
+    a.status = &c.result->status;
+    REF_CHECK(launch_pairs(c.shape, a, c.sched.G, c.stream));
+    const int nb = (int)c.sched.blocks.size();
+    k_ref_reduce<<<nb, c.sched.BI, 0, c.stream>>>(c.partial, c.blocks, c.sched.BI, c.sc,
+                                                    reinterpret_cast<float4*>(Force), c.blk, c.ticket, c.result);
+    REF_CHECK(cudaGetLastError());
+  }
   // one copy into page-locked memory (three into the caller's and the stack
   // waited for the stream one after another; with the frame by value and the
   // pressure in the reduction, 155 -> 123 us a call at N = 8000)

@@ -99,6 +99,8 @@ struct StateArgs {
   int nsys;                    // boxes
   int obs_slot;                // fused EVN: first block-partial slot of this step's K, V, W (0 or 4, by parity)
   double* row_part;            // row step (lj_rows.cu): 8 partial sums per CTA, in place of blk_part
+  float4* force4;              // MODE_FORCES_ONLY of the row and unordered-pair kernels: (F, sum r^-12 - r^-6),
+  float* pressure;             // and (4/6) sum s r^2, as calculateNForces returns them (ticket: blk_cnt[0])
   int ticket;                  // fused: glob_cnt index of this step's pending-observables tickets (2 or 3)
 };
 
@@ -126,6 +128,9 @@ struct NewtonArgs {
   int n, ntasks;
 };
 cudaError_t newton_setup(int* ctas_per_sm);
+// The j sums are 10 KB a particle at 2^18 (2.7 GB) and grow with n; larger
+// boxes keep the stream-K kernel.
+constexpr int kNewtonMaxN = 1 << 18;
 constexpr int kNewtonWarps = 4;  // tasks of a CTA
 cudaError_t launch_newton(const NewtonArgs& a, cudaStream_t st);
 cudaError_t launch_newton_sum(const StateArgs& s, const NewtonArgs& a, int mode, cudaStream_t st);
@@ -137,6 +142,7 @@ struct RowPlan {
 };
 RowPlan plan_rows(int n, int sms);
 cudaError_t rows_setup();
+// MODE_FORCES_ONLY: forces of s.q alone (force4, pressure; no box, state or observables).
 cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, cudaStream_t st);
 // parts: CTAs (row step) or tiles whose sums of tv^2 make chi
 cudaError_t launch_rows_close(const StateArgs& s, int n, int parts, cudaStream_t st);

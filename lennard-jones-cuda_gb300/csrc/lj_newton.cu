@@ -207,13 +207,13 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
   __shared__ double red[5];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = warp % 5, u = warp / 5;
   const int n = a.n, t = blockIdx.x, i = t * 32 + lane;
-  if (t == (n + 31) / 32) {
+  if (MODE != MODE_FORCES_ONLY && t == (n + 31) / 32) {
     extern __shared__ double shd[];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     pending_observables(s, 0, 1, shd);
     return;
   }
-  const BoxArgs box = s.boxes[0];
+  const BoxArgs box = MODE == MODE_FORCES_ONLY ? BoxArgs{} : s.boxes[0];
   const int tb = t / kI, first = a.block_part[2 * tb], count = a.block_part[2 * tb + 1];
   const float* jp = a.jpart + ((size_t)kI * ((size_t)tb * (tb + 1) / 2) + (size_t)(t - tb * kI) * (tb + 1)) * 160 + c * 32 + lane;
   const float* ip = a.ipart + (size_t)first * 5 * kNewtonBlock + c * kNewtonBlock + (t - tb * kI) * 32 + lane;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
   const bool mine = u == 0 && i < n;
   const size_t k3 = (size_t)min(c, 2) * s.npad + min(i, n - 1);
   double x = 0.0, v = 0.0, fn = 0.0;
-  if (mine && c < 3) {
+  if (MODE != MODE_FORCES_ONLY && mine && c < 3) {
     x = s.x[k3];
     v = s.v[k3];
     fn = s.f[k3];
@@ -262,11 +262,17 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
       s.v[k3] = v;
       predict_coord(s, sc, box, c, i, drift_pos(box, x, v, F));
       p0 = v * v;
-    } else {
+    } else if (MODE == MODE_TVN) {
       const double tv = fma(box.qdt, fn + F, v);
       s.tf[k3] = F;
       p0 = tv * tv;
+    } else {
+      reinterpret_cast<float*>(s.force4 + i)[c] = (float)F;
     }
+  } else if (MODE == MODE_FORCES_ONLY && mine && c == 3) {
+    const double A = value(3), B = value(4);
+    s.force4[i].w = (float)(A - B);
+    p0 = fma(12.0, A, -6.0 * B);
   } else if (mine && c == 3) {
     const double A = value(3), B = value(4);
     p0 = box.eps4 * (A - B);
@@ -283,6 +289,10 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
     }
   }
   __syncthreads();
+  if (MODE == MODE_FORCES_ONLY) {
+    forces_only_finish(s, red[3]);
+    return;
+  }
   if (threadIdx.x != 0) return;
   double* const o = s.row_part + (size_t)t * 8;
   if (MODE == MODE_EVN) {
@@ -311,8 +321,11 @@ cudaError_t launch_newton(const NewtonArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_newton_sum(const StateArgs& s, const NewtonArgs& a, int mode, cudaStream_t st) {
-  return launch_dependent(mode == MODE_EVN ? k_newton_sum<MODE_EVN> : k_newton_sum<MODE_TVN>, (a.n + 31) / 32 + 1,
-                          160 * kSum, sizeof(double) * 3 * 32, st, s, a);
+  auto* k = mode == MODE_EVN   ? k_newton_sum<MODE_EVN>
+            : mode == MODE_TVN ? k_newton_sum<MODE_TVN>
+                               : k_newton_sum<MODE_FORCES_ONLY>;
+  return launch_dependent(k, (a.n + 31) / 32 + (mode == MODE_FORCES_ONLY ? 0 : 1), 160 * kSum, sizeof(double) * 3 * 32,
+                          st, s, a);
 }
 
 }  // namespace ljgb

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   int4* const sq = reinterpret_cast<int4*>(smem_raw);              // all n records
   float* const part = reinterpret_cast<float*>(smem_raw + sizeof(int4) * (size_t)n);
 
-  if ((int)blockIdx.x == ctas) {
+  if (MODE != MODE_FORCES_ONLY && (int)blockIdx.x == ctas) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (MODE == MODE_EVN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     pending_observables(s, 0, 1, reinterpret_cast<double*>(smem_raw));
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
     fence_mbar_init();
   }
   for (int k = tid; k < slots * 10; k += kRowThreads) part[k] = 0.0f;
-  const BoxArgs box = s.boxes[0];
+  const BoxArgs box = MODE == MODE_FORCES_ONLY ? BoxArgs{} : s.boxes[0];
   __syncthreads();
   // What the previous step's kernels write is read from here on.
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   const bool mine = c < 4 && r < nr;
   const size_t k3 = (size_t)min(c, 2) * s.npad + i0 + min(r, nr - 1);
   double x = 0.0, v = 0.0, fn = 0.0;
-  if (mine && c < 3) {
+  if (MODE != MODE_FORCES_ONLY && mine && c < 3) {
     x = s.x[k3];
     v = s.v[k3];
     fn = s.f[k3];
@@ -211,11 +211,17 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
         s.v[k3] = v;
         predict_coord(s, sc, box, c, i0 + r, drift_pos(box, x, v, F));
         p0 = v * v;
-      } else {
+      } else if (MODE == MODE_TVN) {
         const double tv = fma(box.qdt, fn + F, v);
         s.tf[k3] = F;
         p0 = tv * tv;
+      } else {
+        reinterpret_cast<float*>(s.force4 + i0 + r)[c] = (float)F;
       }
+    } else if (MODE == MODE_FORCES_ONLY) {
+      const double A = row_sum(3), B = row_sum(4);
+      s.force4[i0 + r].w = (float)(A - B);
+      p0 = fma(12.0, A, -6.0 * B);
     } else {
       const double A = row_sum(3), B = row_sum(4);
       p0 = box.eps4 * (A - B);
@@ -226,7 +232,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   }
   if (c < 4) {  // whole warps
     const int wi = r / 32;
-    if (MODE == MODE_EVN || c < 3) p0 = warp_sum(p0);
+    if (MODE == MODE_EVN || (MODE == MODE_TVN) == (c < 3)) p0 = warp_sum(p0);
     if (MODE == MODE_EVN && c == 3) p1 = warp_sum(p1);
     if (lane == 0) {
       red[c][wi] = p0;
@@ -235,7 +241,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
     }
   }
   __syncthreads();
-  if (w == 0 && lane < 3) {
+  if (MODE == MODE_FORCES_ONLY) {
+    forces_only_finish(s, red[3][0] + red[3][1]);
+  } else if (w == 0 && lane < 3) {
     auto both = [&](int k) { return red[k][0] + red[k][1]; };
     double* const o = s.row_part + (size_t)blockIdx.x * 8;
     if (MODE == MODE_EVN) {
@@ -332,12 +340,15 @@ cudaError_t rows_setup() {
   constexpr int kMost = sizeof(int4) * kNewtonMinN + sizeof(float) * 10 * (kRowWarps + kMaxRows / 2);
   cudaError_t e = cudaFuncSetAttribute(k_rows<MODE_EVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows<MODE_TVN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_rows<MODE_FORCES_ONLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   return e;
 }
 
 cudaError_t launch_rows(const StateArgs& s, const RowPlan& p, int n, int mode, cudaStream_t st) {
-  return launch_dependent(mode == MODE_EVN ? k_rows<MODE_EVN> : k_rows<MODE_TVN>, p.ctas + 1, kRowThreads, p.smem, st,
-                          s, n, p.rows, p.ctas);
+  auto* k = mode == MODE_EVN ? k_rows<MODE_EVN> : mode == MODE_TVN ? k_rows<MODE_TVN> : k_rows<MODE_FORCES_ONLY>;
+  return launch_dependent(k, p.ctas + (mode == MODE_FORCES_ONLY ? 0 : 1), kRowThreads, p.smem, st, s, n, p.rows,
+                          p.ctas);
 }
 
 cudaError_t launch_rows_close(const StateArgs& s, int n, int parts, cudaStream_t st) {

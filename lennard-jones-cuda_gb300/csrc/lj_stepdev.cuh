@@ -351,4 +351,26 @@ __device__ __noinline__ void fused_block_step(const StateArgs& s, int B, double*
   }
 }
 
+// End of a MODE_FORCES_ONLY kernel: the CTA's share of sum_i sum_j s r^2 (in
+// thread 0) into row_part; the last CTA adds them: pressure = (4/6) of the sum
+// (MDSystem.cu:105-108, 136).  Block-wide call.
+__device__ __forceinline__ void forces_only_finish(const StateArgs& s, double share) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    s.row_part[(size_t)blockIdx.x * 8] = share;
+    __threadfence();
+    last = atomicAdd(s.blk_cnt, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  double sum = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) sum += __ldcg(s.row_part + (size_t)b * 8);
+  sum = warp_sum(sum);
+  if (threadIdx.x == 0) {
+    *s.pressure = (float)(sum * 4.0 / 6.0);
+    s.blk_cnt[0] = 0;
+  }
+}
+
 }  // namespace ljgb

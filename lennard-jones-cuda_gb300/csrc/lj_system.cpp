@@ -70,9 +70,6 @@ thread_local std::string g_create_error;
 // weight ragged tiles in the stream-K split.
 constexpr int kTileOverhead = 8;
 constexpr int kMaxSegmentsPerBlock = 8;
-// The unordered-pair step's j sums are 10 KB a particle at N = 2^18 (2.7 GB)
-// and grow with N; larger boxes keep the stream-K kernel.
-constexpr int kNewtonMaxN = 1 << 18;
 
 // Owned device array.  Movable, not copyable; freed on destruction (or
 // explicitly).
