@@ -504,70 +504,66 @@ __device__ __forceinline__ bool ge_nonneg(double d, double e) {
   return __double_as_longlong(d) >= __double_as_longlong(e);
 }
 
+// Number of the nalpha ascending sides that are <= d (d >= 0), by bisection.
+__device__ __forceinline__ int sides_within(const CounterDev& cd, double d) {
+  int lo = 0, hi = cd.nalpha;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ge_nonneg(d, cd.tl[mid])) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // One launch per step, graph-capturable (everything that changes per step
 // lives in st, the kCtr* words).  Whether the step is counted (every
 // `every`-th step) is read at the start by every CTA; st is written only by
 // the last CTA to finish, after every CTA has taken its ticket.  A counted
-// step: each CTA histograms its particles in shared memory and writes its
-// counts to part[block][bin]; the last CTA sums the blocks' counts into the
-// step's ring row (written whole: no clearing pass) and advances the row.
-__global__ void k_counters(StateArgs s, const CounterDev* cs, int nc, int nbins, int* st, int* ring, int* part,
-                           int n) {
-  extern __shared__ int shc[];
+// step: a thread per particle and a grid row per counter, counts collected per
+// CTA in shared memory and added to the step's ring row, which was zero; the
+// last CTA clears the next row (the ring has one more than the host reads) and
+// advances to it.  Bound by its chain of dependent loads and FP64 divides.  (A
+// thread per particle walking through all counters, n / 256 CTAs, and the last
+// CTA adding the others' rows: 12 us at N = 512 with five counters; so 6.)
+__global__ void k_counters(StateArgs s, const CounterDev* cs, int nbins, int* st, int* ring, int n) {
+  __shared__ int shc[kMaxCounterAlphas];
   __shared__ bool last;
-  const int phase = st[kCtrPhase] + 1;
+  const int phase = st[kCtrPhase] + 1, row = st[kCtrNext];
   const bool counted = phase >= st[kCtrEvery];
   if (counted) {
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) shc[b] = 0;
+    const CounterDev& cd = cs[blockIdx.y];
+    for (int b = threadIdx.x; b < cd.nalpha; b += blockDim.x) shc[b] = 0;
     __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
       const double L = s.boxes[0].L;
-      double x[3], v[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        x[c] = s.x[(size_t)c * s.npad + i];
-        v[c] = s.v[(size_t)c * s.npad + i];
+      int k;
+      if (cd.type < 3) {
+        k = bin_trunc_div2(s.x[(size_t)cd.type * s.npad + i], L, cd.alpha_step, cd.inv_bc);
+      } else if (cd.type == 3) {
+        k = 0;
+        for (int c = 0; c < 3; ++c)  // (* 2 is / 0.5, exactly)
+          k = max(k, sides_within(cd, fabs(s.x[(size_t)c * s.npad + i] - 0.5 * L) * 2.0));
+      } else {
+        k = bin_trunc_div2(fabs(s.v[(size_t)(cd.type - 4) * s.npad + i]), cd.vmax, cd.alpha_step, cd.inv_bc);
       }
-      for (int q = 0; q < nc; ++q) {
-        const CounterDev& cd = cs[q];
-        int k;
-        if (cd.type < 3) {
-          k = bin_trunc_div2(x[cd.type], L, cd.alpha_step, cd.inv_bc);
-        } else if (cd.type == 3) {
-          k = 0;
-          for (int c = 0; c < 3; ++c) {
-            const double d = fabs(x[c] - 0.5 * L) * 2.0;  // = / 0.5, exactly
-            int kc = 0;
-            while (kc < cd.nalpha && ge_nonneg(d, cd.tl[kc])) ++kc;
-            k = kc > k ? kc : k;
-          }
-        } else {
-          k = bin_trunc_div2(fabs(v[cd.type - 4]), cd.vmax, cd.alpha_step, cd.inv_bc);
-        }
-        if (k >= 0 && k < cd.nalpha) atomicAdd(&shc[cd.bin0 + k], 1);
-      }
+      if (k >= 0 && k < cd.nalpha) atomicAdd(&shc[k], 1);
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) part[(size_t)blockIdx.x * nbins + b] = shc[b];
+    for (int b = threadIdx.x; b < cd.nalpha; b += blockDim.x)
+      if (shc[b]) atomicAdd(ring + (size_t)row * nbins + cd.bin0 + b, shc[b]);
   }
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&st[kCtrTicket], 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&st[kCtrTicket], 1) == (int)(gridDim.x * gridDim.y) - 1;
   __syncthreads();
   if (!last) return;
-  __threadfence();
-  const int row = st[kCtrNext];
+  const int next = counted ? (row == st[kCtrCap] ? 0 : row + 1) : row;
   if (counted)
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
-      int sum = 0;
-      for (int k = 0; k < (int)gridDim.x; ++k) sum += __ldcg(part + (size_t)k * nbins + b);
-      ring[(size_t)row * nbins + b] = sum;
-    }
+    for (int b = threadIdx.x; b < nbins; b += blockDim.x) ring[(size_t)next * nbins + b] = 0;
   if (threadIdx.x == 0) {
     st[kCtrTicket] = 0;
     st[kCtrPhase] = counted ? 0 : phase;
-    if (counted) st[kCtrNext] = row + 1 == st[kCtrCap] ? 0 : row + 1;
+    st[kCtrNext] = next;
   }
 }
 
@@ -868,11 +864,9 @@ cudaError_t launch_predict(const StateArgs& s, int nblocks, int bi, cudaStream_t
   return cudaGetLastError();
 }
 
-int counters_blocks(int n) { return (n + 255) / 256; }
-
-cudaError_t launch_counters(const StateArgs& s, const CounterDev* cs, int nc, int nbins, int* state, int* ring,
-                            int* part, int n, cudaStream_t st) {
-  k_counters<<<counters_blocks(n), 256, sizeof(int) * nbins, st>>>(s, cs, nc, nbins, state, ring, part, n);
+cudaError_t launch_counters(const StateArgs& s, const CounterDev* cs, int nc, int nbins, int* state, int* ring, int n,
+                            cudaStream_t st) {
+  k_counters<<<dim3((unsigned)(n + 127) / 128, nc), 128, 0, st>>>(s, cs, nbins, state, ring, n);
   return cudaGetLastError();
 }
 

@@ -210,12 +210,10 @@ struct CounterDev {
 enum : int { kCtrNext = 0, kCtrPhase = 1, kCtrEvery = 2, kCtrCap = 3, kCtrTicket = 4, kCtrWords = 8 };
 // One step of the counters in one launch (graph-capturable: everything that
 // changes per step lives in `state`): the histogram of the counters' bin
-// indices over the particles of box 0, per CTA into part (counters_blocks(n)
-// x nbins ints), summed by the last CTA into the step's ring row when the
-// step is counted.
-int counters_blocks(int n);
-cudaError_t launch_counters(const StateArgs& s, const CounterDev* cs, int nc, int nbins, int* state, int* ring,
-                            int* part, int n, cudaStream_t st);
+// indices over the particles of box 0 into the step's ring row when the step
+// is counted.  Row kCtrNext is zero before the launch.
+cudaError_t launch_counters(const StateArgs& s, const CounterDev* cs, int nc, int nbins, int* state, int* ring, int n,
+                            cudaStream_t st);
 cudaError_t launch_unpack(const double* in, double* out, int n, int npad, cudaStream_t st);
 cudaError_t launch_selftest_wait(int* status, cudaStream_t st);
 // Up to three (N,3) interleaved <-> component-major [3][npad] transposes in one launch.

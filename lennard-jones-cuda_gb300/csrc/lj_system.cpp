@@ -264,12 +264,12 @@ struct lj_system {
   int rec_cap = 0;
 
   // per-step subsystem counters (lj_counters_configure): one row of
-  // counter_bins ints per step in a ring of counter_cap rows
+  // counter_bins ints per step in a ring of counter_cap + 1 rows (the spare one
+  // is the next step's, kept at zero)
   std::vector<CounterDev> counters;
   DevBuf<CounterDev> dcounters;
   DevBuf<int> counter_ring;
   DevBuf<int> counter_state;     // kCtr* words: the device's copy of the bookkeeping below
-  DevBuf<int> counter_part;      // per-CTA counts of the counting launch
   int counter_bins = 0, counter_cap = 0;
   int counter_every = 1;         // count after every counter_every-th step
   long long counter_phase = 0;   // steps since the last counted one
@@ -867,7 +867,7 @@ lj_status flush_observables(lj_system* s) {
 lj_status enqueue_after_step(lj_system* s, const RdfPass& rdf, int* kernels) {
   if (s->counter_cap > 0) {
     LJ_CUDA(s, launch_counters(state_args(s), s->dcounters.p, (int)s->counters.size(), s->counter_bins,
-                               s->counter_state.p, s->counter_ring.p, s->counter_part.p, s->ntotal, s->stream));
+                               s->counter_state.p, s->counter_ring.p, s->ntotal, s->stream));
     *kernels += 1;
   }
   if (s->rdf_acc) {
@@ -1235,7 +1235,6 @@ lj_status lj_destroy(lj_system* s) {
   s->dcounters.free();
   s->counter_ring.free();
   s->counter_state.free();
-  s->counter_part.free();
   s->rdf_sum.free();
   s->qhist.free();
   s->h_cta_block.free();
@@ -1882,15 +1881,15 @@ lj_status lj_counters_configure(lj_system* s, const lj_counter* counters, int32_
   words[kCtrNext] = 0;
   words[kCtrPhase] = 0;
   words[kCtrEvery] = s->counter_every;
-  words[kCtrCap] = ring_steps;
+  words[kCtrCap] = ring_steps;  // the last row's index: one spare row
   words[kCtrTicket] = 0;
   cudaError_t e = s->dcounters.alloc(s->counters.size());
-  if (e == cudaSuccess) e = s->counter_ring.alloc((size_t)bins * ring_steps);
+  if (e == cudaSuccess) e = s->counter_ring.alloc((size_t)bins * ((size_t)ring_steps + 1));
   if (e == cudaSuccess) e = s->counter_state.alloc(kCtrWords);
-  if (e == cudaSuccess) e = s->counter_part.alloc((size_t)counters_blocks(s->ntotal) * bins);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->dcounters.p, s->counters.data(), sizeof(CounterDev) * s->counters.size(),
                         cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->counter_ring.p, 0, sizeof(int) * bins, s->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->counter_state.p, words, sizeof(words), cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -1900,7 +1899,6 @@ lj_status lj_counters_configure(lj_system* s, const lj_counter* counters, int32_
     s->dcounters.free();
     s->counter_ring.free();
     s->counter_state.free();
-    s->counter_part.free();
   }
   LJ_CUDA(s, e);
   s->counter_cap = ring_steps;
@@ -1942,8 +1940,8 @@ lj_status lj_counters_read(lj_system* s, int32_t* counts, int32_t max_steps, int
   const int B = s->counter_bins;
   // the rows are contiguous in the ring up to its end, then from its start
   for (int k = 0; k < n;) {
-    const long long row = (s->counter_tail + k) % s->counter_cap;
-    const int run = (int)std::min<long long>(n - k, s->counter_cap - row);
+    const long long rows = (long long)s->counter_cap + 1, row = (s->counter_tail + k) % rows;
+    const int run = (int)std::min<long long>(n - k, rows - row);
     LJ_CUDA(s, cudaMemcpyAsync(counts + (size_t)k * B, s->counter_ring.p + (size_t)row * B,
                                sizeof(int) * B * (size_t)run, cudaMemcpyDeviceToHost, s->stream));
     k += run;
