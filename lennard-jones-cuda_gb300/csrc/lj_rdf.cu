@@ -40,9 +40,18 @@ __device__ __forceinline__ float bin_pos(float x, float k2, float inv_w) {
 template <int MODE>
 __device__ float bin_bound(float k2, float inv_w, float limit) {
   int lo = 0, hi = 0x7f800000;
+  auto reaches = [&](int bits) { return bin_pos<MODE>(__int_as_float(bits), k2, inv_w) >= limit; };
+  // the real quotient is a few ulps away from it, unless a product over- or
+  // underflows: a few tests instead of 31, which every CTA would wait for
+  // (N = 16384, 256 linear bins: 121 us a call without, 113 with)
+  const int near = __float_as_int(MODE == 2 ? limit / k2 : limit / inv_w / k2);
+  if (near > 64 && near < 0x7f000000) {
+    if (reaches(near + 16)) hi = near + 16;
+    if (!reaches(near - 16)) lo = near - 16;
+  }
   while (lo < hi) {
     const int mid = lo + (hi - lo) / 2;
-    if (bin_pos<MODE>(__int_as_float(mid), k2, inv_w) >= limit) hi = mid;
+    if (reaches(mid)) hi = mid;
     else lo = mid + 1;
   }
   return __int_as_float(lo);
@@ -72,7 +81,8 @@ __device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float bou
 // issue (no memory traffic: the shadow stays in L2): 11 instructions for a pair
 // past the bound, which most are.  N = 16384, 256 clamped bins, us a call: 234
 // over ordered pairs, 131 over unordered ones, 119 with the bound in place of
-// the products and a counter.  A CTA owns a contiguous range of (block, 32-j
+// the products and a counter, 113 with
+// bin_bound's bracket.  A CTA owns a contiguous range of (block, 32-j
 // chunk) units (build_rdf_ranges), flushing its shared histogram once: a grid
 // of single tiles would flush 256 bins thousands of times.
 template <int MODE>
