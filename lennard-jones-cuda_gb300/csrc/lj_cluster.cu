@@ -226,16 +226,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_cluster(StateArgs s, int n, int
     const double(*vel)[kCtaRows] = sh.vel[step & 1];
     const double vx = vel[0][lane], vy = vel[1][lane], vz = vel[2][lane];
     const FloatAcc a = sh.pot[step & 1][0][lane], b = sh.pot[step & 1][1][lane];
-    const double A = (double)a.hi + (double)a.lo, B = (double)b.hi + (double)b.lo;
+    const double A = widen(a.hi) + widen(a.lo), B = widen(b.hi) + widen(b.lo);
     e = box.eps4 * (A - B);
     vir = box.eps4 * fma(12.0, A, -6.0 * B);
-    const double K = warp_sum(fma(vx, vx, fma(vy, vy, vz * vz))), E = warp_sum(e), W = warp_sum(vir);
-    if (lane == 0) {
-      double* const to = cluster.map_shared_rank(sh.kvw[step & 1][rank], 0);
-      to[0] = K;
-      to[1] = E;
-      to[2] = W;
-    }
+    const double r = warp_sums<3>({fma(vx, vx, fma(vy, vy, vz * vz)), e, vir});
+    double* const to = cluster.map_shared_rank(sh.kvw[step & 1][rank], 0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (lane == sums_lane(k)) to[k] = r;
   };
   auto observe = [&](int step) {
     double kvw[3];
@@ -280,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cluster(StateArgs s, int n, int
     double F = 0.0;
     if (mine && w < 3) {
       const FloatAcc a = row_sum(w);
-      F = fscale * ((double)a.hi + (double)a.lo);
+      F = fscale * (widen(a.hi) + widen(a.lo));
     } else if (mine) {
       sh.pot[cur][0][lane] = row_sum(3);
       sh.pot[cur][1][lane] = row_sum(4);
@@ -315,11 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cluster(StateArgs s, int n, int
       apply_bc1(box.bc, box.L, x, v);
       const double xp = drift_pos(box, x, v, F);
       if (mine) {
-        if (box.bc == 1) {
-          const double u = (xp - origin) * invP;
-          if (!(u >= 0.0 && u < 0.4999)) atomicOr(s.status, LJ_DEVFLAG_ESCAPED);
-        }
-        const int qn = fixed_coord_scaled(box.bc == 0 ? xp : xp - origin, qscale);
+        const int qn = predicted_fixed(s, box.bc, origin, qscale, xp);
         reinterpret_cast<int*>(&sh.next[lane])[w] = qn;
         sh.vel[cur][w][lane] = v;
         if (step == nsteps - 1) reinterpret_cast<int*>(s.q + i0 + lane)[w] = qn;

@@ -28,20 +28,17 @@ namespace ljgb {
 // Cost: one FP64 multiply, one conversion and a few integer operations (FP64
 // runs at 1/64 of the FP32 rate on this part).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int32_t fixed_coord_scaled(double dx, double scale) {
-  const double t = dx * scale;
+__device__ __forceinline__ int32_t fixed_of_scaled(double t) {
   const uint32_t u = (uint32_t)(unsigned long long)llrint(t);
   const uint32_t r = u % 3u;
   const uint32_t q = r == 0u ? u : (r == 1u ? u - 1u : u + 1u);
   return (int32_t)q;
 }
 
+__device__ __forceinline__ int32_t fixed_coord_scaled(double dx, double scale) { return fixed_of_scaled(dx * scale); }
+
 __device__ __forceinline__ int32_t fixed_coord(double x, double origin, double invP) {
-  const double t = (x - origin) * (invP * 4294967296.0);
-  const uint32_t u = (uint32_t)(unsigned long long)llrint(t);
-  const uint32_t r = u % 3u;
-  const uint32_t q = r == 0u ? u : (r == 1u ? u - 1u : u + 1u);
-  return (int32_t)q;
+  return fixed_coord_scaled(x - origin, invP * 4294967296.0);
 }
 
 // Wrapping difference of two fixed-point coordinates (the minimum image).
@@ -159,6 +156,19 @@ __device__ __forceinline__ void two_sum_add(FloatAcc& a, float t) {
   a.lo = __fadd_rn(a.lo, e);
 }
 
+// (double)f with the exponent re-based by integer operations: exact like the
+// conversion, which takes the FP64 pipe for 16 cycles a warp (this: 2) and 80
+// cycles of latency (12).  Zeros keep their sign; subnormals, infinities and
+// NaN, which sums do not hold in a run that goes well, take the conversion.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu, sign = u & 0x80000000u;
+  if (m - 0x00800000u < 0x7f000000u || m == 0u)
+    return __hiloint2double((int)(sign | (m ? (m >> 3) + 0x38000000u : 0u)), (int)(u << 29));
+  double r;
+  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(r) : "f"(f));
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 reductions.
 // ---------------------------------------------------------------------------
@@ -168,6 +178,28 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Warp sums of two to four values at once: after the first exchange half the
+// lanes carry one value and half another, after the second a quarter each, so 5
+// to 7 FP64 additions (16 cycles each on an SM) take the place of 10 to 20.
+// Value k is returned in lane sums_lane(k).  Fixed order.
+__device__ __forceinline__ constexpr int sums_lane(int k) { return (k & 1) * 16 + (k >> 1) * 8; }
+template <int NV>
+__device__ __forceinline__ double warp_sums(const double (&v)[NV]) {
+  static_assert(NV >= 2 && NV <= 4, "two to four values");
+  const int lane = threadIdx.x & 31;
+  auto merge = [&](double a, double b, int bit) {  // a for the lanes with bit clear, b for the others
+    const bool hi = lane & bit;
+    return (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, bit);
+  };
+  double r = merge(v[0], v[1], 16);
+  if (NV == 2) r += __shfl_xor_sync(0xffffffffu, r, 8);
+  else if (NV == 3) r = merge(r, v[2 % NV] + __shfl_xor_sync(0xffffffffu, v[2 % NV], 16), 8);
+  else r = merge(r, merge(v[2 % NV], v[3 % NV], 16), 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
+}
+
 // Block-wide sum of NV doubles per thread, result valid in thread 0.
 // Fixed reduction order (warp tree, then warps in index order): the result
 // is independent of scheduling.  `sh` needs NV * 32 doubles.
@@ -175,11 +207,14 @@ template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nw = (blockDim.x + 31) >> 5;
+  if constexpr (NV == 1) {
+    v[0] = warp_sum(v[0]);
+    if (lane == 0) sh[warp] = v[0];
+  } else {
+    const double r = warp_sums(v);
 #pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = warp_sum(v[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh[k * 32 + warp] = v[k];
+    for (int k = 0; k < NV; ++k)
+      if (lane == sums_lane(k)) sh[k * 32 + warp] = r;
   }
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -342,9 +342,7 @@ __global__ void k_predict(StateArgs s) {
     const size_t k = (size_t)c * s.npad + p;
     xp[c] = drift_pos(box, s.x[k], s.v[k], s.f[k]);
   }
-  const DevScalars& sc = s.sc[bi.sys];
-  check_wall_frame(s, box.bc, sc, xp[0], xp[1], xp[2]);
-  s.q[p] = shadow_of(sc, xp[0], xp[1], xp[2]);
+  s.q[p] = predicted_shadow(s, s.sc[bi.sys], box.bc, xp);
 }
 
 // Close of a fused TVN step (MDSystem.cpp:469-506, :578-579).  The pair
@@ -358,6 +356,10 @@ __global__ void k_predict(StateArgs s) {
 // them in a CTA that has finished its pair work (pending_observables), or
 // the read-back launch / k_obs_finalize does before the host reads them.
 // This takes a serial last-CTA stage off the step's critical path.
+// Bound by the FP64 pipe (2 lanes a cycle on an SM): 36 instructions a warp of
+// a periodic box (49 before the sums shared their exchanges and chi's factors
+// were formed once a CTA), 40 of a walled one (64 before its frame test used
+// the bits): 256 boxes, 540,000 particles, 75 -> 58 us.
 __global__ void k_tvn_close(StateArgs s) {
   __shared__ double sh[3 * 32];
   // Launched as a programmatic dependent of the pair kernel: the CTAs start
@@ -395,7 +397,17 @@ __global__ void k_tvn_close(StateArgs s) {
   // block epilogues): every CTA of the box forms the same sum in the same
   // order (as k_tvn_finish does), so no CTA of the pair kernel has to wait
   // for the box's last block to compute it.
-  __shared__ double chi_sh, tkin_sh;
+  __shared__ double chi_sh, tkin_sh, a1_sh, b1h_sh;
+  auto set_chi = [&](double tv2) {  // one thread
+    double Tkin;
+    const double chi = tvn_chi(box, tv2, &Tkin);
+    chi_sh = chi;
+    tkin_sh = Tkin;
+    // chi dt tF with tF = (F_n + F_{n+1}) / 2 formed as (chi dt / 2)(F_n + F_{n+1}):
+    // the same bits (the halvings are exact), one FP64 operation fewer
+    a1_sh = 2. * chi - 1.;
+    b1h_sh = 0.5 * (chi * box.dt);
+  };
   if (b1 - b0 <= 32) {
     // Boxes of at most 32 blocks (batches of small boxes): warp 0 alone.
     // box_sum would give every block value to one thread of warp 0 and zeros
@@ -405,26 +417,15 @@ __global__ void k_tvn_close(StateArgs s) {
     if (tid < 32) {
       double v = b0 + tid < b1 ? __ldcg(s.blk_part + (size_t)(b0 + tid) * 8 + 3) : 0.0;
       v = warp_sum(v);
-      if (tid == 0) {
-        double Tkin;
-        chi_sh = tvn_chi(box, 0.0 + v, &Tkin);
-        tkin_sh = Tkin;
-      }
+      if (tid == 0) set_chi(0.0 + v);
     }
     __syncthreads();
   } else {
     const double tv2 = box_sum(s, b0, b1, 3, sh);
-    if (tid == 0) {
-      double Tkin;
-      chi_sh = tvn_chi(box, tv2, &Tkin);
-      tkin_sh = Tkin;
-    }
+    if (tid == 0) set_chi(tv2);
     __syncthreads();
   }
-  const double chi = chi_sh;
-  // chi dt tF with tF = (F_n + F_{n+1}) / 2 formed as (chi dt / 2)(F_n + F_{n+1}):
-  // the same bits (the halvings are exact), one FP64 operation fewer
-  const double a1 = 2. * chi - 1., b1h = 0.5 * (chi * box.dt);
+  const double a1 = a1_sh, b1h = b1h_sh;
   double part[3] = {0.0, 0.0, 0.0};
   if (valid) {
     double x[3], v[3];
@@ -443,8 +444,7 @@ __global__ void k_tvn_close(StateArgs s) {
       s.f[k] = f1[c];
       xp[c] = drift_pos(box, x[c], v[c], f1[c]);
     }
-    check_wall_frame(s, box.bc, sc, xp[0], xp[1], xp[2]);
-    s.q_next[p] = shadow_of_bc(sc, box.bc, xp[0], xp[1], xp[2]);
+    s.q_next[p] = predicted_shadow(s, sc, box.bc, xp);
     part[0] = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));  // K and V shares, halved once per block below
     part[1] = ep;
     part[2] = wp;
@@ -461,7 +461,7 @@ __global__ void k_tvn_close(StateArgs s) {
       const int par = s.ticket - 2;  // this step's parity
       sc.Tkin = tkin_sh;
       sc.Tkin_rec[par] = tkin_sh;
-      sc.chi = chi;
+      sc.chi = chi_sh;
       sc.obs_slot[par] = s.obs_slot;
       sc.obs_nblk[par] = 0;
       sc.obs_pending[par] = MODE_TVN;

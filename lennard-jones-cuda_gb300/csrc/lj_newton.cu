@@ -197,12 +197,13 @@ __global__ void __launch_bounds__(32 * kWarps, 3) k_newton(NewtonArgs a) {
 // One tile of 32 particles: its parts added in FP32 TwoSum (value c by kSum
 // warps, every kSum-th part each; fixed order), then the step's second half
 // with a thread per particle and component, as in k_rows.  One more CTA forms
-// the observables the previous step left pending.
+// the observables the previous step left pending.  4 CTAs an SM: N = 16384
+// fits into one wave (12.0 us; at 60 registers and 3 an SM 15.8).
 namespace {
 constexpr int kSum = 2;
 }
 template <int MODE>
-__global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonArgs a) {
+__global__ void __launch_bounds__(160 * kSum, 4) k_newton_sum(StateArgs s, NewtonArgs a) {
   __shared__ FloatAcc part[kSum][5][32];
   __shared__ double red[5];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = warp % 5, u = warp / 5;
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
       two_sum_add(r, part[m][k][lane].hi);
       r.lo += part[m][k][lane].lo;
     }
-    return (double)r.hi + (double)r.lo;
+    return widen(r.hi) + widen(r.lo);
   };
   DevScalars& sc = s.sc[0];
   double p0 = 0.0, p1 = 0.0;
@@ -280,13 +281,13 @@ __global__ void __launch_bounds__(160 * kSum) k_newton_sum(StateArgs s, NewtonAr
     s.e[i] = p0;
     s.w[i] = p1;
   }
-  if (u == 0 && c < 4) {
+  if (u == 0 && c < 3) {
     p0 = warp_sum(p0);
     if (lane == 0) red[c] = p0;
-    if (c == 3) {
-      p1 = warp_sum(p1);
-      if (lane == 0) red[4] = p1;
-    }
+  } else if (u == 0 && c == 3) {
+    const double r = warp_sums<2>({p0, p1});
+    if (lane == sums_lane(0)) red[3] = r;
+    if (lane == sums_lane(1)) red[4] = r;
   }
   __syncthreads();
   if (MODE == MODE_FORCES_ONLY) {

@@ -222,12 +222,9 @@ __global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair6
       s.e[at] = e;
       s.w[at] = w;
     }
-    e = warp_sum(e);
-    w = warp_sum(w);
-    if (lane == 0) {
-      s.blk_part[(size_t)B * 8 + 1] = 0.5 * e;
-      s.blk_part[(size_t)B * 8 + 2] = w;
-    }
+    const double r = warp_sums<2>({e, w});
+    if (lane == sums_lane(0)) s.blk_part[(size_t)B * 8 + 1] = 0.5 * r;
+    if (lane == sums_lane(1)) s.blk_part[(size_t)B * 8 + 2] = r;
   }
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
     const int g = r >> 1, w1 = warp_of_unit((g + 1) * C - 1, U);
     const float* p = part + g * 10 + (r & 1) * 5 + k;
     for (int ww = warp_of_unit(g * C, U); ww <= w1; ++ww) two_sum_add(a, p[ww * 10]);
-    return (double)a.hi + (double)a.lo;
+    return widen(a.hi) + widen(a.lo);
   };
   double p0 = 0.0, p1 = 0.0;  // c < 3: v^2 (EVN) or tv^2; c = 3: e, w
   if (mine) {
@@ -232,8 +232,12 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
   }
   if (c < 4) {  // whole warps
     const int wi = r / 32;
-    if (MODE == MODE_EVN || (MODE == MODE_TVN) == (c < 3)) p0 = warp_sum(p0);
-    if (MODE == MODE_EVN && c == 3) p1 = warp_sum(p1);
+    if (MODE == MODE_EVN && c == 3) {
+      p0 = warp_sums<2>({p0, p1});
+      p1 = __shfl_sync(0xffffffffu, p0, sums_lane(1));
+    } else if (MODE == MODE_EVN || (MODE == MODE_TVN) == (c < 3)) {
+      p0 = warp_sum(p0);
+    }
     if (lane == 0) {
       red[c][wi] = p0;
       if (c == 3) red[4][wi] = p1;
@@ -277,19 +281,14 @@ __global__ void __launch_bounds__(128) k_rows_close(StateArgs s, int n, int ctas
   } else {
     double tv2 = 0.0;
     for (int b = lane; b < ctas; b += 32) tv2 += __ldcg(s.row_part + (size_t)b * 8 + 3);
-    double e = valid ? s.e[i] : 0.0, ww = valid ? s.w[i] : 0.0;
-    tv2 = warp_sum(tv2);
+    const double r = warp_sums<3>({tv2, valid ? s.e[i] : 0.0, valid ? s.w[i] : 0.0});
     if (lane == 0) {
       double Tkin;
-      chi_sh = tvn_chi(box, tv2, &Tkin);
+      chi_sh = tvn_chi(box, r, &Tkin);
       tkin_sh = Tkin;
     }
-    e = warp_sum(e);
-    ww = warp_sum(ww);
-    if (lane == 0) {
-      vw[0] = e;
-      vw[1] = ww;
-    }
+    if (lane == sums_lane(1)) vw[0] = r;
+    if (lane == sums_lane(2)) vw[1] = r;
   }
   __syncthreads();
   if (c < 3) {

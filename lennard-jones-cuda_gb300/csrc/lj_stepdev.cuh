@@ -78,26 +78,32 @@ __device__ __forceinline__ int4 shadow_of(const DevScalars& sc, double x, double
                    fixed_coord(z, sc.origin[2], sc.invP), 0);
 }
 
-// shadow_of for a box of boundary bc with the frame scale formed once; a
-// periodic box's frame has origin 0, so its subtraction is skipped (x - 0 is
-// x exactly): the same bits as shadow_of.
-__device__ __forceinline__ int4 shadow_of_bc(const DevScalars& sc, int bc, double x, double y, double z) {
-  const double scale = sc.invP * 4294967296.0;
-  if (bc == 0) return make_int4(fixed_coord_scaled(x, scale), fixed_coord_scaled(y, scale), fixed_coord_scaled(z, scale), 0);
-  return make_int4(fixed_coord_scaled(x - sc.origin[0], scale), fixed_coord_scaled(y - sc.origin[1], scale),
-                   fixed_coord_scaled(z - sc.origin[2], scale), 0);
+// Fixed-point coordinate of component c in the box's frame, with the test of
+// check_wall_frame: the scaled offset is that test's u times 2^32 exactly, and
+// is compared on its bits (positive order; a NaN is flagged in both forms).  A
+// periodic box's frame has origin 0, so its subtraction is skipped (x - 0 is x
+// exactly).
+__device__ __forceinline__ int predicted_fixed(const StateArgs& s, int bc, double origin, double scale, double x) {
+  const double t = (bc == 0 ? x : x - origin) * scale;
+  if (bc == 1) {
+    const long long hi = __double_as_longlong(0.4999 * 4294967296.0);
+    if (neg_bits(t) || __double_as_longlong(t) >= hi) atomicOr(s.status, LJ_DEVFLAG_ESCAPED);
+  }
+  return fixed_of_scaled(t);
 }
+__device__ __forceinline__ double frame_scale(const DevScalars& sc) { return sc.invP * 4294967296.0; }
 
-// check_wall_frame and shadow_of_bc for component c of particle p alone.
+// Component c of particle p of the next step's shadow, from its predicted x.
 __device__ __forceinline__ void predict_coord(const StateArgs& s, const DevScalars& sc, const BoxArgs& box, int c,
                                               int p, double x) {
-  const double o = box.bc == 0 ? 0.0 : sc.origin[c];
-  if (box.bc == 1) {
-    const double u = (x - o) * sc.invP;
-    if (!(u >= 0.0 && u < 0.4999)) atomicOr(s.status, LJ_DEVFLAG_ESCAPED);
-  }
-  const double scale = sc.invP * 4294967296.0;
-  reinterpret_cast<int*>(s.q_next + p)[c] = fixed_coord_scaled(box.bc == 0 ? x : x - o, scale);
+  reinterpret_cast<int*>(s.q_next + p)[c] = predicted_fixed(s, box.bc, sc.origin[c], frame_scale(sc), x);
+}
+
+// The particle's whole record.
+__device__ __forceinline__ int4 predicted_shadow(const StateArgs& s, const DevScalars& sc, int bc, const double (&x)[3]) {
+  const double scale = frame_scale(sc);
+  return make_int4(predicted_fixed(s, bc, sc.origin[0], scale, x[0]), predicted_fixed(s, bc, sc.origin[1], scale, x[1]),
+                   predicted_fixed(s, bc, sc.origin[2], scale, x[2]), 0);
 }
 
 // Sum of blk_part[b][slot] over the blocks of one box, fixed order, valid in
@@ -258,7 +264,7 @@ __device__ __forceinline__ void segment_sums(const StateArgs& s, const BlockInfo
     for (int c = 0; c < 5; ++c) two_sum_add(acc[c], __ldcg(s.partial + base + (size_t)c * s.bi_threads));
   }
 #pragma unroll
-  for (int c = 0; c < 5; ++c) S[c] = (double)acc[c].hi + (double)acc[c].lo;
+  for (int c = 0; c < 5; ++c) S[c] = widen(acc[c].hi) + widen(acc[c].lo);
 }
 
 // Fused second half of a step for block B, run by the CTA that wrote the last
@@ -319,8 +325,7 @@ __device__ __noinline__ void fused_block_step(const StateArgs& s, int B, double*
         xp[c] = drift_pos(box, x, v, Fn1[c]);
         vv = fma(v, v, vv);
       }
-      check_wall_frame(s, box.bc, sc, xp[0], xp[1], xp[2]);
-      s.q_next[p] = shadow_of_bc(sc, box.bc, xp[0], xp[1], xp[2]);
+      s.q_next[p] = predicted_shadow(s, sc, box.bc, xp);
       part[0] = vv;  // K and V shares, halved once per block below
       part[1] = e;
       part[2] = w;
