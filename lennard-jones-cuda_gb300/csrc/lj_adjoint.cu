@@ -54,8 +54,8 @@ struct AdjBox {
 // The pair pass's work split (Pair64Plan of one box) and sums.
 struct AdjPass {
   const Pair64Task* tasks;
-  int ntasks, tiles, groups, group, parts;
-  double* part;  // [tile][groups + 1][3][32]: F (forward), or dl/dx + H z
+  int ntasks, tiles, groups, group, parts, split, turns;  // turns = 32 / split
+  double* part;  // [tile][(groups + 1) split][3][32]: F (forward), or dl/dx + H z
   double* scal;  // [task][kScalars]
 };
 
@@ -89,6 +89,7 @@ __device__ __forceinline__ int adj_turns(const AdjBox& b, const double* x, const
     xj[c] = x[(size_t)c * b.npad + j];
     if (HVP) zj[c] = z[(size_t)c * b.npad + j];
   }
+  __builtin_assume((r1 - r0) % 2 == 0);  // Pair64Plan::parts sees to it
 #pragma unroll 2
   for (int r = r0; r < r1; ++r) {
     double d[3] = {xi[0] - xj[0], xi[1] - xj[1], xi[2] - xj[2]};
@@ -159,10 +160,9 @@ __device__ __forceinline__ void store_adj(double* to, int at, const AdjSums& s) 
 // One task: a square of tiles by one warp, or of one tile by `parts` warps.
 template <bool HVP, bool UNIT>
 __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, const double* x, const double* z,
-                                         double cF, double cA, double* sh) {
+                                         double cF, double cA, const Pair64Task tk, double* sh) {
   const int lane = threadIdx.x & 31;
-  const Pair64Task tk = a.tasks[blockIdx.x];
-  const int slots = a.groups + 1;
+  const int slots = (a.groups + 1) * a.split;
   constexpr int kS = HVP ? kScalars : 2;
   double S[kScalars] = {0.0, 0.0, 0.0, 0.0, 0.0};
   auto load = [&](const double* from, int t, double (&to)[3]) {
@@ -173,7 +173,8 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
   double xi[3], zi[3] = {0.0, 0.0, 0.0};
   if (a.parts > 1) {
     const int w = threadIdx.x >> 5, ta = tk.ga, tb = tk.gb;
-    const int first = ta == tb ? 1 : 0, turns = (ta == tb ? 16 : 32) / a.parts;
+    const int turns = (ta == tb ? min(16, a.turns) : a.turns) / a.parts;
+    const int first = (ta == tb ? 1 : 0) + a.turns * tk.slot;
     load(x, ta, xi);
     if (HVP) load(z, ta, zi);
     AdjSums I{}, J{};
@@ -191,8 +192,8 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
     for (int k = threadIdx.x; k < 192 + kS; k += blockDim.x) {
       double v = 0.0;
       for (int p = 0; p < a.parts; ++p) v += sh[p * (192 + kScalars) + k];
-      if (k < 96) a.part[((size_t)ta * slots + tb + 1) * 96 + k] = v;
-      else if (k < 192) a.part[((size_t)tb * slots + ta) * 96 + k - 96] = v;
+      if (k < 96) a.part[((size_t)ta * slots + (tb + 1) * a.split + tk.slot) * 96 + k] = v;
+      else if (k < 192) a.part[((size_t)tb * slots + ta * a.split + tk.slot) * 96 + k - 96] = v;
       else a.scal[(size_t)blockIdx.x * kScalars + k - 192] = v;
     }
     return;
@@ -204,8 +205,8 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
     if (HVP) load(z, ta, zi);
     AdjSums I{};
     for (int tb = max(ta, b0); tb < b1; ++tb) {
-      const int r0 = ta == tb ? 1 : 0, r1 = ta == tb ? 17 : 32;
-      double* const jslot = a.part + ((size_t)tb * slots + tk.ga) * 96;
+      const int r0 = (ta == tb ? 1 : 0) + a.turns * tk.slot, r1 = r0 + (ta == tb ? min(16, a.turns) : a.turns);
+      double* const jslot = a.part + ((size_t)tb * slots + tk.ga * a.split + tk.slot) * 96;
       const int at = (lane + r0) & 31;
       AdjSums J{};
       if (ta > a0) J = AdjSums{jslot[at], jslot[32 + at], jslot[64 + at]};  // earlier rows' sums
@@ -213,7 +214,7 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
       store_adj(jslot, jl, J);
       __syncwarp();
     }
-    store_adj(a.part + ((size_t)ta * slots + tk.gb + 1) * 96, lane, I);
+    store_adj(a.part + ((size_t)ta * slots + (tk.gb + 1) * a.split + tk.slot) * 96, lane, I);
   }
 #pragma unroll
   for (int m = 0; m < kS; ++m) S[m] = warp_sum(S[m]);
@@ -228,9 +229,10 @@ template <bool HVP>
 __global__ void __launch_bounds__(256) k_adj_pairs(AdjBox b, AdjPass a, const double* __restrict__ x,
                                                    const double* __restrict__ z, double cF, double cA) {
   extern __shared__ double sh[];  // parts > 1: parts x (2 x 3 x 32 + kScalars)
+  const Pair64Task tk = a.tasks[blockIdx.x];
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (b.sigma2 == 1.0) adj_task<HVP, true>(b, a, x, z, cF, cA, sh);
-  else adj_task<HVP, false>(b, a, x, z, cF, cA, sh);
+  if (b.sigma2 == 1.0) adj_task<HVP, true>(b, a, x, z, cF, cA, tk, sh);
+  else adj_task<HVP, false>(b, a, x, z, cF, cA, tk, sh);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
@@ -248,7 +250,7 @@ __device__ __forceinline__ double adj_tile_sums(const AdjPass& a, double (&scal)
   __shared__ double sum[3 * kSumWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
   if (warp < 3 * kSumWarps) {
-    const int c = warp % 3, u = warp / 3, slots = a.groups + 1;
+    const int c = warp % 3, u = warp / 3, slots = (a.groups + 1) * a.split;
     const double* p = a.part + (size_t)t * slots * 96 + c * 32 + lane;
     double q0 = 0.0, q1 = 0.0;
     for (int k = u; k < slots; k += 8 * kSumWarps) {
@@ -526,18 +528,20 @@ lj_status lj_adjoint_create(const lj_config* cfg, int32_t checkpoint_every, lj_a
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device) != cudaSuccess)
     return bail(LJ_ERR_NO_DEVICE);
-  const Pair64Plan plan = plan_pairs64({a->n}, sms);
+  const Pair64Plan plan = plan_pairs64({a->n}, sms, 41, 3);  // of 30 and 55 operations a turn
   if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(LJ_ERR_CUDA);
   const size_t s3 = xyz(a);
   if (a->x.alloc(s3) || a->v.alloc(s3) || a->x0.alloc(s3) || a->v0.alloc(s3) || a->Xb.alloc(s3) ||
       a->bb.alloc(s3) || a->z.alloc(s3) || a->hostio.alloc(s3) || a->part.alloc((size_t)plan.slots * 96) ||
       a->scal.alloc(plan.tasks.size() * kScalars) || a->tasks.alloc(plan.tasks.size()))
     return bail(LJ_ERR_OUT_OF_MEMORY);
+  if (cudaMemsetAsync(a->part.p, 0, sizeof(double) * (size_t)plan.slots * 96, a->stream) != cudaSuccess)
+    return bail(LJ_ERR_CUDA);
   if (cudaMemcpyAsync(a->tasks.p, plan.tasks.data(), sizeof(Pair64Task) * plan.tasks.size(), cudaMemcpyHostToDevice,
                       a->stream) != cudaSuccess)
     return bail(LJ_ERR_CUDA);
-  a->pass = AdjPass{a->tasks.p, (int)plan.tasks.size(), plan.boxes[0].tiles, plan.boxes[0].groups,
-                    plan.group, plan.parts,             a->part.p,           a->scal.p};
+  a->pass = AdjPass{a->tasks.p, (int)plan.tasks.size(), plan.boxes[0].tiles, plan.boxes[0].groups, plan.group,
+                    plan.parts, plan.split, 32 / plan.split, a->part.p, a->scal.p};
   std::vector<double> pos((size_t)3 * a->n), vel((size_t)3 * a->n);
   if (!sample_initial_state(a->n, L, cfg->temperature, cfg->lattice, cfg->jitter, cfg->sigma, cfg->seed, pos.data(),
                             vel.data()))

@@ -132,11 +132,14 @@ struct BoxArgs {
 
 // FP64 pair pass over unordered pairs (lj_pairs64.cu).  Each box's particles
 // form tiles of 32 (the FP64 handles' i-blocks), `group` tiles a square side;
-// a tile's sums lie in groups + 1 slots of 5 x 32 doubles: slot ga from the
-// squares (ga, its own group), slot gb + 1 from (its own group, gb).  parts:
-// warps that share a square (1 unless group is 1).
+// a tile's sums lie in (groups + 1) split slots of 5 x 32 doubles: slots
+// ga split .. from the squares (ga, its own group), (gb + 1) split .. from (its
+// own group, gb).  split: tasks of a square of two tiles, each of 32 / split
+// turns from its slot's number times that on (a tile against itself has half
+// the turns and tasks; its other slots stay zero); parts: warps that share a
+// task.  Both 1 unless group is 1.
 struct Pair64Task {
-  int sys, ga, gb;
+  int sys, ga, gb, slot;
 };
 struct Pair64Box {
   int p0, n, tiles, groups;

@@ -159,7 +159,7 @@ struct Pair64Args {
   const Pair64Box* boxes64;
   const BoxArgs* boxes;
   double* part;
-  int ntasks, group, parts, nsys;
+  int ntasks, group, parts, split, turns, nsys;  // turns = 32 / split
 };
 // BoxArgs::image_lo / image_hi of a period L (bits of two separations).
 void fp64_image_bounds(double L, double invL, long long* lo, long long* hi);

@@ -48,6 +48,7 @@ __device__ __forceinline__ int pairs64_turns(const double4_32a* xd, const BoxArg
   int jl = (lane + r0) & 31;
   const double4_32a xj4 = xd[min(tb * 32 + jl, n - 1)];
   double xj = xj4.x, yj = xj4.y, zj = xj4.z;
+  __builtin_assume((r1 - r0) % 2 == 0);  // Pair64Plan::parts sees to it
 #pragma unroll 2
   for (int r = r0; r < r1; ++r) {
     double d[3] = {xi.x - xj, xi.y - yj, xi.z - zj};
@@ -93,11 +94,12 @@ __device__ __forceinline__ void pairs64_task(const Pair64Args& a, const Pair64Ta
                                              const BoxArgs& box, double* sh) {
   const int lane = threadIdx.x & 31;
   const double4_32a* xd = a.xd + bt.p0;
-  const int slots = bt.groups + 1;  // of one tile
+  const int slots = (bt.groups + 1) * a.split;  // of one tile
   double* const part = a.part + (size_t)bt.tile0_slot * 160;
   if (a.parts > 1) {
     const int w = threadIdx.x >> 5, ta = tk.ga, tb = tk.gb;
-    const int first = ta == tb ? 1 : 0, turns = (ta == tb ? 16 : 32) / a.parts;
+    const int turns = (ta == tb ? min(16, a.turns) : a.turns) / a.parts;
+    const int first = (ta == tb ? 1 : 0) + a.turns * tk.slot;
     Sums64 I{}, J{};
     const int jl = pairs64_turns<PERIODIC, UNIT>(xd, box, bt.n, ta, tb, first + w * turns, first + (w + 1) * turns,
                                                  xd[min(ta * 32 + lane, bt.n - 1)], I, J);
@@ -108,8 +110,8 @@ __device__ __forceinline__ void pairs64_task(const Pair64Args& a, const Pair64Ta
       double v = 0.0;
       for (int p = 0; p < a.parts; ++p) v += sh[p * 320 + k];
       // i sums: tile ta, slot of the square's column; j sums: tile tb, slot of its row
-      if (k < 160) part[((size_t)ta * slots + tb + 1) * 160 + k] = v;
-      else part[((size_t)tb * slots + ta) * 160 + k - 160] = v;
+      if (k < 160) part[((size_t)ta * slots + (tb + 1) * a.split + tk.slot) * 160 + k] = v;
+      else part[((size_t)tb * slots + ta * a.split + tk.slot) * 160 + k - 160] = v;
     }
     return;
   }
@@ -119,8 +121,8 @@ __device__ __forceinline__ void pairs64_task(const Pair64Args& a, const Pair64Ta
     const double4_32a xi = xd[min(ta * 32 + lane, bt.n - 1)];
     Sums64 I{};
     for (int tb = max(ta, b0); tb < b1; ++tb) {
-      const int r0 = ta == tb ? 1 : 0, r1 = ta == tb ? 17 : 32;
-      double* const jslot = part + ((size_t)tb * slots + tk.ga) * 160;
+      const int r0 = (ta == tb ? 1 : 0) + a.turns * tk.slot, r1 = r0 + (ta == tb ? min(16, a.turns) : a.turns);
+      double* const jslot = part + ((size_t)tb * slots + tk.ga * a.split + tk.slot) * 160;
       const int at = (lane + r0) & 31;
       Sums64 J{};
       if (ta > a0)  // earlier rows' sums
@@ -129,7 +131,7 @@ __device__ __forceinline__ void pairs64_task(const Pair64Args& a, const Pair64Ta
       store_sums(jslot, jl, J);
       __syncwarp();  // the next row's lanes read each other's sums
     }
-    store_sums(part + ((size_t)ta * slots + tk.gb + 1) * 160, lane, I);
+    store_sums(part + ((size_t)ta * slots + (tk.gb + 1) * a.split + tk.slot) * 160, lane, I);
   }
 }
 
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair6
   const BlockInfo bi = s.blocks[B];
   const Pair64Box bt = a.boxes64[bi.sys];
   const BoxArgs box = s.boxes[bi.sys];
-  const int slots = bt.groups + 1;
+  const int slots = (bt.groups + 1) * a.split;
   const double* p = a.part + ((size_t)bt.tile0_slot + (size_t)(bi.i0 / 32) * slots) * 160 + c * 32 + lane;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   double q0 = 0., q1 = 0.;

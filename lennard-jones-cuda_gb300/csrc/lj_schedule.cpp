@@ -139,7 +139,7 @@ bool build_rdf_ranges(int n, int ctas, RdfRanges* out) {
   return true;
 }
 
-Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops, int slot_ops) {
   Pair64Plan p;
   auto squares = [&](long long group) {
     long long t = 0;
@@ -150,8 +150,23 @@ Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
     return t;
   };
   while (squares(2ll * p.group) >= 80ll * sms) p.group *= 2;
-  if (p.group == 1)
-    while (p.parts < 8 && squares(1) * p.parts < 8ll * sms) p.parts *= 2;
+  if (p.group == 1) {
+    long long off = 0, diag = 0, tiles = 0;
+    for (int k : n) {
+      diag += (k + 31) / 32;
+      tiles = std::max<long long>(tiles, (k + 31) / 32);
+    }
+    off = squares(1) - diag;
+    auto per_sm = [&](long long t) { return (t + sms - 1) / sms; };
+    auto cost = [&](int split) {
+      long long turns = 32 / split * per_sm(split * off + (split / 2) * diag);
+      if (split == 1) turns = std::max(32 * per_sm(off), 16 * per_sm(2 * off + diag));
+      return turns * turn_ops + (tiles + 1) * split * slot_ops;
+    };
+    for (int split : {2, 4})
+      if (50 * cost(split) <= 49 * cost(p.split)) p.split = split;
+    while (p.parts < (p.split == 4 ? 4 : 8) && (p.split * off + std::max(p.split / 2, 1) * diag) * p.parts < 8ll * sms) p.parts *= 2;
+  }
   int p0 = 0;
   for (int k : n) {
     Pair64Box b{};
@@ -160,7 +175,7 @@ Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
     b.tiles = (k + 31) / 32;
     b.groups = (b.tiles + p.group - 1) / p.group;
     b.tile0_slot = p.slots;
-    p.slots += (long long)b.tiles * (b.groups + 1);
+    p.slots += (long long)b.tiles * (b.groups + 1) * p.split;
     p.boxes.push_back(b);
     p0 += k;
   }
@@ -169,7 +184,7 @@ Pair64Plan plan_pairs64(const std::vector<int>& n, int sms) {
     for (int k = 0; k < (int)n.size(); ++k)
       for (int ga = 0; ga < p.boxes[k].groups; ++ga)
         for (int gb = diag ? ga : ga + 1; gb < (diag ? ga + 1 : p.boxes[k].groups); ++gb)
-          p.tasks.push_back(Pair64Task{k, ga, gb});
+          for (int h = 0; h < (diag ? std::max(p.split / 2, 1) : p.split); ++h) p.tasks.push_back(Pair64Task{k, ga, gb, h});
   return p;
 }
 

@@ -58,15 +58,22 @@ bool build_rdf_ranges(int n, int ctas, RdfRanges* out);
 // Squares and tasks of the FP64 pair pass for boxes of sizes n (Pair64Task).
 // The square side grows while there are still about 80 tasks an SM: a tile
 // then has at most ~256 slots, so the sums stay at 10 KB a particle whatever
-// N is.  With fewer than 8 tasks an SM the turns of a task are shared by 2, 4
-// or 8 warps: N = 512 gives 136 tasks for 152 SMs.
+// N is.  Squares of one tile are split into 2 or 4 tasks where that takes 2% off
+// the SM with the most work, at `turn_ops` FP64 instructions a turn and
+// `slot_ops` for adding one more slot of a tile: N = 200 gives 28 squares for 152
+// SMs or 98 quarters, N = 1000 528 squares, 4 on some SMs, or 1024 halves, 7 at
+// most.  us for 20 steps, whole -> split: FP64 EVN N = 200 480 -> 358, N = 600
+// 648 -> 608, N = 1250 1343 -> 1271; adjoint N = 200 1045 -> 656, N = 600 1680
+// -> 1349, N = 1000 2788 -> 2636.  With fewer than 8 tasks an SM the turns of a
+// task are shared by 2, 4 or 8 warps, two turns each at least: N = 512 gives 136
+// tasks.
 struct Pair64Plan {
-  int group = 1, parts = 1;
+  int group = 1, parts = 1, split = 1;
   long long slots = 0;
   std::vector<Pair64Task> tasks;
   std::vector<Pair64Box> boxes;
 };
-Pair64Plan plan_pairs64(const std::vector<int>& n, int sms);
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops = 28, int slot_ops = 5);
 
 // Tasks of the unordered-pair kernel for n particles and `warps` warps: equal
 // shares (+-1) of the (block, tile) sequence.  The i sums of (task, block) are

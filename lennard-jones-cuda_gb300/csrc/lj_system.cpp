@@ -254,7 +254,7 @@ struct lj_system {
   DevBuf<float> newton_j, newton_i;
   DevBuf<float> partial;  // MIXED: nseg x 5 x BI
   // FP64 pair pass: tasks, boxes and sums (Pair64Args)
-  int p64_group = 1, p64_parts = 1;
+  int p64_group = 1, p64_parts = 1, p64_split = 1;
   DevBuf<Pair64Task> p64_tasks;
   DevBuf<Pair64Box> p64_boxes;
   DevBuf<double> p64_part;
@@ -378,7 +378,8 @@ PairArgs pair_args(lj_system* s) {
 
 Pair64Args pair64_args(const lj_system* s) {
   return Pair64Args{s->xd.p,       s->p64_tasks.p,        s->p64_boxes.p, s->dboxes.p,
-                    s->p64_part.p, (int)s->p64_tasks.n, s->p64_group,   s->p64_parts,  s->nsys};
+                    s->p64_part.p, (int)s->p64_tasks.n, s->p64_group,   s->p64_parts,  s->p64_split,
+                    32 / s->p64_split, s->nsys};
 }
 
 int nblocks(const lj_system* s) { return (int)s->sched.blocks.size(); }
@@ -497,6 +498,7 @@ lj_status build_and_swap_schedule(lj_system* s) {
     LJ_CUDA(s, p64_tasks.alloc(p64.tasks.size()));
     LJ_CUDA(s, p64_boxes.alloc(p64.boxes.size()));
     LJ_CUDA(s, p64_part.alloc((size_t)p64.slots * 5 * 32));
+    LJ_CUDA(s, cudaMemsetAsync(p64_part.p, 0, sizeof(double) * (size_t)p64.slots * 5 * 32, s->stream));
     LJ_CUDA(s, cudaMemcpyAsync(p64_tasks.p, p64.tasks.data(), sizeof(Pair64Task) * p64.tasks.size(),
                                cudaMemcpyHostToDevice, s->stream));
     LJ_CUDA(s, cudaMemcpyAsync(p64_boxes.p, p64.boxes.data(), sizeof(Pair64Box) * p64.boxes.size(),
@@ -533,6 +535,7 @@ lj_status build_and_swap_schedule(lj_system* s) {
   s->p64_part.swap(p64_part);
   s->p64_group = p64.group;
   s->p64_parts = p64.parts;
+  s->p64_split = p64.split;
   s->sched = std::move(sch);
   s->BI = threads;
   s->pred_ready = false;
@@ -2094,7 +2097,7 @@ lj_status lj_split_info(lj_system* s, int32_t* cap, int32_t* ctas, int32_t* max_
     for (const BlockInfo& b : s->sched.blocks) m = std::max(m, b.seg_count);
     if (fp64)
       for (const lj_config& c : s->cfg)
-        m = std::max(m, (((c.n + 31) / 32 + s->p64_group - 1) / s->p64_group + 1));
+        m = std::max(m, (((c.n + 31) / 32 + s->p64_group - 1) / s->p64_group + 1) * s->p64_split);
     *max_segments = m;
   }
   return LJ_OK;
