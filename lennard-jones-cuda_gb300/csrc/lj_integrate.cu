@@ -329,8 +329,8 @@ __global__ void k_observables(StateArgs s) {
   observables_box<MODE>(s, blockIdx.x, sh);
 }
 
-// Predictor of the fused step: the shadow of x + dt v + dt^2 F / 2 (the
-// positions the next pair kernel evaluates), periodic and walled boxes.
+// Predictor of a step whose drift is the previous one's last act: the shadow of
+// x + dt v + dt^2 F / 2 (the positions the next pair kernel evaluates).
 __global__ void k_predict(StateArgs s) {
   const BlockInfo bi = s.blocks[blockIdx.x];
   if ((int)threadIdx.x >= bi.n_i) return;
@@ -342,7 +342,8 @@ __global__ void k_predict(StateArgs s) {
     const size_t k = (size_t)c * s.npad + p;
     xp[c] = drift_pos(box, s.x[k], s.v[k], s.f[k]);
   }
-  s.q[p] = predicted_shadow(s, s.sc[bi.sys], box.bc, xp);
+  if (s.prec) s.xd[p] = make_double4_32a(xp[0], xp[1], xp[2], 0.0);
+  else s.q[p] = predicted_shadow(s, s.sc[bi.sys], box.bc, xp);
 }
 
 // Close of a fused TVN step (MDSystem.cpp:469-506, :578-579).  The pair

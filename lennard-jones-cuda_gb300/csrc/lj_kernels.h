@@ -164,8 +164,12 @@ struct Pair64Args {
 // BoxArgs::image_lo / image_hi of a period L (bits of two separations).
 void fp64_image_bounds(double L, double invL, long long* lo, long long* hi);
 cudaError_t launch_pairs64(const Pair64Args& a, cudaStream_t st);
-// With the observables of every box, except for MODE_TVN.
-cudaError_t launch_reduce64(const StateArgs& s, const Pair64Args& a, int nblocks, int mode, cudaStream_t st);
+// Its sums, the step's second half and the observables of every box (MODE_TVN:
+// two launches).  carried: the pass ran at the drift that the previous step (or
+// launch_predict) left in xd, and this one leaves the next; qhist (carried
+// steps of periodic boxes, may be null): the new positions' fixed-point shadow.
+cudaError_t launch_reduce64(const StateArgs& s, const Pair64Args& a, int nblocks, int mode, bool carried, int4* qhist,
+                            cudaStream_t st);
 
 cudaError_t launch_drift_mode(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st);
 cudaError_t launch_bbox(const StateArgs& s, int nblocks, int bi, cudaStream_t st);

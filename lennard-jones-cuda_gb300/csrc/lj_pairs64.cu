@@ -155,21 +155,55 @@ __global__ void __launch_bounds__(256) k_pairs64(Pair64Args a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// End of a kernel with a CTA per tile: the CTA that finishes a box's last tile
+// goes on to the box's observables (a launch of their own took 5 us).
+// Block-wide call.
+template <int MODE>
+__device__ __forceinline__ void finish_box(const StateArgs& s, const BlockInfo& bi, int tiles, const BoxArgs& box) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  const int b0 = blockIdx.x - bi.i0 / 32, lane = threadIdx.x & 31;  // b0: the box's first block
+  if (threadIdx.x == 0) last = atomicAdd(s.blk_cnt + b0, 1) == tiles - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) s.blk_cnt[b0] = 0;
+  if (threadIdx.x >= 32) return;
+  double kvw[3] = {0.0, 0.0, 0.0};
+  for (int k = lane; k < tiles; k += 32)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) kvw[m] += __ldcg(s.blk_part + (size_t)(b0 + k) * 8 + m);
+#pragma unroll
+  for (int m = 0; m < 3; ++m) kvw[m] = warp_sum(kvw[m]);
+  if (lane == 0) write_observables<MODE>(s, bi.sys, box, kvw[0], kvw[1], kvw[2], -1);
+}
+
+// What a finished step leaves of component c for the next pair pass, the next
+// step's drift, and for the histogram (periodic boxes), the position's
+// fixed-point shadow.
+__device__ __forceinline__ void carry64(const StateArgs& s, const BoxArgs& box, int sys, int4* qhist, int c, int at,
+                                        double x, double v, double F) {
+  reinterpret_cast<double*>(s.xd + at)[c] = drift_pos(box, x, v, F);
+  if (qhist) reinterpret_cast<int*>(qhist + at)[c] = fixed_coord_scaled(x, frame_scale(s.sc[sys]));
+}
+
 // One tile of 32 particles: the sums over its slots (value c of a particle by
 // four warps, a quarter of the slots each; fixed order), then, a component
 // per warp, what k_reduce does for the mixed path: (EVN) the second half-kick
 // and boundaries, (TVN) the averaged force and the half-kicked velocity whose
 // kinetic temperature sets chi.  Block partials [0] K, [1] V, [2] W, [3]
-// sum tv^2.  Except for TVN, the CTA that finishes a box's last tile goes on
-// to the box's observables (a launch of their own took 5 us).
+// sum tv^2.
+// CARRIED: x, v and F are those of the step's start and the shadow held the
+// drift; the drift is taken here, and the next one's shadow left behind (a
+// launch for the drift: 4.5 us a step).
 // Latency is what bounds it: the slots' loads, then a serial chain of FP64
 // operations (a warp's takes 16 clocks of the SM's pipe alone).
 constexpr int kSumWarps = 4;  // warps per value
-template <int MODE>
-__global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair64Args a) {
+template <int MODE, bool CARRIED>
+__global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair64Args a, int4* qhist) {
   __shared__ double sum[kSumWarps][5][32];
   __shared__ double ksum[3], tsum[3];
-  __shared__ int last;
   const int B = blockIdx.x, warp = threadIdx.x >> 5, c = warp % 5, u = warp / 5, lane = threadIdx.x & 31;
   const BlockInfo bi = s.blocks[B];
   const Pair64Box bt = a.boxes64[bi.sys];
@@ -177,38 +211,47 @@ __global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair6
   const int slots = (bt.groups + 1) * a.split;
   const double* p = a.part + ((size_t)bt.tile0_slot + (size_t)(bi.i0 / 32) * slots) * 160 + c * 32 + lane;
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  const bool valid = lane < bi.n_i;
+  const int at = bi.p0 + bi.i0 + lane;
+  const size_t k3 = (size_t)min(c, 2) * s.npad + (valid ? at : bi.p0 + bi.i0);
+  double x = 0.0, v = 0.0, fn = 0.0;
+  if (u == 0 && c < 3) {
+    x = s.x[k3];
+    v = s.v[k3];
+    if (CARRIED) fn = s.f[k3];
+    else if (MODE == MODE_TVN) fn = s.tf[k3];  // F_n / 2
+  }
   double q0 = 0., q1 = 0.;
   for (int k = u; k < slots; k += 8 * kSumWarps) {
-    double v[8];
+    double val[8];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) v[m] = k + m * kSumWarps < slots ? p[(size_t)(k + m * kSumWarps) * 160] : 0.0;
-    q0 += (v[0] + v[2]) + (v[4] + v[6]);
-    q1 += (v[1] + v[3]) + (v[5] + v[7]);
+    for (int m = 0; m < 8; ++m) val[m] = k + m * kSumWarps < slots ? p[(size_t)(k + m * kSumWarps) * 160] : 0.0;
+    q0 += (val[0] + val[2]) + (val[4] + val[6]);
+    q1 += (val[1] + val[3]) + (val[5] + val[7]);
   }
   sum[u][c][lane] = q0 + q1;
   __syncthreads();
   auto total = [&](int k) { return (sum[0][k][lane] + sum[1][k][lane]) + (sum[2][k][lane] + sum[3][k][lane]); };
-  const bool valid = lane < bi.n_i;
-  const int at = bi.p0 + bi.i0 + lane;
   double vv = 0.0, tv2 = 0.0;
   if (u == 0 && c < 3) {
     if (valid) {
-      const size_t k3 = (size_t)c * s.npad + at;
       const double F = box.fscale64 * total(c);
       s.f[k3] = F;
-      double v = s.v[k3];
+      if (CARRIED) x = drift_pos(box, x, v, fn);
       if (MODE == MODE_FORCES_ONLY) {
         vv = v * v;
       } else if (MODE == MODE_EVN) {
-        double x = s.x[k3];
+        if (CARRIED) v = fma(box.hdt, fn, v);
         v = fma(box.hdt, F, v);
         apply_bc1(box.bc, box.L, x, v);
         s.v[k3] = v;
-        if (box.bc == 0) s.x[k3] = x;
+        if (CARRIED || box.bc == 0) s.x[k3] = x;
+        if (CARRIED) carry64(s, box, bi.sys, qhist, c, at, x, v, F);
         vv = v * v;
       } else {  // TVN
-        const double tf = s.tf[k3] + 0.5 * F;
+        const double tf = (CARRIED ? 0.5 * fn : fn) + 0.5 * F;
         s.tf[k3] = tf;
+        if (CARRIED) s.x[k3] = x;
         const double tv = fma(box.hdt, tf, v);
         tv2 = tv * tv;
       }
@@ -230,26 +273,62 @@ __global__ void __launch_bounds__(160 * kSumWarps) k_reduce64(StateArgs s, Pair6
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    s.blk_part[(size_t)B * 8 + 0] = MODE == MODE_TVN ? 0.0 : 0.5 * (ksum[0] + ksum[1] + ksum[2]);
-    s.blk_part[(size_t)B * 8 + 3] = MODE == MODE_TVN ? tsum[0] + tsum[1] + tsum[2] : 0.0;
+    if (MODE == MODE_TVN) s.blk_part[(size_t)B * 8 + 3] = tsum[0] + tsum[1] + tsum[2];
+    else s.blk_part[(size_t)B * 8 + 0] = 0.5 * (ksum[0] + ksum[1] + ksum[2]);
   }
-  if (MODE == MODE_TVN) return;  // K follows from chi (k_tvn_finish)
-  __threadfence();
+  if (MODE != MODE_TVN) finish_box<MODE>(s, bi, bt.tiles, box);  // (TVN: K follows from chi)
+}
+
+// TVN velocity update (MDSystem.cpp:498-506) of a tile, a component per warp:
+// chi = sqrt(T0 / Tkin(tv)) by the fourth warp, v = (2 chi - 1) v + chi dt tF,
+// boundaries, K, the box's observables, and what is carried to the next step.
+// (Two launches before, a thread per particle and then the observables.)
+template <bool CARRIED>
+__global__ void __launch_bounds__(128) k_close64(StateArgs s, Pair64Args a, int4* qhist) {
+  __shared__ double chi_sh, ksum[3];
+  const int B = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const BlockInfo bi = s.blocks[B];
+  const BoxArgs box = s.boxes[bi.sys];
+  const int tiles = a.boxes64[bi.sys].tiles, b0 = B - bi.i0 / 32;
+  const bool valid = lane < bi.n_i;
+  const int at = bi.p0 + bi.i0 + lane;
+  const size_t k3 = (size_t)min(c, 2) * s.npad + (valid ? at : bi.p0 + bi.i0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  double x = 0.0, v = 0.0, tf = 0.0, F = 0.0;
+  if (c < 3) {
+    x = s.x[k3];
+    v = s.v[k3];
+    tf = s.tf[k3];
+    if (CARRIED) F = s.f[k3];
+  } else {
+    double tv2 = 0.0;
+    for (int k = lane; k < tiles; k += 32) tv2 += __ldcg(s.blk_part + (size_t)(b0 + k) * 8 + 3);
+    tv2 = warp_sum(tv2);
+    if (lane == 0) {
+      double Tkin;
+      chi_sh = tvn_chi(box, tv2, &Tkin);
+      if (B == b0) {
+        s.sc[bi.sys].Tkin = Tkin;
+        s.sc[bi.sys].chi = chi_sh;
+      }
+    }
+  }
   __syncthreads();
-  const int b0 = B - bi.i0 / 32;  // the box's first block
-  if (threadIdx.x == 0) last = atomicAdd(s.blk_cnt + b0, 1) == bt.tiles - 1;
+  if (c < 3) {
+    const double chi = chi_sh;
+    v = fma(2. * chi - 1., v, chi * box.dt * tf);
+    apply_bc1(box.bc, box.L, x, v);
+    if (valid) {
+      s.v[k3] = v;
+      if (box.bc == 0) s.x[k3] = x;
+      if (CARRIED) carry64(s, box, bi.sys, qhist, c, at, x, v, F);
+    }
+    const double vv = warp_sum(valid ? v * v : 0.0);
+    if (lane == 0) ksum[c] = vv;
+  }
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (threadIdx.x == 0) s.blk_cnt[b0] = 0;
-  if (threadIdx.x >= 32) return;
-  double kvw[3] = {0.0, 0.0, 0.0};
-  for (int k = lane; k < bt.tiles; k += 32)
-#pragma unroll
-    for (int m = 0; m < 3; ++m) kvw[m] += __ldcg(s.blk_part + (size_t)(b0 + k) * 8 + m);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) kvw[m] = warp_sum(kvw[m]);
-  if (lane == 0) write_observables<MODE>(s, bi.sys, box, kvw[0], kvw[1], kvw[2], -1);
+  if (threadIdx.x == 0) s.blk_part[(size_t)B * 8 + 0] = 0.5 * (ksum[0] + ksum[1] + ksum[2]);
+  finish_box<MODE_TVN>(s, bi, tiles, box);
 }
 
 }  // namespace
@@ -264,11 +343,14 @@ cudaError_t launch_pairs64(const Pair64Args& a, cudaStream_t st) {
   return launch_dependent(k_pairs64, a.ntasks, 32 * a.parts, a.parts > 1 ? sizeof(double) * 320 * a.parts : 0, st, a);
 }
 
-cudaError_t launch_reduce64(const StateArgs& s, const Pair64Args& a, int nblocks, int mode, cudaStream_t st) {
-  auto* k = mode == MODE_FORCES_ONLY ? k_reduce64<MODE_FORCES_ONLY>
-            : mode == MODE_EVN       ? k_reduce64<MODE_EVN>
-                                     : k_reduce64<MODE_TVN>;
-  return launch_dependent(k, nblocks, 160 * kSumWarps, 0, st, s, a);
+cudaError_t launch_reduce64(const StateArgs& s, const Pair64Args& a, int nblocks, int mode, bool carried, int4* qhist,
+                            cudaStream_t st) {
+  auto* k = mode == MODE_FORCES_ONLY ? k_reduce64<MODE_FORCES_ONLY, false>
+            : mode == MODE_EVN       ? (carried ? k_reduce64<MODE_EVN, true> : k_reduce64<MODE_EVN, false>)
+                                     : (carried ? k_reduce64<MODE_TVN, true> : k_reduce64<MODE_TVN, false>);
+  cudaError_t e = launch_dependent(k, nblocks, 160 * kSumWarps, 0, st, s, a, qhist);
+  if (e != cudaSuccess || mode != MODE_TVN) return e;
+  return launch_dependent(carried ? k_close64<true> : k_close64<false>, nblocks, 128, 0, st, s, a, qhist);
 }
 
 }  // namespace ljgb

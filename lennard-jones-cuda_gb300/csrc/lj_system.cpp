@@ -235,7 +235,7 @@ struct lj_system {
   DevBuf<int> blk_cnt, glob_cnt;  // fused-step completion counters
   int qpar = 0;             // which of q / q2 holds the current shadow
   bool obs_maybe_pending = false;  // a fused step left observables pending (DevScalars::obs_pending)
-  bool pred_ready = false;  // current shadow = predictor x + dt v + dt^2 F/2 for pred_dt
+  bool pred_ready = false;  // current shadow (q or xd) = predictor x + dt v + dt^2 F/2 for pred_dt
   double pred_dt = 0.0;
   DevBuf<BlockInfo> blocks;
   DevBuf<int> cta_tile_begin, cta_lo, cta_block, cta_jt, sys_block_first;
@@ -584,22 +584,32 @@ lj_status enqueue_pairs(lj_system* s) {
   return LJ_OK;
 }
 
-// ... TVN's rescale and the observables (k_reduce64 forms them itself unless
-// the rescale has to come first); *kernels counts the launches.
+// FP64 steps carry the drift: a step's second half leaves the next step's
+// positions in the shadow, and a step is the pair pass and that second half.
+// (The pass needs no fixed-point frame.  Histograms do, so walled and open boxes
+// that accumulate them after every step rebuild their frames in between.)  us a
+// step, N = 100, drift on its own -> carried: EVN 18 -> 13, TVN 22 -> 17; with
+// walls, whose frames took two more launches, 34 -> 14 and 38 -> 16.
+bool carries64(const lj_system* s) { return s->prec == LJ_PREC_FP64 && !(s->any_nonperiodic && s->rdf_acc); }
+
+// ... with TVN's rescale and the observables; *kernels counts the launches.
 lj_status enqueue_reduce(lj_system* s, int mode, int* kernels) {
   const StateArgs a = state_args(s);
-  const bool fp64 = s->prec == LJ_PREC_FP64;
-  if (fp64) LJ_CUDA(s, launch_reduce64(a, pair64_args(s), nblocks(s), mode, s->stream));
-  else LJ_CUDA(s, launch_reduce(a, nblocks(s), s->BI, mode, s->stream));
+  if (s->prec == LJ_PREC_FP64) {
+    const bool carried = mode != MODE_FORCES_ONLY && carries64(s);
+    LJ_CUDA(s, launch_reduce64(a, pair64_args(s), nblocks(s), mode, carried,
+                               carried && s->rdf_acc ? s->qhist.p : nullptr, s->stream));
+    *kernels += mode == MODE_TVN ? 2 : 1;
+    return LJ_OK;
+  }
+  LJ_CUDA(s, launch_reduce(a, nblocks(s), s->BI, mode, s->stream));
   *kernels += 1;
   if (mode == MODE_TVN) {
     LJ_CUDA(s, launch_tvn_finish(a, nblocks(s), s->BI, s->stream));
     *kernels += 1;
   }
-  if (!fp64 || mode == MODE_TVN) {
-    LJ_CUDA(s, launch_observables(a, s->nsys, mode, s->stream));
-    *kernels += 1;
-  }
+  LJ_CUDA(s, launch_observables(a, s->nsys, mode, s->stream));
+  *kernels += 1;
   return LJ_OK;
 }
 
@@ -663,12 +673,14 @@ lj_status enqueue_step(lj_system* s, int mode, cudaEvent_t* ev, bool capture, in
   int k = 0;
   const unsigned flags = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[0], s->stream, flags));
-  LJ_CUDA(s, launch_drift_mode(a, nb, s->BI, mode, s->stream));
-  ++k;
-  if (s->any_nonperiodic) {
-    LJ_CUDA(s, launch_frame(a, s->nsys, true, s->stream));
-    LJ_CUDA(s, launch_quantize(a, nb, s->BI, true, s->stream));
-    k += 2;
+  if (!carries64(s)) {
+    LJ_CUDA(s, launch_drift_mode(a, nb, s->BI, mode, s->stream));
+    ++k;
+    if (s->any_nonperiodic) {
+      LJ_CUDA(s, launch_frame(a, s->nsys, true, s->stream));
+      LJ_CUDA(s, launch_quantize(a, nb, s->BI, true, s->stream));
+      k += 2;
+    }
   }
   if (ev) LJ_CUDA(s, cudaEventRecordWithFlags(ev[1], s->stream, flags));
   lj_status pst = enqueue_pairs(s);
@@ -874,11 +886,14 @@ lj_status enqueue_after_step(lj_system* s, const RdfPass& rdf, int* kernels) {
     *kernels += 1;
   }
   if (s->rdf_acc) {
-    StateArgs a = state_args(s);
-    a.q = s->qhist.p;
-    LJ_CUDA(s, launch_quantize(a, nblocks(s), s->BI, false, s->stream));
+    if (!carries64(s)) {  // (those leave it themselves)
+      StateArgs a = state_args(s);
+      a.q = s->qhist.p;
+      LJ_CUDA(s, launch_quantize(a, nblocks(s), s->BI, false, s->stream));
+      *kernels += 1;
+    }
     LJ_CUDA(s, launch_rdf(rdf, s->hist_grid, s->stream));
-    *kernels += 2;
+    *kernels += 1;
   }
   return LJ_OK;
 }
@@ -1521,15 +1536,16 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
     lj_status st = flush_observables(s);
     if (st) return st;
   }
-  if (fused && (!s->pred_ready || s->pred_dt != dt)) {
+  if ((fused || carries64(s)) && (!s->pred_ready || s->pred_dt != dt)) {
     LJ_CUDA(s, launch_predict(state_args(s), nblocks(s), s->BI, s->stream));
     s->launches += 1;
     s->pred_ready = true;
     s->pred_dt = dt;
   }
-  // The row step's launches go to the stream directly: each is a programmatic
-  // dependent of the one before, across steps too, which graphs of one step
-  // would not be.
+  if (!fused && !carries64(s)) s->pred_ready = false;  // these steps move the shadow themselves
+  // The row and the carried FP64 step's launches go to the stream directly: each
+  // is a programmatic dependent of the one before, across steps too, which graphs
+  // of one step would not be.
   // (A stream being captured keeps the graphs' route: single launches would be
   // recorded with this call's step parity.)
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1547,15 +1563,16 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
     }
     return LJ_OK;
   }
-  const bool direct = fused && use_rows(s) && plain;
+  const bool direct = plain && (fused ? use_rows(s) : carries64(s));
   for (int k = 0; k < nsteps; ++k) {
     if (direct) {
       int kernels = 0;
-      lj_status st = enqueue_rows(s, mode, nullptr, 0, &kernels);
+      lj_status st = fused ? enqueue_rows(s, mode, nullptr, 0, &kernels)
+                           : enqueue_step(s, mode, nullptr, true, &kernels);
       if (st) return st;
       s->launches += kernels;
-      s->qpar ^= 1;
-      s->obs_maybe_pending = true;
+      if (fused) s->qpar ^= 1;
+      if (fused) s->obs_maybe_pending = true;
       continue;
     }
     GraphEntry* ge = nullptr;
