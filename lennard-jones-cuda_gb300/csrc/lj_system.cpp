@@ -1644,18 +1644,21 @@ lj_status lj_set_recording(lj_system* s, int32_t cap) {
 static lj_status read_records(lj_system* s, int box, lj_observables* out, int32_t max, int32_t* count) {
   if (!s || !count || max < 0 || box < 0 || box >= s->nsys) return LJ_ERR_INVALID;
   DeviceGuard device_guard(s->device);
-  lj_status st = check_status(s);
+  // status and scalars with one synchronisation
+  lj_status st = s->rec_cap ? fetch_scalars(s) : check_status(s);
   if (st) return st;
   *count = 0;
   if (s->rec_cap == 0) return LJ_OK;
-  std::vector<DevScalars> sc;
-  if ((st = read_scalars(s, sc))) return st;
-  std::vector<DevRecord> rec(s->rec_cap);
-  LJ_CUDA(s, cudaMemcpy(rec.data(), s->records.p + (size_t)box * s->rec_cap, sizeof(DevRecord) * s->rec_cap,
-                        cudaMemcpyDeviceToHost));
-  const long long total = sc[box].rec_count;
+  const long long total = s->h_sc.p[box].rec_count;
   const long long have = std::min<long long>(total, s->rec_cap);
   const long long first = total - have;
+  if (have == 0 || max == 0) return LJ_OK;
+  // a ring that has not come round yet holds what is wanted at its start
+  const long long used = first > 0 ? s->rec_cap : std::min<long long>(have, max);
+  std::vector<DevRecord> rec((size_t)used);
+  LJ_CUDA(s, cudaMemcpyAsync(rec.data(), s->records.p + (size_t)box * s->rec_cap, sizeof(DevRecord) * rec.size(),
+                             cudaMemcpyDeviceToHost, s->stream));
+  LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   int n = 0;
   for (long long k = first; k < total && n < max; ++k, ++n) {
     const DevRecord& r = rec[k % s->rec_cap];

@@ -57,6 +57,21 @@ class Observables(C.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
+_OBS_DTYPE = np.dtype([(name, np.int64 if t is C.c_int64 else np.float64) for name, t in Observables._fields_])
+
+
+class _ObservablesArray:
+    """n lj_observables (uninitialised) as a numpy array the library writes to;
+    dicts(k) is what as_dict() of the first k gives."""
+
+    def __init__(self, n: int):
+        self.a = np.empty(n or 1, _OBS_DTYPE)
+        self.p = self.a.ctypes.data_as(C.POINTER(Observables))
+
+    def dicts(self, k: int):
+        return [dict(zip(_OBS_DTYPE.names, row)) for row in self.a[:k].tolist()]
+
+
 class Counter(C.Structure):
     """lj_counter (include/lj_gb300.h): type 0-2 slab, 3 cube, 4-6 |v| component."""
     _fields_ = [("type", C.c_int32), ("nalpha", C.c_int32), ("alpha_step", C.c_double), ("vmax", C.c_double)]
@@ -388,24 +403,24 @@ class System:
         return o.as_dict()
 
     def batch_observables(self):
-        arr = (Observables * self.nsys)()
-        self._c(load().lj_batch_observables(self.h, arr))
-        return [a.as_dict() for a in arr]
+        arr = _ObservablesArray(self.nsys)
+        self._c(load().lj_batch_observables(self.h, arr.p))
+        return arr.dicts(self.nsys)
 
     def set_recording(self, cap: int):
         self._c(load().lj_set_recording(self.h, int(cap)))
 
     def records(self, max_records: int = 1 << 20):
-        arr = (Observables * max_records)()
+        arr = _ObservablesArray(max_records)
         cnt = C.c_int32()
-        self._c(load().lj_get_records(self.h, arr, max_records, C.byref(cnt)))
-        return [arr[k].as_dict() for k in range(cnt.value)]
+        self._c(load().lj_get_records(self.h, arr.p, max_records, C.byref(cnt)))
+        return arr.dicts(cnt.value)
 
     def batch_records(self, box: int, max_records: int = 1 << 20):
-        arr = (Observables * max_records)()
+        arr = _ObservablesArray(max_records)
         cnt = C.c_int32()
-        self._c(load().lj_batch_records(self.h, int(box), arr, max_records, C.byref(cnt)))
-        return [arr[k].as_dict() for k in range(cnt.value)]
+        self._c(load().lj_batch_records(self.h, int(box), arr.p, max_records, C.byref(cnt)))
+        return arr.dicts(cnt.value)
 
     def reset_averaging(self):
         self._c(load().lj_reset_averaging(self.h))
