@@ -230,9 +230,9 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
 
 // Launch as a programmatic dependent of the kernel queued before.
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch_dependent(void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

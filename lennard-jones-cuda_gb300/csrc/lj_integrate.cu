@@ -201,6 +201,7 @@ __global__ void k_frame(StateArgs s, int only_nonperiodic) {
 __global__ void k_quantize(StateArgs s, int only_nonperiodic) {
   const int B = blockIdx.x;
   const BlockInfo bi = s.blocks[B];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (only_nonperiodic && s.boxes[bi.sys].bc == 0) return;
   if ((int)threadIdx.x >= bi.n_i) return;
   const int p = bi.p0 + bi.i0 + threadIdx.x;
@@ -529,6 +530,7 @@ __device__ __forceinline__ int sides_within(const CounterDev& cd, double d) {
 __global__ void k_counters(StateArgs s, const CounterDev* cs, int nbins, int* st, int* ring, int n) {
   __shared__ int shc[kMaxCounterAlphas];
   __shared__ bool last;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int phase = st[kCtrPhase] + 1, row = st[kCtrNext];
   const bool counted = phase >= st[kCtrEvery];
   if (counted) {
@@ -671,6 +673,7 @@ __device__ __forceinline__ void mailbox_row(const Mailbox& mb, const StateArgs& 
 }
 
 __global__ void k_pack_multi(XyzArrays a, int count, int n, int npad, Mailbox mb, StateArgs s) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if ((int)blockIdx.y == count) {
     mailbox_row(mb, s);
   } else {
@@ -792,8 +795,7 @@ cudaError_t launch_pack_multi(const XyzArrays& a, int count, int n, int npad, co
   if (rows <= 0) return cudaSuccess;
   int gx = (3 * n + 255) / 256;
   if (mb && mb->finalize && gx < s.nsys) gx = s.nsys;
-  k_pack_multi<<<dim3(gx, rows), 256, 0, st>>>(a, count, n, npad, mb ? *mb : Mailbox{}, s);
-  return cudaGetLastError();
+  return launch_dependent(k_pack_multi, dim3(gx, rows), 256, 0, st, a, count, n, npad, mb ? *mb : Mailbox{}, s);
 }
 
 cudaError_t launch_upload_stage(const double* pos, const double* vel, int n, int npad, double* spos, double* svel,
@@ -837,8 +839,7 @@ cudaError_t launch_frame(const StateArgs& s, int nsys, bool only_nonperiodic, cu
 }
 
 cudaError_t launch_quantize(const StateArgs& s, int nblocks, int bi, bool only_nonperiodic, cudaStream_t st) {
-  k_quantize<<<nblocks, bi, 0, st>>>(s, only_nonperiodic ? 1 : 0);
-  return cudaGetLastError();
+  return launch_dependent(k_quantize, nblocks, bi, 0, st, s, only_nonperiodic ? 1 : 0);
 }
 
 cudaError_t launch_reduce(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st) {
@@ -867,8 +868,7 @@ cudaError_t launch_predict(const StateArgs& s, int nblocks, int bi, cudaStream_t
 
 cudaError_t launch_counters(const StateArgs& s, const CounterDev* cs, int nc, int nbins, int* state, int* ring, int n,
                             cudaStream_t st) {
-  k_counters<<<dim3((unsigned)(n + 127) / 128, nc), 128, 0, st>>>(s, cs, nbins, state, ring, n);
-  return cudaGetLastError();
+  return launch_dependent(k_counters, dim3((n + 127) / 128, nc), 128, 0, st, s, cs, nbins, state, ring, n);
 }
 
 cudaError_t launch_obs_finalize(const StateArgs& s, int nsys, cudaStream_t st) {

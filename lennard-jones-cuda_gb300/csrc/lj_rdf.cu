@@ -81,10 +81,10 @@ __device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float bou
 // issue (no memory traffic: the shadow stays in L2): 11 instructions for a pair
 // past the bound, which most are.  N = 16384, 256 clamped bins, us a call: 234
 // over ordered pairs, 131 over unordered ones, 119 with the bound in place of
-// the products and a counter, 113 with
-// bin_bound's bracket.  A CTA owns a contiguous range of (block, 32-j
-// chunk) units (build_rdf_ranges), flushing its shared histogram once: a grid
-// of single tiles would flush 256 bins thousands of times.
+// the products and a counter, 113 with bin_bound's bracket.  A CTA owns a
+// contiguous range of (block, 32-j chunk) units (build_rdf_ranges), flushing its
+// shared histogram once: a grid of single tiles would flush 256 bins thousands
+// of times.
 template <int MODE>
 __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
   extern __shared__ unsigned shist[];
@@ -93,9 +93,10 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
   const int tid = threadIdx.x, lane = tid & 31;
   const HistArgs h = a.hist;
   const int last = h.nb - 1;
+  for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const float k2 = a.sc->k2;
   const float bound = bin_bound<MODE>(k2, h.inv_w, MODE == 2 ? h.rmax2 : (float)(MODE == 1 ? h.nb : last));
-  for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
   unsigned npairs = 0;  // of this thread's i, since the last flush
   auto flush = [&]() {
     __syncthreads();
@@ -162,10 +163,8 @@ int rdf_ctas_per_sm() { return 6; }
 
 cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st) {
   const size_t smem = sizeof(unsigned) * (size_t)a.hist.nb;
-  if (a.hist.mode == 0) k_rdf<0><<<grid, kRdfBlock, smem, st>>>(a);
-  else if (a.hist.mode == 1) k_rdf<1><<<grid, kRdfBlock, smem, st>>>(a);
-  else k_rdf<2><<<grid, kRdfBlock, smem, st>>>(a);
-  return cudaGetLastError();
+  auto* k = a.hist.mode == 0 ? k_rdf<0> : a.hist.mode == 1 ? k_rdf<1> : k_rdf<2>;
+  return launch_dependent(k, grid, kRdfBlock, smem, st, a);
 }
 
 }  // namespace ljgb
