@@ -86,6 +86,7 @@ __global__ void k_drift(StateArgs s) {
   __shared__ double sh[6 * 32];
   const int B = blockIdx.x;
   const BlockInfo bi = s.blocks[B];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool valid = (int)threadIdx.x < bi.n_i;
   const int p = bi.p0 + bi.i0 + threadIdx.x;
   const BoxArgs box = s.boxes[bi.sys];
@@ -142,6 +143,7 @@ __global__ void k_bbox(StateArgs s) {
 __global__ void k_frame(StateArgs s, int only_nonperiodic) {
   __shared__ double sh[32];
   const int sys = blockIdx.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const BoxArgs box = s.boxes[sys];
   if (only_nonperiodic && box.bc == 0) return;
   const int b0 = s.sys_block_first[sys], b1 = s.sys_block_first[sys + 1];
@@ -222,6 +224,7 @@ __global__ void k_reduce(StateArgs s) {
   const int tid = threadIdx.x;
   const bool valid = tid < bi.n_i;
   const int p = bi.p0 + bi.i0 + tid;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const BoxArgs box = s.boxes[bi.sys];
   double part[4] = {0., 0., 0., 0.};
   if (valid) {
@@ -287,6 +290,7 @@ __global__ void k_tvn_finish(StateArgs s) {
   const int tid = threadIdx.x;
   const BoxArgs box = s.boxes[bi.sys];
   const int b0 = s.sys_block_first[bi.sys], b1 = s.sys_block_first[bi.sys + 1];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const double tv2 = box_sum(s, b0, b1, 3, sh);
   if (tid == 0) {
     double Tkin;
@@ -327,6 +331,7 @@ __global__ void k_tvn_finish(StateArgs s) {
 template <int MODE>
 __global__ void k_observables(StateArgs s) {
   __shared__ double sh[3 * 32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   observables_box<MODE>(s, blockIdx.x, sh);
 }
 
@@ -365,15 +370,17 @@ __global__ void k_predict(StateArgs s) {
 __global__ void k_tvn_close(StateArgs s) {
   __shared__ double sh[3 * 32];
   // Launched as a programmatic dependent of the pair kernel: the CTAs start
-  // while the pair grid drains.  What the pair kernel does not write (the
-  // block table, the box, x, v and F_n) is loaded before waiting for its
-  // writes (F_{n+1} in tf, e, w, the blocks' sums) to become visible.
+  // while the pair grid drains.  Only what no step writes (the block table, the
+  // box) is loaded before the wait: the pair kernel may itself have started
+  // while the previous step's close, which wrote x, v and F_n, was draining.
   const int B = blockIdx.x;
   const BlockInfo bi = s.blocks[B];
   const int tid = threadIdx.x;
   const BoxArgs box = s.boxes[bi.sys];
   const bool valid = tid < bi.n_i;
   const int p = bi.p0 + bi.i0 + (valid ? tid : 0);
+  const int b0 = s.sys_block_first[bi.sys], b1 = s.sys_block_first[bi.sys + 1];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   double xn[3], vn[3], fn[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -382,8 +389,6 @@ __global__ void k_tvn_close(StateArgs s) {
     vn[c] = s.v[k];
     fn[c] = s.f[k];
   }
-  const int b0 = s.sys_block_first[bi.sys], b1 = s.sys_block_first[bi.sys + 1];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   DevScalars& sc = s.sc[bi.sys];
   // The pair kernel's results for this particle, loaded before chi's sum so
   // that both wait on memory together.
@@ -823,9 +828,7 @@ cudaError_t launch_upload_commit(const StateArgs& s, int nblocks, int bi, const 
 }
 
 cudaError_t launch_drift_mode(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st) {
-  if (mode == MODE_EVN) k_drift<MODE_EVN><<<nblocks, bi, 0, st>>>(s);
-  else k_drift<MODE_TVN><<<nblocks, bi, 0, st>>>(s);
-  return cudaGetLastError();
+  return launch_dependent(mode == MODE_EVN ? k_drift<MODE_EVN> : k_drift<MODE_TVN>, nblocks, bi, 0, st, s);
 }
 
 cudaError_t launch_bbox(const StateArgs& s, int nblocks, int bi, cudaStream_t st) {
@@ -834,8 +837,7 @@ cudaError_t launch_bbox(const StateArgs& s, int nblocks, int bi, cudaStream_t st
 }
 
 cudaError_t launch_frame(const StateArgs& s, int nsys, bool only_nonperiodic, cudaStream_t st) {
-  k_frame<<<nsys, kObsThreads, 0, st>>>(s, only_nonperiodic ? 1 : 0);
-  return cudaGetLastError();
+  return launch_dependent(k_frame, nsys, kObsThreads, 0, st, s, only_nonperiodic ? 1 : 0);
 }
 
 cudaError_t launch_quantize(const StateArgs& s, int nblocks, int bi, bool only_nonperiodic, cudaStream_t st) {
@@ -843,22 +845,19 @@ cudaError_t launch_quantize(const StateArgs& s, int nblocks, int bi, bool only_n
 }
 
 cudaError_t launch_reduce(const StateArgs& s, int nblocks, int bi, int mode, cudaStream_t st) {
-  if (mode == MODE_FORCES_ONLY) k_reduce<MODE_FORCES_ONLY><<<nblocks, bi, 0, st>>>(s);
-  else if (mode == MODE_EVN) k_reduce<MODE_EVN><<<nblocks, bi, 0, st>>>(s);
-  else k_reduce<MODE_TVN><<<nblocks, bi, 0, st>>>(s);
-  return cudaGetLastError();
+  auto* k = mode == MODE_FORCES_ONLY ? k_reduce<MODE_FORCES_ONLY> : mode == MODE_EVN ? k_reduce<MODE_EVN> : k_reduce<MODE_TVN>;
+  return launch_dependent(k, nblocks, bi, 0, st, s);
 }
 
 cudaError_t launch_tvn_finish(const StateArgs& s, int nblocks, int bi, cudaStream_t st) {
-  k_tvn_finish<<<nblocks, bi, 0, st>>>(s);
-  return cudaGetLastError();
+  return launch_dependent(k_tvn_finish, nblocks, bi, 0, st, s);
 }
 
 cudaError_t launch_observables(const StateArgs& s, int nsys, int mode, cudaStream_t st) {
-  if (mode == MODE_FORCES_ONLY) k_observables<MODE_FORCES_ONLY><<<nsys, kObsThreads, 0, st>>>(s);
-  else if (mode == MODE_EVN) k_observables<MODE_EVN><<<nsys, kObsThreads, 0, st>>>(s);
-  else k_observables<MODE_TVN><<<nsys, kObsThreads, 0, st>>>(s);
-  return cudaGetLastError();
+  auto* k = mode == MODE_FORCES_ONLY ? k_observables<MODE_FORCES_ONLY>
+            : mode == MODE_EVN       ? k_observables<MODE_EVN>
+                                     : k_observables<MODE_TVN>;
+  return launch_dependent(k, nsys, kObsThreads, 0, st, s);
 }
 
 cudaError_t launch_predict(const StateArgs& s, int nblocks, int bi, cudaStream_t st) {

@@ -304,12 +304,14 @@ __device__ __forceinline__ void pairs_body(const PairArgs& a, const StateArgs& s
 template <int THREADS, int TILE, int STAGES, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_pairs_mixed(PairArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   pairs_body<THREADS, TILE, STAGES, 0>(a, StateArgs{}, smem_raw);
 }
 
 template <int THREADS, int TILE, int STAGES, int MINB, int EPI>
 __global__ void __launch_bounds__(THREADS, MINB) k_pairs_mixed_fused(FusedPairArgs f) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   pairs_body<THREADS, TILE, STAGES, EPI>(f.pair, f.st, smem_raw);
 }
 
@@ -322,16 +324,15 @@ template <int THREADS, int TILE, int STAGES, int MINB>
 cudaError_t launch_mixed_t(const PairArgs& a, int grid, cudaStream_t st) {
   // <= 48 KB: 16 B x STAGES x TILE staging, no opt-in needed.
   const size_t smem = sizeof(int4) * STAGES * TILE;
-  k_pairs_mixed<THREADS, TILE, STAGES, MINB><<<grid, THREADS, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_dependent(k_pairs_mixed<THREADS, TILE, STAGES, MINB>, grid, THREADS, smem, st, a);
 }
 
 template <int THREADS, int TILE, int STAGES, int MINB>
 cudaError_t launch_fused_t(int mode, const FusedPairArgs& f, int grid, cudaStream_t st) {
   const size_t smem = sizeof(int4) * STAGES * TILE;
-  if (mode == MODE_EVN) k_pairs_mixed_fused<THREADS, TILE, STAGES, MINB, MODE_EVN><<<grid, THREADS, smem, st>>>(f);
-  else k_pairs_mixed_fused<THREADS, TILE, STAGES, MINB, MODE_TVN><<<grid, THREADS, smem, st>>>(f);
-  return cudaGetLastError();
+  auto* k = mode == MODE_EVN ? k_pairs_mixed_fused<THREADS, TILE, STAGES, MINB, MODE_EVN>
+                             : k_pairs_mixed_fused<THREADS, TILE, STAGES, MINB, MODE_TVN>;
+  return launch_dependent(k, grid, THREADS, smem, st, f);
 }
 
 template <int THREADS, int TILE, int STAGES, int MINB>

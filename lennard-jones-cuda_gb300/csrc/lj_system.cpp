@@ -1541,11 +1541,12 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
     s->pred_dt = dt;
   }
   if (!fused && !carries64(s)) s->pred_ready = false;  // these steps move the shadow themselves
-  // The row and the carried FP64 step's launches go to the stream directly, with
-  // the counters' and the histogram's: each is a programmatic dependent of the one
-  // before, across steps too, which graphs of one step would not be (20 FP64
-  // steps of 512 particles with both: 763 -> 724 us).
-  // (A stream being captured keeps the graphs' route: single launches would be
+  // The launches go to the stream directly: each is a programmatic dependent of
+  // the one before, across steps too, which graphs of one step would not be (us,
+  // graphs -> so: 20 FP64 steps of 512 particles with counters and histogram 763
+  // -> 724, a step of an open box of 400 36.3 -> 32.5, ten steps of 8 boxes of
+  // 100 to 300 in all 255 -> 228).  (A profiled step keeps its graph for the
+  // events; a stream being captured does too, as single launches would be
   // recorded with this call's step parity.)
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
@@ -1562,16 +1563,15 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
     }
     return LJ_OK;
   }
-  const bool direct = plain && (fused ? use_rows(s) : carries64(s));
   RdfPass rdf{};
-  if (direct && s->rdf_acc) {
+  if (plain && s->rdf_acc) {
     lj_status st = rdf_pass(s, s->qhist.p, s->rdf_args, &rdf);
     if (st) return st;
   }
   for (int k = 0; k < nsteps; ++k) {
-    if (direct) {
+    if (plain) {
       int kernels = 0;
-      lj_status st = fused ? enqueue_rows(s, mode, nullptr, 0, &kernels)
+      lj_status st = fused ? enqueue_step_fused(s, mode, nullptr, true, &kernels)
                            : enqueue_step(s, mode, nullptr, true, &kernels);
       if (!st) st = enqueue_after_step(s, rdf, &kernels);
       if (st) return st;
