@@ -273,7 +273,7 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
   if (want_rdf)
-    REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}},
+    REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}, {}, nullptr},
                          c.rdf_grid, c.stream));
   if (c.rows.ctas > 0 || c.newton > 0) {
     StateArgs st{};

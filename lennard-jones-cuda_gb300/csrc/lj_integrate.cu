@@ -668,13 +668,7 @@ __device__ __forceinline__ void mailbox_row(const Mailbox& mb, const StateArgs& 
   } else {
     for (int k = threadIdx.x; k < mb.sc_nwords; k += blockDim.x) mb.sc_out[k] = mb.sc[k];
   }
-  if (threadIdx.x == 0) {
-    mb.words_out[0] = *(volatile const int*)mb.status;
-    if (mb.bad) {
-      mb.words_out[1] = *mb.bad;
-      *mb.bad = 0x7f7f7f7f;  // read: ready for the next upload's check
-    }
-  }
+  if (threadIdx.x == 0) mail_status(mb);
 }
 
 __global__ void k_pack_multi(XyzArrays a, int count, int n, int npad, Mailbox mb, StateArgs s) {

@@ -38,6 +38,25 @@ struct PairArgs {
 };
 
 
+// Small device words copied by the pack launch: the status word (and the
+// upload check's bad index, if bad is set, which is then reset to 0x7f7f7f7f)
+// to words_out[0..1], and sc_nwords 32-bit words of the scalar block to sc_out.
+struct Mailbox {
+  const int* status;
+  int* bad;
+  int* words_out;
+  const int* sc;
+  int* sc_out;
+  int sc_nwords;
+  int finalize;  // != 0: compute the observables the last fused TVN step left pending first (one CTA per box)
+  int* ticket;   // finalize with several boxes: the last box's CTA copies the status words (0 between launches)
+  // seq != 0: the launch's last CTA writes seq into words_out[2] once every
+  // store of the launch is visible to the host (grid_ticket: CTAs done, 0
+  // between launches), so the host can wait on that word alone.
+  int* grid_ticket;
+  int seq;
+};
+
 // Pair histogram of one box of n particles (lj_rdf.cu) over the fixed-point
 // shadow q: adds the counts of all ordered pairs to h.counts.  The ranges are
 // those of build_rdf_ranges for at most rdf_ctas_per_sm() CTAs an SM.
@@ -49,6 +68,10 @@ struct RdfPass {
   const int* cta_chunk;    // first j-chunk of that block
   const int* cta_units;    // chunks the CTA covers
   HistArgs hist;
+  // with mail.seq != 0 the last CTA hands the counts and the status words over:
+  // counts_out is host memory, mail.grid_ticket 0 between launches
+  Mailbox mail;
+  unsigned long long* counts_out;
 };
 int rdf_ctas_per_sm();
 cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st);
@@ -224,24 +247,6 @@ cudaError_t launch_selftest_wait(int* status, cudaStream_t st);
 struct XyzArrays {
   const double* src[3];
   double* dst[3];
-};
-// Small device words copied by the pack launch: the status word (and the
-// upload check's bad index, if bad is set, which is then reset to 0x7f7f7f7f)
-// to words_out[0..1], and sc_nwords 32-bit words of the scalar block to sc_out.
-struct Mailbox {
-  const int* status;
-  int* bad;
-  int* words_out;
-  const int* sc;
-  int* sc_out;
-  int sc_nwords;
-  int finalize;  // != 0: compute the observables the last fused TVN step left pending first (one CTA per box)
-  int* ticket;   // finalize with several boxes: the last box's CTA copies the status words (0 between launches)
-  // seq != 0: the launch's last CTA writes seq into words_out[2] once every
-  // store of the launch is visible to the host (grid_ticket: CTAs done, 0
-  // between launches), so the host can wait on that word alone.
-  int* grid_ticket;
-  int seq;
 };
 // `s` is read only with mb->finalize.
 cudaError_t launch_pack_multi(const XyzArrays& a, int count, int n, int npad, const Mailbox* mb, const StateArgs& s,

@@ -11,6 +11,7 @@
 #include "lj_device.cuh"
 #include "lj_kernels.h"
 #include "lj_schedule.h"
+#include "lj_stepdev.cuh"
 
 namespace ljgb {
 namespace {
@@ -85,7 +86,9 @@ __device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float bou
 // contiguous range of (block, 32-j chunk) units (build_rdf_ranges), flushing its
 // shared histogram once: a grid of single tiles would flush 256 bins thousands
 // of times.
-template <int MODE>
+// MAIL: the last CTA hands the counts to the host (rdf_counts of 500 particles
+// 42 -> 30 us, of 16384 113 -> 102, against two copies behind the pass).
+template <int MODE, bool MAIL>
 __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
   extern __shared__ unsigned shist[];
   __shared__ int4 tile[kTile];
@@ -153,6 +156,21 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
     }
   }
   flush();
+  if (!MAIL) return;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) sirec[0].x = atomicAdd(a.mail.grid_ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!sirec[0].x) return;
+  __threadfence();
+  for (int b = tid; b < h.nb; b += kRdfBlock) a.counts_out[b] = __ldcg(h.counts + b);
+  if (tid == 0) {
+    *a.mail.grid_ticket = 0;
+    mail_status(a.mail);
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (tid == 0) *(volatile int*)(a.mail.words_out + 2) = a.mail.seq;
 }
 
 }  // namespace
@@ -163,7 +181,10 @@ int rdf_ctas_per_sm() { return 6; }
 
 cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st) {
   const size_t smem = sizeof(unsigned) * (size_t)a.hist.nb;
-  auto* k = a.hist.mode == 0 ? k_rdf<0> : a.hist.mode == 1 ? k_rdf<1> : k_rdf<2>;
+  const bool mail = a.mail.seq != 0;
+  auto* k = a.hist.mode == 0   ? (mail ? k_rdf<0, true> : k_rdf<0, false>)
+            : a.hist.mode == 1 ? (mail ? k_rdf<1, true> : k_rdf<1, false>)
+                               : (mail ? k_rdf<2, true> : k_rdf<2, false>);
   return launch_dependent(k, grid, kRdfBlock, smem, st, a);
 }
 

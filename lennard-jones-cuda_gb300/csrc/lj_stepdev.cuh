@@ -356,6 +356,15 @@ __device__ __noinline__ void fused_block_step(const StateArgs& s, int B, double*
   }
 }
 
+// The status word and a queued upload's check to the host.  One thread.
+__device__ __forceinline__ void mail_status(const Mailbox& mb) {
+  mb.words_out[0] = *(volatile const int*)mb.status;
+  if (mb.bad) {
+    mb.words_out[1] = *mb.bad;
+    *mb.bad = 0x7f7f7f7f;  // read: ready for the next upload's check
+  }
+}
+
 // End of a MODE_FORCES_ONLY kernel: the CTA's share of sum_i sum_j s r^2 (in
 // thread 0) into row_part; the last CTA adds them: pressure = (4/6) of the sum
 // (MDSystem.cu:105-108, 136).  Block-wide call.

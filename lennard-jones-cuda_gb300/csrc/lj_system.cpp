@@ -282,6 +282,7 @@ struct lj_system {
   long long rdf_samples = 0;
   // CTA ranges of the pair-histogram pass (they depend on N alone)
   int hist_grid = 0;  // 0: not built yet
+  PinnedBuf<unsigned long long> h_hist;  // counts of a histogram call, written by its pass
   DevBuf<int> h_cta_block, h_cta_chunk, h_cta_units;
 
   cudaStream_t own_stream = nullptr;
@@ -634,7 +635,7 @@ lj_status rdf_pass(lj_system* s, const int4* q, const HistArgs& h, RdfPass* out)
     s->h_cta_units.swap(cu);
     s->hist_grid = r.G;
   }
-  *out = RdfPass{q, s->sc.p, s->cfg[0].n, s->h_cta_block.p, s->h_cta_chunk.p, s->h_cta_units.p, h};
+  *out = RdfPass{q, s->sc.p, s->cfg[0].n, s->h_cta_block.p, s->h_cta_chunk.p, s->h_cta_units.p, h, {}, nullptr};
   return LJ_OK;
 }
 
@@ -1272,6 +1273,7 @@ lj_status lj_destroy(lj_system* s) {
   s->status.free();
   s->records.free();
   s->hist.free();
+  s->h_hist.free();
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   delete s;
   return LJ_OK;
@@ -1823,9 +1825,11 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   if (!(width > 0)) return fail(s, LJ_ERR_INVALID, "bin width must be > 0");
   if (s->nsys != 1) return fail(s, LJ_ERR_UNSUPPORTED, "RDF counts apply to single-box handles");
   DeviceGuard device_guard(s->device);
-  lj_status st = enqueue_shadow(s);
+  // (pending observables may flag the status, which comes back with the counts)
+  lj_status st = flush_observables(s);
   if (st) return st;
   LJ_CUDA(s, cudaMemsetAsync(s->hist.p, 0, sizeof(unsigned long long) * nbins, s->stream));
+  if ((st = enqueue_shadow(s))) return st;
   HistArgs h{};
   h.mode = mode;
   h.nb = nbins;
@@ -1844,10 +1848,30 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   RdfPass p{};
   st = rdf_pass(s, pair_args(s).q, h, &p);
   if (st) return st;
+  if (!s->h_hist.p) LJ_CUDA(s, s->h_hist.alloc(kMaxHistBins));
+  if (s->h_words.dev && s->h_hist.dev) {
+    // the pass's last CTA hands counts and status over: no copy is queued, and
+    // the host waits on the completion word (as for the read-back launch)
+    p.mail.status = s->status.p;
+    p.mail.bad = s->upload_check_pending ? s->bad.p : nullptr;
+    if (p.mail.bad) s->bad_clean = true;
+    p.mail.words_out = static_cast<int*>(s->h_words.dev);
+    p.mail.grid_ticket = s->mb_ticket.p + 1;
+    s->mb_seq = s->mb_seq == INT32_MAX ? 1 : s->mb_seq + 1;
+    p.mail.seq = s->mb_seq;
+    p.counts_out = static_cast<unsigned long long*>(s->h_hist.dev);
+    *(volatile int*)(s->h_words.p + 2) = 0;
+    LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
+    s->launches += 1;
+    s->mb_wait = p.mail.seq;
+    st = finish_status(s);
+    std::memcpy(counts, s->h_hist.p, sizeof(unsigned long long) * nbins);
+    return st;
+  }
   LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
   s->launches += 1;
   // the status word first: the copy into pageable memory returns once both are there
-  if ((st = flush_observables(s)) || (st = enqueue_status_read(s))) return st;
+  if ((st = enqueue_status_read(s))) return st;
   LJ_CUDA(s, cudaMemcpyAsync(counts, s->hist.p, sizeof(unsigned long long) * nbins, cudaMemcpyDeviceToHost,
                              s->stream));
   return finish_status(s);
