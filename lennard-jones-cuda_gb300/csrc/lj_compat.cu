@@ -269,9 +269,9 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   if (!ensure_ctx(n, block_size > 0 ? block_size : 128)) return false;
   CompatCtx& c = g_ctx;
   const float4* pos = reinterpret_cast<const float4*>(Pos);
-  REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
+  REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));
   if (want_rdf)
     REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}, {}, nullptr},
                          c.rdf_grid, c.stream));
