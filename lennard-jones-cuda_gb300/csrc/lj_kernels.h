@@ -94,6 +94,15 @@ cudaError_t launch_pairs_fused(int shape, int mode, const FusedPairArgs& a, int 
 // Integrator / reduction kernels (lj_integrate.cu).  All operate on the
 // i-block decomposition: grid = number of blocks, blockDim = BI.
 // ---------------------------------------------------------------------------
+// Where the last CTA of a MODE_FORCES_ONLY launch copies a call's results:
+// `words` of src to host memory at dst, then a 1 into *done.
+struct ResultMail {
+  const int* src;
+  int* dst;
+  int words;
+  int* done;
+};
+
 struct StateArgs {
   double* x;        // 3 x Npad, component-major (x | y | z)
   double* v;        // 3 x Npad
@@ -124,6 +133,7 @@ struct StateArgs {
   double* row_part;            // row step (lj_rows.cu): 8 partial sums per CTA, in place of blk_part
   float4* force4;              // MODE_FORCES_ONLY of the row and unordered-pair kernels: (F, sum r^-12 - r^-6),
   float* pressure;             // and (4/6) sum s r^2, as calculateNForces returns them (ticket: blk_cnt[0])
+  const ResultMail* mail;      // MODE_FORCES_ONLY: may be null
   int ticket;                  // fused: glob_cnt index of this step's pending-observables tickets (2 or 3)
 };
 

@@ -385,6 +385,14 @@ __device__ __forceinline__ void forces_only_finish(const StateArgs& s, double sh
     *s.pressure = (float)(sum * 4.0 / 6.0);
     s.blk_cnt[0] = 0;
   }
+  if (!s.mail) return;
+  const ResultMail m = *s.mail;
+  __threadfence();
+  __syncwarp();
+  for (int k = threadIdx.x; k < m.words; k += 32) m.dst[k] = __ldcg(m.src + k);
+  __threadfence_system();
+  __syncwarp();
+  if (threadIdx.x == 0) *(volatile int*)m.done = 1;
 }
 
 }  // namespace ljgb
