@@ -3,7 +3,7 @@
  *
  * One handle (lj_system) owns one simulation box on one GPU: FP64 positions
  * and velocities resident in HBM, the FP32/fixed-point shadow the pair
- * kernel reads, forces, observables and the step graphs.  Every entry point
+ * kernel reads, forces and observables.  Every entry point
  * returns an lj_status (0 = LJ_OK) and never exits the process; the message
  * of the last failure on a handle is available from lj_last_error().
  *
@@ -173,7 +173,7 @@ lj_status lj_compute_forces(lj_system* sys);
 /* MDSystem::Integrate(dt) nsteps times (MDSystem.cpp:438-583): velocity
  * Verlet (EVN) or constant-kinetic-temperature Verlet (TVN), boundary
  * handling, observables and running averages every step.  Enqueued on the
- * handle's stream as CUDA graphs; returns once enqueued.  Errors of the
+ * handle's stream; returns once enqueued.  Errors of the
  * device work surface at the next lj_sync / lj_get_* call. */
 lj_status lj_step(lj_system* sys, double dt, int32_t nsteps);
 
@@ -253,7 +253,8 @@ lj_status lj_split_info(lj_system* sys, int32_t* cap, int32_t* ctas, int32_t* ma
 /* Device-time profiling.  When enabled, each pair-kernel launch inside
  * lj_step / lj_compute_forces is bracketed by CUDA events on the handle's
  * stream; lj_profile_read returns the launch count and summed milliseconds
- * of the pair kernel and of the whole step graph since the last reset. */
+ * of the pair kernel (with the launch that sums its parts, where there is one)
+ * and of the whole step since the last reset. */
 lj_status lj_profile_enable(lj_system* sys, int32_t on);
 lj_status lj_profile_read(lj_system* sys, int64_t* pair_launches, double* pair_ms,
                           int64_t* steps, double* step_ms);

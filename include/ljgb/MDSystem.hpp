@@ -133,7 +133,7 @@ class MDSystem {
   void setBoundaryCondition(int cond);
 
   // ---- extensions ----
-  // n steps in one call (one graph launch per step, observables read once).
+  // n steps in one call (observables read once).
   void Integrate(double dt, int nsteps);
   void setHostMirror(bool on) { m_mirror = on; }
   bool hostMirror() const { return m_mirror; }

@@ -330,10 +330,9 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
     REF_CHECK(cudaGetLastError());
   }
   // The results come by the launch's own stores and its completion word (N =
-  // 8000 with RDF: 98.5 us a call with a copy behind it, 95 so; N = 1000 without 39
-  // -> 28); a word that
-  // does not come within 20 ms, and the stream-K kernel's results, by a copy into
-  // page-locked memory.
+  // 8000 with RDF: 98.5 us a call with a copy behind it, 95 so; N = 1000 without
+  // 39 -> 28).  If the word does not come within 20 ms, and with the stream-K
+  // kernel, they come by a copy into page-locked memory.
   RefResult* const r = c.host_result;
   bool here = false;
   if (c.mail) {

@@ -49,7 +49,7 @@ enum : int {
 
 // Per-system frame of the fixed-point shadow and the scalar state that the
 // kernels update on the device.  One per simulated box; kept in device memory
-// so captured step graphs read current values.
+// so queued and captured launches read current values.
 struct DevScalars {
   // fixed-point frame: q = frac((x - origin)/P) * 2^32
   double origin[3];

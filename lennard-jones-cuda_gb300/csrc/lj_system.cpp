@@ -4,7 +4,8 @@
 // One lj_system owns one or more boxes (a batch shares one persistent pair
 // launch per step).  Host code never loops over particles except to sample the
 // initial state; all per-step work runs in the kernels of lj_pairs.cu and
-// lj_integrate.cu, enqueued on the handle's stream as captured CUDA graphs.
+// lj_integrate.cu, enqueued on the handle's stream one after another (profiled
+// steps: as captured CUDA graphs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1548,8 +1549,9 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
   // graphs -> so: 20 FP64 steps of 512 particles with counters and histogram 763
   // -> 724, a step of an open box of 400 36.3 -> 32.5, ten steps of 8 boxes of
   // 100 to 300 in all 255 -> 228).  (A profiled step keeps its graph for the
-  // events; a stream being captured does too, as single launches would be
-  // recorded with this call's step parity.)
+  // events.  On a stream that is being captured the graphs' route refuses the
+  // call, as it always did: single launches would be recorded with this call's
+  // step parity.)
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
   const bool plain = !s->profiling && capture == cudaStreamCaptureStatusNone;

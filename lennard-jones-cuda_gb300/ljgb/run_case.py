@@ -4,8 +4,7 @@
         --tvn --fcc --jitter 0.02 --steps 10
 
 The counterpart of the reference's task drivers (src/tasks/*) for quick runs
-and for profiling a fixed workload (every step is one CUDA-graph launch of
-the drift / pair / reduce / thermostat / observable kernels).
+and for profiling a fixed workload.
 """
 import argparse
 import os
