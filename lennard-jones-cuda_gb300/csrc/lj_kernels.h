@@ -74,6 +74,25 @@ struct RdfPass {
   unsigned long long* counts_out;
 };
 int rdf_ctas_per_sm();
+// The same by tiles of neighbours (four launches, always with a.mail).  Sorting
+// costs about 20 us, so the line lies where the pairs left out are worth more.
+// us a call at reach / L, all pairs -> near tiles, particles in lattice order
+// (shuffled: 5 to 20% more for all pairs, the same for near tiles): N = 8192 at
+// 0.15 40 -> 47; N = 16384 at 0.15 95 -> 56, 0.25 108 -> 95, 0.35 120 -> 129; N =
+// 32768 at 0.15 296 -> 144, 0.35 380 -> 368, 0.4 402 -> 443; N = 40000 at 0.15 435
+// -> 183, 0.35 556 -> 442.  (A droplet within the reach leaves nothing out.)
+struct RdfNear {
+  int* cells;    // kRdfCells, 0 before
+  int* rank;     // n: place within the cell
+  int4* sorted;  // n
+  uint2* box;    // 3 per tile of 32
+};
+constexpr int kRdfCells = 4096;
+constexpr int kRdfNearMaxN = 1 << 20;  // a CTA's 32-bit counts
+inline bool rdf_near(int n, double reach, double L) {
+  return n >= 16384 && n <= kRdfNearMaxN && reach <= (n >= 32768 ? 0.35 : 0.25) * L;
+}
+cudaError_t launch_rdf_near(const RdfPass& a, const RdfNear& s, bool periodic, int grid, cudaStream_t st);
 cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st);
 
 struct PairShape {

@@ -75,6 +75,25 @@ __device__ __forceinline__ void bin_pair(const int4 qi, const int4 qj, float bou
   }
 }
 
+// The pass's end: its last CTA hands counts and status words to the host.
+__device__ __forceinline__ void mail_counts(const RdfPass& a, int* flag) {
+  const int tid = threadIdx.x;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) *flag = atomicAdd(a.mail.grid_ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!*flag) return;
+  __threadfence();
+  for (int b = tid; b < a.hist.nb; b += kRdfBlock) a.counts_out[b] = __ldcg(a.hist.counts + b);
+  if (tid == 0) {
+    *a.mail.grid_ticket = 0;
+    mail_status(a.mail);
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (tid == 0) *(volatile int*)(a.mail.words_out + 2) = a.mail.seq;
+}
+
 // Each unordered pair once: block b of 256 i's (one per thread) runs over the
 // j's from its own first particle on and skips j <= i inside its own square;
 // the wrapping difference is antisymmetric, so (j, i) falls into the bin of
@@ -156,21 +175,154 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf(RdfPass a) {
     }
   }
   flush();
-  if (!MAIL) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) sirec[0].x = atomicAdd(a.mail.grid_ticket, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!sirec[0].x) return;
-  __threadfence();
-  for (int b = tid; b < h.nb; b += kRdfBlock) a.counts_out[b] = __ldcg(h.counts + b);
-  if (tid == 0) {
-    *a.mail.grid_ticket = 0;
-    mail_status(a.mail);
+  if (MAIL) mail_counts(a, &sirec[0].x);
+}
+
+// ---------------------------------------------------------------------------
+// Short-ranged histograms of large boxes: the particles are sorted into cells
+// of 1/16 of the frame in Morton order, so 32 consecutive ones (a tile) lie
+// together, and pairs of tiles that are too far apart are left out.  The test
+// is exact: the gap of two tiles' bounds, circular as the wrapping difference
+// is, goes through the pairs' own roundings, which are monotonic.
+// ---------------------------------------------------------------------------
+constexpr int kCells = kRdfCells;
+
+// shift: 28 where the frame is the whole 32-bit circle (periodic), 27 where
+// the positions lie in its lower half.
+__device__ __forceinline__ int cell_of(const int4 q, int shift) {
+  auto spread = [](unsigned c) { return (c & 1u) | (c & 2u) << 2 | (c & 4u) << 4 | (c & 8u) << 6; };
+  return (int)(spread((unsigned)q.x >> shift & 15u) | spread((unsigned)q.y >> shift & 15u) << 1 |
+               spread((unsigned)q.z >> shift & 15u) << 2);
+}
+
+__global__ void __launch_bounds__(kRdfBlock) k_rdf_cells(const int4* q, int n, int shift, RdfNear s) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int i = blockIdx.x * kRdfBlock + threadIdx.x;
+  if (i < n) s.rank[i] = atomicAdd(&s.cells[cell_of(q[i], shift)], 1);
+}
+
+// Every CTA forms the cells' first places itself (a launch less).
+__global__ void __launch_bounds__(kRdfBlock) k_rdf_scatter(const int4* q, int n, int shift, RdfNear s) {
+  __shared__ int first[kCells];
+  __shared__ int wsum[kRdfBlock / 32];
+  constexpr int kPer = kCells / kRdfBlock;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int c[kPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; k += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(s.cells + tid * kPer + k);
+    c[k] = v.x;
+    c[k + 1] = v.y;
+    c[k + 2] = v.z;
+    c[k + 3] = v.w;
   }
-  __threadfence_system();
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) sum += c[k];
+  int incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) wsum[w] = incl;
   __syncthreads();
-  if (tid == 0) *(volatile int*)(a.mail.words_out + 2) = a.mail.seq;
+  int at = incl - sum;
+  for (int k = 0; k < w; ++k) at += wsum[k];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    first[tid * kPer + k] = at;
+    at += c[k];
+  }
+  __syncthreads();
+  const int i = blockIdx.x * kRdfBlock + tid;
+  if (i >= n) return;
+  const int4 r = q[i];
+  s.sorted[first[cell_of(r, shift)] + s.rank[i]] = r;
+}
+
+// Bounds of each tile: a warp a tile.
+__global__ void __launch_bounds__(kRdfBlock) k_rdf_boxes(int n, RdfNear s) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int t = (blockIdx.x * kRdfBlock + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (t * 32 >= n) return;
+  const int4 r = s.sorted[min(t * 32 + lane, n - 1)];
+  const unsigned v[3] = {(unsigned)r.x, (unsigned)r.y, (unsigned)r.z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const uint2 b = make_uint2(__reduce_min_sync(0xffffffffu, v[c]), __reduce_max_sync(0xffffffffu, v[c]));
+    if (lane == 0) s.box[t * 3 + c] = b;
+  }
+}
+
+// Least circular distance of two intervals.
+__device__ __forceinline__ unsigned gap(uint2 a, uint2 b) {
+  const unsigned lo = max(a.x, b.x), hi = min(a.y, b.y);
+  if (lo <= hi) return 0u;
+  return min(lo - hi, 0u - (max(a.y, b.y) - min(a.x, b.x)));
+}
+
+// A unit is a tile of i's (one a lane) against a group of 8 tiles of j's, from
+// its own tile on; units go round the warps of the grid.  Bound by issue as
+// k_rdf where the reach is long, by the tiles' loads where it is short.
+template <int MODE>
+__global__ void __launch_bounds__(kRdfBlock, 6) k_rdf_near(RdfPass a, RdfNear s) {
+  extern __shared__ unsigned shist[];
+  __shared__ int4 tile[kRdfBlock / 32][32];
+  __shared__ int4 sirec[kRdfBlock];
+  constexpr int kGroup = 8;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const HistArgs h = a.hist;
+  const int last = h.nb - 1;
+  for (int b = tid; b < h.nb; b += kRdfBlock) shist[b] = 0u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float k2 = a.sc->k2;
+  const float bound = bin_bound<MODE>(k2, h.inv_w, MODE == 2 ? h.rmax2 : (float)(MODE == 1 ? h.nb : last));
+  __syncthreads();
+  const int tiles = (a.n + 31) / 32, groups = (tiles + kGroup - 1) / kGroup;
+  for (long long u = (long long)w * gridDim.x + blockIdx.x; u < (long long)tiles * groups;
+       u += (long long)gridDim.x * (kRdfBlock / 32)) {
+    const int I = (int)(u / groups), g = (int)(u - (long long)I * groups);
+    if ((g + 1) * kGroup <= I) continue;
+    const int mine = g * kGroup + lane;
+    bool near = false;
+    if (lane < kGroup && mine >= I && mine < tiles) {
+      const float gx = __uint2float_rn(gap(s.box[I * 3], s.box[mine * 3]));
+      const float gy = __uint2float_rn(gap(s.box[I * 3 + 1], s.box[mine * 3 + 1]));
+      const float gz = __uint2float_rn(gap(s.box[I * 3 + 2], s.box[mine * 3 + 2]));
+      near = __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, __fmul_rn(gx, gx))) < bound;
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, near);
+    if (!todo) continue;
+    const int i = I * 32 + lane;
+    const int4 qi = i_record_slots123(s.sorted[min(i, a.n - 1)], &sirec[tid]);
+    for (; todo; todo &= todo - 1) {
+      const int J = g * kGroup + __ffs(todo) - 1, cnt = min(32, a.n - J * 32);
+      __syncwarp();
+      tile[w][lane] = s.sorted[min(J * 32 + lane, a.n - 1)];
+      __syncwarp();
+      if (i >= a.n) continue;
+      if (J > I && cnt == 32) {
+#pragma unroll 8
+        for (int jj = 0; jj < 32; ++jj) bin_pair<MODE>(qi, tile[w][jj], bound, k2, h.inv_w, last, shist);
+      } else {
+        for (int jj = 0; jj < cnt; ++jj)
+          if (J > I || jj > lane) bin_pair<MODE>(qi, tile[w][jj], bound, k2, h.inv_w, last, shist);
+      }
+    }
+  }
+  __syncthreads();
+  unsigned counted = 0;
+  for (int b = tid; b < h.nb; b += kRdfBlock)
+    if (shist[b]) {
+      counted += shist[b];
+      atomicAdd(h.counts + b, 2ull * shist[b]);
+    }
+  if (MODE == 0) {  // the last bin's are all pairs less the counted ones
+    const unsigned binned = __reduce_add_sync(0xffffffffu, counted);
+    if (lane == 0 && binned) atomicAdd(h.counts + last, 0ull - 2ull * binned);
+    if (tid == 0 && blockIdx.x == 0) atomicAdd(h.counts + last, (unsigned long long)a.n * (a.n - 1));
+  }
+  mail_counts(a, &sirec[0].x);
 }
 
 }  // namespace
@@ -186,6 +338,16 @@ cudaError_t launch_rdf(const RdfPass& a, int grid, cudaStream_t st) {
             : a.hist.mode == 1 ? (mail ? k_rdf<1, true> : k_rdf<1, false>)
                                : (mail ? k_rdf<2, true> : k_rdf<2, false>);
   return launch_dependent(k, grid, kRdfBlock, smem, st, a);
+}
+
+cudaError_t launch_rdf_near(const RdfPass& a, const RdfNear& s, bool periodic, int grid, cudaStream_t st) {
+  const int shift = periodic ? 28 : 27, nb = (a.n + kRdfBlock - 1) / kRdfBlock;
+  cudaError_t e = launch_dependent(k_rdf_cells, nb, kRdfBlock, 0, st, a.q, a.n, shift, s);
+  if (e == cudaSuccess) e = launch_dependent(k_rdf_scatter, nb, kRdfBlock, 0, st, a.q, a.n, shift, s);
+  if (e == cudaSuccess) e = launch_dependent(k_rdf_boxes, nb, kRdfBlock, 0, st, a.n, s);
+  if (e != cudaSuccess) return e;
+  auto* k = a.hist.mode == 0 ? k_rdf_near<0> : a.hist.mode == 1 ? k_rdf_near<1> : k_rdf_near<2>;
+  return launch_dependent(k, grid, kRdfBlock, sizeof(unsigned) * (size_t)a.hist.nb, st, a, s);
 }
 
 }  // namespace ljgb

@@ -283,6 +283,9 @@ struct lj_system {
   long long rdf_samples = 0;
   // CTA ranges of the pair-histogram pass (they depend on N alone)
   int hist_grid = 0;  // 0: not built yet
+  DevBuf<int> near_cells, near_rank;  // short-ranged histograms of large boxes (RdfNear)
+  DevBuf<int4> near_sorted;
+  DevBuf<uint2> near_box;
   PinnedBuf<unsigned long long> h_hist;  // counts of a histogram call, written by its pass
   DevBuf<int> h_cta_block, h_cta_chunk, h_cta_units;
 
@@ -1275,6 +1278,10 @@ lj_status lj_destroy(lj_system* s) {
   s->records.free();
   s->hist.free();
   s->h_hist.free();
+  s->near_cells.free();
+  s->near_rank.free();
+  s->near_sorted.free();
+  s->near_box.free();
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   delete s;
   return LJ_OK;
@@ -1830,6 +1837,20 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   // (pending observables may flag the status, which comes back with the counts)
   lj_status st = flush_observables(s);
   if (st) return st;
+  if (!s->h_hist.p) LJ_CUDA(s, s->h_hist.alloc(kMaxHistBins));
+  const bool mapped = s->h_words.dev && s->h_hist.dev;
+  const int n = s->cfg[0].n;
+  const double rmax = mode == 2 ? nbins * width : std::sqrt(nbins * width);
+  const bool near_tiles = mapped && rdf_near(n, rmax, s->boxes[0].L);
+  if (near_tiles) {
+    if (!s->near_cells.p) {
+      LJ_CUDA(s, s->near_rank.alloc(n));
+      LJ_CUDA(s, s->near_sorted.alloc(n));
+      LJ_CUDA(s, s->near_box.alloc(3 * (size_t)((n + 31) / 32)));
+      LJ_CUDA(s, s->near_cells.alloc(kRdfCells));
+    }
+    LJ_CUDA(s, cudaMemsetAsync(s->near_cells.p, 0, sizeof(int) * kRdfCells, s->stream));
+  }
   LJ_CUDA(s, cudaMemsetAsync(s->hist.p, 0, sizeof(unsigned long long) * nbins, s->stream));
   if ((st = enqueue_shadow(s))) return st;
   HistArgs h{};
@@ -1850,8 +1871,7 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   RdfPass p{};
   st = rdf_pass(s, pair_args(s).q, h, &p);
   if (st) return st;
-  if (!s->h_hist.p) LJ_CUDA(s, s->h_hist.alloc(kMaxHistBins));
-  if (s->h_words.dev && s->h_hist.dev) {
+  if (mapped) {
     // the pass's last CTA hands counts and status over: no copy is queued, and
     // the host waits on the completion word (as for the read-back launch)
     p.mail.status = s->status.p;
@@ -1863,8 +1883,14 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
     p.mail.seq = s->mb_seq;
     p.counts_out = static_cast<unsigned long long*>(s->h_hist.dev);
     *(volatile int*)(s->h_words.p + 2) = 0;
-    LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
-    s->launches += 1;
+    if (near_tiles) {
+      const RdfNear near{s->near_cells.p, s->near_rank.p, s->near_sorted.p, s->near_box.p};
+      LJ_CUDA(s, launch_rdf_near(p, near, s->boxes[0].bc == 0, s->num_sms * rdf_ctas_per_sm(), s->stream));
+      s->launches += 4;
+    } else {
+      LJ_CUDA(s, launch_rdf(p, s->hist_grid, s->stream));
+      s->launches += 1;
+    }
     s->mb_wait = p.mail.seq;
     st = finish_status(s);
     std::memcpy(counts, s->h_hist.p, sizeof(unsigned long long) * nbins);
