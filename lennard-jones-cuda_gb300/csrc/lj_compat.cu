@@ -107,8 +107,9 @@ struct CompatCtx {
   // ... or the stream-K kernel's schedule
   BlockInfo* blocks = nullptr;
   int *ctb = nullptr, *clo = nullptr, *cb = nullptr, *cj = nullptr;
-  int rdf_grid = 0;
+  int rdf_grid = 0, num_sms = 0;
   int *rb = nullptr, *rc = nullptr, *ru = nullptr;  // ranges of the histogram pass
+  RdfNear near{};                                   // large boxes: its tiles of neighbours
   float* partial = nullptr;
   double* blk = nullptr;
   RefResult* result = nullptr;       // device
@@ -131,6 +132,10 @@ struct CompatCtx {
     cudaFree(rb);
     cudaFree(rc);
     cudaFree(ru);
+    cudaFree(near.cells);
+    cudaFree(near.rank);
+    cudaFree(near.sorted);
+    cudaFree(near.box);
     cudaFree(partial);
     cudaFree(blk);
     cudaFree(result);
@@ -199,6 +204,7 @@ bool ensure_ctx(int n, int block_hint) {
   c.n = n;
   c.shape = shape;
   c.nb_bbox = (n + kBlk - 1) / kBlk;
+  c.num_sms = sms;
   // Buffers of the new context; on any failure everything allocated so far
   // is freed and the layer is left without a context (the next call retries).
   auto build = [&]() -> bool {
@@ -213,6 +219,12 @@ bool ensure_ctx(int n, int block_hint) {
     REF_CHECK(device_alloc((void**)&c.rb, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.rc, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.ru, sizeof(int) * rr.G));
+    if (rdf_near(n, 0.0, 1.0)) {
+      REF_CHECK(device_alloc((void**)&c.near.cells, sizeof(int) * kRdfCells));
+      REF_CHECK(device_alloc((void**)&c.near.rank, sizeof(int) * n));
+      REF_CHECK(device_alloc((void**)&c.near.sorted, sizeof(int4) * n));
+      REF_CHECK(device_alloc((void**)&c.near.box, sizeof(uint2) * 3 * (size_t)((n + 31) / 32)));
+    }
     // 8 doubles per CTA, i-block, tile or bounding-box CTA, whichever are most
     REF_CHECK(device_alloc((void**)&c.blk, sizeof(double) * 8 * (size_t)std::max({nb, c.nb_bbox, (n + 31) / 32, sms})));
     if (stream_k) {
@@ -287,11 +299,16 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   CompatCtx& c = g_ctx;
   const float4* pos = reinterpret_cast<const float4*>(Pos);
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
+  const bool near = want_rdf && rdf_near(n, std::sqrt((double)kRefBins * dr2), L);
+  if (near) REF_CHECK(cudaMemsetAsync(c.near.cells, 0, sizeof(int) * kRdfCells, c.stream));
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
   REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));
-  if (want_rdf)
-    REF_CHECK(launch_rdf(RdfPass{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}, {}, nullptr},
-                         c.rdf_grid, c.stream));
+  const RdfPass rdf{c.q, c.sc, n, c.rb, c.rc, c.ru, HistArgs{0, kRefBins, 1.0f / dr2, 0.0f, c.result->hist}, {}, nullptr};
+  if (near) {
+    REF_CHECK(launch_rdf_near(rdf, c.near, periodic != 0, c.num_sms * rdf_ctas_per_sm(), c.stream));
+  } else if (want_rdf) {
+    REF_CHECK(launch_rdf(rdf, c.rdf_grid, c.stream));
+  }
   // set by the last CTA once the results are in host memory
   volatile int* const done = reinterpret_cast<volatile int*>(c.host_result + 1);
   if (c.rows.ctas > 0 || c.newton > 0) {

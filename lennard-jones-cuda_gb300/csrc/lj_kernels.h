@@ -74,7 +74,7 @@ struct RdfPass {
   unsigned long long* counts_out;
 };
 int rdf_ctas_per_sm();
-// The same by tiles of neighbours (four launches, always with a.mail).  Sorting
+// The same by tiles of neighbours (four launches; without a.mail mode 0 alone).  Sorting
 // costs about 20 us, so the line lies where the pairs left out are worth more.
 // us a call at reach / L, all pairs -> near tiles, particles in lattice order
 // (shuffled: 5 to 20% more for all pairs, the same for near tiles): N = 8192 at

@@ -264,7 +264,7 @@ __device__ __forceinline__ unsigned gap(uint2 a, uint2 b) {
 // A unit is a tile of i's (one a lane) against a group of 8 tiles of j's, from
 // its own tile on; units go round the warps of the grid.  Bound by issue as
 // k_rdf where the reach is long, by the tiles' loads where it is short.
-template <int MODE>
+template <int MODE, bool MAIL>
 __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf_near(RdfPass a, RdfNear s) {
   extern __shared__ unsigned shist[];
   __shared__ int4 tile[kRdfBlock / 32][32];
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kRdfBlock, 6) k_rdf_near(RdfPass a, RdfNear s)
     if (lane == 0 && binned) atomicAdd(h.counts + last, 0ull - 2ull * binned);
     if (tid == 0 && blockIdx.x == 0) atomicAdd(h.counts + last, (unsigned long long)a.n * (a.n - 1));
   }
-  mail_counts(a, &sirec[0].x);
+  if (MAIL) mail_counts(a, &sirec[0].x);
 }
 
 }  // namespace
@@ -346,7 +346,12 @@ cudaError_t launch_rdf_near(const RdfPass& a, const RdfNear& s, bool periodic, i
   if (e == cudaSuccess) e = launch_dependent(k_rdf_scatter, nb, kRdfBlock, 0, st, a.q, a.n, shift, s);
   if (e == cudaSuccess) e = launch_dependent(k_rdf_boxes, nb, kRdfBlock, 0, st, a.n, s);
   if (e != cudaSuccess) return e;
-  auto* k = a.hist.mode == 0 ? k_rdf_near<0> : a.hist.mode == 1 ? k_rdf_near<1> : k_rdf_near<2>;
+  // (a pass that leaves its counts on the device is calculateNForces', mode 0)
+  auto* k = a.mail.seq == 0     ? k_rdf_near<0, false>
+            : a.hist.mode == 0 ? k_rdf_near<0, true>
+            : a.hist.mode == 1 ? k_rdf_near<1, true>
+                               : k_rdf_near<2, true>;
+  if (a.mail.seq == 0 && a.hist.mode != 0) return cudaErrorInvalidValue;
   return launch_dependent(k, grid, kRdfBlock, sizeof(unsigned) * (size_t)a.hist.nb, st, a, s);
 }
 

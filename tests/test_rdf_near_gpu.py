@@ -2,6 +2,8 @@
 counts are whole numbers, so equal to the exact emulation (periodic boxes), and
 to the full pass elsewhere -- the same box with more bins, which reach too far
 for tiles to be left out."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -54,3 +56,26 @@ def test_near_tiles_match_the_full_pass(ljgb_mod, boundary, mode):
     if mode == 0:
         assert near.sum() == full.sum() == N * (N - 1)
     s.close()
+
+
+@pytest.mark.parametrize("n", [16385, 20001])
+def test_reference_call_counts(ljgb_mod, oracle_mod, n):
+    lib = ljgb_mod.load()
+    pos, _, L = _positions("shuffled", n, 0.5, n)
+    p4, L = np.zeros((n, 4), np.float32), float(np.float32(L))
+    p4[:, :3] = pos
+    d_pos, d_frc, rdf, press = C.c_void_p(), C.c_void_p(), np.zeros(256, np.int32), C.c_float()
+    lib.allocateArray(C.byref(d_pos), n)
+    lib.allocateArray(C.byref(d_frc), n)
+    lib.copyArrayToDevice(d_pos, p4.ctypes.data, n)
+    ks = L / 4294967296.0
+    want = oracle_mod.emu_rdf_r2(oracle_mod.emu_fixed(p4[:, :3].astype(np.float64), L), np.float32(ks * ks),
+                                 np.float32(1.0) / np.float32(0.1), 256, 0)
+    for _ in range(2):
+        lib.calculateNForces(d_pos, d_frc, C.byref(press), n, C.c_float(L), 1, rdf.ctypes.data, C.c_float(0.1), 128, 1)
+        assert lib.lj_reference_abi_status() == 0 and np.array_equal(rdf, want)
+    lib.calculateNForces(d_pos, d_frc, C.byref(press), n, C.c_float(L), 0, rdf.ctypes.data, C.c_float(0.1), 128, 1)
+    assert rdf.sum() == n * (n - 1)
+    lib.deleteArray(d_pos)
+    lib.deleteArray(d_frc)
+    lib.threadExit()
