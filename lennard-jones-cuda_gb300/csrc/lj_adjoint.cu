@@ -223,7 +223,7 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
     for (int m = 0; m < kS; ++m) a.scal[(size_t)blockIdx.x * kScalars + m] = S[m];
 }
 
-// FP64-pipe bound.  N = 1000: 37 us forward, 65 us reverse (79 and 142 over
+// FP64-pipe bound.  N = 1000: 34 us forward, 60 us reverse (79 and 142 over
 // ordered pairs).
 template <bool HVP>
 __global__ void __launch_bounds__(256) k_adj_pairs(AdjBox b, AdjPass a, const double* __restrict__ x,

@@ -31,7 +31,7 @@ namespace {
 // unordered pair with sigma = 1 (3 differences, 3 images, 3 r^2, 3 reciprocal,
 // 5 powers and force factor, 6 force sums, 4 energy sums), against 2 x 36 of
 // the loop over ordered pairs that this kernel replaced (IEEE division,
-// product-round-fma images).  N = 2048: 355 -> 115 us; N = 512: 103 -> 14 us.
+// product-round-fma images).  N = 2048: 355 -> 114 us; N = 512: 103 -> 13 us.
 struct Sums64 {
   double x, y, z, a, b;  // s d, (s/r)^12, (s/r)^6
 };
