@@ -50,18 +50,21 @@ __device__ __forceinline__ int fixed_diff(int a, int b) { return (int)((unsigned
 // two operands from registers of opposite parity, which sit in different
 // register-file banks: with both records in slots 0..2 every difference
 // waited on a bank conflict (measured on GB300: 52.5 -> 49.4 cycles per
-// 64-pair warp step of the packed loop).  i_record_slots123 places it.
+// 64-pair warp step of the packed loop).  i_record_slots123 places it by way of
+// *slot, 16 bytes of shared memory that no other thread may touch meanwhile.
 __device__ __forceinline__ int4 i_record_slots123(const int4 q, int4* slot) {
   volatile int4* v = slot;
   v->x = 0;
   v->y = q.x;
   v->z = q.y;
   v->w = q.z;
-  // volatile load: the compiler may not forward the stored registers
+  // volatile load: the compiler may not forward the stored registers, nor move
+  // a later store to the same bytes before it
   int4 r;
   asm volatile("ld.volatile.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "r"((unsigned)__cvta_generic_to_shared(slot)));
+               : "r"((unsigned)__cvta_generic_to_shared(slot))
+               : "memory");
   return r;
 }
 

@@ -138,11 +138,15 @@ __global__ void __launch_bounds__(32 * kWarps, 3) k_newton(NewtonArgs a) {
   int I = tk.block, t = tk.tile, left = tk.count;
   while (left > 0) {
     const int i0 = I * kNewtonBlock, t1 = min(tiles, t + left);
+    // Each i record passes through this lane's own entry of a tile buffer: the
+    // other lanes' last reads of it lie before newton_tile's closing
+    // __syncwarp, and their next ones after the one that follows the tile's own
+    // records.  (Every other array here has lanes reach into each other's.)
     int4 q[kI];
 #pragma unroll
     for (int k = 0; k < kI; ++k) {
       const int4 r = a.q[min(i0 + 32 * k + lane, n - 1)];
-      q[k] = i_record_slots123(r, reinterpret_cast<int4*>(&sh.hi[w][0][0][0]) + lane);
+      q[k] = i_record_slots123(r, &sh.tile[w][0][lane]);
     }
 #pragma unroll
     for (int m = 0; m < kI / 2; ++m)
