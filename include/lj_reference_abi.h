@@ -78,6 +78,12 @@ void threadExit(void);
 int lj_reference_abi_status(void);
 const char* lj_reference_abi_error(void);
 
+/* Testing hook (host side): leaves the cached work buffers as a launch in which
+ * a device-side wait ran out would, the timeout flagged and `tickets` CTAs
+ * counted.  The next calculateNForces reports LJ_ERR_DEVICE_TIMEOUT; the one
+ * after it works again.  0, or LJ_ERR_INVALID before the first call. */
+int lj_debug_reference_abi_timeout(int tickets);
+
 #ifdef __cplusplus
 }
 #endif

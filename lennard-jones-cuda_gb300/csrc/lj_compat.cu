@@ -368,7 +368,12 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   }
   *host_pressure = r->pressure;
   if (r->status) {
-    cudaMemset(&c.result->status, 0, sizeof(int));
+    // A CTA whose wait timed out takes no completion ticket: the count goes back
+    // to 0 as well, behind the launch's last CTA, or the next call's last CTA
+    // would be taken for an earlier one.
+    REF_CHECK(cudaMemsetAsync(&c.result->status, 0, sizeof(int), c.stream));
+    REF_CHECK(cudaMemsetAsync(c.ticket, 0, 2 * sizeof(int), c.stream));
+    REF_CHECK(cudaStreamSynchronize(c.stream));
     g_status = LJ_ERR_DEVICE_TIMEOUT;
     g_error = "calculateNForces: a device-side wait timed out";
     return false;
@@ -464,6 +469,16 @@ void threadExit(void) {
   g_status = 0;
   g_ctx.release();
   record(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+}
+
+int lj_debug_reference_abi_timeout(int tickets) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (!g_ctx.stream) return LJ_ERR_INVALID;
+  const int status = LJ_DEVFLAG_TIMEOUT;
+  if (cudaMemcpy(g_ctx.ticket, &tickets, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(&g_ctx.result->status, &status, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+    return LJ_ERR_CUDA;
+  return LJ_OK;
 }
 
 int lj_reference_abi_status(void) { return g_status; }

@@ -162,6 +162,7 @@ def _declare(L):
         "lj_adjoint_backward": (C.c_int, [_P, _dp, _dp, _P, _P]),
         "lj_reference_abi_status": (C.c_int, []),
         "lj_reference_abi_error": (C.c_char_p, []),
+        "lj_debug_reference_abi_timeout": (C.c_int, [C.c_int]),
     }
     for name, (res, args) in sig.items():
         f = getattr(L, name)
