@@ -42,18 +42,28 @@ static bool allocation_refused() {
   return false;
 }
 
+// A failed allocation is reported by its return value alone: left behind as
+// CUDA's last error, it would be taken for the next launch's.
+static cudaError_t allocated(cudaError_t e, void** p) {
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
+
 namespace ljgb {
 
 cudaError_t device_alloc(void** p, size_t bytes) {
   *p = nullptr;
   if (allocation_refused()) return cudaErrorMemoryAllocation;
-  return cudaMalloc(p, bytes);
+  return allocated(cudaMalloc(p, bytes), p);
 }
 
 cudaError_t pinned_alloc(void** p, size_t bytes) {
   *p = nullptr;
   if (allocation_refused()) return cudaErrorMemoryAllocation;
-  return cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+  return allocated(cudaHostAlloc(p, bytes, cudaHostAllocDefault), p);
 }
 
 }  // namespace ljgb
