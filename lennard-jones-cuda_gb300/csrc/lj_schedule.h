@@ -86,5 +86,8 @@ struct NewtonPlan {
   int iparts = 0;
 };
 NewtonPlan plan_newton(int n, int warps);
+// Whether the plan's sums leave at least as much of the current device's memory
+// free as they take.
+bool newton_fits(const NewtonPlan& p);
 
 }  // namespace ljgb

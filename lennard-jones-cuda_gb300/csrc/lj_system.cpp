@@ -728,13 +728,14 @@ void free_newton(lj_system* s) {
   s->newton_i.free();
 }
 
-// The unordered-pair step's tables and sums, built when the box is created.
-lj_status setup_newton(lj_system* s) {
+// The unordered-pair step's tables and sums.
+lj_status build_newton(lj_system* s) {
   const int n = s->cfg[0].n;
   int per_sm = 0;
   LJ_CUDA(s, newton_setup(&per_sm));
   if (per_sm < 1) return LJ_OK;
   const NewtonPlan p = plan_newton(n, s->num_sms * per_sm * kNewtonWarps);
+  if (!newton_fits(p)) return LJ_ERR_OUT_OF_MEMORY;
   LJ_CUDA(s, s->newton_tasks.alloc(p.tasks.size()));
   LJ_CUDA(s, s->newton_blocks.alloc(p.block_part.size()));
   LJ_CUDA(s, s->newton_j.alloc((size_t)p.jparts * 160));
@@ -746,6 +747,22 @@ lj_status setup_newton(lj_system* s) {
                              cudaMemcpyHostToDevice, s->stream));
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   s->newton = (int)p.tasks.size();
+  return LJ_OK;
+}
+
+// Built for a box in its range unless a stream-K shape was chosen.  Up to 10 KB
+// a particle: a box that cannot have it, or would take more than half of the
+// device's free memory, steps by the stream-K kernel, so this comes last where
+// other buffers are made.
+lj_status setup_newton(lj_system* s) {
+  if (s->nsys != 1 || s->prec != LJ_PREC_MIXED || s->cfg[0].n < kNewtonMinN || s->cfg[0].n > kNewtonMaxN ||
+      s->newton > 0 || s->forced_shape >= 0)
+    return LJ_OK;
+  const std::string err = s->err;
+  const lj_status st = build_newton(s);
+  if (st) free_newton(s);
+  if (st != LJ_ERR_OUT_OF_MEMORY) return st;
+  s->err = err;
   return LJ_OK;
 }
 
@@ -1156,11 +1173,6 @@ lj_status create_impl(const lj_config* cfgs, int nsys, lj_system** out) {
     return bail(fail(s, LJ_ERR_CUDA, "cluster set-up failed"));
   lj_status st = alloc_state(s);
   if (st) return bail(st);
-  if (nsys == 1 && s->prec == LJ_PREC_MIXED && s->cfg[0].n >= kNewtonMinN && s->cfg[0].n <= kNewtonMaxN) {
-    // (without memory for its sums the box steps by the stream-K kernel)
-    if ((st = setup_newton(s)) == LJ_ERR_OUT_OF_MEMORY) free_newton(s);
-    else if (st) return bail(st);
-  }
   st = upload_boxes(s);
   if (st) return bail(st);
   // Shape: the reference's CUDABlockSize picks the nearest i-block size.
@@ -1203,6 +1215,7 @@ lj_status create_impl(const lj_config* cfgs, int nsys, lj_system** out) {
   }
   st = write_scalars(s, sc);
   if (st) return bail(st);
+  if ((st = setup_newton(s))) return bail(st);
   *out = s;
   return LJ_OK;
 }
@@ -2154,7 +2167,8 @@ lj_status lj_set_kernel_shape(lj_system* s, int32_t shape) {
     return st;
   }
   // The i-block length changed: rebuild shadows and the per-block sums.
-  return recompute_forces_keep_scalars(s);
+  if ((st = recompute_forces_keep_scalars(s))) return st;
+  return setup_newton(s);
 }
 
 lj_status lj_set_split_cap(lj_system* s, int32_t cap) {
@@ -2309,6 +2323,7 @@ lj_status lj_autotune(lj_system* s) {
   float rows_ms = 1e30f;
   s->rows_off = false;
   s->forced_shape = -1;  // a block hint gives way to the measurement
+  if ((st = setup_newton(s))) return give_up(st);
   if (use_rows(s) && (st = trial(&rows_ms))) return give_up(st);
   s->rows_off = true;
   int best = 0, best_split = s->split_cap;
