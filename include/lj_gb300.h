@@ -426,6 +426,9 @@ void lj_host_free(void* ptr);
  * histogram range table, record ring or counter table replaces the old one
  * only once complete, and an interrupted autotune puts the state back. */
 lj_status lj_debug_fail_allocations(int64_t after);
+/* The same for allocations of more than `bytes` bytes only, wherever they come:
+ * a large workspace is refused and what takes its place is not.  -1: off. */
+lj_status lj_debug_limit_allocations(int64_t bytes);
 
 /* Library version string and the device architecture it was built for. */
 const char* lj_version(void);

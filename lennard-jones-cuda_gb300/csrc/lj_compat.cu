@@ -152,35 +152,33 @@ CompatCtx g_ctx;
 int g_status = 0;
 std::string g_error;
 
-bool record(cudaError_t e, const char* what) {
+bool record(cudaError_t e, const char* what, bool loud = true) {
   if (e == cudaSuccess) return true;
   g_status = e == cudaErrorMemoryAllocation ? LJ_ERR_OUT_OF_MEMORY : LJ_ERR_CUDA;
   g_error = std::string(what) + ": " + cudaGetErrorString(e);
-  std::fprintf(stderr, "lj_gb300 reference ABI: %s\n", g_error.c_str());
+  if (loud) std::fprintf(stderr, "lj_gb300 reference ABI: %s\n", g_error.c_str());
   return false;
 }
 
+constexpr bool loud = true;  // (build_ctx has one of its own)
 #define REF_CHECK(call) \
-  if (!record((call), #call)) return false
+  if (!record((call), #call, loud)) return false
 
-bool ensure_ctx(int n, int block_hint) {
-  int shape = 0;
-  for (int k = 0; k < kNumShapes; ++k)
-    if (std::abs(kShapes[k].threads - block_hint) < std::abs(kShapes[shape].threads - block_hint)) shape = k;
-  int dev = 0, sms = 0, per_sm = 0;
-  REF_CHECK(cudaGetDevice(&dev));
-  if (g_ctx.n == n && g_ctx.shape == shape && g_ctx.stream && g_ctx.device == dev) return true;
-  if (g_ctx.stream && g_ctx.device != dev) {
-    // The caller switched devices: free the old buffers on their own device.
-    REF_CHECK(cudaSetDevice(g_ctx.device));
-    g_ctx.release();
-    REF_CHECK(cudaSetDevice(dev));
-  } else {
-    g_ctx.release();
-  }
+// A context for n particles on the current device, into g_ctx.  `lean`: without
+// what a call can do without, the unordered pairs' sums (up to 10 KB a particle;
+// the stream-K kernel takes their place) and the histogram's neighbour tiles.
+bool build_ctx(int n, int shape, int dev, bool lean, bool loud) {
+  int sms = 0, per_sm = 0;
   REF_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const RowPlan rows = plan_rows(n, sms);
-  const bool stream_k = n > kNewtonMaxN || (n < kNewtonMinN && rows.ctas == 0);
+  NewtonPlan np;
+  if (!lean && n >= kNewtonMinN && n <= kNewtonMaxN) {
+    int newton_per_sm = 0;
+    REF_CHECK(newton_setup(&newton_per_sm));
+    if (newton_per_sm > 0) np = plan_newton(n, sms * newton_per_sm * kNewtonWarps);
+    if (!newton_fits(np)) np = NewtonPlan();
+  }
+  const bool stream_k = np.tasks.empty() && rows.ctas == 0;
   Schedule s;
   if (stream_k) {
     REF_CHECK(pair_occupancy(shape, &per_sm));
@@ -219,7 +217,7 @@ bool ensure_ctx(int n, int block_hint) {
     REF_CHECK(device_alloc((void**)&c.rb, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.rc, sizeof(int) * rr.G));
     REF_CHECK(device_alloc((void**)&c.ru, sizeof(int) * rr.G));
-    if (rdf_near(n, 0.0, 1.0)) {
+    if (!lean && rdf_near(n, 0.0, 1.0)) {
       REF_CHECK(device_alloc((void**)&c.near.cells, sizeof(int) * kRdfCells));
       REF_CHECK(device_alloc((void**)&c.near.rank, sizeof(int) * n));
       REF_CHECK(device_alloc((void**)&c.near.sorted, sizeof(int4) * n));
@@ -239,20 +237,17 @@ bool ensure_ctx(int n, int block_hint) {
       REF_CHECK(cudaMemcpy(c.clo, s.cta_lo.data(), sizeof(int) * (s.G + 1), cudaMemcpyHostToDevice));
       REF_CHECK(cudaMemcpy(c.cb, s.cta_block.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
       REF_CHECK(cudaMemcpy(c.cj, s.cta_jt.data(), sizeof(int) * s.G, cudaMemcpyHostToDevice));
-    } else if (n < kNewtonMinN) {
+    } else if (rows.ctas > 0) {
       c.rows = rows;
       REF_CHECK(rows_setup());
     } else {
-      int newton_per_sm = 0;
-      REF_CHECK(newton_setup(&newton_per_sm));
-      const NewtonPlan p = plan_newton(n, sms * newton_per_sm * kNewtonWarps);
-      REF_CHECK(device_alloc((void**)&c.newton_tasks, sizeof(NewtonTask) * p.tasks.size()));
-      REF_CHECK(device_alloc((void**)&c.newton_blocks, sizeof(int) * p.block_part.size()));
-      REF_CHECK(device_alloc((void**)&c.newton_j, sizeof(float) * 160 * (size_t)p.jparts));
-      REF_CHECK(device_alloc((void**)&c.newton_i, sizeof(float) * 5 * kNewtonBlock * (size_t)p.iparts));
-      REF_CHECK(cudaMemcpy(c.newton_tasks, p.tasks.data(), sizeof(NewtonTask) * p.tasks.size(), cudaMemcpyHostToDevice));
-      REF_CHECK(cudaMemcpy(c.newton_blocks, p.block_part.data(), sizeof(int) * p.block_part.size(), cudaMemcpyHostToDevice));
-      c.newton = (int)p.tasks.size();
+      REF_CHECK(device_alloc((void**)&c.newton_tasks, sizeof(NewtonTask) * np.tasks.size()));
+      REF_CHECK(device_alloc((void**)&c.newton_blocks, sizeof(int) * np.block_part.size()));
+      REF_CHECK(device_alloc((void**)&c.newton_j, sizeof(float) * 160 * (size_t)np.jparts));
+      REF_CHECK(device_alloc((void**)&c.newton_i, sizeof(float) * 5 * kNewtonBlock * (size_t)np.iparts));
+      REF_CHECK(cudaMemcpy(c.newton_tasks, np.tasks.data(), sizeof(NewtonTask) * np.tasks.size(), cudaMemcpyHostToDevice));
+      REF_CHECK(cudaMemcpy(c.newton_blocks, np.block_part.data(), sizeof(int) * np.block_part.size(), cudaMemcpyHostToDevice));
+      c.newton = (int)np.tasks.size();
     }
     REF_CHECK(device_alloc((void**)&c.result, sizeof(RefResult)));
     REF_CHECK(device_alloc((void**)&c.ticket, 2 * sizeof(int)));
@@ -288,6 +283,35 @@ bool ensure_ctx(int n, int block_hint) {
   return true;
 }
 
+bool ensure_ctx(int n, int block_hint) {
+  int shape = 0;
+  for (int k = 0; k < kNumShapes; ++k)
+    if (std::abs(kShapes[k].threads - block_hint) < std::abs(kShapes[shape].threads - block_hint)) shape = k;
+  int dev = 0;
+  REF_CHECK(cudaGetDevice(&dev));
+  if (g_ctx.n == n && g_ctx.shape == shape && g_ctx.stream && g_ctx.device == dev) return true;
+  if (g_ctx.stream && g_ctx.device != dev) {
+    // The caller switched devices: free the old buffers on their own device.
+    REF_CHECK(cudaSetDevice(g_ctx.device));
+    g_ctx.release();
+    REF_CHECK(cudaSetDevice(dev));
+  } else {
+    g_ctx.release();
+  }
+  // Without the memory for everything, with less (for as long as this context
+  // is kept: until another n, shape or device, or threadExit).
+  const bool can_be_lean = n >= kNewtonMinN;
+  const std::string error = g_error;
+  if (build_ctx(n, shape, dev, false, !can_be_lean)) return true;
+  if (g_status != LJ_ERR_OUT_OF_MEMORY || !can_be_lean) {
+    if (can_be_lean) std::fprintf(stderr, "lj_gb300 reference ABI: %s\n", g_error.c_str());
+    return false;
+  }
+  g_status = 0;
+  g_error = error;
+  return build_ctx(n, shape, dev, true, true);
+}
+
 bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L, int periodic, int* host_RDF,
                  float dr2, int block_size) {
   if (!Pos || !Force || !host_pressure || n < 2) {
@@ -299,7 +323,7 @@ bool calc_forces(float* Pos, float* Force, float* host_pressure, int n, float L,
   CompatCtx& c = g_ctx;
   const float4* pos = reinterpret_cast<const float4*>(Pos);
   const bool want_rdf = host_RDF != nullptr && dr2 > 0.0f;
-  const bool near = want_rdf && rdf_near(n, std::sqrt((double)kRefBins * dr2), L);
+  const bool near = want_rdf && c.near.cells && rdf_near(n, std::sqrt((double)kRefBins * dr2), L);
   if (near) REF_CHECK(cudaMemsetAsync(c.near.cells, 0, sizeof(int) * kRdfCells, c.stream));
   if (want_rdf) REF_CHECK(cudaMemsetAsync(c.result->hist, 0, sizeof(c.result->hist), c.stream));
   REF_CHECK(launch_float4_shadow(pos, n, periodic, (double)L, c.sc, nullptr, c.blk, c.ticket + 1, c.q, c.stream));

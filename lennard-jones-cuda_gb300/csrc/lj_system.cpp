@@ -31,9 +31,13 @@ using namespace ljgb;
 // g_alloc_budget < 0: allocations go to CUDA.  >= 0: that many more succeed,
 // every later one fails with cudaErrorMemoryAllocation (no CUDA call made)
 // until lj_debug_fail_allocations(-1).
+// g_alloc_limit >= 0: so do those of more bytes.
 static std::atomic<long long> g_alloc_budget{-1};
+static std::atomic<long long> g_alloc_limit{-1};
 
-static bool allocation_refused() {
+static bool allocation_refused(size_t bytes) {
+  const long long limit = g_alloc_limit.load();
+  if (limit >= 0 && bytes > (size_t)limit) return true;
   long long b = g_alloc_budget.load();
   while (b >= 0) {
     if (b == 0) return true;
@@ -56,13 +60,13 @@ namespace ljgb {
 
 cudaError_t device_alloc(void** p, size_t bytes) {
   *p = nullptr;
-  if (allocation_refused()) return cudaErrorMemoryAllocation;
+  if (allocation_refused(bytes)) return cudaErrorMemoryAllocation;
   return allocated(cudaMalloc(p, bytes), p);
 }
 
 cudaError_t pinned_alloc(void** p, size_t bytes) {
   *p = nullptr;
-  if (allocation_refused()) return cudaErrorMemoryAllocation;
+  if (allocation_refused(bytes)) return cudaErrorMemoryAllocation;
   return allocated(cudaHostAlloc(p, bytes, cudaHostAllocDefault), p);
 }
 
@@ -70,6 +74,11 @@ cudaError_t pinned_alloc(void** p, size_t bytes) {
 
 extern "C" lj_status lj_debug_fail_allocations(int64_t after) {
   g_alloc_budget.store(after < 0 ? -1 : after);
+  return LJ_OK;
+}
+
+extern "C" lj_status lj_debug_limit_allocations(int64_t bytes) {
+  g_alloc_limit.store(bytes < 0 ? -1 : bytes);
   return LJ_OK;
 }
 
