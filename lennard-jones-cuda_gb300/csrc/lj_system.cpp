@@ -898,6 +898,19 @@ lj_status get_graph(lj_system* s, int mode, GraphEntry** out) {
   return LJ_OK;
 }
 
+// The buffers of the histogram's neighbour tiles, made on the first use.
+bool setup_near(lj_system* s) {
+  if (s->near_cells.p) return true;
+  const int n = s->cfg[0].n;
+  if (s->near_rank.alloc(n) == cudaSuccess && s->near_sorted.alloc(n) == cudaSuccess &&
+      s->near_box.alloc(3 * (size_t)((n + 31) / 32)) == cudaSuccess && s->near_cells.alloc(kRdfCells) == cudaSuccess)
+    return true;
+  s->near_rank.free();
+  s->near_sorted.free();
+  s->near_box.free();
+  return false;
+}
+
 // Computes the observables that fused steps left pending (k_obs_finalize;
 // entries a later pair kernel already consumed are skipped on the device).
 // Called before anything reads or changes the observables, the running sums
@@ -1869,22 +1882,6 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   // (pending observables may flag the status, which comes back with the counts)
   lj_status st = flush_observables(s);
   if (st) return st;
-  if (!s->h_hist.p) LJ_CUDA(s, s->h_hist.alloc(kMaxHistBins));
-  const bool mapped = s->h_words.dev && s->h_hist.dev;
-  const int n = s->cfg[0].n;
-  const double rmax = mode == 2 ? nbins * width : std::sqrt(nbins * width);
-  const bool near_tiles = mapped && rdf_near(n, rmax, s->boxes[0].L);
-  if (near_tiles) {
-    if (!s->near_cells.p) {
-      LJ_CUDA(s, s->near_rank.alloc(n));
-      LJ_CUDA(s, s->near_sorted.alloc(n));
-      LJ_CUDA(s, s->near_box.alloc(3 * (size_t)((n + 31) / 32)));
-      LJ_CUDA(s, s->near_cells.alloc(kRdfCells));
-    }
-    LJ_CUDA(s, cudaMemsetAsync(s->near_cells.p, 0, sizeof(int) * kRdfCells, s->stream));
-  }
-  LJ_CUDA(s, cudaMemsetAsync(s->hist.p, 0, sizeof(unsigned long long) * nbins, s->stream));
-  if ((st = enqueue_shadow(s))) return st;
   HistArgs h{};
   h.mode = mode;
   h.nb = nbins;
@@ -1903,6 +1900,16 @@ lj_status lj_rdf_counts(lj_system* s, int32_t mode, int32_t nbins, double width,
   RdfPass p{};
   st = rdf_pass(s, pair_args(s).q, h, &p);
   if (st) return st;
+  // The call does without what follows if it has to: without page-locked memory
+  // the counts come by a copy, without neighbour tiles all pairs are evaluated.
+  if (!s->h_hist.p) (void)s->h_hist.alloc(kMaxHistBins);
+  const bool mapped = s->h_words.dev && s->h_hist.dev;
+  const int n = s->cfg[0].n;
+  const double rmax = mode == 2 ? nbins * width : std::sqrt(nbins * width);
+  const bool near_tiles = mapped && rdf_near(n, rmax, s->boxes[0].L) && setup_near(s);
+  if (near_tiles) LJ_CUDA(s, cudaMemsetAsync(s->near_cells.p, 0, sizeof(int) * kRdfCells, s->stream));
+  LJ_CUDA(s, cudaMemsetAsync(s->hist.p, 0, sizeof(unsigned long long) * nbins, s->stream));
+  if ((st = enqueue_shadow(s))) return st;
   if (mapped) {
     // the pass's last CTA hands counts and status over: no copy is queued, and
     // the host waits on the completion word (as for the read-back launch)
