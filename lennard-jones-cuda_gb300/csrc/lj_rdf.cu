@@ -38,8 +38,12 @@ __device__ __forceinline__ float bin_pos(float x, float k2, float inv_w) {
 // Smallest x >= 0 whose bin position reaches `limit`, by bisection on the
 // bits: rounded products by positive constants are monotonic in x, so `x <
 // bound` decides as comparing the position itself would, without forming it.
+// 0, so that no pair lies below it, where a factor is infinite (widths below
+// 2^-128, say): separation 0 then has no position, and the others are past every
+// bin.
 template <int MODE>
 __device__ float bin_bound(float k2, float inv_w, float limit) {
+  if (bin_pos<MODE>(0.0f, k2, inv_w) != 0.0f) return 0.0f;
   int lo = 0, hi = 0x7f800000;
   auto reaches = [&](int bits) { return bin_pos<MODE>(__int_as_float(bits), k2, inv_w) >= limit; };
   // the real quotient is a few ulps away from it, unless a product over- or
