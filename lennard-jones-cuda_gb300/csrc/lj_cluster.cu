@@ -66,8 +66,8 @@ __device__ __forceinline__ void cluster_pairs(const int4* rowq, const int4* q, i
                : "r"(smem_addr(rowq + 2 * g + 1)));
   const int ia = i + 2 * g;
   f32x2 f[5] = {0ull, 0ull, 0ull, 0ull, 0ull};
-  // The chunks with the warp's own rows (8 of them: one chunk) and the ragged
-  // last one are masked.
+  // The chunks with the warp's own rows (8 of them, over two chunks where the
+  // CTA's first row is no multiple of 8) and the ragged last one are masked.
   const int own = i >> 3, ragged = (n & 7) ? n >> 3 : -1;
   auto masked = [&](int c) {
     const int j = c * 8 + sub;
@@ -85,7 +85,11 @@ __device__ __forceinline__ void cluster_pairs(const int4* rowq, const int4* q, i
       pair_mixed_rows<false>(qa, qb, q[c * 8 + sub], k2i2, false, false, f[0], f[1], f[2], f[3], f[4]);
     if (c < c1) masked(c++);
   }
-  // row a to lanes 0..3 of each group, row b to lanes 4..7, then within
+  // Row a to lanes 0..3 of each group, row b to lanes 4..7: that makes plain FP32
+  // sums of up to 32 pairs (a lane has 16 j's at most).  The four lanes of a row
+  // meet in TwoSum pairs: values 0, 1 go to the lower two and 2, 3 to the upper,
+  // then one value a lane; value 4 to all.
+  const bool h2 = sub & 2, h1 = sub & 1;
   float v[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
@@ -94,13 +98,19 @@ __device__ __forceinline__ void cluster_pairs(const int4* rowq, const int4* q, i
     const float give = sub < 4 ? b : a;
     v[k] = (sub < 4 ? a : b) + __shfl_xor_sync(0xffffffffu, give, 4);
   }
-#pragma unroll
-  for (int o = 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  if ((lane & 3) == 0)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) out[2 * g + (sub >> 2)][k] = v[k];
+  const f32x2 v01 = pk2(v[0], v[1]), v23 = pk2(v[2], v[3]);
+  Float2Acc p{h2 ? v23 : v01, 0ull};
+  two_sum_add2(p, __shfl_xor_sync(0xffffffffu, h2 ? v01 : v23, 2));
+  FloatAcc v4{v[4], 0.f};
+  two_sum_add(v4, __shfl_xor_sync(0xffffffffu, v4.hi, 2));
+  float x, y, xl, yl;
+  upk2(p.hi, x, y);
+  upk2(p.lo, xl, yl);
+  const FloatAcc one = exchange1(h1 ? FloatAcc{y, yl} : FloatAcc{x, xl}, h1 ? FloatAcc{x, xl} : FloatAcc{y, yl}, 1);
+  v4 = exchange1(v4, v4, 1);
+  float* const row = out[2 * g + (sub >> 2)];
+  row[(h2 ? 2 : 0) + (h1 ? 1 : 0)] = one.hi + one.lo;
+  if ((sub & 3) == 0) row[4] = v4.hi + v4.lo;
 }
 
 // The 16 working warps meet here; the observables' two are left out, whose

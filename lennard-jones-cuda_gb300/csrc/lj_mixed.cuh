@@ -129,6 +129,20 @@ __device__ __forceinline__ void two_sum_add2(Float2Acc& a, f32x2 t) {
   a.lo = add2(a.lo, e);
 }
 
+// What the lane `bit` away gives, added to what this lane keeps.
+__device__ __forceinline__ FloatAcc exchange1(FloatAcc keep, FloatAcc give, int bit) {
+  const float hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
+  two_sum_add(keep, hi);
+  keep.lo = __fadd_rn(keep.lo, lo);
+  return keep;
+}
+__device__ __forceinline__ Float2Acc exchange2(Float2Acc keep, Float2Acc give, int bit) {
+  const f32x2 hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
+  two_sum_add2(keep, hi);
+  keep.lo = add2(keep.lo, lo);
+  return keep;
+}
+
 // pair_mixed2 with the two lanes on two i's (qa, qb in slots 1..3) against one
 // j: the same arithmetic per lane.
 template <bool MASKED>

@@ -37,20 +37,6 @@ __device__ __forceinline__ int4 load_slots(const int4* rec) {
   return r;
 }
 
-// What the lane `bit` away gives, added to what this lane keeps.
-__device__ __forceinline__ FloatAcc exchange1(FloatAcc keep, FloatAcc give, int bit) {
-  const float hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
-  two_sum_add(keep, hi);
-  keep.lo = __fadd_rn(keep.lo, lo);
-  return keep;
-}
-__device__ __forceinline__ Float2Acc exchange2(Float2Acc keep, Float2Acc give, int bit) {
-  const f32x2 hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
-  two_sum_add2(keep, hi);
-  keep.lo = add2(keep.lo, lo);
-  return keep;
-}
-
 // Pairs of two rows with chunks c0 .. c1-1 (32 j's each, one a lane) of the n
 // records st; the lanes' sums added up into out[row * 5 + value].  self: the
 // first row's index (even).

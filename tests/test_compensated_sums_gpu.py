@@ -55,3 +55,9 @@ def _check(ljgb, n, L, centre, push, push_back, pull):
 def test_row_step(ljgb_mod, n):
     """Lanes 1, 2 and 3 of a warp's j's."""
     _check(ljgb_mod, n, 60.0, 0, 33, 66, 99)
+
+
+@pytest.mark.parametrize("n", [256, 400, 512])
+def test_cluster_step(ljgb_mod, n):
+    """Lanes 1, 2 and 3 of a group of eight, in a warp's part of the j's."""
+    _check(ljgb_mod, n, 60.0, 0, 9, 18, 27)
