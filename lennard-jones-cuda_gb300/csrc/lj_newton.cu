@@ -16,7 +16,8 @@
 //     are written once, and k_newton_sum adds a particle's parts in FP32
 //     TwoSum and takes the step's second half.
 // Arithmetic per pair is that of lj_mixed.cuh, sums are folded into TwoSum
-// pairs every 32 pairs of an i and every 64 of a j.
+// pairs every 32 pairs of an i, and a j's forces every 32 with each half of the
+// i's, its energies every 64.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -108,7 +109,17 @@ __device__ __forceinline__ void newton_tile(const int4 (&q)[kI], const int4* til
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       FloatAcc acc = J[k][jl];
-      two_sum_add(acc, lane_sum(g[k]));
+      if (k < 3) {  // forces: the halves (32 pairs each) meet exactly too
+        FloatAcc both;
+        float other;
+        upk2(g[k], both.hi, other);
+        both.lo = 0.f;
+        two_sum_add(both, other);
+        two_sum_add(acc, both.hi);
+        acc.lo = __fadd_rn(acc.lo, both.lo);
+      } else {
+        two_sum_add(acc, lane_sum(g[k]));
+      }
       J[k][jl] = acc;
     }
     __syncwarp();

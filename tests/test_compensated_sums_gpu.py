@@ -61,3 +61,10 @@ def test_row_step(ljgb_mod, n):
 def test_cluster_step(ljgb_mod, n):
     """Lanes 1, 2 and 3 of a group of eight, in a warp's part of the j's."""
     _check(ljgb_mod, n, 60.0, 0, 9, 18, 27)
+
+
+def test_unordered_pair_step(ljgb_mod):
+    """A j of the second block's first tile and i's of the first block: the push
+    and the pull in the two halves of the same eight turns, the push back in
+    another eight."""
+    _check(ljgb_mod, 8192, 100.0, 261, 5, 27, 36)
