@@ -1608,9 +1608,10 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
   if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
   const bool plain = !s->profiling && capture == cudaStreamCaptureStatusNone;
   if (fused && use_rows(s) && s->cluster_ok && plain && s->counter_cap == 0 && !s->rdf_acc) {
-    // Small boxes: all steps in one launch (at most kClusterSteps, ~10 ms, so
-    // that the stream gets its turn).
-    constexpr int kClusterSteps = 4096;
+    // Small boxes: all steps in one launch, of at most kClusterSteps: 2.2 ms (EVN,
+    // N = 128) to 6.1 ms (TVN, N = 512), after which the stream and a host that
+    // waits for a completion word (20 ms) get their turn.
+    constexpr int kClusterSteps = 1024;
     lj_status st = flush_observables(s);
     if (st) return st;
     for (int done = 0; done < nsteps; done += kClusterSteps) {
