@@ -225,9 +225,12 @@ __device__ __forceinline__ void adj_task(const AdjBox& b, const AdjPass& a, cons
 
 // FP64-pipe bound.  N = 1000: 34 us forward, 60 us reverse (79 and 142 over
 // ordered pairs).
+// x and z are written by the launch before, which this one may overlap until the
+// wait: no __restrict__, whose promise of data that stays constant for the whole
+// kernel would let them be read through the non-coherent path.
 template <bool HVP>
-__global__ void __launch_bounds__(256) k_adj_pairs(AdjBox b, AdjPass a, const double* __restrict__ x,
-                                                   const double* __restrict__ z, double cF, double cA) {
+__global__ void __launch_bounds__(256) k_adj_pairs(AdjBox b, AdjPass a, const double* x, const double* z, double cF,
+                                                   double cA) {
   extern __shared__ double sh[];  // parts > 1: parts x (2 x 3 x 32 + kScalars)
   const Pair64Task tk = a.tasks[blockIdx.x];
   asm volatile("griddepcontrol.wait;" ::: "memory");

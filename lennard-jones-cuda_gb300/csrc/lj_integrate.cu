@@ -721,8 +721,8 @@ __global__ void k_upload_stage(const double* __restrict__ pos, const double* __r
 // nothing).  With `predict` (periodic boxes on the fused step) the same thread
 // then writes the next pair kernel's shadow x + dt v + dt^2 F / 2, as
 // k_predict does, so the first step after an upload needs no predictor launch.
-__global__ void k_upload_commit(StateArgs s, const double* __restrict__ spos, const double* __restrict__ svel,
-                                const int* bad, int predict) {
+// (No __restrict__: the stage may still be writing spos and svel as this starts.)
+__global__ void k_upload_commit(StateArgs s, const double* spos, const double* svel, const int* bad, int predict) {
   // Launched as a programmatic dependent of k_upload_stage: what the stage
   // does not write (block table, state, forces) is loaded before waiting for
   // its grid to complete.
