@@ -2176,13 +2176,13 @@ lj_status lj_set_kernel_shape(lj_system* s, int32_t shape) {
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_shape;
   s->forced_shape = shape;
-  s->rows_off = false;
   s->shape = shape < 0 ? 0 : shape;
   lj_status st = setup_schedule(s);
   if (st) {
     s->forced_shape = old_forced;
     return st;
   }
+  s->rows_off = false;
   // The i-block length changed: rebuild shadows and the per-block sums.
   if ((st = recompute_forces_keep_scalars(s))) return st;
   return setup_newton(s);
@@ -2195,13 +2195,13 @@ lj_status lj_set_split_cap(lj_system* s, int32_t cap) {
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_split;
   s->forced_split = cap;
-  s->rows_off = false;
   s->split_cap = cap > 0 ? cap : kMaxSegmentsPerBlock;
   lj_status st = setup_schedule(s);
   if (st) {
     s->forced_split = old_forced;
     return st;
   }
+  s->rows_off = false;
   // The partial segments were re-cut: rebuild the per-block sums.
   return recompute_forces_keep_scalars(s);
 }
