@@ -2173,11 +2173,14 @@ lj_status lj_set_kernel_shape(lj_system* s, int32_t shape) {
   if (shape < -1 || shape >= kNumShapes) return fail(s, LJ_ERR_INVALID, "shape %d out of range", shape);
   if (s->prec == LJ_PREC_FP64) return LJ_OK;  // one FP64 shape
   DeviceGuard device_guard(s->device);
+  // the last step's observables come from the block sums that are replaced
+  lj_status st = flush_observables(s);
+  if (st) return st;
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_shape;
   s->forced_shape = shape;
   s->shape = shape < 0 ? 0 : shape;
-  lj_status st = setup_schedule(s);
+  st = setup_schedule(s);
   if (st) {
     s->forced_shape = old_forced;
     return st;
@@ -2192,11 +2195,13 @@ lj_status lj_set_split_cap(lj_system* s, int32_t cap) {
   if (!s) return LJ_ERR_INVALID;
   if (cap < 0 || cap > 1024) return fail(s, LJ_ERR_INVALID, "split cap %d out of range [0, 1024]", cap);
   DeviceGuard device_guard(s->device);
+  lj_status st = flush_observables(s);
+  if (st) return st;
   LJ_CUDA(s, cudaStreamSynchronize(s->stream));
   const int old_forced = s->forced_split;
   s->forced_split = cap;
   s->split_cap = cap > 0 ? cap : kMaxSegmentsPerBlock;
-  lj_status st = setup_schedule(s);
+  st = setup_schedule(s);
   if (st) {
     s->forced_split = old_forced;
     return st;
