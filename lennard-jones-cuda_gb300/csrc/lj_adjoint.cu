@@ -531,11 +531,15 @@ lj_status lj_adjoint_create(const lj_config* cfg, int32_t checkpoint_every, lj_a
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device) != cudaSuccess)
     return bail(LJ_ERR_NO_DEVICE);
-  const Pair64Plan plan = plan_pairs64({a->n}, sms, 41, 3);  // of 30 and 55 operations a turn
   if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(LJ_ERR_CUDA);
   const size_t s3 = xyz(a);
+  Pair64Plan plan;  // of 30 and 55 operations a turn
+  const cudaError_t sums = plan_pairs64_within({a->n}, sms, 41, 3, 3, &plan, [&](const Pair64Plan& p) {
+    return a->part.alloc((size_t)p.slots * 96);
+  });
+  if (sums != cudaSuccess) return bail(sums == cudaErrorMemoryAllocation ? LJ_ERR_OUT_OF_MEMORY : LJ_ERR_CUDA);
   if (a->x.alloc(s3) || a->v.alloc(s3) || a->x0.alloc(s3) || a->v0.alloc(s3) || a->Xb.alloc(s3) ||
-      a->bb.alloc(s3) || a->z.alloc(s3) || a->hostio.alloc(s3) || a->part.alloc((size_t)plan.slots * 96) ||
+      a->bb.alloc(s3) || a->z.alloc(s3) || a->hostio.alloc(s3) ||
       a->scal.alloc(plan.tasks.size() * kScalars) || a->tasks.alloc(plan.tasks.size()))
     return bail(LJ_ERR_OUT_OF_MEMORY);
   if (cudaMemsetAsync(a->part.p, 0, sizeof(double) * (size_t)plan.slots * 96, a->stream) != cudaSuccess)

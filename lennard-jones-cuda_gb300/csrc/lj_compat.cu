@@ -176,7 +176,7 @@ bool build_ctx(int n, int shape, int dev, bool lean, bool loud) {
     int newton_per_sm = 0;
     REF_CHECK(newton_setup(&newton_per_sm));
     if (newton_per_sm > 0) np = plan_newton(n, sms * newton_per_sm * kNewtonWarps);
-    if (!newton_fits(np)) np = NewtonPlan();
+    if (!leaves_room(np.bytes())) np = NewtonPlan();
   }
   const bool stream_k = np.tasks.empty() && rows.ctas == 0;
   Schedule s;

@@ -39,6 +39,8 @@ class DeviceGuard {
 // exhausting a GPU.
 cudaError_t device_alloc(void** p, size_t bytes);
 cudaError_t pinned_alloc(void** p, size_t bytes);
+// Whether `bytes` more leave at least as much of the current device's memory free.
+bool leaves_room(size_t bytes);
 
 // Device-side status flags (DevScalars::status).
 enum : int {

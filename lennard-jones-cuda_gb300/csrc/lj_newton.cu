@@ -25,7 +25,6 @@
 #include "lj_device.cuh"
 #include "lj_kernels.h"
 #include "lj_mixed.cuh"
-#include "lj_schedule.h"
 #include "lj_stepdev.cuh"
 
 namespace ljgb {
@@ -325,15 +324,6 @@ __global__ void __launch_bounds__(160 * kSum, 4) k_newton_sum(StateArgs s, Newto
   } else {
     o[3] = red[0] + red[1] + red[2];
   }
-}
-
-bool newton_fits(const NewtonPlan& p) {
-  size_t free_bytes = 0, total = 0;
-  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return true;  // the allocations will tell
-  }
-  return sizeof(float) * (160 * (size_t)p.jparts + 5 * kNewtonBlock * (size_t)p.iparts) <= free_bytes / 2;
 }
 
 cudaError_t newton_setup(int* ctas_per_sm) {

@@ -139,8 +139,9 @@ bool build_rdf_ranges(int n, int ctas, RdfRanges* out) {
   return true;
 }
 
-Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops, int slot_ops) {
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops, int slot_ops, int group) {
   Pair64Plan p;
+  p.group = group;
   auto squares = [&](long long group) {
     long long t = 0;
     for (int k : n) {

@@ -73,7 +73,24 @@ struct Pair64Plan {
   std::vector<Pair64Task> tasks;
   std::vector<Pair64Box> boxes;
 };
-Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops = 28, int slot_ops = 5);
+// `group` > 1: at least that side, for sums that have to take less memory.
+Pair64Plan plan_pairs64(const std::vector<int>& n, int sms, int turn_ops = 28, int slot_ops = 5, int group = 1);
+// The plan of the smallest side for which take(plan) has cudaSuccess, given that
+// only a lack of memory is worth another try; a plan whose sums (`values` a
+// particle and slot) would leave less memory free than they take is not tried
+// while a larger side is left.
+template <typename Take>
+cudaError_t plan_pairs64_within(const std::vector<int>& n, int sms, int turn_ops, int slot_ops, int values,
+                                Pair64Plan* p, Take take) {
+  for (int group = 1;; group = 2 * p->group) {
+    *p = plan_pairs64(n, sms, turn_ops, slot_ops, group);
+    bool last = true;
+    for (const Pair64Box& b : p->boxes) last &= b.groups == 1;
+    if (!last && !leaves_room(sizeof(double) * 32 * values * (size_t)p->slots)) continue;
+    const cudaError_t e = take(*p);
+    if (e != cudaErrorMemoryAllocation || last) return e;
+  }
+}
 
 // Tasks of the unordered-pair kernel for n particles and `warps` warps: equal
 // shares (+-1) of the (block, tile) sequence.  The i sums of (task, block) are
@@ -84,10 +101,8 @@ struct NewtonPlan {
   std::vector<int> block_part;
   long long jparts = 0;  // parts of the j sums
   int iparts = 0;
+  size_t bytes() const { return sizeof(float) * 5 * (32 * (size_t)jparts + kNewtonBlock * (size_t)iparts); }
 };
 NewtonPlan plan_newton(int n, int warps);
-// Whether the plan's sums leave at least as much of the current device's memory
-// free as they take.
-bool newton_fits(const NewtonPlan& p);
 
 }  // namespace ljgb

@@ -70,6 +70,13 @@ cudaError_t pinned_alloc(void** p, size_t bytes) {
   return allocated(cudaHostAlloc(p, bytes, cudaHostAllocDefault), p);
 }
 
+bool leaves_room(size_t bytes) {
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess) return bytes <= free_bytes / 2;
+  (void)cudaGetLastError();
+  return true;  // the allocation will tell
+}
+
 }  // namespace ljgb
 
 extern "C" lj_status lj_debug_fail_allocations(int64_t after) {
@@ -497,7 +504,6 @@ lj_status build_and_swap_schedule(lj_system* s) {
   for (int k = 0; k < s->nsys; ++k) nbt += (n[k] + threads - 1) / threads;
   const int G = fp64 ? 1 : (int)std::min<long long>((long long)s->num_sms * blocks_per_sm, nbt * s->split_cap);
   Pair64Plan p64;
-  if (fp64) p64 = plan_pairs64(n, s->num_sms);
   Schedule sch;
   if (!build_schedule(n.data(), s->nsys, threads, tile, G, kTileOverhead, &sch))
     return fail(s, LJ_ERR_INVALID, "cannot build the pair schedule");
@@ -519,9 +525,11 @@ lj_status build_and_swap_schedule(lj_system* s) {
   DevBuf<Pair64Box> p64_boxes;
   DevBuf<double> p64_part;
   if (fp64) {
+    LJ_CUDA(s, plan_pairs64_within(n, s->num_sms, 28, 5, 5, &p64, [&](const Pair64Plan& p) {
+              return p64_part.alloc((size_t)p.slots * 5 * 32);
+            }));
     LJ_CUDA(s, p64_tasks.alloc(p64.tasks.size()));
     LJ_CUDA(s, p64_boxes.alloc(p64.boxes.size()));
-    LJ_CUDA(s, p64_part.alloc((size_t)p64.slots * 5 * 32));
     LJ_CUDA(s, cudaMemsetAsync(p64_part.p, 0, sizeof(double) * (size_t)p64.slots * 5 * 32, s->stream));
     LJ_CUDA(s, cudaMemcpyAsync(p64_tasks.p, p64.tasks.data(), sizeof(Pair64Task) * p64.tasks.size(),
                                cudaMemcpyHostToDevice, s->stream));
@@ -744,7 +752,7 @@ lj_status build_newton(lj_system* s) {
   LJ_CUDA(s, newton_setup(&per_sm));
   if (per_sm < 1) return LJ_OK;
   const NewtonPlan p = plan_newton(n, s->num_sms * per_sm * kNewtonWarps);
-  if (!newton_fits(p)) return LJ_ERR_OUT_OF_MEMORY;
+  if (!leaves_room(p.bytes())) return LJ_ERR_OUT_OF_MEMORY;
   LJ_CUDA(s, s->newton_tasks.alloc(p.tasks.size()));
   LJ_CUDA(s, s->newton_blocks.alloc(p.block_part.size()));
   LJ_CUDA(s, s->newton_j.alloc((size_t)p.jparts * 160));
