@@ -136,12 +136,6 @@ __device__ __forceinline__ FloatAcc exchange1(FloatAcc keep, FloatAcc give, int 
   keep.lo = __fadd_rn(keep.lo, lo);
   return keep;
 }
-__device__ __forceinline__ Float2Acc exchange2(Float2Acc keep, Float2Acc give, int bit) {
-  const f32x2 hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
-  two_sum_add2(keep, hi);
-  keep.lo = add2(keep.lo, lo);
-  return keep;
-}
 
 // pair_mixed2 with the two lanes on two i's (qa, qb in slots 1..3) against one
 // j: the same arithmetic per lane.

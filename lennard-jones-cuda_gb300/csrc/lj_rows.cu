@@ -67,38 +67,40 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
 #pragma unroll
     for (int k = 0; k < 5; ++k) two_sum_add2(acc[k], f[k]);
   }
-  // The lanes' sums meet as TwoSum pairs too: row 0 goes to the lower half of the
-  // warp and row 1 to the upper, then values 0, 1 to the lower eight of the
-  // sixteen lanes and 2, 3 to the upper, then one value a lane, and at last
-  // value 4 to every other pair of lanes (fixed order).  12 exchanges; plain
-  // FP32 ones lose what meets a larger term in another lane, and are 0.35 us of a
-  // step faster (N = 2001 EVN, 20 steps: 185 us, so 192).
-  const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
-  float kh[5], kl[5], gh[5], gl[5];  // kept and given
+  // The lanes' forces meet as TwoSum pairs too, their energies (compensated so
+  // far) in plain FP32, five additions where the stream-K kernel has one a chunk
+  // over a tile.  Row 0 goes to the lower half of the warp and row 1 to the
+  // upper; then value 0 or 1 (3 or 4) is kept by every other eight lanes, and
+  // that or value 2 by every other four (fixed order).  All five values plain,
+  // 0.3 us of a step faster at N = 2001 (20 EVN steps: 185 us, so 191), lose a
+  // force that meets a larger one in another lane.
+  const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+  FloatAcc f[3];
+  float ke[2];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    float ha, hb, la, lb;
-    upk2(acc[k].hi, ha, hb);
-    upk2(acc[k].lo, la, lb);
-    kh[k] = h16 ? hb : ha;
-    kl[k] = h16 ? lb : la;
-    gh[k] = h16 ? ha : hb;
-    gl[k] = h16 ? la : lb;
+  for (int k = 0; k < 3; ++k) {
+    FloatAcc a, b;
+    upk2(acc[k].hi, a.hi, b.hi);
+    upk2(acc[k].lo, a.lo, b.lo);
+    f[k] = exchange1(h16 ? b : a, h16 ? a : b, 16);
   }
-  Float2Acc v01 = exchange2(Float2Acc{pk2(kh[0], kh[1]), pk2(kl[0], kl[1])}, Float2Acc{pk2(gh[0], gh[1]), pk2(gl[0], gl[1])}, 16);
-  Float2Acc v23 = exchange2(Float2Acc{pk2(kh[2], kh[3]), pk2(kl[2], kl[3])}, Float2Acc{pk2(gh[2], gh[3]), pk2(gl[2], gl[3])}, 16);
-  FloatAcc v4 = exchange1(FloatAcc{kh[4], kl[4]}, FloatAcc{gh[4], gl[4]}, 16);
-  v01 = exchange2(h8 ? v23 : v01, h8 ? v01 : v23, 8);
-  v4 = exchange1(v4, v4, 8);
-  float x, y, xl, yl;
-  upk2(v01.hi, x, y);
-  upk2(v01.lo, xl, yl);
-  FloatAcc v = exchange1(h4 ? FloatAcc{y, yl} : FloatAcc{x, xl}, h4 ? FloatAcc{x, xl} : FloatAcc{y, yl}, 4);
-  v4 = exchange1(v4, v4, 4);
-  v = exchange1(h2 ? v4 : v, h2 ? v : v4, 2);
-  v = exchange1(v, v, 1);
-  if ((lane & 1) == 0 && (!h2 || (lane & 12) == 0))
-    out[(h16 ? 5 : 0) + (h2 ? 4 : (h8 ? 2 : 0) + (h4 ? 1 : 0))] = v.hi + v.lo;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    float a, b;
+    upk2(add2(acc[3 + k].hi, acc[3 + k].lo), a, b);
+    ke[k] = (h16 ? b : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : b, 16);
+  }
+  FloatAcc v = exchange1(h8 ? f[1] : f[0], h8 ? f[0] : f[1], 8);
+  const FloatAcc v2 = exchange1(f[2], f[2], 8);
+  float e = (h8 ? ke[1] : ke[0]) + __shfl_xor_sync(0xffffffffu, h8 ? ke[0] : ke[1], 8);
+  v = exchange1(h4 ? v2 : v, h4 ? v : v2, 4);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) v = exchange1(v, v, o);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  float* const row = out + (h16 ? 5 : 0);
+  if ((lane & 3) == 0 && !(h4 && h8)) row[h4 ? 2 : h8 ? 1 : 0] = v.hi + v.lo;
+  if ((lane & 7) == 0) row[h8 ? 4 : 3] = e;
 }
 
 // The warp that works on unit u when U units are cut evenly over the warps.
