@@ -253,6 +253,15 @@ def flops_per_pair(launches_per_step: float) -> float:
     return FLOPS_PER_UNORDERED_PAIR / 2 if launches_per_step > 2.5 else FLOPS_PER_PAIR
 
 
+def kernel_that_ran(launches_per_step: float, shape: dict) -> dict:
+    """The pair kernel of a TVN step and its geometry: the unordered-pair kernel's
+    (lj_newton.cu: CTAs of 128 threads, 8 i's each, tiles of 32 j's), or the
+    stream-K shape that is set."""
+    if flops_per_pair(launches_per_step) != FLOPS_PER_PAIR:
+        return {"kernel": "k_newton", "threads": 128, "ipt": 8, "tile": 32}
+    return dict(shape, kernel="k_pairs_mixed_fused")
+
+
 def read_traffic():
     """Per-launch DRAM bytes of the pair kernel from the committed ncu summary."""
     path = os.path.join(REPO, "profiles", "unordered_pairs_ncu.md")
@@ -360,7 +369,7 @@ def extra_configs(torch, ljgb, oracle, dev, flush, peak):
     g.close()
     out["large_262144"] = {
         "workload": "N=262144 rho*=1.1 T*=1.0 FCC+0.01 dt=0.004 TVN", "ms_per_step": ms / steps,
-        "kernel_shape": tune["shapes"][tune["active"]],
+        "kernel_shape": kernel_that_ran(launches / steps, tune["shapes"][tune["active"]]),
         "pair_interactions_per_s": n * (n - 1) * steps / (ms * 1e-3), "pair_kernel_ms": pair_ms,
         "fp32_frac": flops_per_pair(launches / steps) * n * (n - 1) / (pair_ms * 1e-3) / 1e12 / peak,
         "subset_vs_fp64_oracle": {"rows": [i0, i0 + 4096], "gate_max": float((d / np.maximum(mag, rms)).max()),
@@ -504,7 +513,7 @@ def gpu_arm(args, rank, world, local_rank):
             "value": value, "unit": "pair-interactions/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32-pairs/f64-state", "data": "synthetic (seeded FCC+jitter)",
-            "config": bench_config(world), "kernel_shape": shape,
+            "config": bench_config(world), "kernel_shape": kernel_that_ran(launches / args.steps, shape),
             "steps_per_s": 1e3 / ms_step,
             "e2e": {"value": e2e_value, "unit": "pair-interactions/s", "h2d_bytes_per_step":
                     e2e_bytes["h2d_bytes_per_step"], "d2h_bytes_per_step": e2e_bytes["d2h_bytes_per_step"],
@@ -514,7 +523,7 @@ def gpu_arm(args, rank, world, local_rank):
             "accuracy": acc,
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "k_newton" if per_pair != FLOPS_PER_PAIR else "k_pairs_mixed_fused",
+                         "kernel": kernel_that_ran(launches / args.steps, shape)["kernel"],
                          "flops_per_pair": per_pair,
                          "pair_kernel_ms": pair_ms, "step_ms_profiled": step_ms_prof,
                          "step_frac": per_pair * pairs_step / (ms_step * 1e-3) / 1e12 / peak,

@@ -184,10 +184,11 @@ struct ClusterObs {
 // nsteps steps of box 0.  s.q holds the first step's predicted shadow and
 // receives the one after the last.
 //
-// What bounds a step is latency, in clocks at N = 400 (EVN, 7300 in all): pair
-// phase 3800 (13 pairs a lane and their reduction), sums and ~12 dependent
-// FP64 operations of 64 clocks 2100, records sent and barrier 1300; TVN adds a
-// barrier, two FP64 sums over the rows and chi's rsqrt, 4000.  The sums for
+// What bounds a step is latency, in clocks of rank 0's first warp at N = 400 (EVN,
+// 7570 in all): pair phase 4250 (13 pairs a lane and their reduction), sums and ~12
+// dependent FP64 operations of 64 clocks 1870, records sent and barrier 1450; TVN
+// (11 800) adds a barrier (1000), two FP64 sums over the rows and chi's rsqrt
+// (3070).  N = 128: 1370 + 2010 + 1050; N = 512: 5070 + 1790 + 1400.  The sums for
 // the observables run beside the next step.  us a step, lj_rows.cu -> this
 // one: EVN N = 128 5.4 -> 2.3, N = 256 5.4 -> 2.8, N = 400 5.5 -> 3.8, N = 512
 // 5.6 -> 4.1; TVN N = 256 8.3 -> 4.7, N = 400 9.6 -> 5.7.  16 SMs are too few
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cluster(StateArgs s, int n, int
   const int i0 = rank * rows, nr = max(0, min(rows, n - i0));
   const BoxArgs box = s.boxes[0];
   DevScalars& sc = s.sc[0];
-  const double fscale = sc.fscale, qscale = sc.invP * 4294967296.0, invP = sc.invP;
+  const double fscale = sc.fscale, qscale = sc.invP * 4294967296.0;
   const f32x2 k2i2 = pk2(sc.k2inv, sc.k2inv);
   const bool worker = w < kPairWarps;
 

@@ -75,12 +75,15 @@ struct RdfPass {
 };
 int rdf_ctas_per_sm();
 // The same by tiles of neighbours (four launches; without a.mail mode 0 alone).  Sorting
-// costs about 20 us, so the line lies where the pairs left out are worth more.
-// us a call at reach / L, all pairs -> near tiles, particles in lattice order
-// (shuffled: 5 to 20% more for all pairs, the same for near tiles): N = 8192 at
-// 0.15 40 -> 47; N = 16384 at 0.15 95 -> 56, 0.25 108 -> 95, 0.35 120 -> 129; N =
+// costs about 20 us, which the pairs left out have to be worth.  us a call at
+// reach / L, all pairs -> near tiles, particles in lattice order (shuffled: 5 to
+// 20% more for all pairs, the same for near tiles): N = 8192 at 0.15 41 -> 47, 0.25
+// 44 -> 55; N = 10000 48 -> 68, 52 -> 78; N = 12000 62 -> 62, 69 -> 75; N = 14000 79
+// -> 54, 88 -> 76; N = 16384 at 0.15 95 -> 56, 0.25 108 -> 95, 0.35 120 -> 129; N =
 // 32768 at 0.15 296 -> 144, 0.35 380 -> 368, 0.4 402 -> 443; N = 40000 at 0.15 435
-// -> 183, 0.35 556 -> 442.  (A droplet within the reach leaves nothing out.)
+// -> 183, 0.35 556 -> 442.  The two cross between 12000 and 14000, by how the
+// sorted tiles fall; the line lies above, at 16384, where near tiles win throughout.
+// (A droplet within the reach leaves nothing out.)
 struct RdfNear {
   int* cells;    // kRdfCells, 0 before
   int* rank;     // n: place within the cell
