@@ -106,8 +106,8 @@ __device__ __forceinline__ void cluster_pairs(const int4* rowq, const int4* q, i
   float x, y, xl, yl;
   upk2(p.hi, x, y);
   upk2(p.lo, xl, yl);
-  const FloatAcc one = exchange1(h1 ? FloatAcc{y, yl} : FloatAcc{x, xl}, h1 ? FloatAcc{x, xl} : FloatAcc{y, yl}, 1);
-  v4 = exchange1(v4, v4, 1);
+  const FloatAcc one = exchange1(FloatAcc{x, xl}, FloatAcc{y, yl}, h1, 1);
+  v4 = exchange1(v4, v4, false, 1);
   float* const row = out[2 * g + (sub >> 2)];
   row[(h2 ? 2 : 0) + (h1 ? 1 : 0)] = one.hi + one.lo;
   if ((sub & 3) == 0) row[4] = v4.hi + v4.lo;

@@ -129,9 +129,14 @@ __device__ __forceinline__ void two_sum_add2(Float2Acc& a, f32x2 t) {
   a.lo = add2(a.lo, e);
 }
 
-// What the lane `bit` away gives, added to what this lane keeps.
-__device__ __forceinline__ FloatAcc exchange1(FloatAcc keep, FloatAcc give, int bit) {
-  const float hi = __shfl_xor_sync(0xffffffffu, give.hi, bit), lo = __shfl_xor_sync(0xffffffffu, give.lo, bit);
+// Lanes with `second` keep b and give a to the lane `bit` away, the others keep a
+// and give b; returns what is kept plus what the other lane gives.
+__device__ __forceinline__ FloatAcc exchange1(const FloatAcc a, const FloatAcc b, bool second, int bit) {
+  FloatAcc keep;
+  keep.hi = second ? b.hi : a.hi;
+  keep.lo = second ? b.lo : a.lo;
+  const float hi = __shfl_xor_sync(0xffffffffu, second ? a.hi : b.hi, bit);
+  const float lo = __shfl_xor_sync(0xffffffffu, second ? a.lo : b.lo, bit);
   two_sum_add(keep, hi);
   keep.lo = __fadd_rn(keep.lo, lo);
   return keep;

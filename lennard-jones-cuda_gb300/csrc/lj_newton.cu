@@ -132,8 +132,8 @@ __device__ __forceinline__ void newton_tile(const int4 (&q)[kI], const int4* til
 // spends 28 and 14 per 2).  12 warps an SM at 168 registers: with 16 warps at
 // 128 the loop spilled and ran 7% slower; unrolled 4 turns (1: 25% slower, 8:
 // 1% faster on the largest boxes and 7% slower at N = 16384).  us a TVN step,
-// stream-K -> this kernel and its sums: N = 16384 185 -> 153, N = 65536 2700
-// -> 2060, N = 262144 42.9 -> 31.7 ms.
+// stream-K -> this kernel and its sums: N = 16384 185 -> 154, N = 65536 2700
+// -> 2080, N = 262144 42.9 -> 31.9 ms.
 __global__ void __launch_bounds__(32 * kWarps, 3) k_newton(NewtonArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NewtonShared& sh = *reinterpret_cast<NewtonShared*>(smem_raw);

@@ -40,6 +40,10 @@ __device__ __forceinline__ int4 load_slots(const int4* rec) {
 // Pairs of two rows with chunks c0 .. c1-1 (32 j's each, one a lane) of the n
 // records st; the lanes' sums added up into out[row * 5 + value].  self: the
 // first row's index (even).
+// UNROLL: chunks in flight.  The registers that the second half holds meanwhile
+// decide: us a step, 4 / 8, TVN N = 4000 19.3 / 19.7, N = 8000 49.7 / 51.0; EVN N =
+// 2001 7.9 / 8.1, N = 4000 16.3 / 16.0, N = 8000 49.0 / 47.5.
+template <int UNROLL>
 __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, int n, int c0, int c1, int self,
                                             f32x2 k2i2, float* out) {
   const int lane = threadIdx.x & 31;
@@ -54,7 +58,7 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
     f32x2 f[5] = {0ull, 0ull, 0ull, 0ull, 0ull};
     if (c < special) {
       const int ce = min(special, c + kRowFold);
-#pragma unroll 8
+#pragma unroll UNROLL
       for (; c < ce; ++c)
         pair_mixed_rows<false>(qa, qb, st[c * 32 + lane], k2i2, false, false, f[0], f[1], f[2], f[3], f[4]);
     } else {
@@ -72,7 +76,7 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
   // over a tile.  Row 0 goes to the lower half of the warp and row 1 to the
   // upper; then value 0 or 1 (3 or 4) is kept by every other eight lanes, and
   // that or value 2 by every other four (fixed order).  All five values plain,
-  // 0.3 us of a step faster at N = 2001 (20 EVN steps: 185 us, so 191), lose a
+  // 0.3 us of an EVN step faster at N = 2001 (20 steps: 185 us, so 191), lose a
   // force that meets a larger one in another lane.
   const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
   FloatAcc f[3];
@@ -82,7 +86,7 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
     FloatAcc a, b;
     upk2(acc[k].hi, a.hi, b.hi);
     upk2(acc[k].lo, a.lo, b.lo);
-    f[k] = exchange1(h16 ? b : a, h16 ? a : b, 16);
+    f[k] = exchange1(a, b, h16, 16);
   }
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -90,12 +94,12 @@ __device__ __forceinline__ void row_portion(const int4* rowq, const int4* st, in
     upk2(add2(acc[3 + k].hi, acc[3 + k].lo), a, b);
     ke[k] = (h16 ? b : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : b, 16);
   }
-  FloatAcc v = exchange1(h8 ? f[1] : f[0], h8 ? f[0] : f[1], 8);
-  const FloatAcc v2 = exchange1(f[2], f[2], 8);
+  FloatAcc v = exchange1(f[0], f[1], h8, 8);
+  const FloatAcc v2 = exchange1(f[2], f[2], false, 8);
   float e = (h8 ? ke[1] : ke[0]) + __shfl_xor_sync(0xffffffffu, h8 ? ke[0] : ke[1], 8);
-  v = exchange1(h4 ? v2 : v, h4 ? v : v2, 4);
+  v = exchange1(v, v2, h4, 4);
 #pragma unroll
-  for (int o = 2; o > 0; o >>= 1) v = exchange1(v, v, o);
+  for (int o = 2; o > 0; o >>= 1) v = exchange1(v, v, false, o);
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
   float* const row = out + (h16 ? 5 : 0);
@@ -121,7 +125,7 @@ __device__ __forceinline__ int warp_of_unit(int u, int U) { return ((u + 1) * kR
 // lj_pairs.cu; below ~2000 the fixed parts (launch, first copy, reductions, a
 // chain of ~15 FP64 operations), ~5 us.  us a step, stream-K kernel -> this
 // one, on GB300: EVN N = 400 14.4 -> 5.5, N = 1000 16.4 -> 6.2, N = 2001 20.5
-// -> 8.7; TVN N = 256 18.4 -> 8.3, N = 4000 30.8 -> 20.5, N = 8000 70 -> 52.
+// -> 8.1; TVN N = 256 18.4 -> 8.3, N = 4000 30.8 -> 19.3, N = 8000 70 -> 49.7.
 template <int MODE>
 __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int rows, int ctas) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_rows(StateArgs s, int n, int
     const int hi = (w + 1) * U / kRowWarps;
     for (int u = w * U / kRowWarps; u < hi;) {
       const int g = u / C, c0 = u - g * C, c1 = min(C, c0 + hi - u);
-      row_portion(srow + 2 * g, sq, n, c0, c1, i0 + 2 * g, k2i2, part + (w + g) * 10);
+      row_portion<MODE == MODE_TVN ? 4 : 8>(srow + 2 * g, sq, n, c0, c1, i0 + 2 * g, k2i2, part + (w + g) * 10);
       u += c1 - c0;
     }
   } else if (lane == 0) {
