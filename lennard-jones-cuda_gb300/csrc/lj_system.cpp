@@ -1579,6 +1579,13 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
   if (!(dt > 0) || !std::isfinite(dt)) return fail(s, LJ_ERR_INVALID, "dt must be > 0");
   if (nsteps == 0) return LJ_OK;
   DeviceGuard device_guard(s->device);
+  // Not on a stream that is being captured: the launches would be recorded with
+  // this call's step parity, and nothing may be queued or marked as done before
+  // the refusal.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+  else if (capture != cudaStreamCaptureStatusNone)
+    return fail(s, LJ_ERR_CUDA, "lj_step: the handle's stream is being captured");
   bool changed = false;
   for (auto& b : s->boxes)
     if (b.dt != dt) {
@@ -1609,12 +1616,8 @@ lj_status lj_step(lj_system* s, double dt, int32_t nsteps) {
   // graphs -> so: 20 FP64 steps of 512 particles with counters and histogram 763
   // -> 724, a step of an open box of 400 36.3 -> 32.5, ten steps of 8 boxes of
   // 100 to 300 in all 255 -> 228).  (A profiled step keeps its graph for the
-  // events.  On a stream that is being captured the graphs' route refuses the
-  // call, as it always did: single launches would be recorded with this call's
-  // step parity.)
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
-  const bool plain = !s->profiling && capture == cudaStreamCaptureStatusNone;
+  // events.)
+  const bool plain = !s->profiling;
   if (fused && use_rows(s) && s->cluster_ok && plain && s->counter_cap == 0 && !s->rdf_acc) {
     // Small boxes: all steps in one launch, of at most kClusterSteps: 2.2 ms (EVN,
     // N = 128) to 6.1 ms (TVN, N = 512), after which the stream and a host that
