@@ -2272,6 +2272,20 @@ lj_status lj_autotune(lj_system* s) {
   const int qpar = s->qpar;
   const bool was_profiling = s->profiling;
   s->profiling = false;
+  // the trials are no samples: counters and the summed histogram rest meanwhile
+  struct Samples {
+    lj_system* s;
+    int cap;
+    bool rdf;
+    explicit Samples(lj_system* sys) : s(sys), cap(sys->counter_cap), rdf(sys->rdf_acc) {
+      s->counter_cap = 0;
+      s->rdf_acc = false;
+    }
+    ~Samples() {
+      s->counter_cap = cap;
+      s->rdf_acc = rdf;
+    }
+  } samples(s);
   auto restore = [&]() -> lj_status {
     for (int k = 0; k < 6; ++k)
       LJ_CUDA(s, cudaMemcpyAsync(cur[k], snap[k].p, sizeof(double) * cnt[k], cudaMemcpyDeviceToDevice, s->stream));
