@@ -18,7 +18,7 @@
  *    reset the device for the whole process (MDSystem.cu:294-297);
  *  - `blockSize` (CUDABlockSize) selects the nearest i-block size of the
  *    kernel shapes that boxes of more than 2^18 particles use (smaller ones
- *    have kernels of their own); `q` stays unused as in the reference;
+ *    have kernels of their own, from 8192 on given the memory); `q` stays unused as in the reference;
  *  - no per-call cudaMalloc/cudaFree: work buffers are cached per particle
  *    count (MDSystem.cu:265-287 allocated two RDF arrays on every call).
  */

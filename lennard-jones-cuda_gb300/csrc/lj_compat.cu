@@ -6,7 +6,8 @@
 // calculateNForces: float4 positions -> fixed-point shadow (frame from L or
 // from the bounding box for non-periodic boxes) -> the pair kernels of a step
 // without the step (the row kernel below kNewtonMinN particles, unordered pairs
-// up to kNewtonMaxN, the stream-K kernel above) -> per-particle float4 forces
+// up to kNewtonMaxN, the stream-K kernel above, and where the unordered pairs'
+// sums cannot be had) -> per-particle float4 forces
 // and one FP64 virial sum; the 256-bin r^2 RDF, where it is asked for, is the histogram
 // kernel's (lj_rdf.cu): a call of N = 8000 took 203 us with both in one kernel and
 // took 155 us in two, since the force loop evaluates ordered pairs and the
